@@ -7,6 +7,7 @@ raised.  The library is looked up next to this file; it is built in-tree by
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_void_p
@@ -49,6 +50,16 @@ _SIGNATURES = {
     "fox_dq_convert": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _F, c_float, _T4P]),
     "fox_attn_fwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P,
                              _F, _F, _F, c_float, _T4P, _F, _F, _F]),
+    "fox_attn_fwd_parts": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P,
+                                   _F, _F, _F, c_float, _T4P, _F, _F, c_int64, _F]),
+    "fox_norm_parts": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
+    "fox_attn_prologue": (c_int, [c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _F, c_int64,
+                                  c_int64, c_int64, _F, _F, _T4P, _F, c_int64, _T4P, _F, c_int64]),
+    "fox_attn_index": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, _F, c_float, _F,
+                               c_int64, _F, c_int64, c_float, _F, _F, _F]),
+    "fox_bwd_prepare": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _F, _F, _F]),
+    "fox_bwd_finish": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _F, _F, c_int, _F,
+                               c_int64, c_int64, c_int64, _F, c_int64, c_int64, c_int64, _F, c_float, _T4P]),
     "fox_attn_decode": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P, _F, _F, _F,
                                 c_float, _T4P, _F, _F, c_int64]),
     "fox_attn_decode_workspace_floats": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
@@ -147,60 +158,53 @@ def tma_ready(x: torch.Tensor) -> bool:
     return all((x.stride(i) * es) % 16 == 0 and x.stride(i) > 0 or x.shape[i] == 1 for i in range(x.dim() - 1))
 
 
+# ------------------------------------------------------------------ native host side
+_host = None
+
+
+def host():
+    """The host extension ``_fox_host`` (building it first when the file is absent)."""
+    global _host
+    if _host is None:
+        load()      # the kernels' library first: the extension is linked to it
+        with _lock:
+            if _host is None:
+                path = _build.HOST_PATH
+                if not os.path.exists(path) and os.environ.get("FOX_B200_NO_BUILD") != "1":
+                    try:
+                        _build.build()
+                    except Exception as exc:
+                        raise FoxError(f"cannot build {path}: {exc}") from exc
+                spec = importlib.util.spec_from_file_location("_fox_host", path)
+                try:
+                    mod = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(mod)
+                except (ImportError, OSError) as exc:
+                    raise FoxError(f"{path} cannot be loaded ({exc}); run `python -m forgetting_transformer_b200.build`") from exc
+                mod.set_error(FoxError)
+                _host = mod
+    return _host
+
+
 # ------------------------------------------------------------------ status words
-_status = {}
+def _ordinal(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
 
 
 def status_buffer(device: torch.device) -> torch.Tensor:
-    """Per-device int32[4] the attention kernels report a failed bounded wait in."""
-    key = (device.index if device.index is not None else torch.cuda.current_device())
-    buf = _status.get(key)
-    if buf is None:
-        buf = torch.zeros(4, dtype=torch.int32, device=device)
-        _status[key] = buf
-    return buf
-
-
-_readback = {}   # device ordinal -> (pinned int32[4], event of the last queued copy)
-
-
-def queue_status_readback(device: torch.device) -> None:
-    """Queue, on the current stream, a copy of the device's status words to pinned host memory (no
-    synchronisation); ``poll_status`` looks at it once it has landed.  Skipped while a CUDA graph is being
-    captured."""
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    buf = _status.get(key)
-    if buf is None or torch.cuda.is_current_stream_capturing():
-        return
-    slot = _readback.get(key)
-    if slot is None:
-        slot = (torch.zeros(4, dtype=torch.int32).pin_memory(), torch.cuda.Event())
-        _readback[key] = slot
-    slot[0].copy_(buf, non_blocking=True)
-    slot[1].record()
+    """Per-device int32[4] in pinned host memory that the attention kernels report a failed bounded wait in."""
+    return host().status_words(_ordinal(device))
 
 
 def poll_status(device: torch.device) -> None:
-    """Non-synchronising check: raises FoxError when the last status readback that has completed shows that a
-    bounded wait inside a kernel ran out (the results of that step are incomplete)."""
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    slot = _readback.get(key)
-    if slot is None or torch.cuda.is_current_stream_capturing() or not slot[1].query():
-        return
-    vals = slot[0].tolist()
-    if vals[0] != 0:
-        slot[0].zero_()
-        _status[key].zero_()
-        raise FoxError(f"kernel wait timed out in an earlier step: site={vals[0]} cta={vals[1]} thread={vals[2]} "
-                       f"detail={vals[3]}")
+    """Non-synchronising check, made by every forward after a backward: raises FoxError when a bounded wait inside a
+    kernel of an earlier step has run out (the results of that step are incomplete)."""
+    host().status_poll(_ordinal(device))
 
 
 def check_status(device=None) -> None:
     """Synchronising check of the kernels' status words; raises if a wait ran out."""
-    for key, buf in list(_status.items()):
-        if device is not None and torch.device(device).index not in (None, key):
-            continue
-        vals = buf.tolist()
-        if vals[0] != 0:
-            buf.zero_()
-            raise FoxError(f"kernel wait timed out: site={vals[0]} cta={vals[1]} thread={vals[2]} detail={vals[3]}")
+    if _host is None and device is None:
+        return
+    index = None if device is None else torch.device(device).index
+    host().status_check(-1 if index is None else index)

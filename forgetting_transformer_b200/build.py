@@ -1,47 +1,91 @@
-"""Builds the CUDA library in-tree: ``python -m forgetting_transformer_b200.build``.
+"""Builds the native code in-tree: ``python -m forgetting_transformer_b200.build``.
 
-One ``nvcc`` invocation compiles every kernel file for sm_100a only (SASS, no PTX)
-into ``forgetting_transformer_b200/libfox_b200.so``, which exports the C ABI
-declared in ``include/fox_b200.h``.  nvcc cross-compiles, so no GPU is needed.
+Two shared objects next to this file, both git-ignored:
+
+* ``libfox_b200.so``: every kernel file compiled by ``nvcc`` for sm_100a only (SASS, no PTX); exports the C ABI declared
+  in ``include/fox_b200.h``.  nvcc cross-compiles, so no GPU is needed.
+* ``_fox_host.so``: the operators' host side as a Python extension (``g++`` against the installed PyTorch's headers),
+  linked to the first.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libfox_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_fox_host.so")
 SOURCES = ["fox_scan.cu", "fox_attn_fwd.cu", "fox_attn_bwd.cu", "fox_attn_bwd_dq.cu", "fox_attn_bwd_kv.cu", "fox_decode.cu", "fox_normgate.cu", "fox_rmsnorm.cu", "fox_shift.cu", "fox_glu.cu", "fox_ce.cu", "fox_noalloc.cu"]
 HEADERS = ["fox_common.cuh", "fox_host.h", os.path.join("..", "..", "include", "fox_b200.h")]
+HOST_SOURCES = ["host_module.cpp", "host_attention.cpp"]
+HOST_HEADERS = ["host_common.h", "host_attention.h", os.path.join("..", "..", "include", "fox_b200.h")]
 
 
-def _sources():
-    return [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
+def _paths(names):
+    return [p for p in (os.path.join(CSRC, s) for s in names) if os.path.exists(p)]
+
+
+def _stale(target, deps) -> bool:
+    if not os.path.exists(target):
+        return True
+    t = os.path.getmtime(target)
+    return any(os.path.getmtime(d) > t for d in deps)
 
 
 def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = _sources() + [os.path.join(CSRC, h) for h in HEADERS]
-    return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
+    return _stale(LIB_PATH, _paths(SOURCES + HEADERS)) or _stale(HOST_PATH, _paths(HOST_SOURCES + HOST_HEADERS))
+
+
+def _run(cmd, verbose=False):
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    if verbose:
+        sys.stderr.write(res.stderr)
+
+
+def _compile_all(sources, compile_cmd, link_cmd, target, libs=(), verbose=False):
+    """Each source to an object file of its own, side by side, then one link (to a temporary name that replaces the
+    target, so that a process which has the old file mapped keeps it)."""
+    with tempfile.TemporaryDirectory(dir=PKG_DIR, prefix=".build_") as tmp:
+        objs = [os.path.join(tmp, os.path.basename(s) + ".o") for s in sources]
+        with ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as pool:
+            list(pool.map(lambda so: _run(compile_cmd + ["-c", so[0], "-o", so[1]], verbose), zip(sources, objs)))
+        part = os.path.join(tmp, os.path.basename(target))
+        _run(link_cmd + ["-shared", "-o", part] + objs + list(libs))
+        os.replace(part, target)
+
+
+def _build_kernels(verbose):
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    flags = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
+    _compile_all(_paths(SOURCES), flags + (["-Xptxas", "-v"] if verbose else []), flags, LIB_PATH, verbose=verbose)
+
+
+def _build_host(verbose):
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    # (not $CXX: the extension has to share the process's libstdc++, which a compiler that only has the static one breaks)
+    cxx = os.environ.get("FOX_B200_CXX", "g++")
+    inc = include_paths() + [sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+    flags = [cxx, "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f for i in inc for f in ("-isystem", i)]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    libs = ["-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
+            "-L" + PKG_DIR, "-l:libfox_b200.so", "/usr/local/cuda/lib64/libcudart.so", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib]
+    _compile_all(_paths(HOST_SOURCES), flags, [cxx], HOST_PATH, libs, verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not is_stale():
-        return LIB_PATH
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [
-        nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
-        "-shared", "-Xcompiler", "-fPIC", "-o", LIB_PATH,
-    ] + (["-Xptxas", "-v"] if verbose else []) + _sources()
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
-    if verbose:
-        sys.stderr.write(res.stderr)
+    if force or _stale(LIB_PATH, _paths(SOURCES + HEADERS)):
+        _build_kernels(verbose)
+    if force or _stale(HOST_PATH, _paths(HOST_SOURCES + HOST_HEADERS)):
+        _build_host(verbose)
     return LIB_PATH
 
 

@@ -73,6 +73,7 @@ struct BwdParams {
   int* status;
   long long* trace;          // optional (debug builds of the kernel only): clock64 stamps of CTA (0,0,0)
   int H, M, N;
+  bool tma_out;              // dK / dV leave through shared memory and TMA stores
   float sm_scale, qk_scale;
 };
 
@@ -728,7 +729,7 @@ fox_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       constexpr int kCols = D / kPer;
       const int which = g / kPer, part_c = (g % kPer) * kCols;
       const bool keep = j_ok && n_tiles > 0;
-      const bool via_tma = p.end_index != nullptr;
+      const bool via_tma = p.tma_out;
       const uint32_t tcol = tbase + lane_base + (which == 0 ? kColDK : kColDV) + part_c;
       const float sc = which == 0 ? p.sm_scale : 1.f;
       uint16_t* orow = (which == 0
@@ -797,12 +798,13 @@ static long long* g_bwd_trace = nullptr;
 template <int D, bool kBf16>
 static int launch_bwd(int device, cudaStream_t stream, int64_t B, int64_t H, int64_t M, int64_t N,
                       const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v, const fox_tensor4* d_o,
-                      const BwdParams& prm) {
+                      int64_t Dt, const BwdParams& prm) {
+  // Dt <= D: the tensors' own head dim; the TMA unit fills the columns past it with zeros and clips them from stores
   CUtensorMap tmQ, tmK, tmV, tmDO;
-  Tensor4 tq{q->ptr, B, H, M, D, q->sb, q->sh, q->st};
-  Tensor4 tk{k->ptr, B, H, N, D, k->sb, k->sh, k->st};
-  Tensor4 tv{v->ptr, B, H, N, D, v->sb, v->sh, v->st};
-  Tensor4 tdo{d_o->ptr, B, H, M, D, d_o->sb, d_o->sh, d_o->st};
+  Tensor4 tq{q->ptr, B, H, M, Dt, q->sb, q->sh, q->st};
+  Tensor4 tk{k->ptr, B, H, N, Dt, k->sb, k->sh, k->st};
+  Tensor4 tv{v->ptr, B, H, N, Dt, v->sb, v->sh, v->st};
+  Tensor4 tdo{d_o->ptr, B, H, M, Dt, d_o->sb, d_o->sh, d_o->st};
   if (!tma_compatible(tq, 2) || !tma_compatible(tk, 2) || !tma_compatible(tv, 2) || !tma_compatible(tdo, 2))
     return FOX_ERR_ALIGNMENT;
   int rc;
@@ -811,8 +813,8 @@ static int launch_bwd(int device, cudaStream_t stream, int64_t B, int64_t H, int
   if ((rc = cached_tmap_4d(&tmV, tv, 2, false, kBf16, 64, 128, true))) return rc;
   if ((rc = cached_tmap_4d(&tmDO, tdo, 2, false, kBf16, 64, 128, true))) return rc;
   CUtensorMap tmDK, tmDV;
-  Tensor4 tdk{prm.dk, B, H, N, D, prm.dk_sb, prm.dk_sh, prm.dk_st};
-  Tensor4 tdv{prm.dv, B, H, N, D, prm.dv_sb, prm.dv_sh, prm.dv_st};
+  Tensor4 tdk{prm.dk, B, H, N, Dt, prm.dk_sb, prm.dk_sh, prm.dk_st};
+  Tensor4 tdv{prm.dv, B, H, N, Dt, prm.dv_sb, prm.dv_sh, prm.dv_st};
   if (!tma_compatible(tdk, 2) || !tma_compatible(tdv, 2)) return FOX_ERR_ALIGNMENT;
   if ((rc = cached_tmap_4d(&tmDK, tdk, 2, false, kBf16, 64, 128, true))) return rc;
   if ((rc = cached_tmap_4d(&tmDV, tdv, 2, false, kBf16, 64, 128, true))) return rc;
@@ -882,7 +884,8 @@ extern "C" int fox_attn_bwd(int device, void* stream, int dtype, int64_t B, int6
     return FOX_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || M <= 0 || N <= 0 || M > N || H > 65535 || B > 65535) return FOX_ERR_BAD_ARG;
   if (N > 2147483647LL) return FOX_ERR_TOO_LARGE;   // row indices are 32-bit inside the kernels (M <= N)
-  if (D != 64 && D != 128) return FOX_ERR_HEAD_DIM;
+  // head dims 16 and 32 run through the D = 64 one-pass kernel (dq_accum then has 64 columns)
+  if (D != 64 && D != 128 && !((D == 16 || D == 32) && dq_accum_zeroed)) return FOX_ERR_HEAD_DIM;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
   const fox_tensor4* outs[2] = {dk, dv};
   for (int i = 0; i < 2; ++i)
@@ -904,6 +907,7 @@ extern "C" int fox_attn_bwd(int device, void* stream, int dtype, int64_t B, int6
   prm.trace = nullptr;
 #endif
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
+  prm.tma_out = end_index != nullptr || D < 64;
   prm.sm_scale = sm_scale;
   prm.qk_scale = sm_scale * 1.4426950408889634f;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -916,9 +920,9 @@ extern "C" int fox_attn_bwd(int device, void* stream, int dtype, int64_t B, int6
   if (key_side_kernel)
     return launch_bwd_kv(device, st, bf, (int)D, B, H, M, N, q, k, v, d_o, log_lambda, L, delta, seq_start, end_index,
                          sm_scale, dlam_col, dk, dv, status);
-  if (D == 64)
-    return bf ? launch_bwd<64, true>(device, st, B, H, M, N, q, k, v, d_o, prm)
-              : launch_bwd<64, false>(device, st, B, H, M, N, q, k, v, d_o, prm);
-  return bf ? launch_bwd<128, true>(device, st, B, H, M, N, q, k, v, d_o, prm)
-            : launch_bwd<128, false>(device, st, B, H, M, N, q, k, v, d_o, prm);
+  if (D <= 64)
+    return bf ? launch_bwd<64, true>(device, st, B, H, M, N, q, k, v, d_o, D, prm)
+              : launch_bwd<64, false>(device, st, B, H, M, N, q, k, v, d_o, D, prm);
+  return bf ? launch_bwd<128, true>(device, st, B, H, M, N, q, k, v, d_o, D, prm)
+            : launch_bwd<128, false>(device, st, B, H, M, N, q, k, v, d_o, D, prm);
 }

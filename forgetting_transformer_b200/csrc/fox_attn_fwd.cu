@@ -44,7 +44,8 @@ struct FwdParams {
   int* status;
   int H, M, N;
   float qk_scale;              // sm_scale * log2(e)
-  const float* k_norm_max;     // (B,H) max_t ||k[b,h,t,:]||_2, or nullptr: lets a tile skip its maximum pass
+  const float* k_norm_max;     // (B,H,n_norm_parts) max_t ||k[b,h,t,:]||_2 in parts, or nullptr: lets a tile skip its maximum pass
+  int n_norm_parts;            // <= 32
 };
 
 // How many of every 4 column pairs take the FMA-pipe exponential instead of the ex2 unit (measured best:
@@ -339,6 +340,9 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     float qbound = INFINITY;
     if (p.k_norm_max != nullptr && n_tiles > 1) {
       ok = mbar_wait(&bar_q_full, 0, abortp, p.status, kSiteQFull);
+      float kn = lane < p.n_norm_parts ? p.k_norm_max[bh * p.n_norm_parts + lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) kn = fmaxf(kn, __shfl_xor_sync(0xffffffffu, kn, o));
       float ss = 0.f;
 #pragma unroll
       for (int sub = 0; sub < kSub; ++sub) {
@@ -352,7 +356,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           ss = fmaf(f3.x, f3.x, ss); ss = fmaf(f3.y, f3.y, ss);
         }
       }
-      qbound = sqrtf(ss) * p.k_norm_max[bh] * fabsf(p.qk_scale) * 1.0001f + a_i;
+      qbound = sqrtf(ss) * kn * fabsf(p.qk_scale) * 1.0001f + a_i;
     }
     constexpr float kSkipShift = kBf16 ? kSkipShiftBf16 : kSkipShiftFp16;
     constexpr int kPolyQ = (D == 64) ? FOX_POLYQ64 : FOX_POLYQ128;
@@ -582,18 +586,20 @@ extern "C" int fox_debug_read_fwd_trace(long long* host) {
 
 template <bool kBf16, int D, int BN, int STAGES, int CTAS, int NWG, bool PREF>
 static int launch_fwd_t(int device, cudaStream_t stream, int64_t B, int64_t H, int64_t M, int64_t N, const fox_tensor4* q,
-                      const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
+                      int64_t Dt, const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
+  // Dt <= D: the tensors' own head dim.  The boxes are D columns wide all the same: the TMA unit fills the columns
+  // past Dt with zeros, which change no product, and clips them from the stores.
   CUtensorMap tmQ, tmK, tmV;
-  Tensor4 tq{q->ptr, B, H, M, D, q->sb, q->sh, q->st};
-  Tensor4 tk{k->ptr, B, H, N, D, k->sb, k->sh, k->st};
-  Tensor4 tv{v->ptr, B, H, N, D, v->sb, v->sh, v->st};
+  Tensor4 tq{q->ptr, B, H, M, Dt, q->sb, q->sh, q->st};
+  Tensor4 tk{k->ptr, B, H, N, Dt, k->sb, k->sh, k->st};
+  Tensor4 tv{v->ptr, B, H, N, Dt, v->sb, v->sh, v->st};
   if (!tma_compatible(tq, 2) || !tma_compatible(tk, 2) || !tma_compatible(tv, 2)) return FOX_ERR_ALIGNMENT;
   int rc;
   if ((rc = cached_tmap_4d(&tmQ, tq, 2, false, kBf16, 64, 128, true))) return rc;
   if ((rc = cached_tmap_4d(&tmK, tk, 2, false, kBf16, 64, BN, true))) return rc;
   if ((rc = cached_tmap_4d(&tmV, tv, 2, false, kBf16, 64, BN, true))) return rc;
   CUtensorMap tmO;
-  Tensor4 to{prm.o, B, H, M, D, prm.o_sb, prm.o_sh, prm.o_st};
+  Tensor4 to{prm.o, B, H, M, Dt, prm.o_sb, prm.o_sh, prm.o_st};
   if (!tma_compatible(to, 2)) return FOX_ERR_ALIGNMENT;
   if ((rc = cached_tmap_4d(&tmO, to, 2, false, kBf16, 64, 128, true))) return rc;
   constexpr int smem = 128 * D * 2 + 2 * STAGES * BN * D * 2 + 1024;
@@ -611,13 +617,13 @@ static int launch_fwd_t(int device, cudaStream_t stream, int64_t B, int64_t H, i
 
 template <int... A>
 static int launch_fwd(int device, cudaStream_t stream, int64_t B, int64_t H, int64_t M, int64_t N, const fox_tensor4* q,
-                      const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
-  return launch_fwd_t<true, A...>(device, stream, B, H, M, N, q, k, v, prm);
+                      int64_t Dt, const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
+  return launch_fwd_t<true, A...>(device, stream, B, H, M, N, q, Dt, k, v, prm);
 }
 template <int... A>
 static int launch_fwd_fp16(int device, cudaStream_t stream, int64_t B, int64_t H, int64_t M, int64_t N, const fox_tensor4* q,
-                           const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
-  return launch_fwd_t<false, A...>(device, stream, B, H, M, N, q, k, v, prm);
+                           int64_t Dt, const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
+  return launch_fwd_t<false, A...>(device, stream, B, H, M, N, q, Dt, k, v, prm);
 }
 
 }  // namespace fox
@@ -631,12 +637,21 @@ extern "C" int fox_attn_fwd(int device, void* stream, int dtype, int64_t B, int6
                             const float* log_lambda, const int64_t* seq_start, const int64_t* start_index,
                             float sm_scale, const fox_tensor4* o, float* L, const float* k_norm_max,
                             int32_t* status) {
+  return fox_attn_fwd_parts(device, stream, dtype, B, H, M, N, D, q, k, v, log_lambda, seq_start, start_index, sm_scale, o,
+                            L, k_norm_max, 1, status);
+}
+
+extern "C" int fox_attn_fwd_parts(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N,
+                                  int64_t D, const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v,
+                                  const float* log_lambda, const int64_t* seq_start, const int64_t* start_index,
+                                  float sm_scale, const fox_tensor4* o, float* L, const float* k_norm_parts,
+                                  int64_t n_norm_parts, int32_t* status) {
   using namespace fox;
   if (!q || !k || !v || !o || !q->ptr || !k->ptr || !v->ptr || !o->ptr || !log_lambda || !L || !status)
     return FOX_ERR_BAD_ARG;
   if (B <= 0 || H <= 0 || M <= 0 || N <= 0 || M > N || H > 65535 || B > 65535) return FOX_ERR_BAD_ARG;
   if (N > 2147483647LL) return FOX_ERR_TOO_LARGE;   // row indices are 32-bit inside the kernels (M <= N)
-  if (D != 64 && D != 128) return FOX_ERR_HEAD_DIM;
+  if (D != 16 && D != 32 && D != 64 && D != 128) return FOX_ERR_HEAD_DIM;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
   if (reinterpret_cast<uintptr_t>(o->ptr) % 16 || (o->sb * 2) % 16 || (o->sh * 2) % 16 || (o->st * 2) % 16)
     return FOX_ERR_ALIGNMENT;
@@ -650,20 +665,22 @@ extern "C" int fox_attn_fwd(int device, void* stream, int dtype, int64_t B, int6
   prm.status = status;
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
   prm.qk_scale = sm_scale * 1.4426950408889634f;
-  prm.k_norm_max = k_norm_max;
+  if (k_norm_parts && (n_norm_parts <= 0 || n_norm_parts > 32)) return FOX_ERR_BAD_ARG;
+  prm.k_norm_max = k_norm_parts;
+  prm.n_norm_parts = (int)n_norm_parts;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const bool bf = dtype == FOX_DTYPE_BF16;
 #ifdef FOX_DEBUG
   const int variant = g_fwd_variant;
 #endif
 #define FOX_FWD_LAUNCH(...) \
-  (bf ? launch_fwd<__VA_ARGS__>(device, st, B, H, M, N, q, k, v, prm) : launch_fwd_fp16<__VA_ARGS__>(device, st, B, H, M, N, q, k, v, prm))
+  (bf ? launch_fwd<__VA_ARGS__>(device, st, B, H, M, N, q, D, k, v, prm) : launch_fwd_fp16<__VA_ARGS__>(device, st, B, H, M, N, q, D, k, v, prm))
   //                 D  BN  STAGES CTAS NWG PREF
 #ifdef FOX_DEBUG
   if (D == 64 && variant == 1) return FOX_FWD_LAUNCH(64, 128, 2, 2, 1, false);
   if (D == 128 && variant == 2) return FOX_FWD_LAUNCH(128, 64, 2, 2, 1, false);
 #endif
-  if (D == 64) return FOX_FWD_LAUNCH(64, 128, 2, 2, 2, false);
+  if (D <= 64) return FOX_FWD_LAUNCH(64, 128, 2, 2, 2, false);
   return FOX_FWD_LAUNCH(128, 128, 1, 2, 1, true);
 #undef FOX_FWD_LAUNCH
 }

@@ -10,6 +10,8 @@
 //   _bwd_preprocess ........................ lines 902-943
 //   reverse cumsum of dlog_lambda .......... lines 390-392
 //   vector_norm(...).max(...) .............. lines 95-96
+#include <math.h>
+
 #include "fox_common.cuh"
 #include "fox_host.h"
 
@@ -66,12 +68,11 @@ __device__ __forceinline__ float load_gate(const void* base, int64_t idx) {
 // One CTA per (b,h); chunks of 4096 elements with a carried running total.  With gate logits as input
 // (kIn < 3) the log gates themselves are formed on the fly and, if lf_out is given, written out (unmasked).
 template <int kIn>
-__global__ void __launch_bounds__(kScanThreads)
-fox_cumsum_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
-                  const int64_t* __restrict__ seq_start, const float* __restrict__ carry_in,
-                  float* __restrict__ out, float* __restrict__ total_out, float* __restrict__ lf_out, int H, int N) {
-  __shared__ float red[32];
-  const int bh = blockIdx.x, b = bh / H, h = bh % H;
+__device__ __forceinline__ void cumsum_rows(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
+                                            const int64_t* __restrict__ seq_start, const float* __restrict__ carry_in,
+                                            float* __restrict__ out, float* __restrict__ total_out,
+                                            float* __restrict__ lf_out, int H, int N, int bh, float* red) {
+  const int b = bh / H, h = bh % H;
   const int64_t src0 = b * sb + h * sh;
   float* dst = out + static_cast<int64_t>(bh) * N;
   const int s0 = seq_start ? static_cast<int>(seq_start[b]) : 0;
@@ -102,20 +103,40 @@ fox_cumsum_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t s
   if (total_out && threadIdx.x == 0) total_out[bh] = carry;
 }
 
+template <int kIn>
+__global__ void __launch_bounds__(kScanThreads)
+fox_cumsum_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
+                  const int64_t* __restrict__ seq_start, const float* __restrict__ carry_in,
+                  float* __restrict__ out, float* __restrict__ total_out, float* __restrict__ lf_out, int H, int N) {
+  __shared__ float red[32];
+  cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, carry_in, out, total_out, lf_out, H, N, blockIdx.x, red);
+}
+
 // dlog_fgate[t] = carry_in + sum_{u >= t} (dcol[u] + drow[u - P] if u >= P)
 // Reverse inclusive scan, one CTA per (b,h).  kIn < 3: the chain rule through log sigmoid is applied on the way
 // out, dlogit[t] = dlog_fgate[t] * sigmoid(-logit[t]), written in the logits' dtype with the logits' strides.
+struct RevParams {
+  const float *dcol, *drow, *carry_in;
+  float *out, *total_out;
+  int M, N;
+  const void* logit;       // kIn < 3
+  void* dlogit;
+  int64_t sb, sh, sn;      // strides of logit
+  int64_t osb, osh, osn;   // strides of out / dlogit
+  int H;
+};
+
 template <int kIn>
-__global__ void __launch_bounds__(kScanThreads)
-fox_revcumsum_kernel(const float* __restrict__ dcol, const float* __restrict__ drow,
-                     const float* __restrict__ carry_in, float* __restrict__ out,
-                     float* __restrict__ total_out, int M, int N, const void* __restrict__ logit,
-                     void* __restrict__ dlogit, int64_t sb, int64_t sh, int64_t sn, int H) {
-  __shared__ float red[32];
-  const int bh = blockIdx.x;
+__device__ __forceinline__ void revcumsum_rows(const RevParams& p, int bh, float* red) {
+  const float *dcol = p.dcol, *drow = p.drow, *carry_in = p.carry_in;
+  float *out = p.out, *total_out = p.total_out;
+  const int M = p.M, N = p.N, H = p.H;
+  const void* logit = p.logit;
+  void* dlogit = p.dlogit;
+  const int64_t sb = p.sb, sh = p.sh, sn = p.sn;
   const float* c = dcol + static_cast<int64_t>(bh) * N;
   const float* r = drow ? drow + static_cast<int64_t>(bh) * M : nullptr;
-  float* dst = out + static_cast<int64_t>(bh) * N;
+  const int64_t o0 = static_cast<int64_t>(bh / H) * p.osb + static_cast<int64_t>(bh % H) * p.osh;
   const int P = N - M;
   float carry = carry_in ? carry_in[bh] : 0.f;
   // walk chunks from the right; inside a chunk index i runs right-to-left
@@ -143,15 +164,16 @@ fox_revcumsum_kernel(const float* __restrict__ dcol, const float* __restrict__ d
       if (t >= 0) {
         const float gsum = x[j] + excl;
         if constexpr (kIn == 3) {
-          dst[t] = gsum;
+          out[o0 + static_cast<int64_t>(t) * p.osn] = gsum;
         } else {
           const int64_t idx = static_cast<int64_t>(bh / H) * sb + static_cast<int64_t>(bh % H) * sh + static_cast<int64_t>(t) * sn;
           float xl;
           if constexpr (kIn == 2) xl = reinterpret_cast<const float*>(logit)[idx];
           else xl = unpack2<kIn == 1>(static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(logit)[idx])).x;
           const float dl = gsum / (1.f + expf(xl));     // d/dx log sigmoid(x) = sigmoid(-x)
-          if constexpr (kIn == 2) reinterpret_cast<float*>(dlogit)[idx] = dl;
-          else reinterpret_cast<uint16_t*>(dlogit)[idx] = static_cast<uint16_t>(pack2<kIn == 1>(dl, 0.f) & 0xffffu);
+          const int64_t odx = o0 + static_cast<int64_t>(t) * p.osn;
+          if constexpr (kIn == 2) reinterpret_cast<float*>(dlogit)[odx] = dl;
+          else reinterpret_cast<uint16_t*>(dlogit)[odx] = static_cast<uint16_t>(pack2<kIn == 1>(dl, 0.f) & 0xffffu);
         }
       }
     }
@@ -161,53 +183,112 @@ fox_revcumsum_kernel(const float* __restrict__ dcol, const float* __restrict__ d
 }
 
 // ------------------------------------------------------------ pruning indices
-// One CTA per (b,h).  The scans only look at log_lambda on block boundaries, so
-// those values are staged in shared memory and one thread replays upstream's
-// carried sequential scan on them (bit-identical decisions, no dependent global
-// loads).  start != nullptr: start_index (B,H,ceil(M/BM)); end != nullptr:
-// end_index (B,H,ceil(N/BN)).
-__global__ void __launch_bounds__(256)
-fox_find_index_kernel(const float* __restrict__ lam, const float* __restrict__ thr, int64_t thr_sb,
-                      int64_t thr_sh, int64_t* __restrict__ start, int64_t* __restrict__ end, int H, int M,
-                      int N, int BM, int BN, int nmb, int nnb) {
+// Threshold of one (b,h): a value (kThrTensor: read from a (B,H) view), or upstream's automatic rule
+// -(2 max||q|| max||k|| sm_scale + log N) - 10 evaluated step by step in the input dtype
+// (src/forgetting_transformer/ops/forgetting_attention.py:91-109) from fp32 norm maxima.
+enum ThresholdKind { kThrTensor = 0, kThrScalar = 1, kThrAutoFp16 = 2, kThrAutoBf16 = 3 };
+
+template <bool kBf16>
+__device__ __forceinline__ float round16(float x) {
+  return unpack2<kBf16>(pack2<kBf16>(x, 0.f)).x;
+}
+template <bool kBf16>
+__device__ __forceinline__ float auto_threshold(float qn, float kn, float sm_scale, float log_n) {
+  const float bound = round16<kBf16>(round16<kBf16>(round16<kBf16>(qn) * round16<kBf16>(kn)) * sm_scale);
+  const float s = round16<kBf16>(round16<kBf16>(2.f * bound) + log_n);
+  return round16<kBf16>(-s - 10.f);
+}
+
+struct IndexParams {
+  const float* lam;
+  const float* thr;            // kThrTensor
+  int64_t thr_sb, thr_sh;
+  float thr_value;             // kThrScalar
+  const float *q_parts, *k_parts;   // automatic: per-(b,h) partial norm maxima
+  int n_q_parts, n_k_parts;
+  float sm_scale, log_n;
+  int kind;
+  int64_t *start, *end;
+  float* thr_out;              // (B,H) or nullptr: the threshold that was used
+  int H, M, N, BM, BN, nmb, nnb;
+};
+
+// One CTA of two warps per (b,h).  The scans only look at log_lambda on block boundaries, so those values are
+// staged in shared memory, and a warp replays upstream's carried sequential scan on them: the scan's "advance while
+// the condition holds" is a search for the first block where it fails, which the 32 lanes test 32 blocks at a time
+// (same comparisons on the same values: bit-identical arrays).  Warp 0: start_index (B,H,ceil(M/BM)); warp 1:
+// end_index (B,H,ceil(N/BN)).  Bound by the dependent steps of the scan: one thread per scan took 24 us per call at
+// 128 x 128 blocks.
+__global__ void __launch_bounds__(64)
+fox_find_index_kernel(const IndexParams p) {
   extern __shared__ float sm[];
+  const int nmb = p.nmb, nnb = p.nnb, M = p.M, N = p.N, BM = p.BM, BN = p.BN;
   float* row_first = sm;        // lam[P + mb*BM]            (nmb)
   float* col_last = sm + nmb;   // lam[min(N-1, nb*BN+BN-1)] (nnb)
   float* row_e = col_last + nnb;  // lam[min(mb*BM, M-1)], mb in [0, nmb]  (nmb + 1)
-  const int bh = blockIdx.x, b = bh / H, h = bh % H;
-  const float* l = lam + static_cast<int64_t>(bh) * N;
+  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* l = p.lam + static_cast<int64_t>(bh) * N;
   const int P = N - M;
   for (int i = threadIdx.x; i < nmb; i += blockDim.x) row_first[i] = l[P + i * BM];
   for (int i = threadIdx.x; i < nnb; i += blockDim.x) col_last[i] = l[min(N - 1, i * BN + BN - 1)];
   for (int i = threadIdx.x; i <= nmb; i += blockDim.x) row_e[i] = l[min(min(i * BM, M), M - 1)];
+  float t;
+  if (p.kind == kThrTensor) {
+    t = p.thr[b * p.thr_sb + h * p.thr_sh];
+  } else if (p.kind == kThrScalar) {
+    t = p.thr_value;
+  } else {
+    float qn = 0.f, kn = 0.f;
+    for (int i = lane; i < p.n_q_parts; i += 32) qn = fmaxf(qn, p.q_parts[bh * p.n_q_parts + i]);
+    for (int i = lane; i < p.n_k_parts; i += 32) kn = fmaxf(kn, p.k_parts[bh * p.n_k_parts + i]);
+    for (int o = 16; o > 0; o >>= 1) {
+      qn = fmaxf(qn, __shfl_xor_sync(0xffffffffu, qn, o));
+      kn = fmaxf(kn, __shfl_xor_sync(0xffffffffu, kn, o));
+    }
+    t = p.kind == kThrAutoBf16 ? auto_threshold<true>(qn, kn, p.sm_scale, p.log_n)
+                               : auto_threshold<false>(qn, kn, p.sm_scale, p.log_n);
+  }
+  if (p.thr_out && threadIdx.x == 0) p.thr_out[bh] = t;
   __syncthreads();
-  const float t = thr[b * thr_sb + h * thr_sh];
-  if (threadIdx.x == 0 && start) {
-    int64_t* dst = start + static_cast<int64_t>(bh) * nmb;
+  if (warp == 0 && p.start) {
+    int64_t* dst = p.start + static_cast<int64_t>(bh) * nmb;
     int s = 0;  // in blocks of BN
     for (int mb = 0; mb < nmb; ++mb) {
       const float lo = row_first[mb];
-      // upstream: while (lo - lam[min(N-1, s+BN-1)] < thr) s += BN.  Past the last
-      // block the clamped column stays N-1, which is col_last[nnb-1].
-      int guard = 0;
-      while (lo - col_last[min(s, nnb - 1)] < t && guard < nnb + 2) {
-        ++s;
-        if (s >= nnb) ++guard;
+      // upstream: while (lo - lam[min(N-1, s+BN-1)] < thr) s += BN.  Past the last block the clamped column stays
+      // N-1, which is col_last[nnb-1]: a condition that still holds there holds for ever (upstream would not
+      // return; here s moves on by nnb + 2 blocks past it).
+      bool found = false;
+      for (int s0 = s; s0 < nnb && !found; s0 += 32) {
+        const int c = s0 + lane;
+        const unsigned stop = __ballot_sync(0xffffffffu, c < nnb && !(lo - col_last[min(c, nnb - 1)] < t));
+        if (stop) {
+          s = s0 + __ffs(stop) - 1;
+          found = true;
+        }
       }
-      dst[mb] = static_cast<int64_t>(s) * BN;
+      if (!found && lo - col_last[nnb - 1] < t) s = s < nnb ? 2 * nnb + 1 : s + nnb + 2;
+      if (lane == 0) dst[mb] = static_cast<int64_t>(s) * BN;
     }
   }
-  if (threadIdx.x == 32 && end) {
-    int64_t* dst = end + static_cast<int64_t>(bh) * nnb;
-    int e = 0;  // row index, multiple of BM or M
+  if (warp == 1 && p.end) {
+    int64_t* dst = p.end + static_cast<int64_t>(bh) * nnb;
+    int eb = 0;  // row block: the row index is min(eb * BM, M)
     for (int nb = 0; nb < nnb; ++nb) {
       const float li = col_last[nb];
-      while (e < M) {
-        const int eb = (e + BM - 1) / BM;  // e is k*BM (eb = k) or M (eb = nmb, handled by e < M)
-        if (!(row_e[eb] - li >= t)) break;
-        e = min(e + BM, M);
+      bool found = false;
+      while (eb < nmb && !found) {
+        const int c = eb + lane;
+        const unsigned stop = __ballot_sync(0xffffffffu, c < nmb && !(row_e[min(c, nmb)] - li >= t));
+        if (stop) {
+          eb += __ffs(stop) - 1;
+          found = true;
+        } else {
+          eb = min(eb + 32, nmb);
+        }
       }
-      dst[nb] = e;
+      if (lane == 0) dst[nb] = min(eb * BM, M);
     }
   }
 }
@@ -258,15 +339,87 @@ fox_max_row_norm_kernel(const uint16_t* __restrict__ x, int64_t sb, int64_t sh, 
   if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(out + bh), __float_as_int(best));
 }
 
+// ------------------------------------------------------ before the attention forward
+// The prefix sum of the log gates and the largest key (and, for the automatic threshold, query) row norms in one
+// launch: they are independent, and each alone leaves most of the chip idle (one CTA per (b,h) scans, a scan of
+// 16384 gates takes 10 us).  blockIdx.x = 0 scans; blocks 1 .. n_k (n_k+1 .. n_k+n_q) each take every n_k-th
+// (n_q-th) group of rows and write ONE partial maximum, so nothing has to be zeroed first; the reader takes the
+// maximum of the parts.
+struct NormSource {
+  const uint16_t* x;
+  int64_t sb, sh, st;
+  int T, n_parts;
+  float* parts;   // (B*H, n_parts)
+};
+
+// max over this block's rows of the squared norm, then its root: D / 8 lanes share a row (one 16-byte load each),
+// four rows per iteration with their loads issued first
+template <bool kBf16>
+__device__ __forceinline__ void norm_part(const NormSource& s, int D, int H, int bh, int part, float* red) {
+  const int lanes_per_row = D / 8;
+  const int rows_per_block = kScanThreads / lanes_per_row;
+  const int sub = threadIdx.x % lanes_per_row, r_in = threadIdx.x / lanes_per_row;
+  const uint16_t* base = s.x + (bh / H) * s.sb + (bh % H) * s.sh + sub * 8;
+  const int stride = s.n_parts * rows_per_block;
+  float best = 0.f;
+  constexpr int kU = 4;
+  for (int t0 = part * rows_per_block; t0 < s.T; t0 += kU * stride) {
+    uint4 v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int t = t0 + u * stride + r_in;
+      v[u] = make_uint4(0, 0, 0, 0);
+      if (t < s.T) v[u] = *reinterpret_cast<const uint4*>(base + static_cast<int64_t>(t) * s.st);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack2<kBf16>(w[j]);
+        acc = fmaf(f.x, f.x, acc);
+        acc = fmaf(f.y, f.y, acc);
+      }
+      for (int o = lanes_per_row / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      best = fmaxf(best, acc);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = red[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    // (sqrt is monotone and correctly rounded: same result as the maximum of the roots)
+    if (threadIdx.x == 0) s.parts[static_cast<int64_t>(bh) * s.n_parts + part] = sqrtf(best);
+  }
+}
+
+template <int kIn, bool kBf16>
+__global__ void __launch_bounds__(kScanThreads)
+fox_prologue_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
+                    const int64_t* __restrict__ seq_start, float* __restrict__ lam, const NormSource k,
+                    const NormSource q, int H, int N, int D) {
+  __shared__ float red[32];
+  const int bh = blockIdx.y, x = blockIdx.x;
+  if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+  else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
+  else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
+}
+
 // ------------------------------------------------------ delta = rowsum(O * dO)
 // D / 8 lanes share a row (16 bytes each); a thread takes kDeltaRows rows a block-stride apart and issues all
-// its loads before using any (two loads per thread left the kernel at a third of the copy rate).
+// its loads before using any (two loads per thread left the kernel at a third of the copy rate).  For the one-pass
+// backward the same threads clear the fp32 accumulators of their rows (acc_cols floats a row of dq_acc, dlam_row),
+// which a fill kernel of its own did in front of it.
 constexpr int kDeltaRows = 4;
+constexpr int kAccumCols = 64;
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
 fox_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int64_t o_st,
                  const uint16_t* __restrict__ d_o, int64_t d_sb, int64_t d_sh, int64_t d_st, int H, int M, int D,
-                 float* __restrict__ delta) {
+                 float* __restrict__ delta, float* __restrict__ dq_acc, int acc_cols, float* __restrict__ dlam_row) {
   const int lanes_per_row = D / 8;
   const int rows_per_pass = 256 / lanes_per_row;
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
@@ -282,6 +435,17 @@ fox_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int
     if (row < M) {
       a[i] = *reinterpret_cast<const uint4*>(ob + static_cast<int64_t>(row) * o_st);
       g[i] = *reinterpret_cast<const uint4*>(gb + static_cast<int64_t>(row) * d_st);
+    }
+  }
+  if (dq_acc) {   // (under the loads) whole rows by the lanes that share one, neighbouring lanes 16 bytes apart
+#pragma unroll
+    for (int i = 0; i < kDeltaRows; ++i) {
+      const int row = row0 + i * rows_per_pass;
+      if (row < M) {
+        float4* z = reinterpret_cast<float4*>(dq_acc + (static_cast<int64_t>(bh) * M + row) * acc_cols);
+        for (int c = sub; c < acc_cols / 4; c += lanes_per_row) z[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (sub == 0) dlam_row[static_cast<int64_t>(bh) * M + row] = 0.f;
+      }
     }
   }
 #pragma unroll
@@ -300,25 +464,57 @@ fox_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int
   }
 }
 
-// ------------------------------------------- dq = (fp32 accumulator) * scale
+// ------------------------------------------- after the attention backward
+// The reverse prefix sum of the gate gradient and, for the one-pass backward, dq = (fp32 accumulator) * scale in
+// 16 bits.  One launch: the first scan_blocks CTAs scan (one (b,h) each, started first because they are the long
+// ones), the others convert, each thread 8 channels of kConvRows rows with its loads issued first.
+struct ConvParams {
+  const float* acc;       // (B,H,M,acc_cols)
+  uint16_t* dq;
+  int64_t sb, sh, st;
+  int H, M, D, acc_cols;
+  float scale;
+  int blocks_per_bh, units;   // units = B * H; 0: nothing to convert
+};
+constexpr int kConvRows = 2;
+
 template <bool kBf16>
-__global__ void __launch_bounds__(256)
-fox_dq_convert_kernel(const float* __restrict__ acc, uint16_t* __restrict__ dq, int64_t sb, int64_t sh, int64_t st,
-                      int H, int M, int D, float scale) {
-  const int lanes_per_row = D / 8;
-  const int rows_per_block = 256 / lanes_per_row;
-  const int bh = blockIdx.y, b = bh / H, h = bh % H;
+__device__ __forceinline__ void convert_rows(const ConvParams& p, int block) {
+  const int lanes_per_row = p.D / 8;
+  const int rows_per_pass = kScanThreads / lanes_per_row;
+  const int bh = block / p.blocks_per_bh, b = bh / p.H, h = bh % p.H;
   const int sub = threadIdx.x % lanes_per_row;
-  const int row = blockIdx.x * rows_per_block + threadIdx.x / lanes_per_row;
-  if (row >= M) return;
-  const float4* src = reinterpret_cast<const float4*>(acc + (static_cast<int64_t>(bh) * M + row) * D + sub * 8);
-  const float4 a = src[0], c = src[1];
-  uint4 w;
-  w.x = pack2<kBf16>(a.x * scale, a.y * scale);
-  w.y = pack2<kBf16>(a.z * scale, a.w * scale);
-  w.z = pack2<kBf16>(c.x * scale, c.y * scale);
-  w.w = pack2<kBf16>(c.z * scale, c.w * scale);
-  *reinterpret_cast<uint4*>(dq + b * sb + h * sh + static_cast<int64_t>(row) * st + sub * 8) = w;
+  const int row0 = (block % p.blocks_per_bh) * rows_per_pass * kConvRows + threadIdx.x / lanes_per_row;
+  float4 a[kConvRows], c[kConvRows];
+#pragma unroll
+  for (int i = 0; i < kConvRows; ++i) {
+    const int row = row0 + i * rows_per_pass;
+    if (row < p.M) {
+      const float4* src = reinterpret_cast<const float4*>(p.acc + (static_cast<int64_t>(bh) * p.M + row) * p.acc_cols + sub * 8);
+      a[i] = src[0];
+      c[i] = src[1];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kConvRows; ++i) {
+    const int row = row0 + i * rows_per_pass;
+    if (row < p.M) {
+      uint4 w;
+      w.x = pack2<kBf16>(a[i].x * p.scale, a[i].y * p.scale);
+      w.y = pack2<kBf16>(a[i].z * p.scale, a[i].w * p.scale);
+      w.z = pack2<kBf16>(c[i].x * p.scale, c[i].y * p.scale);
+      w.w = pack2<kBf16>(c[i].z * p.scale, c[i].w * p.scale);
+      *reinterpret_cast<uint4*>(p.dq + b * p.sb + h * p.sh + static_cast<int64_t>(row) * p.st + sub * 8) = w;
+    }
+  }
+}
+
+template <int kIn, bool kBf16>
+__global__ void __launch_bounds__(kScanThreads)
+fox_bwd_finish_kernel(const RevParams rev, const ConvParams conv, int scan_blocks) {
+  __shared__ float red[32];
+  if (static_cast<int>(blockIdx.x) < scan_blocks) revcumsum_rows<kIn>(rev, blockIdx.x, red);
+  else convert_rows<kBf16>(conv, blockIdx.x - scan_blocks);
 }
 
 static inline bool head_dim_ok(int64_t D) { return D == 16 || D == 32 || D == 64 || D == 128; }
@@ -361,14 +557,43 @@ extern "C" int fox_gate_prefix_fwd(int device, void* stream, int dtype, int64_t 
   return launch_rc();
 }
 
+static ConvParams make_conv(int64_t B, int64_t H, int64_t M, int64_t D, const float* acc, int64_t acc_cols, float scale,
+                            const fox_tensor4* dq) {
+  ConvParams c{};
+  c.acc = acc; c.dq = (uint16_t*)dq->ptr; c.sb = dq->sb; c.sh = dq->sh; c.st = dq->st;
+  c.H = (int)H; c.M = (int)M; c.D = (int)D; c.acc_cols = (int)acc_cols; c.scale = scale;
+  const int64_t rows_per_block = kConvRows * kScanThreads / (D / 8);
+  c.blocks_per_bh = (int)((M + rows_per_block - 1) / rows_per_block);
+  c.units = (int)(B * H);
+  return c;
+}
+
+// (reverse scan and / or dQ conversion; every public entry point below ends here)
+static int launch_finish(cudaStream_t st, int gate_kind, bool bf16, const RevParams& rev, int scan_blocks,
+                         const ConvParams& conv) {
+  const int64_t grid = scan_blocks + static_cast<int64_t>(conv.units) * conv.blocks_per_bh;
+  if (grid <= 0 || grid > 2147483647LL) return FOX_ERR_TOO_LARGE;
+  switch (gate_kind) {
+#define FOX_FIN(K)                                                                                          \
+  if (bf16) fox_bwd_finish_kernel<K, true><<<(unsigned)grid, kScanThreads, 0, st>>>(rev, conv, scan_blocks); \
+  else fox_bwd_finish_kernel<K, false><<<(unsigned)grid, kScanThreads, 0, st>>>(rev, conv, scan_blocks)
+    case FOX_DTYPE_FP16: FOX_FIN(0); break;
+    case FOX_DTYPE_BF16: FOX_FIN(1); break;
+    case FOX_DTYPE_FP32: FOX_FIN(2); break;
+    case FOX_GATE_LOG: FOX_FIN(3); break;
+#undef FOX_FIN
+    default: return FOX_ERR_BAD_ARG;
+  }
+  return launch_rc();
+}
+
 extern "C" int fox_revcumsum(int device, void* stream, int64_t B, int64_t H, int64_t M, int64_t N,
                              const float* dlam_col, const float* dlam_row, const float* carry_in,
                              float* dlog_fgate, float* total_out) {
   if (!dlam_col || !dlog_fgate || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  fox_revcumsum_kernel<3><<<(unsigned)(B * H), kScanThreads, 0, (cudaStream_t)stream>>>(
-      dlam_col, dlam_row, carry_in, dlog_fgate, total_out, (int)M, (int)N, nullptr, nullptr, 0, 0, 0, (int)H);
-  return launch_rc();
+  const RevParams rev{dlam_col, dlam_row, carry_in, dlog_fgate, total_out, (int)M, (int)N, nullptr, nullptr, 0, 0, 0, H * N, N, 1, (int)H};
+  return launch_finish((cudaStream_t)stream, FOX_GATE_LOG, false, rev, (int)(B * H), ConvParams{});
 }
 
 extern "C" int fox_gate_prefix_bwd(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N,
@@ -377,14 +602,111 @@ extern "C" int fox_gate_prefix_bwd(int device, void* stream, int dtype, int64_t 
   if (!dlam_col || !fgate_logit || !dfgate_logit || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (dtype != FOX_DTYPE_FP16 && dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP32) return FOX_ERR_BAD_ARG;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  const unsigned grid = (unsigned)(B * H);
+  const RevParams rev{dlam_col, dlam_row, nullptr, nullptr, nullptr, (int)M, (int)N, fgate_logit, dfgate_logit, sb, sh, sn, sb, sh, sn, (int)H};
+  return launch_finish((cudaStream_t)stream, dtype, false, rev, (int)(B * H), ConvParams{});
+}
+
+extern "C" int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
+                              const float* dlam_col, const float* dlam_row, int gate_kind, const void* fgate_logit,
+                              int64_t sb, int64_t sh, int64_t sn, void* dgate, int64_t osb, int64_t osh, int64_t osn,
+                              const float* dq_accum, float scale, const fox_tensor4* dq) {
+  if (!dlam_col || !dgate || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
+  if (gate_kind != FOX_GATE_LOG && !fgate_logit) return FOX_ERR_BAD_ARG;
+  if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
+  if ((dq_accum == nullptr) != (dq == nullptr)) return FOX_ERR_BAD_ARG;
+  if (!head_dim_ok(D)) return FOX_ERR_HEAD_DIM;
+  if (dq && (!aligned16(dq) || reinterpret_cast<uintptr_t>(dq_accum) % 16)) return FOX_ERR_ALIGNMENT;
+  if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
+  const bool log_gate = gate_kind == FOX_GATE_LOG;
+  const RevParams rev{dlam_col, dlam_row, nullptr, log_gate ? (float*)dgate : nullptr, nullptr, (int)M, (int)N,
+                      fgate_logit, dgate, sb, sh, sn, osb, osh, osn, (int)H};
+  ConvParams conv{};
+  if (dq) conv = make_conv(B, H, M, D, dq_accum, D > kAccumCols ? D : kAccumCols, scale, dq);
+  return launch_finish((cudaStream_t)stream, gate_kind, dtype == FOX_DTYPE_BF16, rev, (int)(B * H), conv);
+}
+
+// Parts a (b,h)'s row-norm maximum is split into: about two blocks of 1024 threads per SM over all (b,h), never more
+// than the row groups there are, at most 32 (a warp of the reader takes one each).
+extern "C" int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D) {
+  const int64_t rows_per_block = kScanThreads / (D / 8);
+  int64_t n = (T + rows_per_block - 1) / rows_per_block;
+  const int64_t per_unit = (148 * 2) / (B * H) > 0 ? (148 * 2) / (B * H) : 1;
+  n = n < per_unit ? n : per_unit;
+  return n < 32 ? n : 32;
+}
+
+extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M,
+                                 int64_t N, int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn,
+                                 const int64_t* seq_start, float* log_lambda, const fox_tensor4* k, float* k_parts,
+                                 int64_t n_k_parts, const fox_tensor4* q, float* q_parts, int64_t n_q_parts) {
+  if (!gates || !log_lambda || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
+  if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
+  if (B * H > 65535) return FOX_ERR_TOO_LARGE;   // (b, h) is the grid's y index
+  if (!head_dim_ok(D)) return FOX_ERR_HEAD_DIM;
+  NormSource ks{}, qs{};
+  if (k) {
+    if (!aligned16(k)) return FOX_ERR_ALIGNMENT;
+    if (!k_parts || n_k_parts <= 0) return FOX_ERR_BAD_ARG;
+    ks = NormSource{(const uint16_t*)k->ptr, k->sb, k->sh, k->st, (int)N, (int)n_k_parts, k_parts};
+  }
+  if (q) {
+    if (!aligned16(q)) return FOX_ERR_ALIGNMENT;
+    if (!q_parts || n_q_parts <= 0) return FOX_ERR_BAD_ARG;
+    qs = NormSource{(const uint16_t*)q->ptr, q->sb, q->sh, q->st, (int)M, (int)n_q_parts, q_parts};
+  }
+  if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
+  dim3 grid((unsigned)(1 + ks.n_parts + qs.n_parts), (unsigned)(B * H));
   cudaStream_t st = (cudaStream_t)stream;
-#define FOX_GPB(K) fox_revcumsum_kernel<K><<<grid, kScanThreads, 0, st>>>(dlam_col, dlam_row, nullptr, nullptr, nullptr, (int)M, (int)N, fgate_logit, dfgate_logit, sb, sh, sn, (int)H)
-  if (dtype == FOX_DTYPE_FP16) FOX_GPB(0);
-  else if (dtype == FOX_DTYPE_BF16) FOX_GPB(1);
-  else FOX_GPB(2);
-#undef FOX_GPB
+  const bool bf = dtype == FOX_DTYPE_BF16;
+#define FOX_PRO(K)                                                                                                       \
+  if (bf) fox_prologue_kernel<K, true><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D); \
+  else fox_prologue_kernel<K, false><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D)
+  switch (gate_kind) {
+    case FOX_DTYPE_FP16: FOX_PRO(0); break;
+    case FOX_DTYPE_BF16: FOX_PRO(1); break;
+    case FOX_DTYPE_FP32: FOX_PRO(2); break;
+    case FOX_GATE_LOG: FOX_PRO(3); break;
+    default: return FOX_ERR_BAD_ARG;
+  }
+#undef FOX_PRO
   return launch_rc();
+}
+
+static int launch_index(int device, cudaStream_t st, int64_t B, IndexParams p) {
+  p.nmb = (p.M + p.BM - 1) / p.BM;
+  p.nnb = (p.N + p.BN - 1) / p.BN;
+  const size_t smem = sizeof(float) * (2 * (size_t)p.nmb + (size_t)p.nnb + 1);
+  if (smem > 200 * 1024) return FOX_ERR_TOO_LARGE;
+  if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
+  if (smem > 48 * 1024) {
+    if (cudaFuncSetAttribute(fox_find_index_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return FOX_ERR_LAUNCH;
+  }
+  fox_find_index_kernel<<<(unsigned)(B * p.H), 64, smem, st>>>(p);
+  return launch_rc();
+}
+
+extern "C" int fox_attn_index(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N,
+                              int64_t block_m, int64_t block_n, const float* log_lambda, float threshold,
+                              const float* q_parts, int64_t n_q_parts, const float* k_parts, int64_t n_k_parts,
+                              float sm_scale, int64_t* start_index, int64_t* end_index, float* threshold_out) {
+  if (!log_lambda || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N || block_m <= 0 || block_n <= 0)
+    return FOX_ERR_BAD_ARG;
+  if ((q_parts == nullptr) != (k_parts == nullptr)) return FOX_ERR_BAD_ARG;
+  if (!start_index && !end_index && !threshold_out) return FOX_OK;
+  IndexParams p{};
+  p.lam = log_lambda; p.start = start_index; p.end = end_index; p.thr_out = threshold_out;
+  p.H = (int)H; p.M = (int)M; p.N = (int)N; p.BM = (int)block_m; p.BN = (int)block_n;
+  p.kind = kThrScalar;
+  p.thr_value = threshold;
+  if (q_parts) {
+    p.kind = dtype == FOX_DTYPE_BF16 ? kThrAutoBf16 : kThrAutoFp16;
+    p.q_parts = q_parts; p.n_q_parts = (int)n_q_parts;
+    p.k_parts = k_parts; p.n_k_parts = (int)n_k_parts;
+    p.sm_scale = sm_scale;
+    p.log_n = (float)log((double)N);
+  }
+  return launch_index(device, (cudaStream_t)stream, B, p);
 }
 
 extern "C" int fox_find_index(int device, void* stream, int64_t B, int64_t H, int64_t M, int64_t N,
@@ -393,18 +715,11 @@ extern "C" int fox_find_index(int device, void* stream, int64_t B, int64_t H, in
   if (!log_lambda || !threshold || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N || block_m <= 0 || block_n <= 0)
     return FOX_ERR_BAD_ARG;
   if (!start_index && !end_index) return FOX_OK;
-  const int64_t nmb = (M + block_m - 1) / block_m, nnb = (N + block_n - 1) / block_n;
-  const size_t smem = sizeof(float) * (size_t)(2 * nmb + nnb + 1);
-  if (smem > 200 * 1024) return FOX_ERR_TOO_LARGE;
-  if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(fox_find_index_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return FOX_ERR_LAUNCH;
-  }
-  fox_find_index_kernel<<<(unsigned)(B * H), 256, smem, (cudaStream_t)stream>>>(
-      log_lambda, threshold, thr_sb, thr_sh, start_index, end_index, (int)H, (int)M, (int)N, (int)block_m,
-      (int)block_n, (int)nmb, (int)nnb);
-  return launch_rc();
+  IndexParams p{};
+  p.lam = log_lambda; p.thr = threshold; p.thr_sb = thr_sb; p.thr_sh = thr_sh; p.kind = kThrTensor;
+  p.start = start_index; p.end = end_index;
+  p.H = (int)H; p.M = (int)M; p.N = (int)N; p.BM = (int)block_m; p.BN = (int)block_n;
+  return launch_index(device, (cudaStream_t)stream, B, p);
 }
 
 extern "C" int fox_max_row_norm(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t T, int64_t D,
@@ -428,34 +743,44 @@ extern "C" int fox_max_row_norm(int device, void* stream, int dtype, int64_t B, 
   return launch_rc();
 }
 
-extern "C" int fox_bwd_delta(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
-                             const fox_tensor4* o, const fox_tensor4* d_o, float* delta) {
+static int launch_delta(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
+                        const fox_tensor4* o, const fox_tensor4* d_o, float* delta, float* dq_accum, float* dlam_row) {
   if (!o || !d_o || !delta || B <= 0 || H <= 0 || M <= 0) return FOX_ERR_BAD_ARG;
   if (B > 65535 || H > 65535 || B * H > 65535) return FOX_ERR_TOO_LARGE;   // (b, h) is the grid's y index
   if (!head_dim_ok(D)) return FOX_ERR_HEAD_DIM;
-  if (!aligned16(o) || !aligned16(d_o)) return FOX_ERR_ALIGNMENT;
+  if (!aligned16(o) || !aligned16(d_o) || reinterpret_cast<uintptr_t>(dq_accum) % 16) return FOX_ERR_ALIGNMENT;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   const int rows_per_block = kDeltaRows * 256 / (int)(D / 8);
+  const int acc_cols = (int)(D > kAccumCols ? D : kAccumCols);
   dim3 grid((unsigned)((M + rows_per_block - 1) / rows_per_block), (unsigned)(B * H));
-  if (dtype == FOX_DTYPE_BF16)
-    fox_delta_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)o->ptr, o->sb, o->sh, o->st, (const uint16_t*)d_o->ptr, d_o->sb, d_o->sh, d_o->st, (int)H, (int)M, (int)D, delta);
-  else
-    fox_delta_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)o->ptr, o->sb, o->sh, o->st, (const uint16_t*)d_o->ptr, d_o->sb, d_o->sh, d_o->st, (int)H, (int)M, (int)D, delta);
+#define FOX_DELTA(BF)                                                                                                  \
+  fox_delta_kernel<BF><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)o->ptr, o->sb, o->sh, o->st,             \
+      (const uint16_t*)d_o->ptr, d_o->sb, d_o->sh, d_o->st, (int)H, (int)M, (int)D, delta, dq_accum, acc_cols, dlam_row)
+  if (dtype == FOX_DTYPE_BF16) FOX_DELTA(true);
+  else FOX_DELTA(false);
+#undef FOX_DELTA
   return launch_rc();
+}
+
+extern "C" int fox_bwd_delta(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
+                             const fox_tensor4* o, const fox_tensor4* d_o, float* delta) {
+  return launch_delta(device, stream, dtype, B, H, M, D, o, d_o, delta, nullptr, nullptr);
+}
+
+extern "C" int fox_bwd_prepare(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
+                               const fox_tensor4* o, const fox_tensor4* d_o, float* delta, float* dq_accum,
+                               float* dlam_row) {
+  if (!dq_accum || !dlam_row) return FOX_ERR_BAD_ARG;
+  return launch_delta(device, stream, dtype, B, H, M, D, o, d_o, delta, dq_accum, dlam_row);
 }
 
 extern "C" int fox_dq_convert(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
                               const float* dq_accum, float scale, const fox_tensor4* dq) {
   if (!dq_accum || !dq || B <= 0 || H <= 0 || M <= 0) return FOX_ERR_BAD_ARG;
-  if (B > 65535 || H > 65535 || B * H > 65535) return FOX_ERR_TOO_LARGE;   // (b, h) is the grid's y index
+  if (B > 65535 || H > 65535 || B * H > 65535) return FOX_ERR_TOO_LARGE;
   if (!head_dim_ok(D)) return FOX_ERR_HEAD_DIM;
   if (!aligned16(dq)) return FOX_ERR_ALIGNMENT;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  const int rows_per_block = 256 / (int)(D / 8);
-  dim3 grid((unsigned)((M + rows_per_block - 1) / rows_per_block), (unsigned)(B * H));
-  if (dtype == FOX_DTYPE_BF16)
-    fox_dq_convert_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(dq_accum, (uint16_t*)dq->ptr, dq->sb, dq->sh, dq->st, (int)H, (int)M, (int)D, scale);
-  else
-    fox_dq_convert_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(dq_accum, (uint16_t*)dq->ptr, dq->sb, dq->sh, dq->st, (int)H, (int)M, (int)D, scale);
-  return launch_rc();
+  return launch_finish((cudaStream_t)stream, FOX_GATE_LOG, dtype == FOX_DTYPE_BF16, RevParams{}, 0,
+                       make_conv(B, H, M, D, dq_accum, D, scale, dq));
 }

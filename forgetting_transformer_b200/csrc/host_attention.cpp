@@ -1,0 +1,445 @@
+// forgetting_attention on the host: checks, allocations, launches and the autograd node.
+//
+// Same contract as upstream's ForgettingAttention function and forgetting_attention wrapper
+// (src/forgetting_transformer/ops/forgetting_attention.py:44-455).  A forward is one launch for the prefix sum and the
+// norm maxima, one for the pruning indices when a threshold is given, one for the attention; a backward is one for
+// delta (and clearing the accumulators), one or two for the attention and one for the gate gradient (and dQ's
+// conversion).  Working arrays come from the caching allocator in one piece per direction.
+#include "host_attention.h"
+
+#include <ATen/ExpandUtils.h>
+
+#include <cmath>
+#include <cstdlib>
+#include <sstream>
+
+namespace foxh {
+
+namespace {
+constexpr int64_t kBlock = FOX_FWD_BLOCK_M;
+static_assert(FOX_FWD_BLOCK_M == FOX_BWD_BLOCK_M && FOX_FWD_BLOCK_N == FOX_BWD_BLOCK_N, "one grid for both directions");
+
+bool env_is(const char* name, char c) {
+  const char* v = std::getenv(name);
+  return v && v[0] == c && v[1] == 0;
+}
+bool debug_sync() {
+  static const bool on = env_is("FOX_B200_DEBUG_SYNC", '1');
+  return on;
+}
+}  // namespace
+
+bool default_two_kernel(int64_t D) {
+  static const bool one_pass = env_is("FOX_B200_ONE_PASS_BWD", '1');
+  return D == 128 && !one_pass;
+}
+
+// ---------------------------------------------------------------- argument checks (upstream lines 81-91)
+AttnShape check_attention(const AttnInputs& in) {
+  const bool hf = in.head_first;
+  check_that(in.q.dim() == 4 && in.k.dim() == 4 && in.v.dim() == 4 && in.gate.dim() == 3,
+             "q, k, v must have 4 dimensions and log_fgate 3");
+  const int ih = hf ? 1 : 2, it = hf ? 2 : 1;
+  AttnShape s{in.q.size(0), in.q.size(ih), in.q.size(it), in.k.size(it), in.q.size(3)};
+  check_that(s.D == in.k.size(3) && s.D == in.v.size(3), "feature size of q, k, v should be equal");
+  check_that(s.D == 16 || s.D == 32 || s.D == 64 || s.D == 128, "We only support head dims in {16, 32, 64, 128}");
+  check_that(in.gate.size(0) == s.B && in.gate.size(hf ? 1 : 2) == s.H && in.gate.size(hf ? 2 : 1) == s.N);
+  const auto gt = in.gate.scalar_type();
+  if (in.gate_is_logit) {
+    if (gt != at::kHalf && gt != at::kBFloat16 && gt != at::kFloat)
+      raise_assert("gate logits must be fp16, bf16 or fp32, but got " + std::string(c10::toString(gt)));
+  } else {
+    check_that(gt == at::kFloat,
+               "log_fgate must be in torch.float32. It is best to do this cast before logsigmoid, e.g., "
+               "torch.nn.functional.logsigmoid(fgate_logit.float()).");
+  }
+  check_that(in.k.size(ih) == in.v.size(ih), "num of heads in k and v should be equal");
+  check_that(s.H == in.k.size(ih),
+             "groupped query attention has not been tested. You can uncomment this if you know what you are doing.");
+  check_that(s.M <= s.N, "The key/value tensors must be longer than the query tensor");
+  check_that(in.k.size(0) == s.B && in.v.size(0) == s.B && in.v.size(it) == s.N,
+             "q, k, v should have equal batch sizes and k, v equal lengths");
+  if (in.seq_start.defined()) check_that(in.seq_start.dim() == 1 && in.seq_start.size(0) == s.B);
+  if (!in.q.is_cuda())
+    raise_fox("forgetting_attention needs CUDA tensors on an sm_100 device; there is no CPU path");
+  return s;
+}
+
+Threshold parse_threshold(PyObject* o) {
+  Threshold t;
+  if (o == Py_None) return t;
+  if (PyUnicode_Check(o)) {
+    const char* c = PyUnicode_AsUTF8(o);
+    if (!c || std::string(c) != "auto")
+      raise_assert("adaptive_threshold must be either the string \"auto\", a float, or a Tensor, but got " +
+                   std::string(c ? c : "?") + ".");
+    t.kind = Threshold::kAuto;
+  } else if (THPVariable_Check(o)) {
+    t.kind = Threshold::kTensor;
+    t.tensor = THPVariable_Unpack(o);
+  } else {
+    t.kind = Threshold::kValue;
+    t.value = PyFloat_AsDouble(o);
+    if (PyErr_Occurred()) throw python_error();
+  }
+  return t;
+}
+
+static void gate_strides(const Tensor& g, bool hf, int64_t* st) {
+  st[0] = g.stride(0);
+  st[1] = g.stride(hf ? 1 : 2);
+  st[2] = g.stride(hf ? 2 : 1);
+}
+
+// ---------------------------------------------------------------- forward
+AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs_grad) {
+  const c10::cuda::CUDAGuard guard(in.q.device());
+  const at::AutoDispatchBelowADInplaceOrView no_autograd;
+  const int dev = in.q.device().index();
+  const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const bool hf = in.head_first;
+  const int64_t B = s.B, H = s.H, M = s.M, N = s.N, D = s.D, BH = B * H;
+  status_poll(dev);   // did a kernel of an earlier step give up on a wait? (no synchronisation)
+
+  AttnSaved r;
+  r.shape = s;
+  r.head_first = hf;
+  r.gate_is_logit = in.gate_is_logit;
+  r.sm_scale = in.sm_scale;
+  r.set_gate_layout(in.gate.sizes(), in.gate.is_non_overlapping_and_dense() ? in.gate.strides() : at::IntArrayRef());
+  r.q = tma_view(in.q);
+  r.k = tma_view(in.k);
+  r.v = tma_view(in.v);
+  const int code = dtype_code(r.q.scalar_type());
+  if (in.seq_start.defined()) r.seq_start = in.seq_start.to(in.q.device(), at::kLong).contiguous();
+  const int64_t* seq = r.seq_start.defined() ? r.seq_start.const_data_ptr<int64_t>() : nullptr;
+
+  const bool is_auto = in.threshold.kind == Threshold::kAuto;
+  const bool pruned = in.threshold.kind != Threshold::kNone;
+  // largest key norm per (b,h): the forward kernel's bound that lets most tiles skip the row-maximum pass
+  const bool k_norms = (N >= 8 * kBlock && M > 1) || is_auto;
+  const int64_t n_k = k_norms ? fox_norm_parts(B, H, N, D) : 0, n_q = is_auto ? fox_norm_parts(B, H, M, D) : 0;
+
+  // [log_lambda (B,H,N) | L (B,H,M) | norm parts]
+  r.vectors = at::empty({BH * (N + M + n_k + n_q)}, in.q.options().dtype(at::kFloat));
+  float* lam = r.vectors.mutable_data_ptr<float>();
+  float* L = lam + BH * N;
+  float* k_parts = k_norms ? L + BH * M : nullptr;
+  float* q_parts = is_auto ? k_parts + BH * n_k : nullptr;
+
+  const fox_tensor4 q4 = t4(r.q, hf), k4 = t4(r.k, hf), v4 = t4(r.v, hf);
+  int64_t gs[3];
+  gate_strides(in.gate, hf, gs);
+  const int gate_kind = in.gate_is_logit ? dtype_code(in.gate.scalar_type()) : FOX_GATE_LOG;
+  launch("fox_attn_prologue", st, [&] {
+    return fox_attn_prologue(dev, st, code, gate_kind, B, H, M, N, D, in.gate.data_ptr(), gs[0], gs[1], gs[2], seq, lam,
+                             k_norms ? &k4 : nullptr, k_parts, n_k, is_auto ? &q4 : nullptr, q_parts, n_q);
+  });
+
+  int64_t* start = nullptr;
+  if (pruned) {
+    const int64_t nmb = (M + kBlock - 1) / kBlock, nnb = (N + kBlock - 1) / kBlock;
+    r.index = at::empty({BH * (nmb + (needs_grad ? nnb : 0))}, in.q.options().dtype(at::kLong));
+    start = r.index.mutable_data_ptr<int64_t>();
+    int64_t* end = needs_grad ? start + BH * nmb : nullptr;
+    if (in.threshold.kind == Threshold::kTensor) {
+      r.threshold = in.threshold.tensor.detach().to(in.q.device(), at::kFloat);
+      if (!at::is_expandable_to(r.threshold.sizes(), {B, H})) {
+        std::ostringstream os;
+        os << r.threshold.sizes();
+        throw std::runtime_error(
+            "adaptive_threshold must be either the string \"auto\" or broadcastable to (batch_size, num_heads) = (" +
+            std::to_string(B) + ", " + std::to_string(H) + "), but got torch.Size(" + os.str() + ").");
+      }
+      r.threshold = r.threshold.expand({B, H});
+      launch("fox_find_index", st, [&] {
+        return fox_find_index(dev, st, B, H, M, N, kBlock, kBlock, lam, r.threshold.const_data_ptr<float>(),
+                              r.threshold.stride(0), r.threshold.stride(1), start, end);
+      });
+    } else {
+      r.threshold = at::empty({B, H}, in.q.options().dtype(at::kFloat));
+      launch("fox_find_index", st, [&] {
+        return fox_attn_index(dev, st, code, B, H, M, N, kBlock, kBlock, lam, static_cast<float>(in.threshold.value), q_parts,
+                              n_q, is_auto ? k_parts : nullptr, n_k, static_cast<float>(in.sm_scale), start, end,
+                              r.threshold.mutable_data_ptr<float>());
+      });
+    }
+  }
+
+  r.o = empty_like_tma(r.q);
+  const fox_tensor4 o4 = t4(r.o, hf);
+  if (M == 1 && !needs_grad) {
+    // generation step: one query row against the cache, no gradients -> split-KV kernels
+    int64_t splits = std::max<int64_t>(1, std::min(std::min((N + 511) / 512, (4 * 148 + BH - 1) / BH), int64_t{256}));
+    const int64_t Dk = std::max<int64_t>(D, 64);
+    Tensor q = r.q, k = r.k, v = r.v, o = r.o;
+    if (D < 64) {
+      q = at::constant_pad_nd(q, {0, 64 - D});
+      k = at::constant_pad_nd(k, {0, 64 - D});
+      v = at::constant_pad_nd(v, {0, 64 - D});
+      o = at::empty_like(q);
+    }
+    Tensor work = at::empty({fox_attn_decode_workspace_floats(B, H, Dk, splits)}, in.q.options().dtype(at::kFloat));
+    const fox_tensor4 dq4 = t4(q, hf), dk4 = t4(k, hf), dv4 = t4(v, hf), do4 = t4(o, hf);
+    launch("fox_attn_decode", st, [&] {
+      return fox_attn_decode(dev, st, code, B, H, N, Dk, &dq4, &dk4, &dv4, lam, seq, start, static_cast<float>(in.sm_scale),
+                             &do4, L, work.mutable_data_ptr<float>(), splits);
+    });
+    if (D < 64) r.o = o.narrow(3, 0, D).contiguous();
+    return r;
+  }
+  int32_t* status = status_words(dev);
+  launch("fox_attn_fwd", st, [&] {
+    return fox_attn_fwd_parts(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, lam, seq, start, static_cast<float>(in.sm_scale), &o4,
+                              L, k_parts, n_k, status);
+  });
+  if (debug_sync()) status_check(dev);
+  return r;
+}
+
+// ---------------------------------------------------------------- backward
+AttnGrads attention_backward(const AttnSaved& r, const Tensor& d_o, bool two_kernel) {
+  const c10::cuda::CUDAGuard guard(r.q.device());
+  const at::AutoDispatchBelowADInplaceOrView no_autograd;
+  const int dev = r.q.device().index();
+  const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const bool hf = r.head_first;
+  const int64_t B = r.shape.B, H = r.shape.H, M = r.shape.M, N = r.shape.N, D = r.shape.D, BH = B * H;
+  const int code = dtype_code(r.q.scalar_type());
+  const Tensor g = tma_view(d_o);
+  const float* lam = r.lam();
+  const float* L = r.L();
+  const int64_t* seq = r.seq_start.defined() ? r.seq_start.const_data_ptr<int64_t>() : nullptr;
+  const int64_t nmb = (M + kBlock - 1) / kBlock, nnb = (N + kBlock - 1) / kBlock;
+  two_kernel = two_kernel && D >= 64;
+
+  Tensor index = r.index;
+  if (r.threshold.defined() && !(index.defined() && index.numel() == BH * (nmb + nnb))) {
+    index = at::empty({BH * (nmb + nnb)}, r.q.options().dtype(at::kLong));
+    int64_t* p = index.mutable_data_ptr<int64_t>();
+    launch("fox_find_index", st, [&] {
+      return fox_find_index(dev, st, B, H, M, N, kBlock, kBlock, lam, r.threshold.const_data_ptr<float>(),
+                            r.threshold.stride(0), r.threshold.stride(1), p, p + BH * nmb);
+    });
+  }
+  const int64_t* start = r.threshold.defined() ? index.const_data_ptr<int64_t>() : nullptr;
+  const int64_t* end = start ? start + BH * nmb : nullptr;
+
+  AttnGrads out;
+  out.dq = empty_like_tma(r.q);
+  out.dk = empty_like_tma(r.k);
+  out.dv = empty_like_tma(r.v);
+  // [dq accumulator (B,H,M,max(D,64)), one-pass only | delta, dlam_row (B,H,M) each | dlam_col (B,H,N)]
+  const int64_t acc = two_kernel ? 0 : BH * M * std::max<int64_t>(D, 64);
+  const Tensor work = at::empty({acc + 2 * BH * M + BH * N}, r.q.options().dtype(at::kFloat));
+  float* dq_accum = work.mutable_data_ptr<float>();
+  float* delta = dq_accum + acc;
+  float* dlam_row = delta + BH * M;
+  float* dlam_col = dlam_row + BH * M;
+  const fox_tensor4 q4 = t4(r.q, hf), k4 = t4(r.k, hf), v4 = t4(r.v, hf), o4 = t4(r.o, hf), g4 = t4(g, hf), dq4 = t4(out.dq, hf),
+                    dk4 = t4(out.dk, hf), dv4 = t4(out.dv, hf);
+  const float scale = static_cast<float>(r.sm_scale);
+  int32_t* status = status_words(dev);
+  if (two_kernel) {
+    // key side (dk, dv, column sums) without a dQ product, query side as its own kernel: no fp32 dQ partials to
+    // add-reduce into L2, which is what bounds the one-pass kernel at head dim 128
+    launch("fox_bwd_delta", st, [&] { return fox_bwd_delta(dev, st, code, B, H, M, D, &o4, &g4, delta); });
+    launch("fox_attn_bwd", st, [&] {
+      return fox_attn_bwd(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, &g4, lam, L, delta, seq, end, scale, nullptr, nullptr,
+                          dlam_col, &dk4, &dv4, status);
+    });
+    launch("fox_attn_bwd_dq", st, [&] {
+      return fox_attn_bwd_dq(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, &g4, lam, L, delta, seq, start, scale, &dq4, dlam_row,
+                             status);
+    });
+  } else {
+    launch("fox_bwd_delta", st,
+           [&] { return fox_bwd_prepare(dev, st, code, B, H, M, D, &o4, &g4, delta, dq_accum, dlam_row); });
+    launch("fox_attn_bwd", st, [&] {
+      return fox_attn_bwd(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, &g4, lam, L, delta, seq, end, scale, dq_accum, dlam_row,
+                          dlam_col, &dk4, &dv4, status);
+    });
+  }
+  // reverse prefix sum of the two halves of dlog_lambda (upstream lines 390-392); for gate logits also the chain rule
+  // through log sigmoid, in the logits' dtype and layout
+  int gate_kind = FOX_GATE_LOG;
+  int64_t gs[3] = {0, 0, 0}, os[3];
+  const void* logit = nullptr;
+  if (r.gate_is_logit) {
+    gate_kind = dtype_code(r.gate.scalar_type());
+    gate_strides(r.gate, hf, gs);
+    logit = r.gate.data_ptr();
+    out.dgate = at::empty_like(r.gate);
+  } else {   // in the gates' own layout, which the gradient's accumulation would otherwise copy it into
+    out.dgate = at::empty_strided(r.gate_sizes, r.gate_strides, r.q.options().dtype(at::kFloat));
+  }
+  gate_strides(out.dgate, hf, os);
+  launch("fox_bwd_finish", st, [&] {
+    return fox_bwd_finish(dev, st, code, B, H, M, N, D, dlam_col, dlam_row, gate_kind, logit, gs[0], gs[1], gs[2],
+                          out.dgate.data_ptr(), os[0], os[1], os[2], two_kernel ? nullptr : dq_accum, scale,
+                          two_kernel ? nullptr : &dq4);
+  });
+  status_pending(dev);
+  if (debug_sync()) status_check(dev);
+  return out;
+}
+
+// ---------------------------------------------------------------- autograd node
+namespace {
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+struct AttentionBackward : public torch::autograd::Node {
+  SavedVariable q, k, v, o, gate;   // gate: the logits, where they are what was given
+  AttnSaved rest;                   // (its q, k, v, o, gate are left empty)
+  bool released = false;
+
+  std::string name() const override { return "ForgettingAttentionBackward"; }
+  void release_variables() override {
+    q.reset_data();
+    k.reset_data();
+    v.reset_data();
+    o.reset_data();
+    gate.reset_data();
+    rest.vectors.reset();
+    rest.index.reset();
+    released = true;
+  }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(4);
+    if (!grads[0].defined()) return out;
+    if (released) throw std::runtime_error(torch::autograd::ERR_BACKWARD_TWICE);
+    AttnSaved r = rest;
+    r.q = q.unpack();
+    r.k = k.unpack();
+    r.v = v.unpack();
+    r.o = o.unpack(shared_from_this());
+    if (r.gate_is_logit) r.gate = gate.unpack();
+    AttnGrads g = attention_backward(r, grads[0], default_two_kernel(r.shape.D));
+    if (task_should_compute_output(0)) out[0] = g.dq;
+    if (task_should_compute_output(1)) out[1] = g.dk;
+    if (task_should_compute_output(2)) out[2] = g.dv;
+    if (task_should_compute_output(3)) out[3] = g.dgate;
+    return out;
+  }
+};
+}  // namespace
+
+Tensor attention(const AttnInputs& in) {
+  const AttnShape s = check_attention(in);
+  const bool needs = at::GradMode::is_enabled() && (in.q.requires_grad() || in.k.requires_grad() || in.v.requires_grad() ||
+                                                    in.gate.requires_grad());
+  AttnSaved r = attention_forward(in, s, needs);
+  if (!needs) return r.o;
+  std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(in.q, in.k, in.v, in.gate));
+  Tensor o = r.o;
+  torch::autograd::set_history(o, node);
+  node->q = SavedVariable(r.q, false);
+  node->k = SavedVariable(r.k, false);
+  node->v = SavedVariable(r.v, false);
+  node->o = SavedVariable(o, true);
+  if (in.gate_is_logit) node->gate = SavedVariable(in.gate, false);
+  r.q.reset();
+  r.k.reset();
+  r.v.reset();
+  r.o.reset();
+  node->rest = std::move(r);
+  return o;
+}
+
+}  // namespace foxh
+
+// ---------------------------------------------------------------- Python entry points
+using namespace foxh;
+
+static AttnInputs parse_inputs(PyObject* const* a) {   // q, k, v, gate, head_first, seq_start, sm_scale, threshold, gate_is_logit
+  AttnInputs in;
+  in.q = unpack(a[0], "q");
+  in.k = unpack(a[1], "k");
+  in.v = unpack(a[2], "v");
+  in.gate = unpack(a[3], "log_fgate");
+  in.head_first = PyObject_IsTrue(a[4]) == 1;
+  in.seq_start = unpack_opt(a[5], "seq_start");
+  in.threshold = parse_threshold(a[7]);
+  in.gate_is_logit = a[8] == Py_True;
+  if (a[6] == Py_None) {
+    in.sm_scale = 1. / std::sqrt(static_cast<double>(in.q.size(-1)));
+  } else {
+    in.sm_scale = PyFloat_AsDouble(a[6]);
+    if (PyErr_Occurred()) throw python_error();
+  }
+  return in;
+}
+
+FOX_PY(py_attention) {
+  HANDLE_TH_ERRORS
+  const AttnInputs in = parse_inputs(args);
+  Tensor out;
+  {
+    pybind11::gil_scoped_release no_gil;
+    out = attention(in);
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+static PyObject* tensor_tuple(std::initializer_list<const Tensor*> ts) {   // (an undefined tensor becomes None)
+  PyObject* out = PyTuple_New(static_cast<Py_ssize_t>(ts.size()));
+  Py_ssize_t i = 0;
+  for (const Tensor* t : ts) PyTuple_SET_ITEM(out, i++, THPVariable_Wrap(*t));
+  return out;
+}
+
+// (the nine arguments of attention, needs_grad) -> (out, L, log_lambda, seq_start, threshold, start_index, end_index)
+FOX_PY(py_attention_forward) {
+  HANDLE_TH_ERRORS
+  const AttnInputs in = parse_inputs(args);
+  const bool needs = args[9] == Py_True;
+  AttnSaved r;
+  Tensor L, lam, start, end;
+  {
+    pybind11::gil_scoped_release no_gil;
+    const AttnShape s = check_attention(in);
+    r = attention_forward(in, s, needs);
+    const int64_t BH = s.B * s.H, nmb = (s.M + kBlock - 1) / kBlock, nnb = (s.N + kBlock - 1) / kBlock;
+    lam = r.vectors.narrow(0, 0, BH * s.N).view({s.B, s.H, s.N});
+    L = r.vectors.narrow(0, BH * s.N, BH * s.M).view({s.B, s.H, s.M});
+    if (r.index.defined()) {
+      start = r.index.narrow(0, 0, BH * nmb).view({s.B, s.H, nmb});
+      if (needs) end = r.index.narrow(0, BH * nmb, BH * nnb).view({s.B, s.H, nnb});
+    }
+  }
+  return tensor_tuple({&r.o, &L, &lam, &r.seq_start, &r.threshold, &start, &end});
+  END_HANDLE_TH_ERRORS
+}
+
+// head-first (q, k, v, out, L, log_lambda, seq_start, threshold, dout, gate logits or None, sm_scale, two_kernel)
+// -> (dq, dk, dv, dgate)
+FOX_PY(py_attention_backward) {
+  HANDLE_TH_ERRORS
+  AttnSaved r;
+  r.q = tma_view(unpack(args[0], "q"));
+  r.k = tma_view(unpack(args[1], "k"));
+  r.v = tma_view(unpack(args[2], "v"));
+  r.o = tma_view(unpack(args[3], "out"));
+  r.head_first = true;
+  r.shape = AttnShape{r.q.size(0), r.q.size(1), r.q.size(2), r.k.size(2), r.q.size(3)};
+  r.set_gate_layout({r.shape.B, r.shape.H, r.shape.N}, {});
+  r.separate_L = unpack(args[4], "L").contiguous();
+  r.separate_lam = unpack(args[5], "log_lambda").contiguous();
+  r.seq_start = unpack_opt(args[6], "seq_start");
+  r.threshold = unpack_opt(args[7], "threshold");
+  const Tensor d_o = unpack(args[8], "dout");
+  r.gate = unpack_opt(args[9], "gate logits");
+  r.gate_is_logit = r.gate.defined();
+  r.sm_scale = PyFloat_AsDouble(args[10]);
+  const bool two_kernel = args[11] == Py_True;
+  AttnGrads g;
+  {
+    pybind11::gil_scoped_release no_gil;
+    g = attention_backward(r, d_o, two_kernel);
+  }
+  return tensor_tuple({&g.dq, &g.dk, &g.dv, &g.dgate});
+  END_HANDLE_TH_ERRORS
+}

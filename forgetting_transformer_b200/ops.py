@@ -20,14 +20,20 @@ from . import _lib
 __all__ = ["forgetting_attention", "forgetting_attention_from_gate_logits", "ForgettingAttention", "make_graphed", "FWD_BLOCK",
            "BWD_BLOCK"]
 
-# (BLOCK_M, BLOCK_N) of the kernels; pruning indices are defined on this grid.
-_PADDED_HEAD_DIM = 64   # head dims 16 and 32 are zero-padded to this
 # head dims whose backward runs as a key-side and a query-side kernel instead of the one-pass kernel
 _TWO_KERNEL_BACKWARD_DIMS = set() if os.environ.get("FOX_B200_ONE_PASS_BWD", "0") == "1" else {128}
+# (BLOCK_M, BLOCK_N) of the kernels; pruning indices are defined on this grid.
 FWD_BLOCK = (128, 128)
 BWD_BLOCK = (128, 128)
 
-_DEBUG_SYNC = os.environ.get("FOX_B200_DEBUG_SYNC", "0") == "1"
+_QKV_DTYPES = (torch.float16, torch.bfloat16)
+_host = None
+
+
+def _load_host():
+    global _host
+    _host = _lib.host()
+    return _host
 
 
 class KernelTimer:
@@ -45,31 +51,26 @@ class KernelTimer:
 
     def __enter__(self):
         KernelTimer.active = self
+        _lib.host().timer(True)
         return self
 
     def __exit__(self, *exc):
         KernelTimer.active = None
+        _lib.host().timer(False)
 
     def summary(self):
         torch.cuda.synchronize()
+        self.events += _lib.host().timer_take()
         acc = {}
-        for name, a, b in self.events:
+        for name, ms in self.events:
             n, t = acc.get(name, (0, 0.0))
-            acc[name] = (n + 1, t + a.elapsed_time(b))
+            acc[name] = (n + 1, t + ms)
         return {k: (n, t / n) for k, (n, t) in acc.items()}
 
 
 def _call(name, fn, *args):
-    """Launch one C-ABI entry point, timing it when a KernelTimer is active."""
-    timer = KernelTimer.active
-    if timer is None:
-        _lib.check(fn(*args), name)
-        return
-    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    a.record()
+    """Call one C-ABI entry point, raising on an error code."""
     _lib.check(fn(*args), name)
-    b.record()
-    timer.events.append((name, a, b))
 
 
 def _stream() -> int:
@@ -144,7 +145,8 @@ def find_index(log_lambda: torch.Tensor, threshold: torch.Tensor, M: int, block_
 
 class ForgettingAttention(torch.autograd.Function):
     """Same positional signature as upstream's autograd function (line 73); the three
-    trailing timing arguments are accepted and ignored."""
+    trailing timing arguments are accepted and ignored.  ``forgetting_attention`` itself goes through the same native
+    forward and backward with an autograd node of its own; this class also serves the hidden outputs."""
 
     @staticmethod
     def forward(ctx, q, k, v, log_fgate, seq_start, causal, sm_scale, adaptive_threshold,
@@ -153,110 +155,12 @@ class ForgettingAttention(torch.autograd.Function):
         """``gate_is_logit`` (not part of upstream's signature): ``log_fgate`` holds the gate LOGITS (fp16 / bf16 /
         fp32); log sigmoid and its derivative are folded into the prefix-sum kernels."""
         assert causal, "Only causal attention is supported"
-        Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
-        assert Dq == Dk == Dv, "feature size of q, k, v should be equal"
-        assert Dk in {16, 32, 64, 128}, "We only support head dims in {16, 32, 64, 128}"
-
-        B, H, M, D = q.shape
-        N = k.shape[2]
-        assert log_fgate.shape == (B, H, N)
-        if gate_is_logit:
-            assert log_fgate.dtype in _GATE_DTYPES, f"gate logits must be fp16, bf16 or fp32, but got {log_fgate.dtype}"
-        else:
-            assert log_fgate.dtype == torch.float32, "log_fgate must be in torch.float32. It is best to do this cast before logsigmoid, e.g., torch.nn.functional.logsigmoid(fgate_logit.float())."
-        if sm_scale is None:
-            sm_scale = 1. / math.sqrt(D)
-        Hk, Hv = k.shape[1], v.shape[1]
-        assert Hk == Hv, "num of heads in k and v should be equal"
-        assert H == Hk, "groupped query attention has not been tested. You can uncomment this if you know what you are doing."
-        assert not (M > N), "The key/value tensors must be longer than the query tensor"
-        if isinstance(adaptive_threshold, str):
-            assert adaptive_threshold == "auto", f'adaptive_threshold must be either the string "auto", a float, or a Tensor, but got {adaptive_threshold}.'
-        if seq_start is not None:
-            assert seq_start.shape == (B,)
-        if not q.is_cuda:
-            raise _lib.FoxError("forgetting_attention needs CUDA tensors on an sm_100 device; there is no CPU path")
-        # Head dims 16 and 32 run through the D=64 kernels on zero-padded copies: zero columns change no
-        # dot product, norm or output column, and their gradients are exactly zero and sliced off again.
-        D_in = D
-        if D in (16, 32):
-            q, k, v = [torch.nn.functional.pad(t, (0, _PADDED_HEAD_DIM - D)) for t in (q, k, v)]
-            D = _PADDED_HEAD_DIM
-
-        lib = _lib.load()
-        with torch.cuda.device(q.device):
-            dev = q.device
-            _lib.poll_status(dev)   # did a kernel of an earlier step give up on a wait? (no synchronisation)
-            q, k, v = _tma_view(q), _tma_view(k), _tma_view(v)
-            # largest key norm per (b,h): the forward kernel's bound that lets most tiles skip the row-maximum pass
-            need_auto = isinstance(adaptive_threshold, str)
-            k_norm_max = max_row_norm(k, keep_fp32=True) if ((N >= 8 * FWD_BLOCK[1] and M > 1) or need_auto) else None
-
-            if adaptive_threshold is not None:
-                if isinstance(adaptive_threshold, str):
-                    assert adaptive_threshold == "auto", f'adaptive_threshold must be either the string "auto", a float, or a Tensor, but got {adaptive_threshold}.'
-                    max_q_norm = max_row_norm(q)
-                    max_k_norm = k_norm_max.to(k.dtype)
-                    logit_upper_bound = max_q_norm * max_k_norm * sm_scale
-                    tolerance = -10
-                    adaptive_threshold = -(2 * logit_upper_bound + math.log(N)) + tolerance
-                if isinstance(adaptive_threshold, torch.Tensor):
-                    adaptive_threshold = adaptive_threshold.to(dtype=torch.float, device=dev)
-                else:   # a fill kernel instead of a host-to-device copy: legal inside CUDA-graph capture
-                    adaptive_threshold = torch.full((), float(adaptive_threshold), dtype=torch.float, device=dev)
-                try:
-                    adaptive_threshold = torch.broadcast_to(adaptive_threshold, (B, H))
-                except RuntimeError:
-                    raise RuntimeError(f'adaptive_threshold must be either the string "auto" or broadcastable to (batch_size, num_heads) = ({B}, {H}), but got {adaptive_threshold.size()}.')
-                assert adaptive_threshold.size() == (B, H)
-
-            if seq_start is not None:
-                has_seq_start = True
-                assert seq_start.shape == (B,)
-                seq_start = seq_start.to(device=dev, dtype=torch.long).contiguous()
-            else:
-                has_seq_start = False
-
-            log_lambda = (gate_prefix_from_logits(log_fgate, seq_start) if gate_is_logit
-                          else log_lambda_cumsum(log_fgate, seq_start))
-
-            start_index = None
-            if adaptive_threshold is not None:
-                start_index, _ = find_index(log_lambda, adaptive_threshold, M, *FWD_BLOCK)
-
-            o = torch.empty_like(q)
-            if not _lib.tma_ready(o):
-                o = torch.empty(q.shape, dtype=q.dtype, device=dev)
-            L = torch.empty((B, H, M), device=dev, dtype=torch.float32)
-            if M == 1 and not any(ctx.needs_input_grad[:4]):
-                # generation step: one query row against the cache, no gradients -> split-KV kernels
-                splits = max(1, min((N + 511) // 512, (4 * 148 + B * H - 1) // (B * H), 256))
-                work = torch.empty(lib.fox_attn_decode_workspace_floats(B, H, D, splits), device=dev,
-                                   dtype=torch.float32)
-                _call("fox_attn_decode", lib.fox_attn_decode, dev.index, _stream(), _lib.dtype_code(q.dtype), B, H, N,
-                      D, _lib.t4(q), _lib.t4(k), _lib.t4(v), log_lambda.data_ptr(), _lib.ptr(seq_start),
-                      _lib.ptr(start_index), float(sm_scale), _lib.t4(o), L.data_ptr(), work.data_ptr(), splits)
-                out = o if D_in == D else o[..., :D_in].contiguous()
-                if return_log_normalizer or return_start_index:
-                    return (out, L if return_log_normalizer else None, start_index if return_start_index else None)
-                return out
-            status = _lib.status_buffer(dev)
-            _call("fox_attn_fwd", lib.fox_attn_fwd, dev.index, _stream(), _lib.dtype_code(q.dtype), B, H, M, N, D,
-                  _lib.t4(q), _lib.t4(k), _lib.t4(v), log_lambda.data_ptr(), _lib.ptr(seq_start),
-                  _lib.ptr(start_index), float(sm_scale), _lib.t4(o), L.data_ptr(), _lib.ptr(k_norm_max),
-                  status.data_ptr())
-            if _DEBUG_SYNC:
-                _lib.check_status(dev)
-
-        ctx.save_for_backward(q, k, v, o, L, log_lambda, seq_start, adaptive_threshold)
+        needs_grad = any(ctx.needs_input_grad[:4])
+        out, L, log_lambda, seq_start, threshold, start_index, _ = _lib.host().attention_forward(
+            q, k, v, log_fgate, True, seq_start, sm_scale, adaptive_threshold, gate_is_logit, needs_grad)
+        ctx.save_for_backward(q, k, v, out, L, log_lambda, seq_start, threshold)
         ctx.gate_logit = log_fgate if gate_is_logit else None    # (an input of the function: kept as it is)
-        ctx.sm_scale = sm_scale
-        ctx.has_seq_start = has_seq_start
-        # the query-side backward kernel prunes by the same array when the two block grids agree (not an input or
-        # output of the function, so it is kept on ctx rather than through save_for_backward)
-        ctx.start_index = start_index if FWD_BLOCK == BWD_BLOCK else None
-        ctx.head_dim = D_in
-        out = o if D_in == D else o[..., :D_in].contiguous()
+        ctx.sm_scale = 1. / math.sqrt(q.shape[-1]) if sm_scale is None else sm_scale
         if return_log_normalizer or return_start_index:
             ctx.mark_non_differentiable(*[t for t in (L, start_index) if t is not None])
             return (out, L if return_log_normalizer else None, start_index if return_start_index else None)
@@ -264,93 +168,11 @@ class ForgettingAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, do, *ignored):
-        q, k, v, o, L, log_lambda, seq_start, adaptive_threshold = ctx.saved_tensors
-        sm_scale = ctx.sm_scale
-        B, H, M, D = q.shape
-        N = k.shape[2]
-        lib = _lib.load()
-        # the autograd engine runs this on its own thread: select the device explicitly
-        with torch.cuda.device(q.device):
-            dev = q.device
-            if ctx.head_dim != D:
-                do = torch.nn.functional.pad(do, (0, D - ctx.head_dim))
-            do = _tma_view(do)
-            code = _lib.dtype_code(q.dtype)
-            delta = torch.empty_like(L)
-            _call("fox_bwd_delta", lib.fox_bwd_delta, dev.index, _stream(), code, B, H, M, D, _lib.t4(o),
-                  _lib.t4(do), delta.data_ptr())
-            end_index = None
-            if adaptive_threshold is not None:
-                _, end_index = find_index(log_lambda, adaptive_threshold, M, *BWD_BLOCK, want_start=False,
-                                          want_end=True)
-            dk = torch.empty_like(k)
-            dv = torch.empty_like(v)
-            dq = torch.empty_like(q)
-            if not _lib.tma_ready(dk):
-                dk = torch.empty(k.shape, dtype=k.dtype, device=dev)
-            if not _lib.tma_ready(dv):
-                dv = torch.empty(v.shape, dtype=v.dtype, device=dev)
-            if not _lib.tma_ready(dq):
-                dq = torch.empty(q.shape, dtype=q.dtype, device=dev)
-            dlam_col = torch.empty((B, H, N), dtype=torch.float32, device=dev)
-            status = _lib.status_buffer(dev)
-            if D in _TWO_KERNEL_BACKWARD_DIMS:
-                # key side (dk, dv, column sums) without a dQ product, query side as its own kernel: no fp32
-                # dQ partials to add-reduce into L2, which is what bounds the one-pass kernel at this head dim
-                start_index = None
-                if adaptive_threshold is not None:
-                    start_index = ctx.start_index
-                    if start_index is None:
-                        start_index, _ = find_index(log_lambda, adaptive_threshold, M, *BWD_BLOCK)
-                dlam_row = torch.empty((B, H, M), dtype=torch.float32, device=dev)
-                _call("fox_attn_bwd", lib.fox_attn_bwd, dev.index, _stream(), code, B, H, M, N, D, _lib.t4(q),
-                      _lib.t4(k), _lib.t4(v), _lib.t4(do), log_lambda.data_ptr(), L.data_ptr(), delta.data_ptr(),
-                      _lib.ptr(seq_start), _lib.ptr(end_index), float(sm_scale), None, None,
-                      dlam_col.data_ptr(), _lib.t4(dk), _lib.t4(dv), status.data_ptr())
-                _call("fox_attn_bwd_dq", lib.fox_attn_bwd_dq, dev.index, _stream(), code, B, H, M, N, D, _lib.t4(q),
-                      _lib.t4(k), _lib.t4(v), _lib.t4(do), log_lambda.data_ptr(), L.data_ptr(), delta.data_ptr(),
-                      _lib.ptr(seq_start), _lib.ptr(start_index), float(sm_scale), _lib.t4(dq), dlam_row.data_ptr(),
-                      status.data_ptr())
-                dlog_fgate = _gate_gradient(ctx, lib, dev, B, H, M, N, dlam_col, dlam_row)
-                _lib.queue_status_readback(dev)
-                if _DEBUG_SYNC:
-                    _lib.check_status(dev)
-                if ctx.head_dim != D:
-                    dq, dk, dv = [t[..., :ctx.head_dim].contiguous() for t in (dq, dk, dv)]
-                return dq, dk, dv, dlog_fgate, None, None, None, None, None, None, None, None, None, None
-            # scratch: fp32 dQ accumulator and the query-side log-gate gradient (both reduced into)
-            scratch = torch.zeros(B * H * M * (D + 1), dtype=torch.float32, device=dev)
-            dq_accum = scratch[: B * H * M * D]
-            dlam_row = scratch[B * H * M * D:]
-            _call("fox_attn_bwd", lib.fox_attn_bwd, dev.index, _stream(), code, B, H, M, N, D, _lib.t4(q),
-                  _lib.t4(k), _lib.t4(v), _lib.t4(do), log_lambda.data_ptr(), L.data_ptr(), delta.data_ptr(),
-                  _lib.ptr(seq_start), _lib.ptr(end_index), float(sm_scale), dq_accum.data_ptr(),
-                  dlam_row.data_ptr(), dlam_col.data_ptr(), _lib.t4(dk), _lib.t4(dv), status.data_ptr())
-            _call("fox_dq_convert", lib.fox_dq_convert, dev.index, _stream(), code, B, H, M, D,
-                  dq_accum.data_ptr(), float(sm_scale), _lib.t4(dq))
-            dlog_fgate = _gate_gradient(ctx, lib, dev, B, H, M, N, dlam_col, dlam_row)
-            _lib.queue_status_readback(dev)
-            if _DEBUG_SYNC:
-                _lib.check_status(dev)
-        if ctx.head_dim != D:
-            dq, dk, dv = [t[..., :ctx.head_dim].contiguous() for t in (dq, dk, dv)]
-        return dq, dk, dv, dlog_fgate, None, None, None, None, None, None, None, None, None, None
-
-
-def _gate_gradient(ctx, lib, dev, B, H, M, N, dlam_col, dlam_row):
-    """Reverse prefix sum of the two halves of dlog_lambda (upstream lines 390-392); for gate logits also the
-    chain rule through log sigmoid, in the logits' dtype and layout."""
-    logit = getattr(ctx, "gate_logit", None)
-    if logit is None:
-        dlog_fgate = torch.empty((B, H, N), dtype=torch.float32, device=dev)
-        _call("fox_revcumsum", lib.fox_revcumsum, dev.index, _stream(), B, H, M, N, dlam_col.data_ptr(),
-              dlam_row.data_ptr(), None, dlog_fgate.data_ptr(), None)
-        return dlog_fgate
-    dlogit = torch.empty_strided(logit.shape, logit.stride(), dtype=logit.dtype, device=dev)
-    _call("fox_gate_prefix_bwd", lib.fox_gate_prefix_bwd, dev.index, _stream(), _GATE_DTYPES[logit.dtype], B, H, M, N,
-          dlam_col.data_ptr(), dlam_row.data_ptr(), logit.data_ptr(), logit.stride(0), logit.stride(1),
-          logit.stride(2), dlogit.data_ptr())
-    return dlogit
+        q, k, v, o, L, log_lambda, seq_start, threshold = ctx.saved_tensors
+        grads = _lib.host().attention_backward(q, k, v, o, L, log_lambda, seq_start, threshold, do,
+                                               getattr(ctx, "gate_logit", None), ctx.sm_scale,
+                                               q.shape[-1] in _TWO_KERNEL_BACKWARD_DIMS)
+        return (*grads, None, None, None, None, None, None, None, None, None, None)
 
 
 def forgetting_attention_from_gate_logits(q, k, v, fgate_logit, *, head_first: bool = False,
@@ -361,16 +183,9 @@ def forgetting_attention_from_gate_logits(q, k, v, fgate_logit, *, head_first: b
     gate projection output (fp16 / bf16 / fp32, (B, T, H) or (B, H, T) with ``head_first``, any strides) goes in as
     it is and receives its gradient in its own dtype (upstream forms the log gates with two elementwise kernels in
     front of the operator, modeling_forgetting_transformer.py:343-346).  Everything else as ``forgetting_attention``."""
-    for name, entry in dict(q=q, k=k, v=v).items():
-        assert entry.dtype in [torch.float16, torch.bfloat16], f"Only torch.float16 or torch.bfloat16 are supported for q/k/v, but got {entry.dtype} for {name}."
-    if not head_first:
-        q, k, v = [item.permute(0, 2, 1, 3) for item in (q, k, v)]
-        fgate_logit = fgate_logit.permute(0, 2, 1)
-    out = ForgettingAttention.apply(q, k, v, fgate_logit, seq_start, True, sm_scale, adaptive_threshold,
-                                    False, False, None, False, False, True)
-    if not head_first:
-        out = out.permute(0, 2, 1, 3)
-    return out
+    for name, entry in (("q", q), ("k", k), ("v", v)):
+        assert entry.dtype in _QKV_DTYPES, f"Only torch.float16 or torch.bfloat16 are supported for q/k/v, but got {entry.dtype} for {name}."
+    return (_host or _load_host()).attention(q, k, v, fgate_logit, head_first, seq_start, sm_scale, adaptive_threshold, True)
 
 
 def forgetting_attention(
@@ -390,7 +205,7 @@ def forgetting_attention(
 
     - q (B, Tq, H, D), k/v (B, Tk, H, D) in fp16/bf16 and log_fgate (B, Tk, H) in
       fp32, or with the H and T axes swapped when ``head_first=True``;
-    - Tq <= Tk, causal, D in {16, 32, 64, 128} (16 and 32 run zero-padded through the D=64 kernels);
+    - Tq <= Tk, causal, D in {16, 32, 64, 128} (16 and 32 run through the D=64 kernels, their tiles zero-filled by the copies);
     - ``seq_start`` (B,) long: no attention to positions left of it (left padding);
     - ``sm_scale`` defaults to 1/sqrt(D);
     - ``adaptive_threshold``: "auto", a float or a tensor broadcastable to (B, H);
@@ -398,16 +213,9 @@ def forgetting_attention(
 
     Returns the output in q's layout; differentiable w.r.t. q, k, v and log_fgate.
     """
-    for name, entry in dict(q=q, k=k, v=v).items():
-        assert entry.dtype in [torch.float16, torch.bfloat16], f"Only torch.float16 or torch.bfloat16 are supported for q/k/v, but got {entry.dtype} for {name}."
-    if not head_first:
-        q, k, v = [item.permute(0, 2, 1, 3) for item in (q, k, v)]
-        log_fgate = log_fgate.permute(0, 2, 1)
-    out = ForgettingAttention.apply(q, k, v, log_fgate, seq_start, True, sm_scale, adaptive_threshold,
-                                    False, False, None, False, False)
-    if not head_first:
-        out = out.permute(0, 2, 1, 3)
-    return out
+    for name, entry in (("q", q), ("k", k), ("v", v)):
+        assert entry.dtype in _QKV_DTYPES, f"Only torch.float16 or torch.bfloat16 are supported for q/k/v, but got {entry.dtype} for {name}."
+    return (_host or _load_host()).attention(q, k, v, log_fgate, head_first, seq_start, sm_scale, adaptive_threshold, False)
 
 
 # ---- the FoX layer's glue in front of the operator (modeling_forgetting_transformer.py:366-396) ----

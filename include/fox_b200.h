@@ -46,7 +46,8 @@ extern "C" {
 
 #define FOX_DTYPE_FP16 0
 #define FOX_DTYPE_BF16 1
-#define FOX_DTYPE_FP32 2          /* accepted by fox_cross_entropy_* only */
+#define FOX_DTYPE_FP32 2          /* accepted by fox_cross_entropy_* and as gate_kind only */
+#define FOX_GATE_LOG 3            /* gate_kind: fp32 log gates; the FOX_DTYPE_* values: gate logits of that type */
 
 typedef struct fox_tensor4 {
   void* ptr;
@@ -113,8 +114,25 @@ int fox_find_index(int device, void* stream, int64_t B, int64_t H, int64_t M, in
 int fox_max_row_norm(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t T, int64_t D,
                      const fox_tensor4* x, float* out_zeroed);
 
+/* What the operator needs before its forward kernel, in one launch: the prefix sum of the gates (fox_cumsum_fwd /
+ * fox_gate_prefix_fwd; gate_kind FOX_GATE_LOG or the dtype of gate logits) and, where k (q) is given, the largest row
+ * norm of every (b,h) as n partial maxima, k_parts (B,H,n_k_parts), fully written; n from fox_norm_parts, <= 32. */
+int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D);
+int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M, int64_t N,
+                      int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
+                      float* log_lambda, const fox_tensor4* k, float* k_parts, int64_t n_k_parts, const fox_tensor4* q,
+                      float* q_parts, int64_t n_q_parts);
+
+/* fox_find_index for one threshold value, or (q_parts, k_parts given) for the automatic threshold of
+ * forgetting_attention.py:91-109, evaluated in the input dtype from the norm parts of fox_attn_prologue.
+ * threshold_out (B,H) fp32 or NULL receives the threshold of every (b,h). */
+int fox_attn_index(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t block_m,
+                   int64_t block_n, const float* log_lambda, float threshold, const float* q_parts, int64_t n_q_parts,
+                   const float* k_parts, int64_t n_k_parts, float sm_scale, int64_t* start_index, int64_t* end_index,
+                   float* threshold_out);
+
 /* Forward attention: replaces the _fwd_kernel launch (forgetting_attention.py:186-204, kernel
- * 505-693).  q (B,H,M,D); k, v (B,H,N,D); M <= N; D in {64,128}.  log_lambda from
+ * 505-693).  q (B,H,M,D); k, v (B,H,N,D); M <= N; D in {16,32,64,128}.  log_lambda from
  * fox_cumsum_fwd.  seq_start (B,) int64 or NULL.  start_index from fox_find_index with
  * FOX_FWD_BLOCK_M/N, or NULL for no pruning.  Writes o (same dtype, caller's strides) and the
  * log-normaliser L (B,H,M) fp32 (natural log; -inf for rows left of seq_start, whose output is
@@ -126,6 +144,12 @@ int fox_attn_fwd(int device, void* stream, int dtype, int64_t B, int64_t H, int6
                  const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v, const float* log_lambda,
                  const int64_t* seq_start, const int64_t* start_index, float sm_scale, const fox_tensor4* o,
                  float* L, const float* k_norm_max, int32_t* status);
+/* fox_attn_fwd with k_norm_max as (B,H,n_norm_parts) partial maxima (fox_attn_prologue). */
+int fox_attn_fwd_parts(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
+                 const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v, const float* log_lambda,
+                 const int64_t* seq_start, const int64_t* start_index, float sm_scale, const fox_tensor4* o,
+                 float* L, const float* k_norm_parts,
+                       int64_t n_norm_parts, int32_t* status);
 
 /* Forward attention for ONE query row per (b,h) -- a generation step against a cache of N keys, the
  * seqlen_q = 1 case of the same upstream kernel (forgetting_attention.py:148-153, 591-693; cache:
@@ -145,6 +169,10 @@ int64_t fox_attn_decode_workspace_floats(int64_t B, int64_t H, int64_t D, int64_
 int fox_bwd_delta(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
                   const fox_tensor4* o, const fox_tensor4* d_o, float* delta);
 
+/* fox_bwd_delta that also clears the one-pass backward's accumulators: dq_accum (B,H,M,max(D,64)), dlam_row (B,H,M). */
+int fox_bwd_prepare(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
+                    const fox_tensor4* o, const fox_tensor4* d_o, float* delta, float* dq_accum, float* dlam_row);
+
 /* Backward attention in one pass: replaces the _bwd_kv_kernel and _bwd_q_kernel launches
  * (forgetting_attention.py:313-334, 366-386; kernels 956-1143, 1156-1344).  end_index from
  * fox_find_index with FOX_BWD_BLOCK_M/N, or NULL.  Outputs: dk, dv (input dtype, caller's
@@ -153,7 +181,8 @@ int fox_bwd_delta(int device, void* stream, int dtype, int64_t B, int64_t H, int
  * sum of the fp32 dS values, as fox_attn_bwd_dq's dlam_row, instead of the 16-bit-rounded ones both sums of the
  * one-pass form are built from);
  * and two caller-provided scratch arrays that must be zero on entry and are reduced into:
- * dq_accum (B,H,M,D) fp32 = sum_j dS_ij k_j (unscaled) and dlam_row (B,H,M) fp32 = sum_j dS_ij. */
+ * dq_accum (B,H,M,max(D,64)) fp32 = sum_j dS_ij k_j (unscaled) and dlam_row (B,H,M) fp32 = sum_j dS_ij.
+ * D in {64,128}; in the one-pass form also 16 and 32. */
 int fox_attn_bwd(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
                  const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v, const fox_tensor4* d_o,
                  const float* log_lambda, const float* L, const float* delta, const int64_t* seq_start,
@@ -176,6 +205,14 @@ int fox_attn_bwd_dq(int device, void* stream, int dtype, int64_t B, int64_t H, i
  * and store of forgetting_attention.py:1333-1343). */
 int fox_dq_convert(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,
                    const float* dq_accum, float scale, const fox_tensor4* dq);
+
+/* The end of the backward in one launch: the gate gradient (fox_revcumsum for gate_kind FOX_GATE_LOG, else
+ * fox_gate_prefix_bwd of the logits with strides (sb, sh, sn)) into dgate with strides (osb, osh, osn) and, when dq is
+ * not NULL, dq = dq_accum (B,H,M,max(D,64)) * scale. */
+int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
+                   const float* dlam_col, const float* dlam_row, int gate_kind, const void* fgate_logit, int64_t sb,
+                   int64_t sh, int64_t sn, void* dgate, int64_t osb, int64_t osh, int64_t osn, const float* dq_accum,
+                   float scale, const fox_tensor4* dq);
 
 /* Fused per-head RMSNorm + sigmoid gate, forward: y = x * rstd * w_h * sigmoid(g) with
  * rstd = (mean_d x^2 + eps)^-1/2 per (token, head).  Replaces layer_norm_gated_fwd
