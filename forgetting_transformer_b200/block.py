@@ -19,11 +19,27 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _lib
 from .norm_gate import FusedGroupNormGated, GroupNorm, RMSNorm
 from .ops import (acp_threshold_from_qk_norm, forgetting_attention, forgetting_attention_from_gate_logits,
                   seq_start_from_attention_mask)
 from .glu import swiglu_linear_packed
 from .token_shift import token_shift
+
+_host = None
+
+
+def _load_host():
+    """The native host side, told which classes its block path stands in for."""
+    global _host
+    host = _lib.host()
+    m = torch.nn.modules.module
+    host.set_block_classes(FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear,
+                           m._global_forward_hooks, m._global_forward_pre_hooks, m._global_backward_hooks,
+                           m._global_backward_pre_hooks)
+    _host = host
+    return _host
+
 
 __all__ = ["ShiftLinear", "FoxProAttentionLayer", "FoxMLP", "FoxProBlock"]
 
@@ -174,9 +190,23 @@ class FoxProBlock(nn.Module):
         self.mlp_norm = RMSNorm(hidden_size, eps=norm_eps)
         self.mlp = FoxMLP(hidden_size, intermediate_size)
 
+    def _threshold(self, hidden_states: torch.Tensor) -> Optional[torch.Tensor]:
+        a = self.attn
+        if getattr(a, "log_pruning_tolerance", None) is None or not hasattr(a, "q_norm"):
+            return None
+        return acp_threshold_from_qk_norm(a.q_norm.weight, a.k_norm.weight, a.num_heads, a.head_dim,
+                                          hidden_states.shape[1], a.log_pruning_tolerance)
+
     def forward(self, hidden_states: torch.Tensor, attention_mask: Optional[torch.Tensor] = None,
                 past_key_values=None, layer_idx: int = 0) -> torch.Tensor:
-        """hidden_states (B, T, hidden) in fp16/bf16 (the residual stream is kept in that dtype here)."""
+        """hidden_states (B, T, hidden) in fp16/bf16 (the residual stream is kept in that dtype here).
+
+        Without a cache the whole block runs as one native forward and backward where its parts are the plain modules
+        built here (no hooks, replaced submodules or autocast) in one 16-bit dtype; else module by module."""
+        if past_key_values is None:
+            out = (_host or _load_host()).block(self, hidden_states, attention_mask, self._threshold(hidden_states))
+            if out is not None:
+                return out
         residual = hidden_states
         hidden_states = self.attn(self.attn_norm(hidden_states), attention_mask, past_key_values, layer_idx)
         hidden_states, residual = self.mlp_norm(hidden_states, residual, True)

@@ -19,10 +19,10 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libfox_b200.so")
 HOST_PATH = os.path.join(PKG_DIR, "_fox_host.so")
-SOURCES = ["fox_scan.cu", "fox_attn_fwd.cu", "fox_attn_bwd.cu", "fox_attn_bwd_dq.cu", "fox_attn_bwd_kv.cu", "fox_decode.cu", "fox_normgate.cu", "fox_rmsnorm.cu", "fox_shift.cu", "fox_glu.cu", "fox_ce.cu", "fox_noalloc.cu"]
+SOURCES = ["fox_scan.cu", "fox_attn_fwd.cu", "fox_attn_bwd.cu", "fox_attn_bwd_dq.cu", "fox_attn_bwd_kv.cu", "fox_decode.cu", "fox_normgate.cu", "fox_rmsnorm.cu", "fox_shift.cu", "fox_glu.cu", "fox_ce.cu", "fox_block.cu", "fox_noalloc.cu"]
 HEADERS = ["fox_common.cuh", "fox_host.h", os.path.join("..", "..", "include", "fox_b200.h")]
-HOST_SOURCES = ["host_module.cpp", "host_attention.cpp"]
-HOST_HEADERS = ["host_common.h", "host_attention.h", os.path.join("..", "..", "include", "fox_b200.h")]
+HOST_SOURCES = ["host_module.cpp", "host_attention.cpp", "host_block.cpp", "host_gemm.cpp"]
+HOST_HEADERS = ["host_common.h", "host_attention.h", "host_block.h", "host_gemm.h", os.path.join("..", "..", "include", "fox_b200.h")]
 
 
 def _paths(names):
@@ -76,7 +76,8 @@ def _build_host(verbose):
     flags = [cxx, "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f for i in inc for f in ("-isystem", i)]
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    libs = ["-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
+    blas = os.path.join(os.path.dirname(os.path.dirname(torch.__file__)), "nvidia", "cublas", "lib")   # the one torch loads
+    libs = ["-L" + blas, "-l:libcublasLt.so.12", "-Wl,-rpath," + blas, "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
             "-L" + PKG_DIR, "-l:libfox_b200.so", "/usr/local/cuda/lib64/libcudart.so", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib]
     _compile_all(_paths(HOST_SOURCES), flags, [cxx], HOST_PATH, libs, verbose)
 

@@ -63,7 +63,7 @@ __device__ __forceinline__ void store8(uint16_t* p, const float* f) {
 template <bool kBf16, bool kGate>
 __global__ void fox_normgate_fwd_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ g,
                                         const float* __restrict__ w, uint16_t* __restrict__ y,
-                                        float* __restrict__ rstd, int64_t tokens, int G, int D, float eps) {
+                                        float* __restrict__ rstd, int64_t tokens, int G, int D, float eps, int64_t g_ld) {
   const int lanes = D >> 3;
   const int tid = threadIdx.x;
   const int h = tid / lanes, sub = tid % lanes;
@@ -85,7 +85,7 @@ __global__ void fox_normgate_fwd_kernel(const uint16_t* __restrict__ x, const ui
       xr[u] = gr[u] = make_uint4(0, 0, 0, 0);
       if (active && t < tokens) {
         xr[u] = *reinterpret_cast<const uint4*>(x + t * GD + ch);
-        if (kGate) gr[u] = *reinterpret_cast<const uint4*>(g + t * GD + ch);
+        if (kGate) gr[u] = *reinterpret_cast<const uint4*>(g + t * g_ld + ch);
       }
     }
 #pragma unroll
@@ -115,7 +115,7 @@ __global__ void fox_normgate_bwd_kernel(const uint16_t* __restrict__ x, const ui
                                         const float* __restrict__ w, const float* __restrict__ rstd,
                                         const uint16_t* __restrict__ dy, uint16_t* __restrict__ dx,
                                         uint16_t* __restrict__ dg, float* __restrict__ dw_partial, int64_t tokens,
-                                        int G, int D) {
+                                        int G, int D, int64_t g_ld, int64_t dg_ld) {
   const int lanes = D >> 3;
   const int tid = threadIdx.x;
   const int h = tid / lanes, sub = tid % lanes;
@@ -134,7 +134,7 @@ __global__ void fox_normgate_bwd_kernel(const uint16_t* __restrict__ x, const ui
     float r = 0.f;
     if (active) {
       load8<kBf16>(x + t * GD + ch, xv);
-      if (kGate) load8<kBf16>(g + t * GD + ch, gv);
+      if (kGate) load8<kBf16>(g + t * g_ld + ch, gv);
       load8<kBf16>(dy + t * GD + ch, dyv);
       r = rstd[t * G + h];
     } else {
@@ -161,7 +161,7 @@ __global__ void fox_normgate_bwd_kernel(const uint16_t* __restrict__ x, const ui
 #pragma unroll
       for (int j = 0; j < 8; ++j) dxv[j] = (wdy[j] - xhat[j] * c1) * r;
       store8<kBf16>(dx + t * GD + ch, dxv);
-      if (kGate) store8<kBf16>(dg + t * GD + ch, dgv);
+      if (kGate) store8<kBf16>(dg + t * dg_ld + ch, dgv);
     }
   }
   if (active) {
@@ -182,8 +182,14 @@ using namespace fox;
 
 extern "C" int fox_normgate_fwd(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D,
                                 const void* x, const void* g, const float* w, float eps, void* y, float* rstd) {
+  return fox_normgate_fwd_ld(device, stream, dtype, tokens, G, D, x, g, G * D, w, eps, y, rstd);
+}
+
+extern "C" int fox_normgate_fwd_ld(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D, const void* x,
+                                   const void* g, int64_t g_ld, const float* w, float eps, void* y, float* rstd) {
   if (!x || !w || !y || !rstd || tokens <= 0 || G <= 0) return FOX_ERR_BAD_ARG;
   if (D % 8 || D < 8 || D > 256 || (D & (D - 1))) return FOX_ERR_HEAD_DIM;
+  if (g && (g_ld % 8 || g_ld < G * D)) return FOX_ERR_ALIGNMENT;
   const int threads = normgate_threads(G, D);
   if (threads > 1024) return FOX_ERR_TOO_LARGE;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(y)) % 16)
@@ -192,7 +198,7 @@ extern "C" int fox_normgate_fwd(int device, void* stream, int dtype, int64_t tok
   const int64_t grid = tokens < 148 * 16 ? tokens : 148 * 16;
 #define FOX_NG_FWD(BF, GATE)                                                                      \
   fox_normgate_fwd_kernel<BF, GATE><<<(unsigned)grid, threads, 0, (cudaStream_t)stream>>>(          \
-      (const uint16_t*)x, (const uint16_t*)g, w, (uint16_t*)y, rstd, tokens, (int)G, (int)D, eps)
+      (const uint16_t*)x, (const uint16_t*)g, w, (uint16_t*)y, rstd, tokens, (int)G, (int)D, eps, g_ld)
   if (dtype == FOX_DTYPE_BF16) {
     if (g) FOX_NG_FWD(true, true); else FOX_NG_FWD(true, false);
   } else {
@@ -205,10 +211,18 @@ extern "C" int fox_normgate_fwd(int device, void* stream, int dtype, int64_t tok
 extern "C" int fox_normgate_bwd(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D,
                                 const void* x, const void* g, const float* w, const float* rstd, const void* dy,
                                 void* dx, void* dg, float* dw_partial, int64_t n_partials) {
+  return fox_normgate_bwd_ld(device, stream, dtype, tokens, G, D, x, g, G * D, w, rstd, dy, dx, dg, G * D, dw_partial, n_partials);
+}
+
+extern "C" int fox_normgate_bwd_ld(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D, const void* x,
+                                   const void* g, int64_t g_ld, const float* w, const float* rstd, const void* dy, void* dx,
+                                   void* dg, int64_t dg_ld, float* dw_partial, int64_t n_partials) {
   if (!x || !w || !rstd || !dy || !dx || !dw_partial || tokens <= 0 || G <= 0 || n_partials <= 0)
     return FOX_ERR_BAD_ARG;
   if ((g == nullptr) != (dg == nullptr)) return FOX_ERR_BAD_ARG;
   if (D % 8 || D < 8 || D > 256 || (D & (D - 1))) return FOX_ERR_HEAD_DIM;
+  if (g && (g_ld % 8 || g_ld < G * D)) return FOX_ERR_ALIGNMENT;
+  if (dg && (dg_ld % 8 || dg_ld < G * D)) return FOX_ERR_ALIGNMENT;
   const int threads = normgate_threads(G, D);
   if (threads > 1024) return FOX_ERR_TOO_LARGE;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(dy) |
@@ -218,7 +232,7 @@ extern "C" int fox_normgate_bwd(int device, void* stream, int dtype, int64_t tok
 #define FOX_NG_BWD(BF, GATE)                                                                          \
   fox_normgate_bwd_kernel<BF, GATE><<<(unsigned)n_partials, threads, 0, (cudaStream_t)stream>>>(        \
       (const uint16_t*)x, (const uint16_t*)g, w, rstd, (const uint16_t*)dy, (uint16_t*)dx, (uint16_t*)dg, \
-      dw_partial, tokens, (int)G, (int)D)
+      dw_partial, tokens, (int)G, (int)D, g_ld, dg_ld)
   if (dtype == FOX_DTYPE_BF16) {
     if (g) FOX_NG_BWD(true, true); else FOX_NG_BWD(true, false);
   } else {

@@ -91,12 +91,118 @@ static void gate_strides(const Tensor& g, bool hf, int64_t* st) {
   st[2] = g.stride(hf ? 2 : 1);
 }
 
+// ---------------------------------------------------------------- launches
+int64_t attn_blocks(int64_t n) { return (n + kBlock - 1) / kBlock; }
+
+// largest key norm per (b,h): the forward kernel's bound that lets most tiles skip the row-maximum pass
+AttnNorms attn_norms(const AttnShape& s, bool is_auto) {
+  AttnNorms n;
+  if ((s.N >= 8 * kBlock && s.M > 1) || is_auto) n.n_k = fox_norm_parts(s.B, s.H, s.N, s.D);
+  if (is_auto) n.n_q = fox_norm_parts(s.B, s.H, s.M, s.D);
+  return n;
+}
+
+static void prepare_launch(const AttnCall& c, const AttnNorms& n, float* norms, Threshold::Kind kind, double threshold_value,
+                           float* threshold, int64_t thr_sb, int64_t thr_sh) {
+  const AttnShape& s = c.s;
+  float* k_parts = n.n_k ? norms : nullptr;
+  float* q_parts = n.n_q ? norms + c.BH() * n.n_k : nullptr;
+  launch("fox_attn_prologue", c.st, [&] {
+    return fox_attn_prologue(c.device, c.st, c.code, c.gate_kind, s.B, s.H, s.M, s.N, s.D, c.gate, c.gate_st[0], c.gate_st[1],
+                             c.gate_st[2], c.gate_bias, c.seq_start, c.lam, n.n_k ? &c.k : nullptr, k_parts, n.n_k,
+                             n.n_q ? &c.q : nullptr, q_parts, n.n_q);
+  });
+  if (kind == Threshold::kNone) return;
+  launch("fox_find_index", c.st, [&] {
+    if (kind == Threshold::kTensor)
+      return fox_find_index(c.device, c.st, s.B, s.H, s.M, s.N, kBlock, kBlock, c.lam, threshold, thr_sb, thr_sh, c.start, c.end);
+    return fox_attn_index(c.device, c.st, c.code, s.B, s.H, s.M, s.N, kBlock, kBlock, c.lam, static_cast<float>(threshold_value),
+                          q_parts, n.n_q, q_parts ? k_parts : nullptr, n.n_k, c.sm_scale, c.start, c.end, threshold);
+  });
+}
+
+void attn_forward_launch(const AttnCall& c, const AttnNorms& n, float* norms, Threshold::Kind kind, double threshold_value,
+                         float* threshold, int64_t thr_sb, int64_t thr_sh) {
+  prepare_launch(c, n, norms, kind, threshold_value, threshold, thr_sb, thr_sh);
+  int32_t* status = status_words(c.device);
+  launch("fox_attn_fwd", c.st, [&] {
+    return fox_attn_fwd_parts(c.device, c.st, c.code, c.s.B, c.s.H, c.s.M, c.s.N, c.s.D, &c.q, &c.k, &c.v, c.lam, c.seq_start,
+                              c.start, c.sm_scale, &c.o, c.L, n.n_k ? norms : nullptr, n.n_k, status);
+  });
+  if (debug_sync()) status_check(c.device);
+}
+
+// [dq accumulator (B,H,M,max(D,64)), one-pass only | delta, dlam_row (B,H,M) each | dlam_col (B,H,N)]
+static int64_t accum_floats(const AttnShape& s, bool two_kernel) {
+  return two_kernel ? 0 : s.B * s.H * s.M * std::max<int64_t>(s.D, 64);
+}
+int64_t attn_backward_floats(const AttnShape& s, bool two_kernel) {
+  return accum_floats(s, two_kernel) + s.B * s.H * (2 * s.M + s.N);
+}
+
+void attn_backward_launch(const AttnCall& c, const AttnGradCall& g) {
+  const AttnShape& s = c.s;
+  const int64_t B = s.B, H = s.H, M = s.M, N = s.N, D = s.D, BH = B * H;
+  float* dq_accum = g.work;
+  float* delta = dq_accum + accum_floats(s, g.two_kernel);
+  float* dlam_row = delta + BH * M;
+  float* dlam_col = dlam_row + BH * M;
+  const int dev = c.device;
+  const cudaStream_t st = c.st;
+  int32_t* status = status_words(dev);
+  if (g.two_kernel) {
+    // key side (dk, dv, column sums) without a dQ product, query side as its own kernel: no fp32 dQ partials to
+    // add-reduce into L2, which is what bounds the one-pass kernel at head dim 128
+    launch("fox_bwd_delta", st, [&] { return fox_bwd_delta(dev, st, c.code, B, H, M, D, &c.o, &g.g, delta); });
+    launch("fox_attn_bwd", st, [&] {
+      return fox_attn_bwd(dev, st, c.code, B, H, M, N, D, &c.q, &c.k, &c.v, &g.g, c.lam, c.L, delta, c.seq_start, c.end, c.sm_scale,
+                          nullptr, nullptr, dlam_col, &g.dk, &g.dv, status);
+    });
+    launch("fox_attn_bwd_dq", st, [&] {
+      return fox_attn_bwd_dq(dev, st, c.code, B, H, M, N, D, &c.q, &c.k, &c.v, &g.g, c.lam, c.L, delta, c.seq_start, c.start,
+                             c.sm_scale, &g.dq, dlam_row, status);
+    });
+  } else {
+    launch("fox_bwd_delta", st,
+           [&] { return fox_bwd_prepare(dev, st, c.code, B, H, M, D, &c.o, &g.g, delta, dq_accum, dlam_row); });
+    launch("fox_attn_bwd", st, [&] {
+      return fox_attn_bwd(dev, st, c.code, B, H, M, N, D, &c.q, &c.k, &c.v, &g.g, c.lam, c.L, delta, c.seq_start, c.end, c.sm_scale,
+                          dq_accum, dlam_row, dlam_col, &g.dk, &g.dv, status);
+    });
+  }
+  // reverse prefix sum of the two halves of dlog_lambda (upstream lines 390-392); for gate logits also the chain rule
+  // through log sigmoid, in the logits' dtype and layout
+  launch("fox_bwd_finish", st, [&] {
+    return fox_bwd_finish(dev, st, c.code, B, H, M, N, D, dlam_col, dlam_row, c.gate_kind, c.gate, c.gate_st[0], c.gate_st[1],
+                          c.gate_st[2], c.gate_bias, g.dgate, g.dgate_st[0], g.dgate_st[1], g.dgate_st[2], g.dbias,
+                          g.two_kernel ? nullptr : dq_accum, c.sm_scale, g.two_kernel ? nullptr : &g.dq);
+  });
+  status_pending(dev);
+  if (debug_sync()) status_check(dev);
+}
+
 // ---------------------------------------------------------------- forward
+static AttnCall call_of(const AttnSaved& r, cudaStream_t st) {
+  AttnCall c;
+  c.device = r.q.device().index();
+  c.st = st;
+  c.code = dtype_code(r.q.scalar_type());
+  c.s = r.shape;
+  c.q = t4(r.q, r.head_first);
+  c.k = t4(r.k, r.head_first);
+  c.v = t4(r.v, r.head_first);
+  c.o = t4(r.o, r.head_first);
+  c.sm_scale = static_cast<float>(r.sm_scale);
+  if (r.seq_start.defined()) c.seq_start = r.seq_start.const_data_ptr<int64_t>();
+  c.lam = const_cast<float*>(r.lam());
+  c.L = const_cast<float*>(r.L());
+  return c;
+}
+
 AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs_grad) {
   const c10::cuda::CUDAGuard guard(in.q.device());
   const at::AutoDispatchBelowADInplaceOrView no_autograd;
   const int dev = in.q.device().index();
-  const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
   const bool hf = in.head_first;
   const int64_t B = s.B, H = s.H, M = s.M, N = s.N, D = s.D, BH = B * H;
   status_poll(dev);   // did a kernel of an earlier step give up on a wait? (no synchronisation)
@@ -110,38 +216,22 @@ AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs
   r.q = tma_view(in.q);
   r.k = tma_view(in.k);
   r.v = tma_view(in.v);
-  const int code = dtype_code(r.q.scalar_type());
   if (in.seq_start.defined()) r.seq_start = in.seq_start.to(in.q.device(), at::kLong).contiguous();
-  const int64_t* seq = r.seq_start.defined() ? r.seq_start.const_data_ptr<int64_t>() : nullptr;
-
-  const bool is_auto = in.threshold.kind == Threshold::kAuto;
   const bool pruned = in.threshold.kind != Threshold::kNone;
-  // largest key norm per (b,h): the forward kernel's bound that lets most tiles skip the row-maximum pass
-  const bool k_norms = (N >= 8 * kBlock && M > 1) || is_auto;
-  const int64_t n_k = k_norms ? fox_norm_parts(B, H, N, D) : 0, n_q = is_auto ? fox_norm_parts(B, H, M, D) : 0;
-
+  const AttnNorms norms = attn_norms(s, in.threshold.kind == Threshold::kAuto);
   // [log_lambda (B,H,N) | L (B,H,M) | norm parts]
-  r.vectors = at::empty({BH * (N + M + n_k + n_q)}, in.q.options().dtype(at::kFloat));
-  float* lam = r.vectors.mutable_data_ptr<float>();
-  float* L = lam + BH * N;
-  float* k_parts = k_norms ? L + BH * M : nullptr;
-  float* q_parts = is_auto ? k_parts + BH * n_k : nullptr;
+  r.vectors = at::empty({BH * (N + M) + norms.floats(BH)}, in.q.options().dtype(at::kFloat));
+  float* norm_parts = r.vectors.mutable_data_ptr<float>() + BH * (N + M);
+  r.o = empty_like_tma(r.q);
 
-  const fox_tensor4 q4 = t4(r.q, hf), k4 = t4(r.k, hf), v4 = t4(r.v, hf);
-  int64_t gs[3];
-  gate_strides(in.gate, hf, gs);
-  const int gate_kind = in.gate_is_logit ? dtype_code(in.gate.scalar_type()) : FOX_GATE_LOG;
-  launch("fox_attn_prologue", st, [&] {
-    return fox_attn_prologue(dev, st, code, gate_kind, B, H, M, N, D, in.gate.data_ptr(), gs[0], gs[1], gs[2], seq, lam,
-                             k_norms ? &k4 : nullptr, k_parts, n_k, is_auto ? &q4 : nullptr, q_parts, n_q);
-  });
-
-  int64_t* start = nullptr;
+  AttnCall c = call_of(r, c10::cuda::getCurrentCUDAStream(dev).stream());
+  c.gate = in.gate.data_ptr();
+  gate_strides(in.gate, hf, c.gate_st);
+  if (in.gate_is_logit) c.gate_kind = dtype_code(in.gate.scalar_type());
   if (pruned) {
-    const int64_t nmb = (M + kBlock - 1) / kBlock, nnb = (N + kBlock - 1) / kBlock;
-    r.index = at::empty({BH * (nmb + (needs_grad ? nnb : 0))}, in.q.options().dtype(at::kLong));
-    start = r.index.mutable_data_ptr<int64_t>();
-    int64_t* end = needs_grad ? start + BH * nmb : nullptr;
+    r.index = at::empty({BH * (attn_blocks(M) + (needs_grad ? attn_blocks(N) : 0))}, in.q.options().dtype(at::kLong));
+    c.start = r.index.mutable_data_ptr<int64_t>();
+    c.end = needs_grad ? c.start + BH * attn_blocks(M) : nullptr;
     if (in.threshold.kind == Threshold::kTensor) {
       r.threshold = in.threshold.tensor.detach().to(in.q.device(), at::kFloat);
       if (!at::is_expandable_to(r.threshold.sizes(), {B, H})) {
@@ -152,24 +242,15 @@ AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs
             std::to_string(B) + ", " + std::to_string(H) + "), but got torch.Size(" + os.str() + ").");
       }
       r.threshold = r.threshold.expand({B, H});
-      launch("fox_find_index", st, [&] {
-        return fox_find_index(dev, st, B, H, M, N, kBlock, kBlock, lam, r.threshold.const_data_ptr<float>(),
-                              r.threshold.stride(0), r.threshold.stride(1), start, end);
-      });
     } else {
       r.threshold = at::empty({B, H}, in.q.options().dtype(at::kFloat));
-      launch("fox_find_index", st, [&] {
-        return fox_attn_index(dev, st, code, B, H, M, N, kBlock, kBlock, lam, static_cast<float>(in.threshold.value), q_parts,
-                              n_q, is_auto ? k_parts : nullptr, n_k, static_cast<float>(in.sm_scale), start, end,
-                              r.threshold.mutable_data_ptr<float>());
-      });
     }
   }
-
-  r.o = empty_like_tma(r.q);
-  const fox_tensor4 o4 = t4(r.o, hf);
+  float* thr = pruned ? static_cast<float*>(r.threshold.data_ptr()) : nullptr;
+  const int64_t thr_sb = pruned ? r.threshold.stride(0) : 0, thr_sh = pruned ? r.threshold.stride(1) : 0;
   if (M == 1 && !needs_grad) {
     // generation step: one query row against the cache, no gradients -> split-KV kernels
+    prepare_launch(c, norms, norm_parts, in.threshold.kind, in.threshold.value, thr, thr_sb, thr_sh);
     int64_t splits = std::max<int64_t>(1, std::min(std::min((N + 511) / 512, (4 * 148 + BH - 1) / BH), int64_t{256}));
     const int64_t Dk = std::max<int64_t>(D, 64);
     Tensor q = r.q, k = r.k, v = r.v, o = r.o;
@@ -181,19 +262,14 @@ AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs
     }
     Tensor work = at::empty({fox_attn_decode_workspace_floats(B, H, Dk, splits)}, in.q.options().dtype(at::kFloat));
     const fox_tensor4 dq4 = t4(q, hf), dk4 = t4(k, hf), dv4 = t4(v, hf), do4 = t4(o, hf);
-    launch("fox_attn_decode", st, [&] {
-      return fox_attn_decode(dev, st, code, B, H, N, Dk, &dq4, &dk4, &dv4, lam, seq, start, static_cast<float>(in.sm_scale),
-                             &do4, L, work.mutable_data_ptr<float>(), splits);
+    launch("fox_attn_decode", c.st, [&] {
+      return fox_attn_decode(dev, c.st, c.code, B, H, N, Dk, &dq4, &dk4, &dv4, c.lam, c.seq_start, c.start, c.sm_scale, &do4, c.L,
+                             work.mutable_data_ptr<float>(), splits);
     });
     if (D < 64) r.o = o.narrow(3, 0, D).contiguous();
     return r;
   }
-  int32_t* status = status_words(dev);
-  launch("fox_attn_fwd", st, [&] {
-    return fox_attn_fwd_parts(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, lam, seq, start, static_cast<float>(in.sm_scale), &o4,
-                              L, k_parts, n_k, status);
-  });
-  if (debug_sync()) status_check(dev);
+  attn_forward_launch(c, norms, norm_parts, in.threshold.kind, in.threshold.value, thr, thr_sb, thr_sh);
   return r;
 }
 
@@ -202,85 +278,46 @@ AttnGrads attention_backward(const AttnSaved& r, const Tensor& d_o, bool two_ker
   const c10::cuda::CUDAGuard guard(r.q.device());
   const at::AutoDispatchBelowADInplaceOrView no_autograd;
   const int dev = r.q.device().index();
-  const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
   const bool hf = r.head_first;
-  const int64_t B = r.shape.B, H = r.shape.H, M = r.shape.M, N = r.shape.N, D = r.shape.D, BH = B * H;
-  const int code = dtype_code(r.q.scalar_type());
-  const Tensor g = tma_view(d_o);
-  const float* lam = r.lam();
-  const float* L = r.L();
-  const int64_t* seq = r.seq_start.defined() ? r.seq_start.const_data_ptr<int64_t>() : nullptr;
-  const int64_t nmb = (M + kBlock - 1) / kBlock, nnb = (N + kBlock - 1) / kBlock;
-  two_kernel = two_kernel && D >= 64;
+  const Tensor grad = tma_view(d_o);
+  AttnCall c = call_of(r, c10::cuda::getCurrentCUDAStream(dev).stream());
+  const int64_t nmb = attn_blocks(c.s.M), nnb = attn_blocks(c.s.N);
 
   Tensor index = r.index;
-  if (r.threshold.defined() && !(index.defined() && index.numel() == BH * (nmb + nnb))) {
-    index = at::empty({BH * (nmb + nnb)}, r.q.options().dtype(at::kLong));
-    int64_t* p = index.mutable_data_ptr<int64_t>();
-    launch("fox_find_index", st, [&] {
-      return fox_find_index(dev, st, B, H, M, N, kBlock, kBlock, lam, r.threshold.const_data_ptr<float>(),
-                            r.threshold.stride(0), r.threshold.stride(1), p, p + BH * nmb);
-    });
+  if (r.threshold.defined()) {
+    const bool have = index.defined() && index.numel() == c.BH() * (nmb + nnb);
+    if (!have) index = at::empty({c.BH() * (nmb + nnb)}, r.q.options().dtype(at::kLong));
+    c.start = index.mutable_data_ptr<int64_t>();
+    c.end = c.start + c.BH() * nmb;
+    if (!have)
+      launch("fox_find_index", c.st, [&] {
+        return fox_find_index(dev, c.st, c.s.B, c.s.H, c.s.M, c.s.N, kBlock, kBlock, c.lam, r.threshold.const_data_ptr<float>(),
+                              r.threshold.stride(0), r.threshold.stride(1), c.start, c.end);
+      });
   }
-  const int64_t* start = r.threshold.defined() ? index.const_data_ptr<int64_t>() : nullptr;
-  const int64_t* end = start ? start + BH * nmb : nullptr;
-
   AttnGrads out;
   out.dq = empty_like_tma(r.q);
   out.dk = empty_like_tma(r.k);
   out.dv = empty_like_tma(r.v);
-  // [dq accumulator (B,H,M,max(D,64)), one-pass only | delta, dlam_row (B,H,M) each | dlam_col (B,H,N)]
-  const int64_t acc = two_kernel ? 0 : BH * M * std::max<int64_t>(D, 64);
-  const Tensor work = at::empty({acc + 2 * BH * M + BH * N}, r.q.options().dtype(at::kFloat));
-  float* dq_accum = work.mutable_data_ptr<float>();
-  float* delta = dq_accum + acc;
-  float* dlam_row = delta + BH * M;
-  float* dlam_col = dlam_row + BH * M;
-  const fox_tensor4 q4 = t4(r.q, hf), k4 = t4(r.k, hf), v4 = t4(r.v, hf), o4 = t4(r.o, hf), g4 = t4(g, hf), dq4 = t4(out.dq, hf),
-                    dk4 = t4(out.dk, hf), dv4 = t4(out.dv, hf);
-  const float scale = static_cast<float>(r.sm_scale);
-  int32_t* status = status_words(dev);
-  if (two_kernel) {
-    // key side (dk, dv, column sums) without a dQ product, query side as its own kernel: no fp32 dQ partials to
-    // add-reduce into L2, which is what bounds the one-pass kernel at head dim 128
-    launch("fox_bwd_delta", st, [&] { return fox_bwd_delta(dev, st, code, B, H, M, D, &o4, &g4, delta); });
-    launch("fox_attn_bwd", st, [&] {
-      return fox_attn_bwd(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, &g4, lam, L, delta, seq, end, scale, nullptr, nullptr,
-                          dlam_col, &dk4, &dv4, status);
-    });
-    launch("fox_attn_bwd_dq", st, [&] {
-      return fox_attn_bwd_dq(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, &g4, lam, L, delta, seq, start, scale, &dq4, dlam_row,
-                             status);
-    });
-  } else {
-    launch("fox_bwd_delta", st,
-           [&] { return fox_bwd_prepare(dev, st, code, B, H, M, D, &o4, &g4, delta, dq_accum, dlam_row); });
-    launch("fox_attn_bwd", st, [&] {
-      return fox_attn_bwd(dev, st, code, B, H, M, N, D, &q4, &k4, &v4, &g4, lam, L, delta, seq, end, scale, dq_accum, dlam_row,
-                          dlam_col, &dk4, &dv4, status);
-    });
-  }
-  // reverse prefix sum of the two halves of dlog_lambda (upstream lines 390-392); for gate logits also the chain rule
-  // through log sigmoid, in the logits' dtype and layout
-  int gate_kind = FOX_GATE_LOG;
-  int64_t gs[3] = {0, 0, 0}, os[3];
-  const void* logit = nullptr;
+  AttnGradCall g;
+  g.two_kernel = two_kernel && c.s.D >= 64;
+  const Tensor work = at::empty({attn_backward_floats(c.s, g.two_kernel)}, r.q.options().dtype(at::kFloat));
+  g.work = work.mutable_data_ptr<float>();
+  g.g = t4(grad, hf);
+  g.dq = t4(out.dq, hf);
+  g.dk = t4(out.dk, hf);
+  g.dv = t4(out.dv, hf);
   if (r.gate_is_logit) {
-    gate_kind = dtype_code(r.gate.scalar_type());
-    gate_strides(r.gate, hf, gs);
-    logit = r.gate.data_ptr();
+    c.gate_kind = dtype_code(r.gate.scalar_type());
+    c.gate = r.gate.data_ptr();
+    gate_strides(r.gate, hf, c.gate_st);
     out.dgate = at::empty_like(r.gate);
   } else {   // in the gates' own layout, which the gradient's accumulation would otherwise copy it into
     out.dgate = at::empty_strided(r.gate_sizes, r.gate_strides, r.q.options().dtype(at::kFloat));
   }
-  gate_strides(out.dgate, hf, os);
-  launch("fox_bwd_finish", st, [&] {
-    return fox_bwd_finish(dev, st, code, B, H, M, N, D, dlam_col, dlam_row, gate_kind, logit, gs[0], gs[1], gs[2],
-                          out.dgate.data_ptr(), os[0], os[1], os[2], two_kernel ? nullptr : dq_accum, scale,
-                          two_kernel ? nullptr : &dq4);
-  });
-  status_pending(dev);
-  if (debug_sync()) status_check(dev);
+  g.dgate = out.dgate.data_ptr();
+  gate_strides(out.dgate, hf, g.dgate_st);
+  attn_backward_launch(c, g);
   return out;
 }
 

@@ -49,6 +49,45 @@ struct AttnSaved {
   }
 };
 
+// One call of the kernels on raw device pointers; every array is the caller's.
+struct AttnCall {
+  int device = 0, code = 0;          // FOX_DTYPE_* of q, k, v
+  cudaStream_t st = nullptr;
+  AttnShape s;
+  fox_tensor4 q, k, v, o;
+  float sm_scale = 0.f;
+  const int64_t* seq_start = nullptr;
+  int gate_kind = FOX_GATE_LOG;      // or the dtype of gate logits
+  const void* gate = nullptr;
+  int64_t gate_st[3] = {0, 0, 0};    // b, h, t strides
+  const float* gate_bias = nullptr;
+  float *lam = nullptr, *L = nullptr;              // (B,H,N), (B,H,M)
+  int64_t *start = nullptr, *end = nullptr;        // with a threshold (end: with gradients)
+
+  int64_t BH() const { return s.B * s.H; }
+};
+struct AttnNorms {   // parts of the row-norm maxima a forward needs: n_k, n_q floats per (b,h)
+  int64_t n_k = 0, n_q = 0;
+  int64_t floats(int64_t BH) const { return BH * (n_k + n_q); }
+};
+AttnNorms attn_norms(const AttnShape& s, bool is_auto);
+int64_t attn_blocks(int64_t n);   // tiles of the pruning grid
+
+// norms: attn_norms().floats() floats.  threshold: where kind is not kNone; its (B,H) values for a tensor, or the place
+// that receives them.  splits_work: for a single query without gradients, the decode kernels' workspace.
+void attn_forward_launch(const AttnCall& c, const AttnNorms& n, float* norms, Threshold::Kind kind, double threshold_value,
+                         float* threshold, int64_t thr_sb, int64_t thr_sh);
+struct AttnGradCall {
+  fox_tensor4 g, dq, dk, dv;         // dout and the gradients
+  float* work = nullptr;             // attn_backward_floats()
+  void* dgate = nullptr;
+  int64_t dgate_st[3] = {0, 0, 0};
+  float* dbias = nullptr;            // (B*H) or nullptr
+  bool two_kernel = false;
+};
+int64_t attn_backward_floats(const AttnShape& s, bool two_kernel);
+void attn_backward_launch(const AttnCall& c, const AttnGradCall& g);
+
 struct AttnGrads {
   Tensor dq, dk, dv, dgate;
 };

@@ -102,3 +102,5 @@ inline Tensor unpack_opt(PyObject* o, const char* what) { return o == Py_None ? 
 FOX_PY(py_attention);
 FOX_PY(py_attention_forward);
 FOX_PY(py_attention_backward);
+FOX_PY(py_set_block_classes);
+FOX_PY(py_block);

@@ -115,12 +115,13 @@ int fox_max_row_norm(int device, void* stream, int dtype, int64_t B, int64_t H, 
                      const fox_tensor4* x, float* out_zeroed);
 
 /* What the operator needs before its forward kernel, in one launch: the prefix sum of the gates (fox_cumsum_fwd /
- * fox_gate_prefix_fwd; gate_kind FOX_GATE_LOG or the dtype of gate logits) and, where k (q) is given, the largest row
+ * fox_gate_prefix_fwd; gate_kind FOX_GATE_LOG or the dtype of gate logits, to which gate_bias (H) fp32 is added if
+ * given) and, where k (q) is given, the largest row
  * norm of every (b,h) as n partial maxima, k_parts (B,H,n_k_parts), fully written; n from fox_norm_parts, <= 32. */
 int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D);
 int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M, int64_t N,
-                      int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
-                      float* log_lambda, const fox_tensor4* k, float* k_parts, int64_t n_k_parts, const fox_tensor4* q,
+                      int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn, const float* gate_bias,
+                      const int64_t* seq_start, float* log_lambda, const fox_tensor4* k, float* k_parts, int64_t n_k_parts, const fox_tensor4* q,
                       float* q_parts, int64_t n_q_parts);
 
 /* fox_find_index for one threshold value, or (q_parts, k_parts given) for the automatic threshold of
@@ -207,12 +208,12 @@ int fox_dq_convert(int device, void* stream, int dtype, int64_t B, int64_t H, in
                    const float* dq_accum, float scale, const fox_tensor4* dq);
 
 /* The end of the backward in one launch: the gate gradient (fox_revcumsum for gate_kind FOX_GATE_LOG, else
- * fox_gate_prefix_bwd of the logits with strides (sb, sh, sn)) into dgate with strides (osb, osh, osn) and, when dq is
- * not NULL, dq = dq_accum (B,H,M,max(D,64)) * scale. */
+ * fox_gate_prefix_bwd of the logits with strides (sb, sh, sn), gate_bias added) into dgate with strides (osb, osh, osn),
+ * dbias (B*H) fp32 or NULL = each (b,h)'s sum of it (logits only) and, when dq is not NULL, dq = dq_accum (B,H,M,max(D,64)) * scale. */
 int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
                    const float* dlam_col, const float* dlam_row, int gate_kind, const void* fgate_logit, int64_t sb,
-                   int64_t sh, int64_t sn, void* dgate, int64_t osb, int64_t osh, int64_t osn, const float* dq_accum,
-                   float scale, const fox_tensor4* dq);
+                   int64_t sh, int64_t sn, const float* gate_bias, void* dgate, int64_t osb, int64_t osh, int64_t osn,
+                   float* dbias, const float* dq_accum, float scale, const fox_tensor4* dq);
 
 /* Fused per-head RMSNorm + sigmoid gate, forward: y = x * rstd * w_h * sigmoid(g) with
  * rstd = (mean_d x^2 + eps)^-1/2 per (token, head).  Replaces layer_norm_gated_fwd
@@ -231,6 +232,41 @@ int fox_normgate_fwd(int device, void* stream, int dtype, int64_t tokens, int64_
 int fox_normgate_bwd(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D, const void* x,
                      const void* g, const float* w, const float* rstd, const void* dy, void* dx, void* dg,
                      float* dw_partial, int64_t n_partials);
+
+/* The two above with a row stride (elements, a multiple of 8) of g and dg: a gate that is a column range of a wider
+ * projection. */
+int fox_normgate_fwd_ld(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D, const void* x,
+                        const void* g, int64_t g_ld, const float* w, float eps, void* y, float* rstd);
+int fox_normgate_bwd_ld(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D, const void* x,
+                        const void* g, int64_t g_ld, const float* w, const float* rstd, const void* dy, void* dx,
+                        void* dg, int64_t dg_ld, float* dw_partial, int64_t n_partials);
+
+/* Between a FoX-Pro layer's stacked projection and its attention: y (B*T, ld) 16-bit rows [q | k | v | output gate |
+ * forget gate (H) | k mix (H) | v mix (H) | pad] with C = H*D columns each; token shift of k and v with the mixing
+ * weights sigmoid(k mix), sigmoid(v mix) (token_shift.py:21-158, ShiftLinear, modeling_forgetting_transformer.py:44-95), then per-head RMSNorm of q
+ * and k (layernorm.py:183-245) with fp32 weights wq, wk (C).  mask (B,T) int64 or NULL: 0 = padding, whose k and v rows
+ * count as zero.  q, k, v: (B*T, C); rstd_q, rstd_k (B*T, H) fp32, both or neither; seq_start (B) or NULL receives
+ * T - sum(mask[b]).  C <= 4096. */
+int fox_mix_fwd(int device, void* stream, int dtype, int64_t B, int64_t T, int64_t H, int64_t D, const void* y, int64_t ld,
+                const float* wq, const float* wk, float eps, const int64_t* mask, void* q, void* k, void* v, float* rstd_q,
+                float* rstd_k, int64_t* seq_start);
+/* Backward: the q, k, v, k mix, v mix and pad columns of dy (B*T, ld), and partial sums (n_partials, C) fp32 of the norm
+ * weights' gradients, n_partials from fox_mix_bwd_partials(B*T). */
+int64_t fox_mix_bwd_partials(int64_t tokens);
+int fox_mix_bwd(int device, void* stream, int dtype, int64_t B, int64_t T, int64_t H, int64_t D, const void* y, int64_t ld,
+                const float* wq, const float* wk, const int64_t* mask, const float* rstd_q, const float* rstd_k,
+                const void* dq, const void* dk, const void* dv, void* dy, float* dwq_partial, float* dwk_partial,
+                int64_t n_partials);
+
+/* Parameters laid out in one launch: up to 8 contiguous 16-bit (mat_rows[i], cols) matrices stacked into (rows, cols),
+ * the rows past them zero; up to 6 vectors (vec_dtype[i]: FOX_DTYPE_*) as fp32, one after another. */
+int fox_pack(int device, void* stream, int64_t n_mats, const void* const* mats, const int64_t* mat_rows, int64_t rows,
+             int64_t cols, void* stack, int64_t n_vecs, const void* const* vecs, const int64_t* vec_len,
+             const int32_t* vec_dtype, float* vecs_out);
+
+/* outs[i][c] = sum over rows of parts[i] (rows[i], cols[i]) fp32, in out_dtype[i]; up to 6 arrays. */
+int fox_column_sums(int device, void* stream, int64_t n, const float* const* parts, const int64_t* rows,
+                    const int64_t* cols, const int32_t* out_dtype, void* const* outs);
 
 /* Row-wise RMSNorm with optional residual add, forward: z = x + residual (fp32; residual may be
  * NULL), residual_out = z rounded to the input dtype (may be NULL), rstd = (mean z^2 + eps)^-1/2,
