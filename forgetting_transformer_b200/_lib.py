@@ -62,6 +62,9 @@ _SIGNATURES = {
                                c_int64, c_int64, c_int64, _F, _F, c_int64, c_int64, c_int64, _F, _F, c_float, _T4P]),
     "fox_attn_decode": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P, _F, _F, _F,
                                 c_float, _T4P, _F, _F, c_int64]),
+    "fox_attn_decode_gates": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P, _F, c_int64,
+                                      c_int64, c_int64, _F, c_float, _T4P, _F, _F, c_int64, c_int]),
+    "fox_attn_decode_splits": (c_int64, [c_int64, c_int64, c_int64]),
     "fox_attn_decode_workspace_floats": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
     "fox_attn_bwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P,
                              _T4P, _F, _F, _F, _F, _F, c_float, _F, _F, _F, _T4P, _T4P, _F]),
@@ -80,6 +83,10 @@ _SIGNATURES = {
     "fox_mix_bwd_partials": (c_int64, [c_int64]),
     "fox_mix_bwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _F, c_int64, _F, _F, _F, _F, _F, _F,
                             _F, _F, _F, _F, _F, c_int64]),
+    "fox_step_product": (c_int, [c_int, c_void_p, c_int, c_int, c_int, c_int64, c_int64, _F, c_int, _F, c_int, c_float, c_int64,
+                                 _F, c_int64, c_int64, _F, _F, _F, _F, c_int64]),
+    "fox_step_mix": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, _F, c_int64, _F, c_int, _F, c_int, c_float, _F,
+                             c_int, _F, _F, _F, _F, _F, _F, _F, _F, c_int64, c_int64]),
     "fox_pack": (c_int, [c_int, c_void_p, c_int64, _F, _F, c_int64, c_int64, _F, c_int64, _F, _F, _F, _F]),
     "fox_column_sums": (c_int, [c_int, c_void_p, c_int64, _F, _F, _F, _F, _F]),
     "fox_rmsnorm_fwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, _F, _F, _F, c_float, _F, _F, _F]),

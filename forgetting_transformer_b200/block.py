@@ -20,6 +20,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _lib
+from .cache import FgateCache, _LayerStore
 from .norm_gate import FusedGroupNormGated, GroupNorm, RMSNorm
 from .ops import (acp_threshold_from_qk_norm, forgetting_attention, forgetting_attention_from_gate_logits,
                   seq_start_from_attention_mask)
@@ -35,7 +36,7 @@ def _load_host():
     host = _lib.host()
     m = torch.nn.modules.module
     host.set_block_classes(FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear,
-                           m._global_forward_hooks, m._global_forward_pre_hooks, m._global_backward_hooks,
+                           FgateCache, _LayerStore, m._global_forward_hooks, m._global_forward_pre_hooks, m._global_backward_hooks,
                            m._global_backward_pre_hooks)
     _host = host
     return _host
@@ -205,6 +206,10 @@ class FoxProBlock(nn.Module):
         built here (no hooks, replaced submodules or autocast) in one 16-bit dtype; else module by module."""
         if past_key_values is None:
             out = (_host or _load_host()).block(self, hidden_states, attention_mask, self._threshold(hidden_states))
+            if out is not None:
+                return out
+        elif hidden_states.shape[1] == 1:     # a generated token: appended to the cache and taken through the block natively
+            out = (_host or _load_host()).block_step(self, hidden_states, attention_mask, past_key_values, layer_idx)
             if out is not None:
                 return out
         residual = hidden_states

@@ -181,6 +181,22 @@ void attn_backward_launch(const AttnCall& c, const AttnGradCall& g) {
   if (debug_sync()) status_check(dev);
 }
 
+int64_t attn_decode_floats(const AttnShape& s) {
+  return fox_attn_decode_workspace_floats(s.B, s.H, s.D, fox_attn_decode_splits(s.B, s.H, s.N));
+}
+void attn_decode_launch(const AttnCall& c, bool prefix, float* work, bool programmatic) {
+  const AttnShape& s = c.s;
+  const int64_t splits = fox_attn_decode_splits(s.B, s.H, s.N);
+  launch("fox_attn_decode", c.st, [&] {
+    if (prefix)
+      return fox_attn_decode(c.device, c.st, c.code, s.B, s.H, s.N, s.D, &c.q, &c.k, &c.v, c.lam, c.seq_start, c.start, c.sm_scale,
+                             &c.o, c.L, work, splits);
+    return fox_attn_decode_gates(c.device, c.st, c.code, s.B, s.H, s.N, s.D, &c.q, &c.k, &c.v, static_cast<const float*>(c.gate),
+                                 c.gate_st[0], c.gate_st[1], c.gate_st[2], c.seq_start, c.sm_scale, &c.o, c.L, work, splits,
+                                 programmatic);
+  });
+}
+
 // ---------------------------------------------------------------- forward
 static AttnCall call_of(const AttnSaved& r, cudaStream_t st) {
   AttnCall c;
@@ -249,24 +265,12 @@ AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs
   float* thr = pruned ? static_cast<float*>(r.threshold.data_ptr()) : nullptr;
   const int64_t thr_sb = pruned ? r.threshold.stride(0) : 0, thr_sh = pruned ? r.threshold.stride(1) : 0;
   if (M == 1 && !needs_grad) {
-    // generation step: one query row against the cache, no gradients -> split-KV kernels
-    prepare_launch(c, norms, norm_parts, in.threshold.kind, in.threshold.value, thr, thr_sb, thr_sh);
-    int64_t splits = std::max<int64_t>(1, std::min(std::min((N + 511) / 512, (4 * 148 + BH - 1) / BH), int64_t{256}));
-    const int64_t Dk = std::max<int64_t>(D, 64);
-    Tensor q = r.q, k = r.k, v = r.v, o = r.o;
-    if (D < 64) {
-      q = at::constant_pad_nd(q, {0, 64 - D});
-      k = at::constant_pad_nd(k, {0, 64 - D});
-      v = at::constant_pad_nd(v, {0, 64 - D});
-      o = at::empty_like(q);
-    }
-    Tensor work = at::empty({fox_attn_decode_workspace_floats(B, H, Dk, splits)}, in.q.options().dtype(at::kFloat));
-    const fox_tensor4 dq4 = t4(q, hf), dk4 = t4(k, hf), dv4 = t4(v, hf), do4 = t4(o, hf);
-    launch("fox_attn_decode", c.st, [&] {
-      return fox_attn_decode(dev, c.st, c.code, B, H, N, Dk, &dq4, &dk4, &dv4, c.lam, c.seq_start, c.start, c.sm_scale, &do4, c.L,
-                             work.mutable_data_ptr<float>(), splits);
-    });
-    if (D < 64) r.o = o.narrow(3, 0, D).contiguous();
+    // generation step: one query row against the cache, no gradients -> split-KV kernels.  Only a threshold's index scan
+    // (or gate logits) needs the prefix sum; otherwise the decode kernel works from the gates.
+    const bool prefix = pruned || in.gate_is_logit;
+    if (prefix) prepare_launch(c, norms, norm_parts, in.threshold.kind, in.threshold.value, thr, thr_sb, thr_sh);
+    const Tensor work = at::empty({attn_decode_floats(s)}, r.q.options().dtype(at::kFloat));
+    attn_decode_launch(c, prefix, work.mutable_data_ptr<float>(), false);
     return r;
   }
   attn_forward_launch(c, norms, norm_parts, in.threshold.kind, in.threshold.value, thr, thr_sb, thr_sh);

@@ -74,9 +74,12 @@ AttnNorms attn_norms(const AttnShape& s, bool is_auto);
 int64_t attn_blocks(int64_t n);   // tiles of the pruning grid
 
 // norms: attn_norms().floats() floats.  threshold: where kind is not kNone; its (B,H) values for a tensor, or the place
-// that receives them.  splits_work: for a single query without gradients, the decode kernels' workspace.
+// that receives them.
 void attn_forward_launch(const AttnCall& c, const AttnNorms& n, float* norms, Threshold::Kind kind, double threshold_value,
                          float* threshold, int64_t thr_sb, int64_t thr_sh);
+// one query row without gradients; prefix: c.lam (and c.start) have been formed, else the log gates c.gate are used
+int64_t attn_decode_floats(const AttnShape& s);
+void attn_decode_launch(const AttnCall& c, bool prefix, float* work, bool programmatic);
 struct AttnGradCall {
   fox_tensor4 g, dq, dk, dv;         // dout and the gradients
   float* work = nullptr;             // attn_backward_floats()

@@ -16,7 +16,7 @@ namespace foxh {
 
 // ---------------------------------------------------------------- the module tree
 namespace {
-enum Class { kLayerCls, kMlpCls, kRmsCls, kGroupCls, kGatedCls, kShiftCls, kLinearCls, kClasses };
+enum Class { kLayerCls, kMlpCls, kRmsCls, kGroupCls, kGatedCls, kShiftCls, kLinearCls, kCacheCls, kStoreCls, kClasses };
 PyObject* g_classes[kClasses] = {};
 PyObject* g_global_hooks[4] = {};   // torch.nn's global forward / pre / backward / backward pre hooks
 
@@ -25,7 +25,8 @@ PyObject* g_global_hooks[4] = {};   // torch.nn's global forward / pre / backwar
   X(_modules) X(_parameters) X(_forward_hooks) X(_forward_pre_hooks) X(_backward_hooks) X(_backward_pre_hooks) X(forward)     \
   X(weight) X(bias) X(attn_norm) X(attn) X(mlp_norm) X(mlp) X(q_proj) X(k_proj) X(v_proj) X(o_proj) X(fgate_proj)             \
   X(ogate_proj) X(output_norm) X(q_norm) X(k_norm) X(linear) X(shift_proj) X(gate_proj) X(down_proj) X(eps) X(num_heads)      \
-  X(log_pruning_tolerance) X(qk_norm) X(use_k_shift) X(use_v_shift) X(activation) X(is_rms_norm) X(num_groups)
+  X(log_pruning_tolerance) X(qk_norm) X(use_k_shift) X(use_v_shift) X(activation) X(is_rms_norm) X(num_groups)     \
+  X(_layers) X(key_shift_cache) X(value_shift_cache) X(_seen_tokens) X(k) X(v) X(g) X(length)
 #define FOX_DECL(n) PyObject* s_##n;
 FOX_NAMES(FOX_DECL)
 #undef FOX_DECL
@@ -498,8 +499,8 @@ struct BlockBackward : public torch::autograd::Node {
 // ---------------------------------------------------------------- Python entry points
 using namespace foxh;
 
-// set_block_classes(FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear,
-//                   the four global hook dictionaries of torch.nn.modules.module)
+// set_block_classes(FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear, FgateCache,
+//                   its layer store, the four global hook dictionaries of torch.nn.modules.module)
 FOX_PY(py_set_block_classes) {
   HANDLE_TH_ERRORS
 #define FOX_INTERN(n) s_##n = PyUnicode_InternFromString(#n);
@@ -563,6 +564,170 @@ FOX_PY(py_block) {
       node->s = s;
     }
   }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- one generated token
+namespace {
+// Layer i of an FgateCache: its buffers, length and shift states, where a token fits without growing them.
+struct CacheLayer {
+  Tensor k, v, g, k_state, v_state;
+  int64_t length = 0;
+  Mod cache, store;
+};
+bool list_tensor(const Mod& m, PyObject* name, int64_t i, Tensor& t) {
+  PyObject* l = m.get(name);
+  return l && PyList_Check(l) && i < PyList_GET_SIZE(l) && tensor(PyList_GET_ITEM(l, i), t);
+}
+bool open_cache(PyObject* cache, int64_t i, const Tensor& x, const Block& b, CacheLayer& c) {
+  if (reinterpret_cast<PyObject*>(Py_TYPE(cache)) != g_classes[kCacheCls] || i < 0 || !open(cache, c.cache)) return false;
+  PyObject* layers = c.cache.get(s__layers);
+  if (!layers || !PyList_Check(layers) || i >= PyList_GET_SIZE(layers)) return false;
+  PyObject* store = PyList_GET_ITEM(layers, i);
+  if (reinterpret_cast<PyObject*>(Py_TYPE(store)) != g_classes[kStoreCls] || !open(store, c.store)) return false;
+  PyObject* len = c.store.get(s_length);
+  if (!len || !PyLong_Check(len) || !tensor(c.store.get(s_k), c.k) || !tensor(c.store.get(s_v), c.v) || !tensor(c.store.get(s_g), c.g) ||
+      !list_tensor(c.cache, s_key_shift_cache, i, c.k_state) || !list_tensor(c.cache, s_value_shift_cache, i, c.v_state))
+    return false;
+  c.length = PyLong_AsLongLong(len);
+  const int64_t B = x.size(0);
+  auto plain = [&](const Tensor& t, at::ScalarType dt) { return t.scalar_type() == dt && t.is_contiguous() && t.device() == x.device(); };
+  for (const Tensor* t : {&c.k, &c.v})
+    if (!plain(*t, x.scalar_type()) || t->dim() != 4 || t->size(0) != B || t->size(1) != b.H || t->size(3) != b.D) return false;
+  for (const Tensor* t : {&c.k_state, &c.v_state})
+    if (!plain(*t, x.scalar_type()) || t->numel() != B * b.C) return false;
+  const int64_t cap = c.k.size(2);
+  return plain(c.g, at::kFloat) && c.g.dim() == 3 && c.g.size(0) == B && c.g.size(1) == b.H && c.g.size(2) == cap && c.v.size(2) == cap &&
+         c.length + 1 <= cap;
+}
+
+Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheLayer& c) {
+  using B = Block;
+  const c10::cuda::CUDAGuard guard(x_in.device());
+  const at::AutoDispatchBelowADInplaceOrView no_autograd;
+  const int dev = x_in.device().index();
+  const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
+  const int code = dtype_code(x_in.scalar_type());
+  status_poll(dev);
+  const Tensor x = x_in.contiguous();
+  Tensor out = at::empty(x_in.sizes(), x_in.options()), mask64;
+  if (mask.defined()) mask64 = mask.to(at::kLong).contiguous();
+  const int64_t n = x.size(0), C = b.C, H = b.H, D = b.D, N = c.length + 1, cap = c.k.size(2);
+  const AttnShape as{n, H, 1, N, D};
+  const int64_t ld = (4 * C + 3 * H + 3) / 4 * 4;
+  Tensor memory;
+  float *y, *z, *L, *work;
+  uint16_t *q, *o, *act;
+  int64_t* seq;
+  for (char* base = nullptr;;) {   // first the size, then the pieces
+    Arena m{base};
+    y = m.take<float>(n * ld);
+    z = m.take<float>(n * C);
+    L = m.take<float>(n * H);
+    work = m.take<float>(attn_decode_floats(as));
+    q = m.take<uint16_t>(n * C);
+    o = m.take<uint16_t>(n * C);
+    act = m.take<uint16_t>(n * b.inter);
+    seq = m.take<int64_t>(n);
+    if (base) break;
+    memory = at::empty({static_cast<int64_t>(m.used)}, x.options().dtype(at::kByte));
+    base = static_cast<char*>(memory.data_ptr());
+  }
+  auto dt = [&](B::Param p) { return dtype_code(b.p[p].scalar_type()); };
+  auto ptr = [&](B::Param p) { return b.p[p].const_data_ptr(); };
+
+  const B::Param first[] = {B::kQ, B::kK, B::kV, B::kOGate, B::kFGate, B::kKMix, B::kVMix};
+  const void* mats[7];
+  int64_t rows[7];
+  for (int i = 0; i < 7; ++i) {
+    mats[i] = ptr(first[i]);
+    rows[i] = b.p[first[i]].size(0);
+  }
+  launch("fox_step_product", st, [&] {
+    return fox_step_product(dev, st, code, 0, 0, n, C, x.const_data_ptr(), 0, ptr(B::kAttnNorm), dt(B::kAttnNorm), b.attn_eps, 0, nullptr,
+                            0, 7, mats, rows, nullptr, y, ld);
+  });
+  const bool bias = b.p[B::kFBias].defined();
+  launch("fox_step_mix", st, [&] {
+    return fox_step_mix(dev, st, code, n, H, D, y, ld, ptr(B::kQNorm), dt(B::kQNorm), ptr(B::kKNorm), dt(B::kKNorm), b.qk_eps,
+                        bias ? ptr(B::kFBias) : nullptr, bias ? dt(B::kFBias) : 0,
+                        mask64.defined() ? mask64.const_data_ptr<int64_t>() : nullptr, seq, c.k_state.data_ptr(), c.v_state.data_ptr(), q,
+                        c.k.data_ptr(), c.v.data_ptr(), c.g.mutable_data_ptr<float>(), cap, c.length);
+  });
+  AttnCall a;
+  a.device = dev;
+  a.st = st;
+  a.code = code;
+  a.s = as;
+  a.q = fox_tensor4{q, C, D, D};
+  a.o = fox_tensor4{o, C, D, D};
+  a.k = fox_tensor4{c.k.data_ptr(), H * cap * D, cap * D, D};
+  a.v = fox_tensor4{c.v.data_ptr(), H * cap * D, cap * D, D};
+  a.sm_scale = static_cast<float>(1. / std::sqrt(static_cast<double>(D)));
+  a.seq_start = mask64.defined() ? seq : nullptr;
+  a.gate = c.g.data_ptr();
+  a.gate_st[0] = H * cap;
+  a.gate_st[1] = cap;
+  a.gate_st[2] = 1;
+  a.L = L;
+  attn_decode_launch(a, false, work, true);
+  const void* m1[1] = {ptr(B::kO)};
+  const int64_t r1[1] = {C};
+  launch("fox_step_product", st, [&] {
+    return fox_step_product(dev, st, code, 1, 1, n, C, o, 0, ptr(B::kONorm), dt(B::kONorm), b.o_eps, D, y + 3 * C, ld, 1, m1, r1,
+                            x.const_data_ptr(), z, C);
+  });
+  const void* m2[1] = {ptr(B::kGate)};
+  const int64_t r2[1] = {2 * b.inter};
+  launch("fox_step_product", st, [&] {
+    return fox_step_product(dev, st, code, 0, 2, n, C, z, 1, ptr(B::kMlpNorm), dt(B::kMlpNorm), b.mlp_eps, 0, nullptr, 0, 1, m2, r2, nullptr,
+                            act, b.inter);
+  });
+  const void* m3[1] = {ptr(B::kDown)};
+  launch("fox_step_product", st, [&] {
+    return fox_step_product(dev, st, code, 2, 3, n, b.inter, act, 0, nullptr, 0, 0.f, 0, nullptr, 0, 1, m3, r1, z, out.mutable_data_ptr(), C);
+  });
+  return out;
+}
+}  // namespace
+
+// block_step(self, hidden_states (B, 1, hidden), attention_mask (B, N + 1) or None, cache, layer_idx) -> out, with the token
+// appended to the cache, or None where the modules' own forward has to run
+FOX_PY(py_block_step) {
+  HANDLE_TH_ERRORS
+  Tensor x;
+  Block b;
+  CacheLayer c;
+  const int64_t layer = PyLong_AsLongLong(args[4]);
+  if (PyErr_Occurred()) throw python_error();
+  if (!tensor(args[1], x) || x.dim() != 3 || x.size(1) != 1 || x.size(0) < 1 || x.size(0) > 16 || !read_block(args[0], x, b) || b.pruned ||
+      b.inter % 32 || x.size(0) * (std::max(b.C, b.inter) / 8 + 12) * 16 > 200 * 1024 || !open_cache(args[3], layer, x, b, c))
+    Py_RETURN_NONE;
+  if (at::GradMode::is_enabled()) {
+    bool needs = x.requires_grad();
+    for (const Tensor& t : b.p) needs = needs || (t.defined() && t.requires_grad());
+    if (needs) Py_RETURN_NONE;
+  }
+  const Tensor mask = unpack_opt(args[2], "attention_mask");
+  if (mask.defined()) {
+    const auto d = mask.scalar_type();
+    if (mask.dim() != 2 || mask.size(0) != x.size(0) || mask.size(1) != c.length + 1 || mask.device() != x.device() ||
+        (d != at::kLong && d != at::kBool && d != at::kInt))
+      Py_RETURN_NONE;
+  }
+  Tensor out;
+  {
+    pybind11::gil_scoped_release no_gil;
+    out = step(b, x, mask, c);
+  }
+  auto set = [](const Mod& m, PyObject* name, int64_t v) {
+    PyObject* n = PyLong_FromLongLong(v);
+    PyDict_SetItem(m.dict, name, n);
+    Py_DECREF(n);
+  };
+  set(c.store, s_length, c.length + 1);
+  if (layer == 0) set(c.cache, s__seen_tokens, static_cast<int64_t>(c.cache.number(s__seen_tokens)) + 1);
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }

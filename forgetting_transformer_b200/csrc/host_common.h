@@ -104,3 +104,4 @@ FOX_PY(py_attention_forward);
 FOX_PY(py_attention_backward);
 FOX_PY(py_set_block_classes);
 FOX_PY(py_block);
+FOX_PY(py_block_step);

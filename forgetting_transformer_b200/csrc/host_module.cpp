@@ -172,6 +172,7 @@ static PyMethodDef g_methods[] = {
     FOX_METHOD("attention_backward", py_attention_backward),
     FOX_METHOD("set_block_classes", py_set_block_classes),
     FOX_METHOD("block", py_block),
+    FOX_METHOD("block_step", py_block_step),
     {nullptr, nullptr, 0, nullptr}};
 static PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_fox_host", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

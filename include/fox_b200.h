@@ -164,6 +164,14 @@ int fox_attn_decode(int device, void* stream, int dtype, int64_t B, int64_t H, i
                     const int64_t* seq_start, const int64_t* start_index, float sm_scale, const fox_tensor4* o,
                     float* L, float* workspace, int64_t splits);
 int64_t fox_attn_decode_workspace_floats(int64_t B, int64_t H, int64_t D, int64_t splits);
+/* The same from the log gates (fp32, element strides sb, sh, sn) instead of their prefix sum, without pruning.
+ * splits for both from fox_attn_decode_splits; D in {16,32,64,128}.  programmatic != 0: launched with programmatic stream
+ * serialization behind another kernel of this library. */
+int fox_attn_decode_gates(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t N, int64_t D,
+                          const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v, const float* log_fgate,
+                          int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float sm_scale,
+                          const fox_tensor4* o, float* L, float* workspace, int64_t splits, int programmatic);
+int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N);
 
 /* delta[b,h,m] = sum_d o[b,h,m,d] * d_o[b,h,m,d] in fp32: replaces _bwd_preprocess
  * (forgetting_attention.py:267-277, kernel 902-943). */
@@ -267,6 +275,23 @@ int fox_pack(int device, void* stream, int64_t n_mats, const void* const* mats, 
 /* outs[i][c] = sum over rows of parts[i] (rows[i], cols[i]) fp32, in out_dtype[i]; up to 6 arrays. */
 int fox_column_sums(int device, void* stream, int64_t n, const float* const* parts, const int64_t* rows,
                     const int64_t* cols, const int32_t* out_dtype, void* const* outs);
+
+/* One generated token through a FoX-Pro block (B <= 16 sequences; programmatic stream serialization throughout).
+ * fox_step_product: out = f(in(x) W^T) for up to 7 contiguous 16-bit matrices (mat_rows[i], K), K a multiple of 32, their
+ * outputs side by side.  input 0: rmsnorm(x) norm_w, x (B,K) 16-bit or (x_fp32) fp32; 1: per-head rmsnorm(x) norm_w
+ * sigmoid(gate), head dim D, gate fp32 with row stride gate_ld; 2: x.  output 0: fp32 (B,ldo); 1: fp32, + residual
+ * (16-bit); 2: silu(first half) * second half of one matrix's rows, 16-bit; 3: 16-bit, + residual (fp32). */
+int fox_step_product(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K, const void* x,
+                     int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D, const float* gate,
+                     int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
+                     const void* residual, void* out, int64_t ldo);
+/* y (B,ld) fp32 as fox_mix_fwd's rows: token shift with the states k_state, v_state (B,C) 16-bit, which are replaced by
+ * this token's projections, norms of q and k, and row pos of the caches k, v (B,H,capacity,D), log gates (B,H,capacity);
+ * mask (B,pos+1) int64 or NULL: seq_start (B) receives pos + 1 - its sum. */
+int fox_step_mix(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t D, const float* y, int64_t ld,
+                 const void* wq, int wq_dtype, const void* wk, int wk_dtype, float eps, const void* bias, int bias_dtype,
+                 const int64_t* mask, int64_t* seq_start, void* k_state, void* v_state, void* q, void* k_cache,
+                 void* v_cache, float* g_cache, int64_t capacity, int64_t pos);
 
 /* Row-wise RMSNorm with optional residual add, forward: z = x + residual (fp32; residual may be
  * NULL), residual_out = z rounded to the input dtype (may be NULL), rstd = (mean z^2 + eps)^-1/2,

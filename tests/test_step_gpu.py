@@ -1,0 +1,105 @@
+"""Single-token kernels: the split-KV decode from the gates at the sizes where its ranges, tiles and batches end, and a
+generated token through a block against the modules' own path."""
+import pytest
+import torch
+
+import forgetting_transformer_b200 as fox
+from forgetting_transformer_b200 import _lib
+from oracle import fox_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,N,D", [(1, 2, 1, 64), (1, 1, 127, 16), (2, 3, 129, 32), (1, 1, 1025, 128), (3, 148, 1023, 64),
+                                     (1, 5, 4097, 128), (1, 1, 70000, 64)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_decode_from_gates(B, H, N, D, padded):
+    """out of one query row against the dense fp32 formulation; (B, N, H) gates and permuted keys.  bf16 rounds the
+    result once and takes fp32 products otherwise: every element within 2^-8 of its value and of the row's scale."""
+    g = torch.Generator().manual_seed(N + D)
+    q, k, v = [torch.randn(B, t, H, D, generator=g).bfloat16().cuda() for t in (1, N, N)]
+    lf = torch.nn.functional.logsigmoid(torch.randn(B, N, H, generator=g) + 3).cuda()
+    seq = torch.randint(0, max(1, N // 2), (B,), generator=g).cuda() if padded else None
+    with torch.no_grad():
+        out = fox.forgetting_attention(q, k, v, lf, seq_start=seq)
+    lam = lf.double().cumsum(1)
+    s = torch.einsum("bqhd,bnhd->bhn", q.double(), k.double()) / D ** 0.5 + (lam[:, -1:] - lam).transpose(1, 2)
+    if padded:
+        s.masked_fill_(torch.arange(N, device="cuda")[None, None, :] < seq[:, None, None], float("-inf"))
+    ref = torch.einsum("bhn,bnhd->bhd", s.softmax(-1), v.double())[:, None]
+    err = (out.double() - ref).abs()
+    assert (err <= 2 ** -8 * ref.abs() + 2 ** -8 * ref.pow(2).mean().sqrt()).all(), err.max().item()
+
+
+@pytest.mark.parametrize("B,C,H,I,N", [(1, 256, 4, 512, 1), (2, 512, 4, 1408, 130), (9, 768, 12, 2048, 64), (16, 256, 2, 96, 300)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("padded", [False, True])
+def test_token_through_block_matches_modules(B, C, H, I, N, dtype, padded):
+    """block_step against the same modules called one by one (a forward hook turns the native path off): three tokens;
+    output, cache rows and shift states.  The module path rounds every intermediate to 16 bits: 8 roundings of relative
+    size 2^-9 (bf16) or 2^-12 (fp16) in series bound the difference by about 2^-6 and 2^-9 of the scale."""
+    torch.manual_seed(B + C)
+    blk = fox.FoxProBlock(C, H, I, fgate_bias=2.0).cuda().to(dtype)
+    with torch.no_grad():
+        for m in (blk.attn_norm, blk.mlp_norm, blk.attn.q_norm, blk.attn.k_norm, blk.attn.output_norm):
+            m.weight.uniform_(0.5, 1.5)
+    xs = torch.randn(3, B, 1, C, device="cuda").to(dtype)
+    k, v = torch.randn(2, B, H, N, C // H, device="cuda").to(dtype)
+    g = torch.nn.functional.logsigmoid(torch.randn(B, H, N, device="cuda") + 3)
+    mask = None
+    if padded:
+        mask = torch.ones(B, N + 3, dtype=torch.long, device="cuda")
+        mask[0, :N // 3] = 0
+    res = []
+    for native in (True, False):
+        cache = fox.FgateCache(granule=128)
+        st = blk.attn.init_shift_state(B)
+        for i, t in enumerate(st.values()):
+            t.copy_(torch.linspace(-1 + i, 1, t.numel(), device="cuda").view_as(t))
+        cache.update_shift_cache(st["key_shift"], st["value_shift"], 0)
+        cache.update(k, v, g, 0)
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        with torch.no_grad():
+            outs = [blk(x, None if mask is None else mask[:, :N + 1 + i], cache, 0) for i, x in enumerate(xs)]
+        if hook is not None:
+            hook.remove()
+        assert cache.get_seq_length() == N + 3 and cache._seen_tokens == N + 3
+        res.append(outs + [t.clone() for t in cache[0]] + [st["key_shift"].clone(), st["value_shift"].clone()])
+    torch.cuda.synchronize()
+    _lib.check_status()
+    tol = 2 ** -6 if dtype == torch.bfloat16 else 2 ** -9
+    for a, b in zip(*res):
+        a, b = a.float(), b.float()
+        assert (a - b).abs().max() <= tol * (b.abs().max() + 1)
+        assert (a - b).norm() <= tol * b.norm()
+
+
+@pytest.mark.parametrize("B,T,C,H", [(1, 2, 256, 16), (2, 129, 512, 4), (3, 17, 768, 12)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_block_native_matches_modules(B, T, C, H, padded):
+    """The block as one autograd node against its modules one by one, fp16: output, input gradient and every parameter's.
+    Both round intermediates to 11 bits at a dozen points: relative error of a tensor below 12 * 2^-12."""
+    torch.manual_seed(T)
+    blk = fox.FoxProBlock(C, H, 2 * C, fgate_bias=2.0).cuda().to(torch.float16)
+    x = torch.randn(B, T, C, device="cuda").half().requires_grad_()
+    dy = torch.randn(B, T, C, device="cuda").half()
+    mask = None
+    if padded:
+        mask = torch.ones(B, T, dtype=torch.bool, device="cuda")
+        mask[0, :T // 3] = False
+    res = []
+    for native in (True, False):
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        x.grad = None
+        blk.zero_grad(set_to_none=True)
+        out = blk(x, mask)
+        assert ("FoxProBlockBackward" in out.grad_fn.name()) == native
+        out.backward(dy)
+        res.append([("out", out.detach()), ("x", x.grad)] + [(n, p.grad) for n, p in blk.named_parameters()])
+        if hook is not None:
+            hook.remove()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for (n, a), (_, b) in zip(*res):
+        a, b = a.float(), b.float()
+        assert a.shape == b.shape and (a - b).norm() <= 12 * 2 ** -12 * b.norm() + 1e-6, (n, ((a - b).norm() / b.norm()).item())
