@@ -14,7 +14,8 @@
 //   last warp          : tcgen05.mma issuer (one elected lane)
 // TMEM: S = Q K^T fp32 in columns [0,BN); each slice's probabilities are written back over the slice's own
 // S columns as packed 16-bit pairs and consumed as the TMEM A operand of P V; O_g accumulates in columns
-// [BN + g D, BN + (g+1) D).  D = 64: BN = 128, NWG = 2 (256 columns); D = 128: BN = 128, NWG = 1 (256 columns).
+// [BN + g D, BN + (g+1) D).  D = 64: BN = 128, NWG = 2 (256 columns); D = 128: BN = 64, NWG = 1 and two S buffers
+// (S in columns [0, 64) and [64, 128), O in [128, 256)).
 //
 // KV tiles are visited from the diagonal leftwards: with forget gates the
 // largest logits sit next to the diagonal, so the running row maximum is found
@@ -48,13 +49,14 @@ struct FwdParams {
   int n_norm_parts;            // <= 32
 };
 
-// How many of every 4 column pairs take the FMA-pipe exponential instead of the ex2 unit (measured best:
-// a quarter at D=64, where four softmax warps share a scheduler, half at D=128 with two).
+// How many of every 4 column pairs take the FMA-pipe exponential instead of the ex2 unit (measured best
+// at both head dims: a quarter.  At D=128, B4 H16 T16384: none 4.62, a quarter 4.60, half 4.77 ms; the FMA pipe's
+// form takes five times the issue slots, and at the power cap instructions are what costs).
 #ifndef FOX_POLYQ64
 #define FOX_POLYQ64 1
 #endif
 #ifndef FOX_POLYQ128
-#define FOX_POLYQ128 2
+#define FOX_POLYQ128 1
 #endif
 
 // Debug builds with -DFOX_FWD_TRACE record clock64 stamps of CTA (0,0,0), tiles 32..47:
@@ -71,7 +73,7 @@ enum FwdWaitSite {
   kSiteSFull = 16, kSitePFull = 17, kSiteODone = 18, kSiteDrain = 19, kSiteNegB = 20, kSiteMerge = 21, kSiteEpi = 22
 };
 
-template <int D, bool kBf16, int BN, int STAGES, int CTAS, int NWG, bool PREF>
+template <int D, bool kBf16, int BN, int STAGES, int CTAS, int NWG, int SB, bool PREF>
 __global__ void __launch_bounds__(128 * NWG + 64, CTAS)
 fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -81,6 +83,9 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // running maximum, row sum and O accumulator (independent online-softmax streams, merged in the
   // epilogue), so that several softmax warps per scheduler hide each other's ex2 / TMEM latency without
   // any exchange between the warpgroups inside the loop.
+  // SB = 2: two S buffers, so that the product for tile t + 1 is complete when the softmax of tile t ends and the
+  // products of one buffer (P V of tile t, S of tile t + 2) run under the softmax of the other.
+  static_assert(SB == 1 || (SB == 2 && NWG == 1 && STAGES == 2), "two S buffers: one warpgroup, two K / V stages");
   constexpr int kWG = NWG;
   constexpr int CW = BN / kWG;              // columns per softmax thread
   constexpr int kQBytes = 128 * D * 2;      // Q tile: D/64 swizzled [128][64] sub-tiles
@@ -88,14 +93,14 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr int kSubBytes = BN * 128;       // one K / V sub-tile
   constexpr int kSub = D / 64;
   constexpr uint32_t kFmt = kBf16 ? 1u : 0u;
-  constexpr uint32_t kColO = BN;            // S (fp32) in columns [0, BN), O_g in [BN + g D, BN + (g+1) D)
+  constexpr uint32_t kColO = SB * BN;       // S (fp32) in columns [0, SB BN), O_g in [SB BN + g D, SB BN + (g+1) D)
   constexpr uint32_t kTmemCols = (kColO + kWG * D <= 128) ? 128 : ((kColO + kWG * D <= 256) ? 256 : 512);
   static_assert(kColO + kWG * D <= 512, "TMEM budget");
   constexpr int kTmaWarp = 4 * kWG, kMmaWarp = 4 * kWG + 1;
 
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_q_full, bar_o_done, bar_merge, bar_epi;
-  __shared__ uint64_t bar_s_full[NWG], bar_p_full[NWG];  // per warpgroup
+  __shared__ uint64_t bar_s_full[NWG * SB], bar_p_full[NWG * SB];  // per warpgroup and S buffer
   __shared__ uint64_t bar_k_full[STAGES], bar_k_empty[STAGES], bar_v_full[STAGES], bar_v_empty[STAGES];
   // -b_j = -Lambda_j log2(e) of a tile's columns and the maximum over each warpgroup's slice, staged by the
   // producer warp one tile ahead in a ring of three (slot of tile t is reused for t+3, which the producer
@@ -133,7 +138,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&bar_q_full, 1);
-    for (int g = 0; g < NWG; ++g) {
+    for (int g = 0; g < NWG * SB; ++g) {
       mbar_init(&bar_s_full[g], 1);
       mbar_init(&bar_p_full[g], 128);
     }
@@ -171,7 +176,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int s = 0; s < kSub; ++s) tma_load_4d(sQ + s * 16384, &tmQ, &bar_q_full, s * 64, mb * kFwdBM, h, b);
       }
       __syncwarp();
-      int issued = 0;
+      int issued_k = 0, issued_v = 0;
       // K(it), V(it) per tile, each into stage it % STAGES once the product that read its previous
       // occupant has retired
       auto load_kv = [&](bool is_v, int it) -> bool {
@@ -190,6 +195,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             tma_load_4d((is_v ? sV : sK) + st * kTileBytes + s * kSubBytes, is_v ? &tmV : &tmK, full, s * 64, nb * BN, h, b);
         }
         __syncwarp();
+        (is_v ? issued_v : issued_k) = it + 1;
         return true;
       };
       // gate prefixes of a tile's columns: lane l holds columns 4l .. 4l+3 (lanes < BN/4)
@@ -220,11 +226,16 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       fetch_lam(0);
       stage_negb(0);
       if (n_tiles > 1) fetch_lam(1);
-      for (int it = 0; it < n_tiles; ++it) {
-        if (!load_kv(false, it)) break;
-        ++issued;
+      // (in the order in which the issuer needs them: with two S buffers K runs two tiles ahead of V)
+      bool fed = true;
+      if (SB == 2) {
+        fed = load_kv(false, 0);
+        if (n_tiles > 1) fed = fed && load_kv(false, 1);
+      }
+      for (int it = 0; it < n_tiles && fed; ++it) {
+        if (SB == 1 && !load_kv(false, it)) break;
         if (!load_kv(true, it)) break;  // waits for O += P V of tile it-STAGES
-        ++issued;
+        if (SB == 2 && it + 2 < n_tiles && !load_kv(false, it + 2)) break;
         if (it + 1 < n_tiles) {
           stage_negb(it + 1);
           if (it + 2 < n_tiles) fetch_lam(it + 2);
@@ -236,15 +247,12 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const long long t0 = clock64();
         while (!mbar_try_wait(&bar_q_full, 0) && clock64() - t0 < 200000000LL) {
         }
-        const int last = (issued + 1) / 2;  // tiles with at least one copy issued
-        for (int it = max(last - STAGES - 1, 0); it < last; ++it) {
-          const int st = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          while (!mbar_try_wait(&bar_k_full[st], ph) && clock64() - t0 < 200000000LL) {
+        for (int it = max(issued_k - STAGES, 0); it < issued_k; ++it)
+          while (!mbar_try_wait(&bar_k_full[it % STAGES], (it / STAGES) & 1) && clock64() - t0 < 200000000LL) {
           }
-          while (!mbar_try_wait(&bar_v_full[st], ph) && clock64() - t0 < 200000000LL) {
+        for (int it = max(issued_v - STAGES, 0); it < issued_v; ++it)
+          while (!mbar_try_wait(&bar_v_full[it % STAGES], (it / STAGES) & 1) && clock64() - t0 < 200000000LL) {
           }
-        }
       }
     }
   } else if (warp == kMmaWarp) {
@@ -256,7 +264,53 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const uint64_t dK0 = umma_desc_kmajor(smem_u32(sK));
       const uint64_t dV0 = umma_desc_mnmajor(smem_u32(sV), kSubBytes);
       bool ok = mbar_wait_warp(&bar_q_full, 0, abortp, p.status, kSiteQFull);
-      {
+      if constexpr (SB == 2) {
+        // order: S(0) S(1) | PV(0) S(2) | PV(1) S(3) | ...; S(t + 2) takes the columns of S(t) / P(t) right behind the
+        // P V product that reads them
+        constexpr uint32_t idQK = umma_idesc(kFmt, 128, BN, 0, 0);
+        auto issue_s = [&](int t) -> bool {
+          if (!mbar_wait_warp(&bar_k_full[t & 1], (t >> 1) & 1, abortp, p.status, kSiteKFull, t)) return false;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t dK = umma_desc_advance(dK0, (t & 1) * kTileBytes);
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk)
+              mma_ss_raw(tbase + (t & 1) * BN, umma_desc_advance(dQ, (kk >> 2) * 16384 + (kk & 3) * 32),
+                         umma_desc_advance(dK, (kk >> 2) * kSubBytes + (kk & 3) * 32), idQK, kk > 0);
+            tc_commit_raw(&bar_s_full[t & 1]);
+            tc_commit_raw(&bar_k_empty[t & 1]);
+          }
+          __syncwarp();
+          return true;
+        };
+        ok = ok && issue_s(0);
+        if (n_tiles > 1) ok = ok && issue_s(1);
+        for (int it = 0; it < n_tiles && ok; ++it) {
+          const int bf = it & 1;
+          const uint32_t ph = (it >> 1) & 1;
+          STAMP(8, 0, it);
+          ok = mbar_wait_warp(&bar_v_full[bf], ph, abortp, p.status, kSiteVFull, it);
+          STAMP(8, 1, it);
+          ok = ok && mbar_wait_warp(&bar_p_full[bf], ph, abortp, p.status, kSitePFull, it);
+          if (!ok) break;
+          STAMP(8, 2, it);
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t dV = umma_desc_advance(dV0, bf * kTileBytes);
+#pragma unroll
+            for (int kk = 0; kk < BN / 16; ++kk)
+              mma_ts_raw(tbase + kColO, tbase + bf * BN + kk * 8, umma_desc_advance(dV, kk * 2048), idPV,
+                         (it > 0 || kk > 0) ? 1u : 0u);
+            tc_commit_raw(&bar_v_empty[bf]);
+            // (past the last tile the barrier only tells a thread that rescales O that P V has retired)
+            if (it + 2 >= n_tiles) tc_commit_raw(&bar_s_full[bf]);
+          }
+          __syncwarp();
+          STAMP(8, 3, it);
+          if (it + 2 < n_tiles) ok = issue_s(it + 2);
+          STAMP(8, 4, it);
+        }
+      } else {
         // Every softmax warpgroup g has its own chain S_g -> P_g -> O_g += P_g V_g -> S_g(next tile): the S
         // product is issued per column slice right behind the P V product that frees the slice, so a
         // warpgroup never waits for the other one.
@@ -328,7 +382,6 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const float* lam = p.lam + bh * N;
     const float a_i = row_ok ? (lam[P + row] - lam[min(P + mb * kFwdBM, N - 1)]) * kLog2e : 0.f;  // (see the producer)
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t tS = tbase + lane_base + g * CW;
     const uint32_t tO = tbase + lane_base + kColO + g * D;
 
     float m_ref = -INFINITY, l_sum = 0.f;
@@ -364,9 +417,12 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int it = 0; it < n_tiles && ok; ++it) {
       const int nb = nb_hi - 1 - it;
       const int col0 = nb * BN + g * CW;  // first column of this thread's slice
+      const int sb = (SB == 2) ? (it & 1) : 0;
+      const uint32_t s_par = (SB == 2) ? ((it >> 1) & 1) : (it & 1);
+      const uint32_t tS = tbase + lane_base + sb * BN + g * CW;
       STAMP(warp & 7, 0, it);
       ok = mbar_wait(&bar_negb[it % 3], (it / 3) & 1, abortp, p.status, kSiteNegB, it);
-      ok = mbar_wait(&bar_s_full[g], it & 1, abortp, p.status, kSiteSFull, it) && ok;
+      ok = mbar_wait(&bar_s_full[g * SB + sb], s_par, abortp, p.status, kSiteSFull, it) && ok;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       STAMP(warp & 7, 1, it);
@@ -429,6 +485,14 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (__any_sync(0xffffffffu, need)) {
           const float alpha = (m_new == -INFINITY) ? 1.f : fast_exp2(m_ref - m_new);
           l_sum *= alpha;
+          // With two S buffers S(it) may be complete while O += P V of tile it-1 still runs; S(it+1) is issued (or, at
+          // the end, its barrier committed) right behind that product.
+          if (SB == 2 && it > 0) {
+            ok = mbar_wait(&bar_s_full[sb ^ 1], ((it + 1) >> 1) & 1, abortp, p.status, kSiteSFull, it);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+          }
           if (it > 0) {
             const float2 alpha2 = make_float2(alpha, alpha);
 #pragma unroll
@@ -479,7 +543,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       STAMP(warp & 7, 4, it);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bar_p_full[g]);
+      mbar_arrive(&bar_p_full[g * SB + sb]);
       STAMP(warp & 7, 5, it);
     }
 
@@ -571,9 +635,13 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == kTmaWarp) tmem_dealloc(tbase, kTmemCols);
 }
 
-// Shapes: D=64 -> 128-row KV tiles in two stages, two softmax warpgroups with independent streams;
-// D=128 -> 128-row KV tiles in a single K and a single V buffer (K is free again once S is computed, V once
-// P V is, so the next tile's copies overlap the softmax), one softmax warpgroup, S chunks prefetched.
+// Shapes: D=64 -> 128-row KV tiles in two stages, two softmax warpgroups with independent streams.
+// D=128 -> 64-row KV tiles in two K and two V stages, one softmax warpgroup, two S buffers.  With 128-row tiles and one
+// S buffer a softmax warp waited 1400 of 3700 cycles per tile for P V and the next S, which cannot start before its
+// own P is there; with the tile cut in two halves that take turns it waits 280 of 2060 per half tile (clock stamps),
+// and what is left is the exponential pass.  The 64-column S product costs more shared-memory reads of Q per column,
+// which the wait paid for: B4 H16 T16384, sustained at the power cap, 4.74 -> 4.60 ms (956 TFLOP/s); first launches on a
+// cool chip 4.62 -> 4.2 ms.
 #ifdef FOX_DEBUG
 // Debug builds (-DFOX_DEBUG) only, tuning hook: 1 = D=64 with one warpgroup, 2 = D=128 with 64-row KV tiles in two stages.
 static int g_fwd_variant = 0;
@@ -584,7 +652,7 @@ extern "C" int fox_debug_read_fwd_trace(long long* host) {
 }
 #endif
 
-template <bool kBf16, int D, int BN, int STAGES, int CTAS, int NWG, bool PREF>
+template <bool kBf16, int D, int BN, int STAGES, int CTAS, int NWG, int SB, bool PREF>
 static int launch_fwd_t(int device, cudaStream_t stream, int64_t B, int64_t H, int64_t M, int64_t N, const fox_tensor4* q,
                       int64_t Dt, const fox_tensor4* k, const fox_tensor4* v, const FwdParams& prm) {
   // Dt <= D: the tensors' own head dim.  The boxes are D columns wide all the same: the TMA unit fills the columns
@@ -603,7 +671,7 @@ static int launch_fwd_t(int device, cudaStream_t stream, int64_t B, int64_t H, i
   if (!tma_compatible(to, 2)) return FOX_ERR_ALIGNMENT;
   if ((rc = cached_tmap_4d(&tmO, to, 2, false, kBf16, 64, 128, true))) return rc;
   constexpr int smem = 128 * D * 2 + 2 * STAGES * BN * D * 2 + 1024;
-  auto kern = fox_attn_fwd_kernel<D, kBf16, BN, STAGES, CTAS, NWG, PREF>;
+  auto kern = fox_attn_fwd_kernel<D, kBf16, BN, STAGES, CTAS, NWG, SB, PREF>;
   static bool configured[64] = {};  // per template instance and device
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;
   if (!configured[device]) {
@@ -675,12 +743,12 @@ extern "C" int fox_attn_fwd_parts(int device, void* stream, int dtype, int64_t B
 #endif
 #define FOX_FWD_LAUNCH(...) \
   (bf ? launch_fwd<__VA_ARGS__>(device, st, B, H, M, N, q, D, k, v, prm) : launch_fwd_fp16<__VA_ARGS__>(device, st, B, H, M, N, q, D, k, v, prm))
-  //                 D  BN  STAGES CTAS NWG PREF
+  //                 D  BN  STAGES CTAS NWG SB PREF
 #ifdef FOX_DEBUG
-  if (D == 64 && variant == 1) return FOX_FWD_LAUNCH(64, 128, 2, 2, 1, false);
-  if (D == 128 && variant == 2) return FOX_FWD_LAUNCH(128, 64, 2, 2, 1, false);
+  if (D == 64 && variant == 1) return FOX_FWD_LAUNCH(64, 128, 2, 2, 1, 1, false);
+  if (D == 128 && variant == 2) return FOX_FWD_LAUNCH(128, 128, 1, 2, 1, 1, true);
 #endif
-  if (D <= 64) return FOX_FWD_LAUNCH(64, 128, 2, 2, 2, false);
-  return FOX_FWD_LAUNCH(128, 128, 1, 2, 1, true);
+  if (D <= 64) return FOX_FWD_LAUNCH(64, 128, 2, 2, 2, 1, false);
+  return FOX_FWD_LAUNCH(128, 64, 2, 2, 1, 2, true);
 #undef FOX_FWD_LAUNCH
 }
