@@ -2,6 +2,8 @@
 applied to q and k (upstream layernorm.py:993-1051 as built at modeling_forgetting_transformer.py:264-265)
 and the data-dependent token shift (token_shift.py), against the oracle and against the fixtures
 produced by upstream's own code (tests/golden/glue_refs.npz)."""
+import math
+
 import pytest
 import torch
 
@@ -296,3 +298,49 @@ def test_cross_entropy_against_upstream_kernels_and_oracle(inplace):
     assert _err(x.grad.cpu(), rd) < 4e-3 * rd.abs().max().item()     # one bf16 rounding of the gradient
     mean = fox.FusedCrossEntropyLoss()(logits.cuda(), labels.cuda())
     assert abs(mean.item() - (orc.cross_entropy(logits, labels)[0].sum() / (labels != -100).sum()).item()) < 1e-4
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [1, 5, 8 * 255, 8 * 1024 - 1, 8 * 1024 + 8, 4 * 4096 + 3])
+def test_cross_entropy_at_the_edges_of_its_steps(cols, dtype):
+    """Row lengths around a CTA's step (256 threads x 4 pieces of 16 bytes), classes masked with -inf (whole pieces of
+    them too), rows without a target or without a gradient, label smoothing: against float64."""
+    g = torch.Generator().manual_seed(cols)
+    rows, eps, scale = 9, 0.1, 0.7
+    x = (torch.randn(rows, cols, generator=g) * 3).to(dtype)
+    labels = torch.randint(0, cols, (rows,), generator=g)
+    labels[2] = -100
+    w = torch.rand(rows, generator=g)
+    w[4] = 0.0
+    for smooth in (0.0, eps):
+        x1 = x.clone()
+        if smooth == 0.0 and cols > 64:
+            x1[:, :cols // 2] = -math.inf
+            labels = labels.where(labels == -100, cols - 1 - labels % 3)
+        z = x1.double().requires_grad_()
+        logp = torch.log_softmax(z * scale, -1)
+        keep = labels != -100
+        nll = -logp.gather(1, labels.where(keep, cols - 1)[:, None])[:, 0]
+        ref = ((1 - smooth) * nll - (smooth * logp.mean(-1) if smooth else 0.0)) * keep
+        (ref * w).sum().backward()
+        xc = x1.cuda().requires_grad_()
+        loss, _ = fox.cross_entropy_loss(xc, labels.cuda(), smooth, scale)
+        (loss * w.cuda()).sum().backward()
+        # fp32 sums of up to 16 K terms in pairs, ex2 to 2 ulp; the gradient is rounded once to the logits' type
+        assert _err(loss.double().cpu(), ref.detach()) < 2e-5
+        ulp = {torch.float32: 2e-6, torch.bfloat16: 2 ** -8, torch.float16: 2 ** -10}[dtype]
+        zg = z.grad.nan_to_num(0.0)     # (float64 gives 0 * NaN nowhere here; masked classes have gradient 0)
+        assert (xc.grad.double().cpu() - zg).abs().le(zg.abs() * ulp + 2e-6).all()
+
+
+def test_cross_entropy_gradient_of_rows_that_are_not_finite():
+    """A row with a zero gradient is not read, unless its log-sum-exp says that a logit is NaN or infinite: its gradient
+    is then NaN, as the products give."""
+    x = torch.zeros(4, 4096, device="cuda", dtype=torch.bfloat16)
+    x[1, 100], x[2, 7] = math.nan, math.inf
+    x.requires_grad_()
+    loss, _ = fox.cross_entropy_loss(x, torch.full((4,), -100, device="cuda"))
+    assert (loss == 0).all()
+    loss.sum().backward()
+    assert (x.grad[0] == 0).all() and (x.grad[3] == 0).all()
+    assert x.grad[1, 100].isnan() and x.grad[2, 7].isnan()
