@@ -64,8 +64,13 @@ __device__ __forceinline__ void mix_load(const MixParams& p, int64_t t, bool on,
   }
 }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(512) fox_mix_fwd_kernel(const MixParams p) {
+// kThreads: 256 (rows of up to 2048 channels) or 512.  One CTA of 192 threads per 3 tokens' loads in flight is too little to
+// cover the chain load - sum over a head's lanes - store, so the narrow form takes one token at a time in 64 registers and
+// has 5 CTAs per SM, where two tokens in 116 registers left 2: 16384 x 1536 bf16 96 -> 71.5 us (4.2 TB/s), 2048 x 768 7.5 ->
+// 7.3 us.  (Two tokens in 80 registers: 67 and 8.1 us; one in 48 registers: 91 and 9.5 us; 4 channels a thread, which doubles
+// the instructions for addresses and sums: 199 and 13 us.)
+template <bool kBf16, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) fox_mix_fwd_kernel(const MixParams p) {
   if (static_cast<int>(blockIdx.x) >= p.mix_blocks) {
     __shared__ unsigned long long s_sum;
     const int b = blockIdx.x - p.mix_blocks;
@@ -92,8 +97,9 @@ __global__ void __launch_bounds__(512) fox_mix_fwd_kernel(const MixParams p) {
   }
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * p.rows, t1 = min(t0 + p.rows, p.tokens);
   uint4 kp, vp;
-  mix_load(p, t0 - 1, active && t0 % p.T != 0, ch, C, kp, vp);
-  constexpr int kU = 2;   // tokens whose loads are in flight together
+  int pos = static_cast<int>(t0 % p.T);   // of the token in its sequence
+  mix_load(p, t0 - 1, active && pos != 0, ch, C, kp, vp);
+  constexpr int kU = kThreads == 256 ? 1 : 2;   // tokens whose loads are in flight together
   for (int64_t tb = t0; tb < t1; tb += kU) {
     uint4 qr[kU], kr[kU], vr[kU];
     float ak[kU], av[kU];
@@ -114,7 +120,8 @@ __global__ void __launch_bounds__(512) fox_mix_fwd_kernel(const MixParams p) {
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int64_t t = tb + u;
-      const bool first = t % p.T == 0;   // no token before it
+      const bool first = pos == 0;   // no token before it
+      pos = pos + 1 == p.T ? 0 : pos + 1;
       float q[8], k[8], v[8], kq[8], vq[8];
       blk_unpack<kBf16>(qr[u], q);
       blk_unpack<kBf16>(kr[u], k);
@@ -347,7 +354,8 @@ __global__ void __launch_bounds__(256) fox_pack_kernel(const PackParams p) {
 
 // ------------------------------------------------------------ column sums of a block's partial weight gradients
 // out_i[c] = sum_r part_i[r][c] for up to six arrays in one launch (a reduction kernel and a cast each before).  A CTA
-// takes 32 columns: warp w sums rows w, w + 8, ... with four loads in flight, then the eight warps are joined.
+// takes 32 columns: warp w of 32 sums rows w, w + 32, ... with four loads in flight, then the warps are joined.  (Bound by
+// latency: with 8 warps a CTA walked 592 rows in 19 trips; 14.1 -> 6.1 us at 768 columns, 15.8 -> 8.2 us at 1536.)
 struct SumParams {
   const float* part[kPackVecs];
   int rows[kPackVecs], cols[kPackVecs], dtype[kPackVecs], block0[kPackVecs + 1];
@@ -355,8 +363,8 @@ struct SumParams {
   int n;
 };
 
-__global__ void __launch_bounds__(256) fox_column_sums_kernel(const SumParams p) {
-  __shared__ float s[8][33];
+__global__ void __launch_bounds__(1024) fox_column_sums_kernel(const SumParams p) {
+  __shared__ float s[32][33];
   int i = 0;
   while (i + 1 < p.n && static_cast<int>(blockIdx.x) >= p.block0[i + 1]) ++i;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -364,10 +372,10 @@ __global__ void __launch_bounds__(256) fox_column_sums_kernel(const SumParams p)
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   if (col < cols) {
     const float* src = p.part[i] + col;
-    for (int r = warp; r < rows; r += 32) {
+    for (int r = warp; r < rows; r += 128) {
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (r + 8 * u < rows) acc[u] += src[static_cast<int64_t>(r + 8 * u) * cols];
+        if (r + 32 * u < rows) acc[u] += src[static_cast<int64_t>(r + 32 * u) * cols];
     }
   }
   s[warp][lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
@@ -375,7 +383,7 @@ __global__ void __launch_bounds__(256) fox_column_sums_kernel(const SumParams p)
   if (warp == 0 && col < cols) {
     float x = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) x += s[w][lane];
+    for (int w = 0; w < 32; ++w) x += s[w][lane];
     if (p.dtype[i] == FOX_DTYPE_FP32) static_cast<float*>(p.out[i])[col] = x;
     else static_cast<uint16_t*>(p.out[i])[col] = static_cast<uint16_t>(
         (p.dtype[i] == FOX_DTYPE_BF16 ? pack2<true>(x, 0.f) : pack2<false>(x, 0.f)) & 0xffffu);
@@ -421,8 +429,10 @@ extern "C" int fox_mix_fwd(int device, void* stream, int dtype, int64_t B, int64
   p.seq_start = seq_start;
   p.mix_blocks = (int)((p.tokens + p.rows - 1) / p.rows);
   const unsigned grid = (unsigned)(p.mix_blocks + (seq_start ? B : 0));
-  if (dtype == FOX_DTYPE_BF16) fox_mix_fwd_kernel<true><<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
-  else fox_mix_fwd_kernel<false><<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
+  const int threads = mix_threads(p);
+  auto kern = dtype == FOX_DTYPE_BF16 ? (threads <= 256 ? fox_mix_fwd_kernel<true, 256> : fox_mix_fwd_kernel<true, 512>)
+                                      : (threads <= 256 ? fox_mix_fwd_kernel<false, 256> : fox_mix_fwd_kernel<false, 512>);
+  kern<<<grid, threads, 0, (cudaStream_t)stream>>>(p);
   return blk_rc();
 }
 
@@ -499,6 +509,6 @@ extern "C" int fox_column_sums(int device, void* stream, int64_t n, const float*
   p.block0[n] = (int)block;
   p.n = (int)n;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  fox_column_sums_kernel<<<(unsigned)block, 256, 0, (cudaStream_t)stream>>>(p);
+  fox_column_sums_kernel<<<(unsigned)block, 1024, 0, (cudaStream_t)stream>>>(p);
   return blk_rc();
 }
