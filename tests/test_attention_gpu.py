@@ -572,3 +572,28 @@ def test_cuda_graph_replay_is_bit_identical(D):
         # dq and the gate gradient are sums of fp32 atomics, whose order varies from launch to launch
         _close(xg[0].grad, xe[0].grad, 1e-2, 1e-2, "dq")
         _close(xg[3].grad, xe[3].grad, 1e-2, 1e-2, "dlog_fgate")
+
+
+@pytest.mark.parametrize("M,N", [(2, 2), (64, 64), (65, 65), (128, 128), (3, 130), (129, 193), (100, 449), (257, 1000)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_forward_d128_half_tiles_with_a_moving_maximum(M, N, dtype):
+    """Head dim 128 walks 64-row key tiles through two score buffers: one tile, an odd and an even number of them, ragged
+    last ones.  Keys grow towards the left, so the running maximum moves in every tile and O is rescaled while the
+    product before may still run.  Rows left of seq_start are empty."""
+    g = torch.Generator().manual_seed(M * 1000 + N)
+    B, H, D = 2, 3, 128
+    q = torch.randn(B, H, M, D, generator=g).to(dtype)
+    k = (torch.randn(B, H, N, D, generator=g) * torch.linspace(12.0, 1.0, N)[:, None]).to(dtype)
+    v = torch.randn(B, H, N, D, generator=g).to(dtype)
+    lf = torch.nn.functional.logsigmoid(torch.randn(B, H, N, generator=g) + 6.0)
+    start = torch.tensor([0, N // 3])
+    ref = orc.dense_forgetting_attention(q.double(), k.double(), v.double(), lf.double(), seq_start=start)
+    ref = ref[0] if isinstance(ref, tuple) else ref
+    with torch.no_grad():
+        out = fox.forgetting_attention(q.cuda(), k.cuda(), v.cuda(), lf.cuda(), head_first=True, seq_start=start.cuda())
+    _lib.check_status()
+    # weights that sum to 1, each rounded to 16 bits (2^-9 or 2^-12) before the product and the result once more; logits of
+    # up to 12 * 128 / sqrt(128) * 4 in fp32 add 1e-4; twice that for fp32 sums
+    eps = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    bound = 2 * (2 * eps + 1e-4) * v.float().abs().max().item()
+    assert (out.double().cpu() - ref.double().nan_to_num(0.0)).abs().max().item() < bound
