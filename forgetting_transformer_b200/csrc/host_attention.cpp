@@ -413,9 +413,12 @@ static AttnInputs parse_inputs(PyObject* const* a) {   // q, k, v, gate, head_fi
   return in;
 }
 
+// the nine arguments -> out, or None where the autograd function has to be called
 FOX_PY(py_attention) {
   HANDLE_TH_ERRORS
   const AttnInputs in = parse_inputs(args);
+  for (const Tensor* t : {&in.q, &in.k, &in.v, &in.gate, &in.seq_start, &in.threshold.tensor})
+    if (has_tangent(*t)) Py_RETURN_NONE;
   Tensor out;
   {
     pybind11::gil_scoped_release no_gil;

@@ -141,7 +141,10 @@ bool read_block(PyObject* self, const Tensor& x, Block& b) {
   const Tensor& g = b.p[B::kGate];
   if (g.dim() != 2 || g.size(0) % 16 || !matrix(m, x, g.size(0), C, b.p[B::kGate])) return false;
   b.inter = g.size(0) / 2;
-  return linear(mlp, s_down_proj, x, C, b.inter, b.p[B::kDown]);
+  if (!linear(mlp, s_down_proj, x, C, b.inter, b.p[B::kDown]) || has_tangent(x)) return false;
+  for (const Tensor& t : b.p)
+    if (has_tangent(t)) return false;
+  return true;
 }
 
 // ---------------------------------------------------------------- working memory

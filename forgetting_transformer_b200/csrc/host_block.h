@@ -14,7 +14,7 @@ struct Block {
 };
 
 // Reads the module tree; false where any part of it is not the plain module this code stands in for (another class, a
-// hook, a patched forward, other dtypes or layouts, autocast): the modules' own forward then runs.
+// hook, a patched forward, other dtypes or layouts, autocast, a forward-mode tangent): the modules' own forward then runs.
 bool read_block(PyObject* self, const Tensor& x, Block& b);
 
 }  // namespace foxh

@@ -89,6 +89,10 @@ inline fox_tensor4 t4(const Tensor& x, bool head_first) {
   return fox_tensor4{x.data_ptr(), stride(0), stride(ih), stride(it)};
 }
 
+// A tangent of forward-mode differentiation.  The native nodes have none to give: their callers leave such calls to the
+// Python autograd functions, which refuse them.
+inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
 inline const Tensor& unpack(PyObject* o, const char* what) {
   if (!THPVariable_Check(o)) raise_assert(std::string(what) + " must be a tensor");
   return THPVariable_Unpack(o);

@@ -175,6 +175,20 @@ class ForgettingAttention(torch.autograd.Function):
         return (*grads, None, None, None, None, None, None, None, None, None, None)
 
 
+def _attention(q, k, v, gate, head_first, seq_start, sm_scale, adaptive_threshold, gate_is_logit):
+    """The native node, or the autograd function above for the calls that the node leaves to it (forward-mode
+    tangents, which the function refuses)."""
+    out = (_host or _load_host()).attention(q, k, v, gate, head_first, seq_start, sm_scale, adaptive_threshold, gate_is_logit)
+    if out is not None:
+        return out
+    if not head_first:
+        q, k, v = [t.permute(0, 2, 1, 3) for t in (q, k, v)]
+        gate = gate.permute(0, 2, 1)
+    out = ForgettingAttention.apply(q, k, v, gate, seq_start, True, sm_scale, adaptive_threshold,
+                                    False, False, None, False, False, gate_is_logit)
+    return out if head_first else out.permute(0, 2, 1, 3)
+
+
 def forgetting_attention_from_gate_logits(q, k, v, fgate_logit, *, head_first: bool = False,
                                           seq_start: Optional[torch.Tensor] = None, sm_scale: Optional[float] = None,
                                           adaptive_threshold=None):
@@ -185,7 +199,7 @@ def forgetting_attention_from_gate_logits(q, k, v, fgate_logit, *, head_first: b
     front of the operator, modeling_forgetting_transformer.py:343-346).  Everything else as ``forgetting_attention``."""
     for name, entry in (("q", q), ("k", k), ("v", v)):
         assert entry.dtype in _QKV_DTYPES, f"Only torch.float16 or torch.bfloat16 are supported for q/k/v, but got {entry.dtype} for {name}."
-    return (_host or _load_host()).attention(q, k, v, fgate_logit, head_first, seq_start, sm_scale, adaptive_threshold, True)
+    return _attention(q, k, v, fgate_logit, head_first, seq_start, sm_scale, adaptive_threshold, True)
 
 
 def forgetting_attention(
@@ -215,7 +229,7 @@ def forgetting_attention(
     """
     for name, entry in (("q", q), ("k", k), ("v", v)):
         assert entry.dtype in _QKV_DTYPES, f"Only torch.float16 or torch.bfloat16 are supported for q/k/v, but got {entry.dtype} for {name}."
-    return (_host or _load_host()).attention(q, k, v, log_fgate, head_first, seq_start, sm_scale, adaptive_threshold, False)
+    return _attention(q, k, v, log_fgate, head_first, seq_start, sm_scale, adaptive_threshold, False)
 
 
 # ---- the FoX layer's glue in front of the operator (modeling_forgetting_transformer.py:366-396) ----

@@ -1,0 +1,61 @@
+"""What the native nodes of attention and block must not change: the calls that go to the autograd functions and modules
+instead, what is refused, what is kept for the backward, memory and precision."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+import forgetting_transformer_b200 as fox
+
+pytestmark = pytest.mark.gpu
+
+
+def _qkvg(B=1, H=2, M=256, N=256, D=64, dtype=torch.bfloat16, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    q, k, v = [torch.randn(B, H, t, D, generator=g).to(dtype).cuda() for t in (M, N, N)]
+    return q, k, v, torch.nn.functional.logsigmoid(torch.randn(B, H, N, generator=g) + 3).cuda()
+
+
+def _block(C=256, H=4, inter=512, dtype=torch.bfloat16, **kw):
+    torch.manual_seed(0)
+    return fox.FoxProBlock(C, H, inter, fgate_bias=2.0, **kw).cuda().to(dtype)
+
+
+def _x(T=64, C=256, dtype=torch.bfloat16, seed=1, B=1):
+    return torch.randn(B, T, C, generator=torch.Generator().manual_seed(seed)).to(dtype).cuda()
+
+
+def _cache(blk, B=1, N=16):
+    """A cache of N tokens for layer 0."""
+    H, D = blk.attn.num_heads, blk.attn.head_dim
+    cache, st = fox.FgateCache(), blk.attn.init_shift_state(B)
+    cache.update_shift_cache(st["key_shift"], st["value_shift"], 0)
+    _, k, v, g = _qkvg(B, H, N, N, D, blk.attn.q_proj.weight.dtype)
+    cache.update(k, v, g, 0)
+    return cache
+
+
+@pytest.mark.parametrize("which", range(4))
+@pytest.mark.parametrize("head_first", [True, False])
+def test_forward_mode_is_refused_by_attention(which, head_first):
+    """No forward derivative is built: a dual tensor raises and does not come back without its tangent."""
+    args = [t if head_first else t.transpose(1, 2) for t in _qkvg()]
+    with fwAD.dual_level():
+        args[which] = fwAD.make_dual(args[which], torch.ones_like(args[which]))
+        with pytest.raises(NotImplementedError, match="jvp"):
+            fox.forgetting_attention(*args, head_first=head_first)
+
+
+@pytest.mark.parametrize("T", [1, 64])
+@pytest.mark.parametrize("of", ["input", "weight"])
+def test_forward_mode_is_refused_by_block(T, of):
+    blk, x = _block(), _x(T)
+    with fwAD.dual_level(), torch.no_grad():
+        if of == "input":
+            x = fwAD.make_dual(x, torch.ones_like(x))
+        else:
+            w = blk.mlp_norm.weight.detach()
+            del blk.mlp_norm.weight
+            blk.mlp_norm.weight = fwAD.make_dual(w, torch.ones_like(w))
+            blk.mlp_norm._parameters["weight"] = blk.mlp_norm.weight
+        with pytest.raises(NotImplementedError, match="jvp"):
+            blk(x, None, *((_cache(blk), 0) if T == 1 else ()))
