@@ -416,6 +416,7 @@ static AttnInputs parse_inputs(PyObject* const* a) {   // q, k, v, gate, head_fi
 // the nine arguments -> out, or None where the autograd function has to be called
 FOX_PY(py_attention) {
   HANDLE_TH_ERRORS
+  if (tracing()) Py_RETURN_NONE;
   const AttnInputs in = parse_inputs(args);
   for (const Tensor* t : {&in.q, &in.k, &in.v, &in.gate, &in.seq_start, &in.threshold.tensor})
     if (has_tangent(*t)) Py_RETURN_NONE;

@@ -111,7 +111,7 @@ bool row_norm_size(int64_t C) {   // what fox_rmsnorm is built for
 
 bool read_block(PyObject* self, const Tensor& x, Block& b) {
   using B = Block;
-  if (!g_classes[0] || !x.is_cuda() || x.dim() != 3) return false;
+  if (!g_classes[0] || tracing() || !x.is_cuda() || x.dim() != 3) return false;
   const auto dt = x.scalar_type();
   if ((dt != at::kHalf && dt != at::kBFloat16) || at::autocast::is_autocast_enabled(at::kCUDA)) return false;
   for (PyObject* h : g_global_hooks)

@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <string>
 
@@ -92,6 +93,10 @@ inline fox_tensor4 t4(const Tensor& x, bool head_first) {
 // A tangent of forward-mode differentiation.  The native nodes have none to give: their callers leave such calls to the
 // Python autograd functions, which refuse them.
 inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
+// Under torch.jit.trace a native result would be recorded as the at::empty that made it: uninitialised memory in the
+// traced graph.  The autograd functions are recorded as Python operators.
+inline bool tracing() { return torch::jit::tracer::isTracing(); }
 
 inline const Tensor& unpack(PyObject* o, const char* what) {
   if (!THPVariable_Check(o)) raise_assert(std::string(what) + " must be a tensor");

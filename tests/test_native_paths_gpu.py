@@ -59,3 +59,26 @@ def test_forward_mode_is_refused_by_block(T, of):
             blk.mlp_norm._parameters["weight"] = blk.mlp_norm.weight
         with pytest.raises(NotImplementedError, match="jvp"):
             blk(x, None, *((_cache(blk), 0) if T == 1 else ()))
+
+
+@pytest.mark.parametrize("head_first", [True, False])
+def test_traced_attention_runs_on_other_inputs(head_first):
+    """torch.jit.trace records the call, not the memory its result was made in."""
+    a, b = [[t if head_first else t.transpose(1, 2).contiguous() for t in _qkvg(seed=s)] for s in (1, 2)]
+    f = lambda *t: fox.forgetting_attention(*t, head_first=head_first, adaptive_threshold="auto") * 1.0
+    traced = torch.jit.trace(f, a, check_trace=False)
+    got = traced(*b)
+    assert torch.equal(got, f(*b))
+
+
+@pytest.mark.parametrize("T", [1, 64])
+def test_block_is_not_traced_natively(T):
+    """Under torch.jit.trace the modules run one by one: their recorded operators reach the result."""
+    blk, x = _block().requires_grad_(False), _x(T)     # (a trace takes weights as constants)
+    cache = _cache(blk) if T == 1 else None
+    with torch.no_grad():
+        try:
+            graph = str(torch.jit.trace(lambda x: blk(x, None, cache, 0), (x,), check_trace=False).inlined_graph)
+        except AssertionError:      # (token_shift's check of the head dim refuses the tracer's sizes)
+            return
+    assert "aten::linear" in graph or "aten::matmul" in graph
