@@ -9,6 +9,7 @@
 #include "host_gemm.h"
 
 #include <ATen/autocast_mode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 
 #include <cmath>
 
@@ -114,6 +115,7 @@ bool read_block(PyObject* self, const Tensor& x, Block& b) {
   if (!g_classes[0] || tracing() || !x.is_cuda() || x.dim() != 3) return false;
   const auto dt = x.scalar_type();
   if ((dt != at::kHalf && dt != at::kBFloat16) || at::autocast::is_autocast_enabled(at::kCUDA)) return false;
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;   // (they are there to see the products)
   for (PyObject* h : g_global_hooks)
     if (!empty_dict(h)) return false;
   Mod blk, attn, mlp, m;

@@ -3,6 +3,7 @@ instead, what is refused, what is kept for the backward, memory and precision.""
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
+from torch.utils._python_dispatch import TorchDispatchMode
 
 import forgetting_transformer_b200 as fox
 
@@ -82,3 +83,20 @@ def test_block_is_not_traced_natively(T):
         except AssertionError:      # (token_shift's check of the head dim refuses the tracer's sizes)
             return
     assert "aten::linear" in graph or "aten::matmul" in graph
+
+
+@pytest.mark.parametrize("T", [1, 64])
+def test_dispatch_modes_see_the_products_of_a_block(T):
+    """A mode that counts or replaces operators gets the block's matrix products (7 projections, o_proj, two of the MLP)."""
+    seen = []
+
+    class Record(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func.__name__)
+            return func(*args, **(kwargs or {}))
+
+    blk, x = _block(), _x(T)
+    args = (None, _cache(blk), 0) if T == 1 else ()
+    with torch.no_grad(), Record():
+        blk(x, *args)
+    assert sum(n.split(".")[0] in ("mm", "addmm", "bmm", "matmul", "linear") for n in seen) == 10
