@@ -249,7 +249,7 @@ AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs
     c.start = r.index.mutable_data_ptr<int64_t>();
     c.end = needs_grad ? c.start + BH * attn_blocks(M) : nullptr;
     if (in.threshold.kind == Threshold::kTensor) {
-      r.threshold = in.threshold.tensor.detach().to(in.q.device(), at::kFloat);
+      r.threshold = in.threshold.tensor.to(in.q.device(), at::kFloat);
       if (!at::is_expandable_to(r.threshold.sizes(), {B, H})) {
         std::ostringstream os;
         os << r.threshold.sizes();
@@ -257,13 +257,13 @@ AttnSaved attention_forward(const AttnInputs& in, const AttnShape& s, bool needs
             "adaptive_threshold must be either the string \"auto\" or broadcastable to (batch_size, num_heads) = (" +
             std::to_string(B) + ", " + std::to_string(H) + "), but got torch.Size(" + os.str() + ").");
       }
-      r.threshold = r.threshold.expand({B, H});
     } else {
       r.threshold = at::empty({B, H}, in.q.options().dtype(at::kFloat));
     }
   }
-  float* thr = pruned ? static_cast<float*>(r.threshold.data_ptr()) : nullptr;
-  const int64_t thr_sb = pruned ? r.threshold.stride(0) : 0, thr_sh = pruned ? r.threshold.stride(1) : 0;
+  const Tensor thr_bh = pruned ? r.threshold.expand({B, H}) : Tensor();
+  float* thr = pruned ? static_cast<float*>(thr_bh.data_ptr()) : nullptr;
+  const int64_t thr_sb = pruned ? thr_bh.stride(0) : 0, thr_sh = pruned ? thr_bh.stride(1) : 0;
   if (M == 1 && !needs_grad) {
     // generation step: one query row against the cache, no gradients -> split-KV kernels.  Only a threshold's index scan
     // (or gate logits) needs the prefix sum; otherwise the decode kernel works from the gates.
@@ -293,11 +293,13 @@ AttnGrads attention_backward(const AttnSaved& r, const Tensor& d_o, bool two_ker
     if (!have) index = at::empty({c.BH() * (nmb + nnb)}, r.q.options().dtype(at::kLong));
     c.start = index.mutable_data_ptr<int64_t>();
     c.end = c.start + c.BH() * nmb;
-    if (!have)
+    if (!have) {
+      const Tensor thr = r.threshold.expand({c.s.B, c.s.H});
       launch("fox_find_index", c.st, [&] {
-        return fox_find_index(dev, c.st, c.s.B, c.s.H, c.s.M, c.s.N, kBlock, kBlock, c.lam, r.threshold.const_data_ptr<float>(),
-                              r.threshold.stride(0), r.threshold.stride(1), c.start, c.end);
+        return fox_find_index(dev, c.st, c.s.B, c.s.H, c.s.M, c.s.N, kBlock, kBlock, c.lam, thr.const_data_ptr<float>(), thr.stride(0),
+                              thr.stride(1), c.start, c.end);
       });
+    }
   }
   AttnGrads out;
   out.dq = empty_like_tma(r.q);
@@ -331,19 +333,16 @@ using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
 struct AttentionBackward : public torch::autograd::Node {
-  SavedVariable q, k, v, o, gate;   // gate: the logits, where they are what was given
-  AttnSaved rest;                   // (its q, k, v, o, gate are left empty)
+  // Everything with memory goes through saved variables: they check that nothing was written to in between (a caller's
+  // seq_start or threshold is used as it is where its type allows) and pass the hooks that move or drop saved tensors.
+  // gate: the logits, where they are what was given.
+  SavedVariable q, k, v, o, gate, seq_start, vectors, threshold, index;
+  AttnSaved rest;   // (its tensors are left empty)
   bool released = false;
 
   std::string name() const override { return "ForgettingAttentionBackward"; }
   void release_variables() override {
-    q.reset_data();
-    k.reset_data();
-    v.reset_data();
-    o.reset_data();
-    gate.reset_data();
-    rest.vectors.reset();
-    rest.index.reset();
+    for (SavedVariable* s : {&q, &k, &v, &o, &gate, &seq_start, &vectors, &threshold, &index}) s->reset_data();
     released = true;
   }
   variable_list apply(variable_list&& grads) override {
@@ -356,6 +355,10 @@ struct AttentionBackward : public torch::autograd::Node {
     r.v = v.unpack();
     r.o = o.unpack(shared_from_this());
     if (r.gate_is_logit) r.gate = gate.unpack();
+    r.seq_start = seq_start.unpack();
+    r.vectors = vectors.unpack();
+    r.threshold = threshold.unpack();
+    r.index = index.unpack();
     AttnGrads g = attention_backward(r, grads[0], default_two_kernel(r.shape.D));
     if (task_should_compute_output(0)) out[0] = g.dq;
     if (task_should_compute_output(1)) out[1] = g.dk;
@@ -381,10 +384,11 @@ Tensor attention(const AttnInputs& in) {
   node->v = SavedVariable(r.v, false);
   node->o = SavedVariable(o, true);
   if (in.gate_is_logit) node->gate = SavedVariable(in.gate, false);
-  r.q.reset();
-  r.k.reset();
-  r.v.reset();
-  r.o.reset();
+  node->seq_start = SavedVariable(r.seq_start, false);
+  node->vectors = SavedVariable(r.vectors, false);
+  node->threshold = SavedVariable(r.threshold, false);
+  node->index = SavedVariable(r.index, false);
+  for (Tensor* t : {&r.q, &r.k, &r.v, &r.o, &r.seq_start, &r.vectors, &r.threshold, &r.index}) t->reset();
   node->rest = std::move(r);
   return o;
 }

@@ -29,7 +29,7 @@ struct AttnSaved {
   double sm_scale = 0.;
   Tensor q, k, v, o, gate, seq_start;
   Tensor vectors;                    // [log_lambda (B,H,N) | L (B,H,M) | norm parts]
-  Tensor threshold;                  // (B,H) fp32 view, with a threshold
+  Tensor threshold;                  // fp32, expands to (B,H), with a threshold (a caller's tensor as it is where it can be)
   Tensor index;                      // [start (B,H,ceil(M/128)) | end (B,H,ceil(N/128)), with gradients], with a threshold
   Tensor separate_lam, separate_L;   // instead of `vectors`, where the caller holds the two as tensors
 

@@ -100,3 +100,40 @@ def test_dispatch_modes_see_the_products_of_a_block(T):
     with torch.no_grad(), Record():
         blk(x, *args)
     assert sum(n.split(".")[0] in ("mm", "addmm", "bmm", "matmul", "linear") for n in seen) == 10
+
+
+@pytest.mark.parametrize("cls", [False, True])
+@pytest.mark.parametrize("what", ["seq_start", "threshold"])
+def test_arguments_changed_before_the_backward_are_noticed(what, cls):
+    """The backward masks and prunes by the values of the forward, so a change in between raises."""
+    q, k, v, g = _qkvg(B=2)
+    q.requires_grad_()
+    kw = dict(seq_start=torch.tensor([3, 9], device="cuda"), adaptive_threshold=torch.full((2, 2), -10.0, device="cuda"))
+    out = (fox.ops.ForgettingAttention.apply(q, k, v, g, kw["seq_start"], True, None, kw["adaptive_threshold"]) if cls
+           else fox.forgetting_attention(q, k, v, g, head_first=True, **kw))
+    kw["seq_start" if what == "seq_start" else "adaptive_threshold"].add_(1)
+    with pytest.raises(RuntimeError, match="inplace"):
+        out.sum().backward()
+
+
+def test_saved_tensor_hooks_get_all_that_attention_keeps():
+    """Offloading and checkpointing work on what is saved: every array the node holds passes the hooks, and what they give
+    back is used."""
+    q, k, v, g = _qkvg(B=2)
+    do = torch.randn(q.shape, generator=torch.Generator().manual_seed(9)).to(q.dtype).cuda()
+    seq = torch.tensor([3, 9], device="cuda")
+    grads, sizes = [], []
+    for hooked in (False, True):
+        x = [t.clone().requires_grad_() for t in (q, k, v, g)]
+        pack = lambda t: (sizes.append((t.dtype, t.numel())), t.cpu())[1]
+        with torch.autograd.graph.saved_tensors_hooks(*((pack, lambda t: t.cuda()) if hooked else (lambda t: t,) * 2)):
+            out = fox.forgetting_attention(*x, head_first=True, seq_start=seq, adaptive_threshold=-20.0)
+        out.backward(do)
+        grads.append([t.grad for t in x])
+    assert sum(n for d, n in sizes if d == torch.bfloat16) == 4 * q.numel()
+    assert sum(n for d, n in sizes if d == torch.float32) >= 2 * g.numel()           # gate prefixes, log normalisers
+    assert sum(n for d, n in sizes if d == torch.int64) == 2 + 2 * 4 * (256 // 128)   # seq_start, both index arrays
+    assert torch.equal(grads[0][1], grads[1][1]) and torch.equal(grads[0][2], grads[1][2])
+    for i in (0, 3):    # (sums by fp32 atomics, whose order varies: an ulp of the result's type here and there)
+        a, b = [t[i].float() for t in grads]
+        assert (a - b).norm() <= 2 ** -9 * b.norm()
