@@ -421,6 +421,8 @@ static AttnInputs parse_inputs(PyObject* const* a) {   // q, k, v, gate, head_fi
 FOX_PY(py_attention) {
   HANDLE_TH_ERRORS
   if (tracing()) Py_RETURN_NONE;
+  for (int i = 0; i < 4; ++i)
+    if (THPVariable_Check(args[i]) && !plain_tensor(args[i])) Py_RETURN_NONE;
   const AttnInputs in = parse_inputs(args);
   for (const Tensor* t : {&in.q, &in.k, &in.v, &in.gate, &in.seq_start, &in.threshold.tensor})
     if (has_tangent(*t)) Py_RETURN_NONE;

@@ -69,7 +69,7 @@ bool open_plain(const Mod& parent, PyObject* name, Class cls, Mod& m) {
 }
 
 bool tensor(PyObject* o, Tensor& t) {
-  if (!o || !THPVariable_Check(o)) return false;
+  if (!o || !plain_tensor(o)) return false;
   t = THPVariable_Unpack(o);
   return true;
 }
@@ -530,6 +530,7 @@ FOX_PY(py_block) {
   Tensor x;
   Block b;
   if (!tensor(args[1], x) || !read_block(args[0], x, b)) Py_RETURN_NONE;
+  if (args[2] != Py_None && !plain_tensor(args[2])) Py_RETURN_NONE;
   const Tensor mask = unpack_opt(args[2], "attention_mask"), threshold = unpack_opt(args[3], "threshold");
   if (b.pruned != threshold.defined() || x.size(1) < 2 || x.size(0) < 1) Py_RETURN_NONE;
   if (mask.defined()) {
@@ -714,6 +715,7 @@ FOX_PY(py_block_step) {
     for (const Tensor& t : b.p) needs = needs || (t.defined() && t.requires_grad());
     if (needs) Py_RETURN_NONE;
   }
+  if (args[2] != Py_None && !plain_tensor(args[2])) Py_RETURN_NONE;
   const Tensor mask = unpack_opt(args[2], "attention_mask");
   if (mask.defined()) {
     const auto d = mask.scalar_type();

@@ -98,6 +98,10 @@ inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*le
 // traced graph.  The autograd functions are recorded as Python operators.
 inline bool tracing() { return torch::jit::tracer::isTracing(); }
 
+// A Tensor or Parameter itself.  A subclass (a quantised weight, a distributed or a not yet waited-for tensor) may have
+// other semantics and no storage: its data pointer is null.
+inline bool plain_tensor(PyObject* o) { return THPVariable_CheckExact(o); }
+
 inline const Tensor& unpack(PyObject* o, const char* what) {
   if (!THPVariable_Check(o)) raise_assert(std::string(what) + " must be a tensor");
   return THPVariable_Unpack(o);

@@ -177,7 +177,8 @@ class ForgettingAttention(torch.autograd.Function):
 
 def _attention(q, k, v, gate, head_first, seq_start, sm_scale, adaptive_threshold, gate_is_logit):
     """The native node, or the autograd function above for the calls that the node leaves to it: forward-mode
-    tangents, which the function refuses, and torch.jit.trace, which records it as a Python operator."""
+    tangents, which the function refuses, torch.jit.trace, which records it as a Python operator, and tensor subclasses,
+    which the permutes may turn into plain tensors."""
     out = (_host or _load_host()).attention(q, k, v, gate, head_first, seq_start, sm_scale, adaptive_threshold, gate_is_logit)
     if out is not None:
         return out

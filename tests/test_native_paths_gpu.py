@@ -137,3 +137,44 @@ def test_saved_tensor_hooks_get_all_that_attention_keeps():
     for i in (0, 3):    # (sums by fp32 atomics, whose order varies: an ulp of the result's type here and there)
         a, b = [t[i].float() for t in grads]
         assert (a - b).norm() <= 2 ** -9 * b.norm()
+
+
+class _Wrapped(torch.Tensor):
+    """A tensor without storage of its own, as weight-only quantised weights are: every operator works on what it holds."""
+
+    @staticmethod
+    def __new__(cls, inner):
+        return torch.Tensor._make_wrapper_subclass(cls, inner.size(), strides=inner.stride(), dtype=inner.dtype, device=inner.device)
+
+    def __init__(self, inner):
+        self.inner = inner
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        unwrap = lambda t: t.inner if isinstance(t, cls) else t
+        args, kwargs = torch.utils._pytree.tree_map(unwrap, (args, kwargs or {}))
+        out = func(*args, **kwargs)
+        return cls(out) if func is torch.ops.aten.detach.default else out
+
+
+@pytest.mark.parametrize("which", ["attn.q_proj", "attn.v_proj.shift_proj", "attn.o_proj", "mlp.gate_proj", "mlp.down_proj"])
+@pytest.mark.parametrize("T", [1, 64])
+def test_block_with_a_weight_without_storage(which, T):
+    """The module whose weight is a wrapper runs its own forward, which the subclass takes part in."""
+    blk, x = _block().requires_grad_(False), _x(T)
+    res = []
+    for wrapped in (False, True):
+        args = (None, _cache(blk), 0) if T == 1 else ()
+        if wrapped:
+            m = blk.get_submodule(which)
+            m.weight = torch.nn.Parameter(_Wrapped(m.weight.data), requires_grad=False)
+            assert type(m.weight.data_ptr()) is int and m.weight.data_ptr() == 0
+        res.append(blk(x, *args).float())
+    assert (res[0] - res[1]).norm() <= 2 ** -6 * res[0].norm()     # (native against modules: 8 roundings to 16 bits)
+
+
+def test_attention_on_wrapped_tensors():
+    """(B, T, H, D) calls permute first, which turns a wrapper of this kind into the tensor it holds."""
+    args = [t.transpose(1, 2).contiguous() for t in _qkvg()]
+    ref = fox.forgetting_attention(*args)
+    assert torch.equal(fox.forgetting_attention(*[_Wrapped(t) for t in args]), ref)
