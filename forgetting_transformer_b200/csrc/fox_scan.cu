@@ -354,9 +354,9 @@ fox_max_row_norm_kernel(const uint16_t* __restrict__ x, int64_t sb, int64_t sh, 
 // ------------------------------------------------------ before the attention forward
 // The prefix sum of the log gates and the largest key (and, for the automatic threshold, query) row norms in one
 // launch: they are independent, and each alone leaves most of the chip idle (one CTA per (b,h) scans, a scan of
-// 16384 gates takes 10 us).  blockIdx.x = 0 scans; blocks 1 .. n_k (n_k+1 .. n_k+n_q) each take every n_k-th
+// 16384 gates takes 10 us).  blockIdx.y = 0 scans; blocks 1 .. n_k (n_k+1 .. n_k+n_q) each take every n_k-th
 // (n_q-th) group of rows and write ONE partial maximum, so nothing has to be zeroed first; the reader takes the
-// maximum of the parts.
+// maximum of the parts.  (b, h) is the grid's x index: there may be more than the 65535 that y takes.
 struct NormSource {
   const uint16_t* x;
   int64_t sb, sh, st;
@@ -414,7 +414,7 @@ fox_prologue_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t
                     const float* __restrict__ gate_bias, const int64_t* __restrict__ seq_start, float* __restrict__ lam,
                     const NormSource k, const NormSource q, int H, int N, int D) {
   __shared__ float red[32];
-  const int bh = blockIdx.y, x = blockIdx.x;
+  const int bh = blockIdx.x, x = blockIdx.y;
   if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red,
                                 gate_bias ? gate_bias[bh % H] : 0.f);
   else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
@@ -654,7 +654,7 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
                                  int64_t n_k_parts, const fox_tensor4* q, float* q_parts, int64_t n_q_parts) {
   if (!gates || !log_lambda || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
-  if (B * H > 65535) return FOX_ERR_TOO_LARGE;   // (b, h) is the grid's y index
+  if (B * H > 2147483647LL || n_k_parts > 32767 || n_q_parts > 32767) return FOX_ERR_TOO_LARGE;
   if (!head_dim_ok(D)) return FOX_ERR_HEAD_DIM;
   NormSource ks{}, qs{};
   if (k) {
@@ -668,7 +668,7 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
     qs = NormSource{(const uint16_t*)q->ptr, q->sb, q->sh, q->st, (int)M, (int)n_q_parts, q_parts};
   }
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  dim3 grid((unsigned)(1 + ks.n_parts + qs.n_parts), (unsigned)(B * H));
+  dim3 grid((unsigned)(B * H), (unsigned)(1 + ks.n_parts + qs.n_parts));
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == FOX_DTYPE_BF16;
 #define FOX_PRO(K)                                                                                                       \

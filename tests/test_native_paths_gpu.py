@@ -6,6 +6,7 @@ import torch.autograd.forward_ad as fwAD
 from torch.utils._python_dispatch import TorchDispatchMode
 
 import forgetting_transformer_b200 as fox
+from oracle import fox_oracle as orc
 
 pytestmark = pytest.mark.gpu
 
@@ -178,3 +179,18 @@ def test_attention_on_wrapped_tensors():
     args = [t.transpose(1, 2).contiguous() for t in _qkvg()]
     ref = fox.forgetting_attention(*args)
     assert torch.equal(fox.forgetting_attention(*[_Wrapped(t) for t in args]), ref)
+
+
+@pytest.mark.parametrize("kind", ["log gates", "gate logits", "one row, pruned", "auto"])
+def test_more_than_65535_heads_without_gradients(kind):
+    """4096 sequences of 24 heads: more (b, h) than a grid's y axis has blocks."""
+    q, k, v, g = _qkvg(B=4096, H=24, M=1 if kind == "one row, pruned" else 3, N=5, D=16)
+    kw = dict(head_first=True, adaptive_threshold={"one row, pruned": -200.0, "auto": "auto"}.get(kind))
+    with torch.no_grad():
+        out = (fox.forgetting_attention_from_gate_logits if kind == "gate logits" else fox.forgetting_attention)(q, k, v, g, **kw)
+    lf = torch.nn.functional.logsigmoid(g) if kind == "gate logits" else g
+    for b in (0, 2730, 2731, 4095):     # (65535 = 2730 * 24 + 15)
+        ref = orc.dense_forgetting_attention(*[t[b:b + 1].double().cpu() for t in (q, k, v, lf)])
+        ref = ref[0] if isinstance(ref, tuple) else ref
+        # five weights that sum to 1, rounded to bf16, and the result once more: 2 * 2^-9 of the largest value
+        assert (out[b:b + 1].double().cpu() - ref).abs().max() <= 2 ** -8 * v[b].abs().max()
