@@ -710,6 +710,10 @@ FOX_PY(py_block_step) {
   if (!tensor(args[1], x) || x.dim() != 3 || x.size(1) != 1 || x.size(0) < 1 || x.size(0) > 16 || !read_block(args[0], x, b) || b.pruned ||
       b.inter % 32 || x.size(0) * (std::max(b.C, b.inter) / 8 + 12) * 16 > 200 * 1024 || !open_cache(args[3], layer, x, b, c))
     Py_RETURN_NONE;
+  // (fox_step_product reads norm weights in 16-byte pieces; views of a flat buffer need not start on one.  Seen here, before
+  // the first launch writes to the cache)
+  for (Block::Param w : {Block::kAttnNorm, Block::kONorm, Block::kMlpNorm})
+    if (reinterpret_cast<uintptr_t>(b.p[w].const_data_ptr()) % 16) Py_RETURN_NONE;
   if (at::GradMode::is_enabled()) {
     bool needs = x.requires_grad();
     for (const Tensor& t : b.p) needs = needs || (t.defined() && t.requires_grad());

@@ -194,3 +194,22 @@ def test_more_than_65535_heads_without_gradients(kind):
         ref = ref[0] if isinstance(ref, tuple) else ref
         # five weights that sum to 1, rounded to bf16, and the result once more: 2 * 2^-9 of the largest value
         assert (out[b:b + 1].double().cpu() - ref).abs().max() <= 2 ** -8 * v[b].abs().max()
+
+
+@pytest.mark.parametrize("which", ["attn_norm", "mlp_norm", "attn.output_norm", "attn.q_norm", "attn.fgate_proj"])
+def test_token_step_with_vectors_that_are_not_aligned(which):
+    """Norm weights and biases may be views into a flat buffer."""
+    blk, x = _block(), _x(1)
+    res = []
+    for shifted in (False, True):
+        if shifted:
+            m, name = blk.get_submodule(which), "bias" if which.endswith("proj") else "weight"
+            flat = torch.empty(1 + getattr(m, name).numel(), device="cuda", dtype=torch.bfloat16)
+            flat[1:] = getattr(m, name).data
+            setattr(m, name, torch.nn.Parameter(flat[1:]))
+            assert getattr(m, name).data_ptr() % 16
+        cache = _cache(blk)
+        with torch.no_grad():
+            res.append([blk(x, None, cache, 0)] + [t.clone() for t in cache[0]] + [cache.key_shift_cache[0].clone()])
+    for a, b in zip(*res):      # (native against modules: 8 roundings to 16 bits)
+        assert (a.float() - b.float()).norm() <= 2 ** -6 * a.float().norm()
