@@ -66,20 +66,25 @@ def _build_kernels(verbose):
     _compile_all(_paths(SOURCES), flags + (["-Xptxas", "-v"] if verbose else []), flags, LIB_PATH, verbose=verbose)
 
 
+def _host_libs():
+    """What the extension is linked to: PyTorch's own libraries and the kernels.  The CUDA runtime and cuBLASLt are not named:
+    they are those libtorch_cuda depends on, wherever and in whatever version the installed PyTorch has them."""
+    import torch
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    return ["-Wl,--no-as-needed", "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
+            "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib]
+
+
 def _build_host(verbose):
     import sysconfig
     import torch
     from torch.utils.cpp_extension import include_paths
     # (not $CXX: the extension has to share the process's libstdc++, which a compiler that only has the static one breaks)
     cxx = os.environ.get("FOX_B200_CXX", "g++")
-    inc = include_paths() + [sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+    inc = include_paths("cuda") + [sysconfig.get_paths()["include"]]
     flags = [cxx, "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f for i in inc for f in ("-isystem", i)]
-    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    blas = os.path.join(os.path.dirname(os.path.dirname(torch.__file__)), "nvidia", "cublas", "lib")   # the one torch loads
-    libs = ["-L" + blas, "-l:libcublasLt.so.12", "-Wl,-rpath," + blas, "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
-            "-L" + PKG_DIR, "-l:libfox_b200.so", "/usr/local/cuda/lib64/libcudart.so", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib]
-    _compile_all(_paths(HOST_SOURCES), flags, [cxx], HOST_PATH, libs, verbose)
+    _compile_all(_paths(HOST_SOURCES), flags, [cxx], HOST_PATH, _host_libs(), verbose)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

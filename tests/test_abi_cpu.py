@@ -51,6 +51,18 @@ def test_python_bindings_cover_every_declared_symbol():
     assert set(_declared_symbols()) <= set(_lib._SIGNATURES)
 
 
+def test_host_extension_takes_cuda_libraries_from_pytorch():
+    """No file of one CUDA installation or version is named: only PyTorch's libraries, the kernels and the C++ runtime are
+    needed directly, and the extension loads with them."""
+    import subprocess
+    _lib.host()
+    out = subprocess.run(["readelf", "-d", build.HOST_PATH], capture_output=True, text=True, check=True).stdout
+    needed = re.findall(r"\(NEEDED\).*\[(.*)\]", out)
+    assert "libtorch_cuda.so" in needed
+    for name in needed:
+        assert re.match(r"lib(torch|c10|fox_b200|stdc\+\+|gcc_s|c\b|m\b)|ld-linux", name), name
+
+
 def _inputs(B=1, H=2, M=8, N=8, D=64, dtype=torch.bfloat16):
     q = torch.zeros(B, H, M, D, dtype=dtype)
     k = torch.zeros(B, H, N, D, dtype=dtype)
