@@ -4,21 +4,32 @@ Two shared objects next to this file, both git-ignored:
 
 * ``libfox_b200.so``: every kernel file compiled by ``nvcc`` for sm_100a only (SASS, no PTX); exports the C ABI declared
   in ``include/fox_b200.h``.  nvcc cross-compiles, so no GPU is needed.
-* ``_fox_host.so``: the operators' host side as a Python extension (``g++`` against the installed PyTorch's headers),
-  linked to the first.
+* ``_fox_host.<python>-torch<version>.so``: the operators' host side as a Python extension (``g++`` against the installed
+  PyTorch's headers), linked to the first.  PyTorch's C++ interface changes from version to version: the name holds what the
+  file was built against, so that one built against another PyTorch is not loaded but built anew.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 import tempfile
 from concurrent.futures import ThreadPoolExecutor
+
+import torch
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libfox_b200.so")
-HOST_PATH = os.path.join(PKG_DIR, "_fox_host.so")
+
+
+def host_path(torch_version: str = torch.__version__) -> str:
+    python = sysconfig.get_config_var("SOABI") or sys.implementation.cache_tag
+    return os.path.join(PKG_DIR, f"_fox_host.{python}-torch{torch_version}.so")
+
+
+HOST_PATH = host_path()
 SOURCES = ["fox_scan.cu", "fox_attn_fwd.cu", "fox_attn_bwd.cu", "fox_attn_bwd_dq.cu", "fox_attn_bwd_kv.cu", "fox_decode.cu", "fox_normgate.cu", "fox_rmsnorm.cu", "fox_shift.cu", "fox_glu.cu", "fox_ce.cu", "fox_block.cu", "fox_step.cu", "fox_noalloc.cu"]
 HEADERS = ["fox_common.cuh", "fox_host.h", os.path.join("..", "..", "include", "fox_b200.h")]
 HOST_SOURCES = ["host_module.cpp", "host_attention.cpp", "host_block.cpp", "host_gemm.cpp"]
@@ -69,15 +80,12 @@ def _build_kernels(verbose):
 def _host_libs():
     """What the extension is linked to: PyTorch's own libraries and the kernels.  The CUDA runtime and cuBLASLt are not named:
     they are those libtorch_cuda depends on, wherever and in whatever version the installed PyTorch has them."""
-    import torch
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     return ["-Wl,--no-as-needed", "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
             "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib]
 
 
 def _build_host(verbose):
-    import sysconfig
-    import torch
     from torch.utils.cpp_extension import include_paths
     # (not $CXX: the extension has to share the process's libstdc++, which a compiler that only has the static one breaks)
     cxx = os.environ.get("FOX_B200_CXX", "g++")

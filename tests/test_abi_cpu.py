@@ -63,6 +63,20 @@ def test_host_extension_takes_cuda_libraries_from_pytorch():
         assert re.match(r"lib(torch|c10|fox_b200|stdc\+\+|gcc_s|c\b|m\b)|ld-linux", name), name
 
 
+def test_host_extension_of_another_pytorch_is_not_taken(tmp_path, monkeypatch):
+    """The file that is looked for holds the PyTorch version in its name: with another version installed the present one is
+    neither up to date nor loaded."""
+    assert torch.__version__ in os.path.basename(build.HOST_PATH) and os.path.exists(build.HOST_PATH)
+    other = build.host_path("0.0.1")
+    assert other != build.HOST_PATH and not os.path.exists(other)
+    monkeypatch.setattr(build, "HOST_PATH", other)
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setenv("FOX_B200_NO_BUILD", "1")
+    assert build.is_stale()
+    with pytest.raises(fox.FoxError, match="cannot be loaded"):
+        _lib.host()
+
+
 def _inputs(B=1, H=2, M=8, N=8, D=64, dtype=torch.bfloat16):
     q = torch.zeros(B, H, M, D, dtype=dtype)
     k = torch.zeros(B, H, N, D, dtype=dtype)
