@@ -54,12 +54,12 @@ _SIGNATURES = {
                                    _F, _F, _F, c_float, _T4P, _F, _F, c_int64, _F]),
     "fox_norm_parts": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
     "fox_attn_prologue": (c_int, [c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _F, c_int64,
-                                  c_int64, c_int64, _F, _F, _F, _T4P, _F, c_int64, _T4P, _F, c_int64]),
+                                  c_int64, c_int64, _F, _F, _T4P, _F, c_int64, _T4P, _F, c_int64]),
     "fox_attn_index": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, _F, c_float, _F,
                                c_int64, _F, c_int64, c_float, _F, _F, _F]),
     "fox_bwd_prepare": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _F, _F, _F]),
     "fox_bwd_finish": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _F, _F, c_int, _F,
-                               c_int64, c_int64, c_int64, _F, _F, c_int64, c_int64, c_int64, _F, _F, c_float, _T4P]),
+                               c_int64, c_int64, c_int64, _F, c_int64, c_int64, c_int64, _F, _F, c_float, _T4P]),
     "fox_attn_decode": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P, _F, _F, _F,
                                 c_float, _T4P, _F, _F, c_int64]),
     "fox_attn_decode_gates": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P, _F, c_int64,
@@ -87,7 +87,7 @@ _SIGNATURES = {
                                  _F, c_int64, c_int64, _F, _F, _F, _F, c_int64]),
     "fox_step_mix": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, _F, c_int64, _F, c_int, _F, c_int, c_float, _F,
                              c_int, _F, _F, _F, _F, _F, _F, _F, _F, c_int64, c_int64]),
-    "fox_pack": (c_int, [c_int, c_void_p, c_int64, _F, _F, c_int64, c_int64, _F, c_int64, _F, _F, _F, _F]),
+    "fox_pack": (c_int, [c_int, c_void_p, c_int64, _F, _F, c_int64, c_int64, _F, c_int64, _F, _F, _F, _F, _F, c_int64, c_int64, _F]),
     "fox_column_sums": (c_int, [c_int, c_void_p, c_int64, _F, _F, _F, _F, _F]),
     "fox_rmsnorm_fwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, _F, _F, _F, c_float, _F, _F, _F]),
     "fox_rmsnorm_bwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, _F, _F, _F, _F, _F, _F, _F, c_int64]),

@@ -301,7 +301,9 @@ __global__ void __launch_bounds__(512) fox_mix_bwd_kernel(const MixBwdParams p) 
 
 // ------------------------------------------------------------ parameters of a block, laid out for its products
 // One launch instead of a concatenation and a cast per parameter: the projection weights stacked into one (rows, C)
-// matrix (padding rows zero), the norm weights and the gate bias as fp32.
+// matrix (padding rows zero), the norm weights as fp32, the gate bias as the product's bias vector: added there in fp32 it
+// is rounded once with its projection, where a bias added to a 16-bit projection keeps the projection's rounding error when
+// the two nearly cancel.
 constexpr int kPackMats = 8, kPackVecs = 6;
 struct PackParams {
   const uint16_t* mat[kPackMats];   // (mat_rows[i], C) contiguous
@@ -312,6 +314,9 @@ struct PackParams {
   int vec_len[kPackVecs], vec_off[kPackVecs], vec_dtype[kPackVecs];
   int n_vecs, vec_blocks;
   float* vecs;
+  const uint16_t* bias;     // (n_bias), into bias_out (rows) from bias_row on
+  int n_bias, bias_row;
+  uint16_t* bias_out;       // or nullptr
 };
 
 __global__ void __launch_bounds__(256) fox_pack_kernel(const PackParams p) {
@@ -325,6 +330,9 @@ __global__ void __launch_bounds__(256) fox_pack_kernel(const PackParams p) {
         p.vecs[p.vec_off[i] + e] = x;
       }
     }
+    if (p.bias_out)
+      for (int e = blockIdx.x * 256 + threadIdx.x; e < p.rows; e += p.vec_blocks * 256)
+        p.bias_out[e] = e >= p.bias_row && e - p.bias_row < p.n_bias ? p.bias[e - p.bias_row] : static_cast<uint16_t>(0);
     return;
   }
   const int per_row = p.C / 8;
@@ -466,7 +474,8 @@ extern "C" int fox_mix_bwd(int device, void* stream, int dtype, int64_t B, int64
 
 extern "C" int fox_pack(int device, void* stream, int64_t n_mats, const void* const* mats, const int64_t* mat_rows, int64_t rows,
                         int64_t cols, void* stack, int64_t n_vecs, const void* const* vecs, const int64_t* vec_len,
-                        const int32_t* vec_dtype, float* vecs_out) {
+                        const int32_t* vec_dtype, float* vecs_out, const void* bias, int64_t n_bias, int64_t bias_row,
+                        void* bias_out) {
   if (n_mats < 0 || n_mats > kPackMats || n_vecs < 0 || n_vecs > kPackVecs || cols <= 0 || cols % 8) return FOX_ERR_BAD_ARG;
   PackParams p{};
   int64_t row = 0;
@@ -486,7 +495,12 @@ extern "C" int fox_pack(int device, void* stream, int64_t n_mats, const void* co
     p.vec[i] = vecs[i]; p.vec_len[i] = (int)vec_len[i]; p.vec_off[i] = (int)off; p.vec_dtype[i] = vec_dtype[i];
     off += vec_len[i];
   }
-  p.n_vecs = (int)n_vecs; p.vecs = vecs_out; p.vec_blocks = n_vecs ? 4 : 0;
+  p.n_vecs = (int)n_vecs; p.vecs = vecs_out;
+  if (bias_out) {
+    if (!bias || n_bias <= 0 || bias_row < 0 || bias_row + n_bias > rows) return FOX_ERR_BAD_ARG;
+    p.bias = (const uint16_t*)bias; p.n_bias = (int)n_bias; p.bias_row = (int)bias_row; p.bias_out = (uint16_t*)bias_out;
+  }
+  p.vec_blocks = n_vecs || bias_out ? 4 : 0;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   int64_t blocks = (rows * (cols / 8) + 256 * 4 - 1) / (256 * 4);
   if (blocks > 148 * 8) blocks = 148 * 8;

@@ -53,14 +53,13 @@ __device__ __forceinline__ float block_inclusive_scan(float v, float* red, float
 // returns log sigmoid(x) = min(x, 0) - log1p(exp(-|x|)) in fp32 (the F.logsigmoid(fgate_logit.float()) of
 // upstream's layer, modeling_forgetting_transformer.py:343-346).
 template <int kIn>
-__device__ __forceinline__ float load_gate(const void* base, int64_t idx, float bias = 0.f) {
+__device__ __forceinline__ float load_gate(const void* base, int64_t idx) {
   if constexpr (kIn == 3) {
     return reinterpret_cast<const float*>(base)[idx];
   } else {
     float x;
     if constexpr (kIn == 2) x = reinterpret_cast<const float*>(base)[idx];
     else x = unpack2<kIn == 1>(static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(base)[idx])).x;
-    x += bias;
     return fminf(x, 0.f) - log1pf(expf(-fabsf(x)));
   }
 }
@@ -72,8 +71,7 @@ template <int kIn>
 __device__ __forceinline__ void cumsum_rows(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
                                             const int64_t* __restrict__ seq_start, const float* __restrict__ carry_in,
                                             float* __restrict__ out, float* __restrict__ total_out,
-                                            float* __restrict__ lf_out, int H, int N, int bh, float* red,
-                                            float bias = 0.f) {
+                                            float* __restrict__ lf_out, int H, int N, int bh, float* red) {
   const int b = bh / H, h = bh % H;
   const int64_t src0 = b * sb + h * sh;
   float* dst = out + static_cast<int64_t>(bh) * N;
@@ -86,7 +84,7 @@ __device__ __forceinline__ void cumsum_rows(const void* __restrict__ lf, int64_t
     for (int j = 0; j < kScanPerThread; ++j) {
       const int t = t0 + j;
       float g = 0.f;
-      if (t < N && (t >= s0 || (kIn < 3 && lf_out))) g = load_gate<kIn>(lf, src0 + static_cast<int64_t>(t) * sn, bias);
+      if (t < N && (t >= s0 || (kIn < 3 && lf_out))) g = load_gate<kIn>(lf, src0 + static_cast<int64_t>(t) * sn);
       if (kIn < 3 && lf_out && t < N) lf_out[static_cast<int64_t>(bh) * N + t] = g;
       x[j] = (t < N && t >= s0) ? g : 0.f;
     }
@@ -126,7 +124,6 @@ struct RevParams {
   int64_t sb, sh, sn;      // strides of logit
   int64_t osb, osh, osn;   // strides of out / dlogit
   int H;
-  const float* bias;       // (H) or nullptr: added to the logits
   float* dbias;            // (B*H) or nullptr: sum of each (b,h)'s dlogit
 };
 
@@ -142,7 +139,6 @@ __device__ __forceinline__ void revcumsum_rows(const RevParams& p, int bh, float
   const float* r = drow ? drow + static_cast<int64_t>(bh) * M : nullptr;
   const int64_t o0 = static_cast<int64_t>(bh / H) * p.osb + static_cast<int64_t>(bh % H) * p.osh;
   const int P = N - M;
-  const float bias = kIn < 3 && p.bias ? p.bias[bh % H] : 0.f;
   float dsum = 0.f;
   float carry = carry_in ? carry_in[bh] : 0.f;
   // walk chunks from the right; inside a chunk index i runs right-to-left
@@ -176,7 +172,7 @@ __device__ __forceinline__ void revcumsum_rows(const RevParams& p, int bh, float
           float xl;
           if constexpr (kIn == 2) xl = reinterpret_cast<const float*>(logit)[idx];
           else xl = unpack2<kIn == 1>(static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(logit)[idx])).x;
-          const float dl = gsum / (1.f + expf(xl + bias));     // d/dx log sigmoid(x) = sigmoid(-x)
+          const float dl = gsum / (1.f + expf(xl));     // d/dx log sigmoid(x) = sigmoid(-x)
           dsum += dl;
           const int64_t odx = o0 + static_cast<int64_t>(t) * p.osn;
           if constexpr (kIn == 2) reinterpret_cast<float*>(dlogit)[odx] = dl;
@@ -411,12 +407,11 @@ __device__ __forceinline__ void norm_part(const NormSource& s, int D, int H, int
 template <int kIn, bool kBf16>
 __global__ void __launch_bounds__(kScanThreads)
 fox_prologue_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
-                    const float* __restrict__ gate_bias, const int64_t* __restrict__ seq_start, float* __restrict__ lam,
+                    const int64_t* __restrict__ seq_start, float* __restrict__ lam,
                     const NormSource k, const NormSource q, int H, int N, int D) {
   __shared__ float red[32];
   const int bh = blockIdx.x, x = blockIdx.y;
-  if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red,
-                                gate_bias ? gate_bias[bh % H] : 0.f);
+  if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
   else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
   else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
 }
@@ -605,7 +600,7 @@ extern "C" int fox_revcumsum(int device, void* stream, int64_t B, int64_t H, int
                              float* dlog_fgate, float* total_out) {
   if (!dlam_col || !dlog_fgate || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  const RevParams rev{dlam_col, dlam_row, carry_in, dlog_fgate, total_out, (int)M, (int)N, nullptr, nullptr, 0, 0, 0, H * N, N, 1, (int)H, nullptr, nullptr};
+  const RevParams rev{dlam_col, dlam_row, carry_in, dlog_fgate, total_out, (int)M, (int)N, nullptr, nullptr, 0, 0, 0, H * N, N, 1, (int)H, nullptr};
   return launch_finish((cudaStream_t)stream, FOX_GATE_LOG, false, rev, (int)(B * H), ConvParams{});
 }
 
@@ -615,14 +610,14 @@ extern "C" int fox_gate_prefix_bwd(int device, void* stream, int dtype, int64_t 
   if (!dlam_col || !fgate_logit || !dfgate_logit || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (dtype != FOX_DTYPE_FP16 && dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP32) return FOX_ERR_BAD_ARG;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  const RevParams rev{dlam_col, dlam_row, nullptr, nullptr, nullptr, (int)M, (int)N, fgate_logit, dfgate_logit, sb, sh, sn, sb, sh, sn, (int)H, nullptr, nullptr};
+  const RevParams rev{dlam_col, dlam_row, nullptr, nullptr, nullptr, (int)M, (int)N, fgate_logit, dfgate_logit, sb, sh, sn, sb, sh, sn, (int)H, nullptr};
   return launch_finish((cudaStream_t)stream, dtype, false, rev, (int)(B * H), ConvParams{});
 }
 
 extern "C" int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
                               const float* dlam_col, const float* dlam_row, int gate_kind, const void* fgate_logit,
-                              int64_t sb, int64_t sh, int64_t sn, const float* gate_bias, void* dgate, int64_t osb,
-                              int64_t osh, int64_t osn, float* dbias, const float* dq_accum, float scale, const fox_tensor4* dq) {
+                              int64_t sb, int64_t sh, int64_t sn, void* dgate, int64_t osb, int64_t osh,
+                              int64_t osn, float* dbias, const float* dq_accum, float scale, const fox_tensor4* dq) {
   if (!dlam_col || !dgate || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (gate_kind != FOX_GATE_LOG && !fgate_logit) return FOX_ERR_BAD_ARG;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
@@ -632,7 +627,7 @@ extern "C" int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, in
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   const bool log_gate = gate_kind == FOX_GATE_LOG;
   const RevParams rev{dlam_col, dlam_row, nullptr, log_gate ? (float*)dgate : nullptr, nullptr, (int)M, (int)N,
-                      fgate_logit, dgate, sb, sh, sn, osb, osh, osn, (int)H, gate_bias, dbias};
+                      fgate_logit, dgate, sb, sh, sn, osb, osh, osn, (int)H, dbias};
   ConvParams conv{};
   if (dq) conv = make_conv(B, H, M, D, dq_accum, D > kAccumCols ? D : kAccumCols, scale, dq);
   return launch_finish((cudaStream_t)stream, gate_kind, dtype == FOX_DTYPE_BF16, rev, (int)(B * H), conv);
@@ -650,7 +645,7 @@ extern "C" int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D) {
 
 extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M,
                                  int64_t N, int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn,
-                                 const float* gate_bias, const int64_t* seq_start, float* log_lambda, const fox_tensor4* k, float* k_parts,
+                                 const int64_t* seq_start, float* log_lambda, const fox_tensor4* k, float* k_parts,
                                  int64_t n_k_parts, const fox_tensor4* q, float* q_parts, int64_t n_q_parts) {
   if (!gates || !log_lambda || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
@@ -672,8 +667,8 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == FOX_DTYPE_BF16;
 #define FOX_PRO(K)                                                                                                       \
-  if (bf) fox_prologue_kernel<K, true><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, gate_bias, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D); \
-  else fox_prologue_kernel<K, false><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, gate_bias, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D)
+  if (bf) fox_prologue_kernel<K, true><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D); \
+  else fox_prologue_kernel<K, false><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D)
   switch (gate_kind) {
     case FOX_DTYPE_FP16: FOX_PRO(0); break;
     case FOX_DTYPE_BF16: FOX_PRO(1); break;

@@ -109,7 +109,7 @@ static void prepare_launch(const AttnCall& c, const AttnNorms& n, float* norms, 
   float* q_parts = n.n_q ? norms + c.BH() * n.n_k : nullptr;
   launch("fox_attn_prologue", c.st, [&] {
     return fox_attn_prologue(c.device, c.st, c.code, c.gate_kind, s.B, s.H, s.M, s.N, s.D, c.gate, c.gate_st[0], c.gate_st[1],
-                             c.gate_st[2], c.gate_bias, c.seq_start, c.lam, n.n_k ? &c.k : nullptr, k_parts, n.n_k,
+                             c.gate_st[2], c.seq_start, c.lam, n.n_k ? &c.k : nullptr, k_parts, n.n_k,
                              n.n_q ? &c.q : nullptr, q_parts, n.n_q);
   });
   if (kind == Threshold::kNone) return;
@@ -174,7 +174,7 @@ void attn_backward_launch(const AttnCall& c, const AttnGradCall& g) {
   // through log sigmoid, in the logits' dtype and layout
   launch("fox_bwd_finish", st, [&] {
     return fox_bwd_finish(dev, st, c.code, B, H, M, N, D, dlam_col, dlam_row, c.gate_kind, c.gate, c.gate_st[0], c.gate_st[1],
-                          c.gate_st[2], c.gate_bias, g.dgate, g.dgate_st[0], g.dgate_st[1], g.dgate_st[2], g.dbias,
+                          c.gate_st[2], g.dgate, g.dgate_st[0], g.dgate_st[1], g.dgate_st[2], g.dbias,
                           g.two_kernel ? nullptr : dq_accum, c.sm_scale, g.two_kernel ? nullptr : &g.dq);
   });
   status_pending(dev);

@@ -60,7 +60,6 @@ struct AttnCall {
   int gate_kind = FOX_GATE_LOG;      // or the dtype of gate logits
   const void* gate = nullptr;
   int64_t gate_st[3] = {0, 0, 0};    // b, h, t strides
-  const float* gate_bias = nullptr;
   float *lam = nullptr, *L = nullptr;              // (B,H,N), (B,H,M)
   int64_t *start = nullptr, *end = nullptr;        // with a threshold (end: with gradients)
 

@@ -138,7 +138,7 @@ bool read_block(PyObject* self, const Tensor& x, Block& b) {
     return false;
   if (!open_plain(attn, s_fgate_proj, kLinearCls, m) || !matrix(m, x, H, C, b.p[B::kFGate])) return false;
   PyObject* fb = m.param(s_bias);
-  if (fb && fb != Py_None && !vector(fb, x, H, b.p[B::kFBias])) return false;
+  if (fb && fb != Py_None && (!vector(fb, x, H, b.p[B::kFBias]) || b.p[B::kFBias].scalar_type() != dt)) return false;
   if (!open_plain(mlp, s_gate_proj, kLinearCls, m) || !no_bias(m) || !tensor(m.param(s_weight), b.p[B::kGate])) return false;
   const Tensor& g = b.p[B::kGate];
   if (g.dim() != 2 || g.size(0) % 16 || !matrix(m, x, g.size(0), C, b.p[B::kGate])) return false;
@@ -186,7 +186,8 @@ struct Arena {
 // what the forward leaves for the backward
 struct Acts {
   uint16_t *stack, *hn, *y, *qn, *kn, *vs, *o, *gated, *z, *m, *packed;
-  float *w_attn, *w_q, *w_k, *w_o, *w_mlp, *w_bias;   // parameters as fp32, one after another
+  float *w_attn, *w_q, *w_k, *w_o, *w_mlp;            // norm weights as fp32, one after another
+  uint16_t* bias;                                     // of the stacked product (ld), or null
   float *r_attn, *r_mlp, *r_q, *r_k, *r_o;            // reciprocal norms
   float *lam, *L, *norms;
   int64_t *start, *end, *seq;
@@ -206,12 +207,12 @@ size_t lay_out(const Shape& s, char* base, Acts& a) {
   a.z = m.take<uint16_t>(n * s.C);
   a.m = m.take<uint16_t>(n * s.C);
   a.packed = m.take<uint16_t>(n * 2 * s.inter);
-  a.w_attn = m.take<float>(5 * s.C + s.H);
+  a.w_attn = m.take<float>(5 * s.C);
   a.w_q = a.w_attn + s.C;
   a.w_k = a.w_q + s.C;
   a.w_o = a.w_k + s.C;
   a.w_mlp = a.w_o + s.C;
-  a.w_bias = s.bias ? a.w_mlp + s.C : nullptr;
+  a.bias = s.bias ? m.take<uint16_t>(s.ld) : nullptr;
   a.r_attn = m.take<float>(n);
   a.r_mlp = m.take<float>(n);
   a.r_q = m.take<float>(n * s.H);
@@ -276,7 +277,6 @@ AttnCall attn_call(const Shape& s, const Acts& a, int dev, cudaStream_t st, int 
   c.gate_st[0] = s.T * s.ld;
   c.gate_st[1] = 1;
   c.gate_st[2] = s.ld;
-  c.gate_bias = a.w_bias;
   c.lam = a.lam;
   c.L = a.L;
   c.start = a.start;
@@ -294,17 +294,19 @@ void pack(int dev, cudaStream_t st, const Block& b, const Shape& s, const Acts& 
     mp[i] = b.p[mats[i]].const_data_ptr();
     rows[i] = b.p[mats[i]].size(0);
   }
-  const B::Param vs[] = {B::kAttnNorm, B::kQNorm, B::kKNorm, B::kONorm, B::kMlpNorm, B::kFBias};
-  const int nv = s.bias ? 6 : 5;
-  const void* vp[6];
-  int64_t len[6];
-  int32_t vd[6];
-  for (int i = 0; i < nv; ++i) {
+  const B::Param vs[] = {B::kAttnNorm, B::kQNorm, B::kKNorm, B::kONorm, B::kMlpNorm};
+  const void* vp[5];
+  int64_t len[5];
+  int32_t vd[5];
+  for (int i = 0; i < 5; ++i) {
     vp[i] = b.p[vs[i]].const_data_ptr();
     len[i] = b.p[vs[i]].size(0);
     vd[i] = dtype_code(b.p[vs[i]].scalar_type());
   }
-  launch("fox_pack", st, [&] { return fox_pack(dev, st, 7, mp, rows, s.ld, s.C, a.stack, nv, vp, len, vd, a.w_attn); });
+  launch("fox_pack", st, [&] {
+    return fox_pack(dev, st, 7, mp, rows, s.ld, s.C, a.stack, 5, vp, len, vd, a.w_attn,
+                    s.bias ? b.p[B::kFBias].const_data_ptr() : nullptr, s.H, 4 * s.C, a.bias);
+  });
 }
 
 struct Forward {
@@ -334,7 +336,7 @@ Forward forward(const Block& b, const Shape& s, const Tensor& x_in, const Tensor
   launch("fox_rmsnorm_fwd", st, [&] {
     return fox_rmsnorm_fwd(dev, st, code, s.tokens, s.C, x.const_data_ptr(), nullptr, a.w_attn, b.attn_eps, a.hn, nullptr, a.r_attn);
   });
-  gemm(g, s.tokens, s.ld, s.C, a.hn, s.C, false, a.stack, s.C, true, nullptr, 0, a.y, s.ld);
+  gemm(g, s.tokens, s.ld, s.C, a.hn, s.C, false, a.stack, s.C, true, nullptr, 0, a.y, s.ld, a.bias);
   const int64_t* mask_p = nullptr;
   if (mask.defined()) {
     f.mask = mask.to(at::kLong).contiguous();

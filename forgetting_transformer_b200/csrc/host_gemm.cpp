@@ -55,15 +55,23 @@ constexpr size_t kMostPlans = 4096;
 std::mutex g_plans_mu;
 std::unordered_map<Key, std::shared_ptr<const Plan>, KeyHash> g_plans;
 
-std::shared_ptr<const Plan> make_plan(cublasLtHandle_t h, const Key& key, bool ta, bool tb, bool bf16, uint32_t align) {
+// (of an operation descriptor) the library's matrices are column-major: D^T = op(B)^T op(A)^T, so B is its first operand
+void describe(cublasLtMatmulDesc_t op, bool ta, bool tb, const void* bias) {
+  const cublasOperation_t opb = tb ? CUBLAS_OP_T : CUBLAS_OP_N, opa = ta ? CUBLAS_OP_T : CUBLAS_OP_N;
+  lt(cublasLtMatmulDescSetAttribute(op, CUBLASLT_MATMUL_DESC_TRANSA, &opb, sizeof(opb)), "cublasLtMatmulDescSetAttribute");
+  lt(cublasLtMatmulDescSetAttribute(op, CUBLASLT_MATMUL_DESC_TRANSB, &opa, sizeof(opa)), "cublasLtMatmulDescSetAttribute");
+  if (!bias) return;
+  const cublasLtEpilogue_t add = CUBLASLT_EPILOGUE_BIAS;
+  lt(cublasLtMatmulDescSetAttribute(op, CUBLASLT_MATMUL_DESC_EPILOGUE, &add, sizeof(add)), "cublasLtMatmulDescSetAttribute");
+  lt(cublasLtMatmulDescSetAttribute(op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof(bias)), "cublasLtMatmulDescSetAttribute");
+}
+
+std::shared_ptr<const Plan> make_plan(cublasLtHandle_t h, const Key& key, bool ta, bool tb, bool bf16, uint32_t align, const void* bias) {
   const int64_t m = key.v[0], n = key.v[1], k = key.v[2];
   auto p = std::make_shared<Plan>();
   const cudaDataType_t dt = bf16 ? CUDA_R_16BF : CUDA_R_16F;
   lt(cublasLtMatmulDescCreate(&p->op, CUBLAS_COMPUTE_32F, CUDA_R_32F), "cublasLtMatmulDescCreate");
-  // the library's matrices are column-major: D^T = op(B)^T op(A)^T, so B is its first operand
-  const cublasOperation_t opb = tb ? CUBLAS_OP_T : CUBLAS_OP_N, opa = ta ? CUBLAS_OP_T : CUBLAS_OP_N;
-  lt(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSA, &opb, sizeof(opb)), "cublasLtMatmulDescSetAttribute");
-  lt(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSB, &opa, sizeof(opa)), "cublasLtMatmulDescSetAttribute");
+  describe(p->op, ta, tb, bias);
   lt(cublasLtMatrixLayoutCreate(&p->b, dt, tb ? k : n, tb ? n : k, key.v[4]), "cublasLtMatrixLayoutCreate");
   lt(cublasLtMatrixLayoutCreate(&p->a, dt, ta ? m : k, ta ? k : m, key.v[3]), "cublasLtMatrixLayoutCreate");
   lt(cublasLtMatrixLayoutCreate(&p->c, dt, n, m, key.v[5]), "cublasLtMatrixLayoutCreate");
@@ -90,7 +98,7 @@ std::shared_ptr<const Plan> make_plan(cublasLtHandle_t h, const Key& key, bool t
 }  // namespace
 
 void gemm(const Gemm& g, int64_t m, int64_t n, int64_t k, const void* A, int64_t lda, bool ta, const void* B, int64_t ldb, bool tb,
-          const void* C, int64_t ldc, void* D, int64_t ldd) {
+          const void* C, int64_t ldc, void* D, int64_t ldd, const void* bias) {
   const bool bf16 = g.code == FOX_DTYPE_BF16;
   if (!C) {
     C = D;
@@ -102,7 +110,7 @@ void gemm(const Gemm& g, int64_t m, int64_t n, int64_t k, const void* A, int64_t
                          reinterpret_cast<uintptr_t>(D) | 256;
   const uint32_t align = static_cast<uint32_t>(bits & (~bits + 1));
   const Key key{{m, n, k, lda, ldb, ldc, ldd,
-                 static_cast<int64_t>(g.device) | (ta ? 64 : 0) | (tb ? 128 : 0) | (bf16 ? 256 : 0) | (beta != 0.f ? 512 : 0) |
+                 static_cast<int64_t>(g.device) | (ta ? 64 : 0) | (tb ? 128 : 0) | (bf16 ? 256 : 0) | (beta != 0.f ? 512 : 0) | (bias ? 1024 : 0) |
                      (static_cast<int64_t>(align) << 16)}};
   const cublasLtHandle_t h = handle(g.device);
   std::shared_ptr<const Plan> p;
@@ -112,12 +120,20 @@ void gemm(const Gemm& g, int64_t m, int64_t n, int64_t k, const void* A, int64_t
     if (it != g_plans.end()) p = it->second;
   }
   if (!p) {
-    p = make_plan(h, key, ta, tb, bf16, align);
+    p = make_plan(h, key, ta, tb, bf16, align, bias);
     std::lock_guard<std::mutex> lock(g_plans_mu);
     if (g_plans.size() >= kMostPlans) g_plans.clear();
     g_plans.emplace(key, p);
   }
-  lt(cublasLtMatmul(h, p->op, &alpha, B, p->b, A, p->a, &beta, C, p->c, D, p->d, &p->algo, g.work, kGemmWorkspace, g.st),
+  // (the remembered descriptor is shared and holds another call's bias pointer: a bias takes one of its own)
+  cublasLtMatmulDescOpaque_t own;
+  cublasLtMatmulDesc_t op = p->op;
+  if (bias) {
+    lt(cublasLtMatmulDescInit(&own, CUBLAS_COMPUTE_32F, CUDA_R_32F), "cublasLtMatmulDescInit");
+    op = &own;
+    describe(op, ta, tb, bias);
+  }
+  lt(cublasLtMatmul(h, op, &alpha, B, p->b, A, p->a, &beta, C, p->c, D, p->d, &p->algo, g.work, kGemmWorkspace, g.st),
      "cublasLtMatmul");
 }
 

@@ -115,13 +115,12 @@ int fox_max_row_norm(int device, void* stream, int dtype, int64_t B, int64_t H, 
                      const fox_tensor4* x, float* out_zeroed);
 
 /* What the operator needs before its forward kernel, in one launch: the prefix sum of the gates (fox_cumsum_fwd /
- * fox_gate_prefix_fwd; gate_kind FOX_GATE_LOG or the dtype of gate logits, to which gate_bias (H) fp32 is added if
- * given) and, where k (q) is given, the largest row
- * norm of every (b,h) as n partial maxima, k_parts (B,H,n_k_parts), fully written; n from fox_norm_parts, <= 32. */
+ * fox_gate_prefix_fwd; gate_kind FOX_GATE_LOG or the dtype of gate logits) and, where k (q) is given, the largest row norm of
+ * every (b,h) as n partial maxima, k_parts (B,H,n_k_parts), fully written; n from fox_norm_parts, <= 32. */
 int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D);
 int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M, int64_t N,
-                      int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn, const float* gate_bias,
-                      const int64_t* seq_start, float* log_lambda, const fox_tensor4* k, float* k_parts, int64_t n_k_parts, const fox_tensor4* q,
+                      int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
+                      float* log_lambda, const fox_tensor4* k, float* k_parts, int64_t n_k_parts, const fox_tensor4* q,
                       float* q_parts, int64_t n_q_parts);
 
 /* fox_find_index for one threshold value, or (q_parts, k_parts given) for the automatic threshold of
@@ -216,11 +215,11 @@ int fox_dq_convert(int device, void* stream, int dtype, int64_t B, int64_t H, in
                    const float* dq_accum, float scale, const fox_tensor4* dq);
 
 /* The end of the backward in one launch: the gate gradient (fox_revcumsum for gate_kind FOX_GATE_LOG, else
- * fox_gate_prefix_bwd of the logits with strides (sb, sh, sn), gate_bias added) into dgate with strides (osb, osh, osn),
+ * fox_gate_prefix_bwd of the logits with strides (sb, sh, sn)) into dgate with strides (osb, osh, osn),
  * dbias (B*H) fp32 or NULL = each (b,h)'s sum of it (logits only) and, when dq is not NULL, dq = dq_accum (B,H,M,max(D,64)) * scale. */
 int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N, int64_t D,
                    const float* dlam_col, const float* dlam_row, int gate_kind, const void* fgate_logit, int64_t sb,
-                   int64_t sh, int64_t sn, const float* gate_bias, void* dgate, int64_t osb, int64_t osh, int64_t osn,
+                   int64_t sh, int64_t sn, void* dgate, int64_t osb, int64_t osh, int64_t osn,
                    float* dbias, const float* dq_accum, float scale, const fox_tensor4* dq);
 
 /* Fused per-head RMSNorm + sigmoid gate, forward: y = x * rstd * w_h * sigmoid(g) with
@@ -267,10 +266,11 @@ int fox_mix_bwd(int device, void* stream, int dtype, int64_t B, int64_t T, int64
                 int64_t n_partials);
 
 /* Parameters laid out in one launch: up to 8 contiguous 16-bit (mat_rows[i], cols) matrices stacked into (rows, cols),
- * the rows past them zero; up to 6 vectors (vec_dtype[i]: FOX_DTYPE_*) as fp32, one after another. */
+ * the rows past them zero; up to 6 vectors (vec_dtype[i]: FOX_DTYPE_*) as fp32, one after another; and, where bias_out (rows)
+ * is given, the n_bias 16-bit values of bias from bias_row on, zeros around them. */
 int fox_pack(int device, void* stream, int64_t n_mats, const void* const* mats, const int64_t* mat_rows, int64_t rows,
              int64_t cols, void* stack, int64_t n_vecs, const void* const* vecs, const int64_t* vec_len,
-             const int32_t* vec_dtype, float* vecs_out);
+             const int32_t* vec_dtype, float* vecs_out, const void* bias, int64_t n_bias, int64_t bias_row, void* bias_out);
 
 /* outs[i][c] = sum over rows of parts[i] (rows[i], cols[i]) fp32, in out_dtype[i]; up to 6 arrays. */
 int fox_column_sums(int device, void* stream, int64_t n, const float* const* parts, const int64_t* rows,

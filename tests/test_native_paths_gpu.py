@@ -213,3 +213,30 @@ def test_token_step_with_vectors_that_are_not_aligned(which):
             res.append([blk(x, None, cache, 0)] + [t.clone() for t in cache[0]] + [cache.key_shift_cache[0].clone()])
     for a, b in zip(*res):      # (native against modules: 8 roundings to 16 bits)
         assert (a.float() - b.float()).norm() <= 2 ** -6 * a.float().norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gate_bias_is_added_before_the_projection_is_rounded(dtype):
+    """Projections near -40 and a bias of 40: the logits lie near 0, where a projection rounded to 16 bits on its own is wrong
+    by up to half an ulp of 40 (0.125 in bf16, 0.016 in fp16).  Native and module by module each round a logit once, so the
+    gates' share of the results differs by the dozen roundings of the chain."""
+    C, H, T = 256, 4, 300
+    blk, x, dy = _block(C, H, 512, dtype), _x(T, C, dtype), _x(T, C, dtype, seed=2)
+    with torch.no_grad():
+        x[..., 0] = 8.0
+        h = blk.attn_norm(x)[..., 0].float()
+        blk.attn.fgate_proj.weight[:, 0] = -40.0 / h.mean()
+        blk.attn.fgate_proj.bias.fill_(40.0)
+    res = []
+    for native in (True, False):
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        blk.zero_grad(set_to_none=True)
+        out = blk(x)
+        out.backward(dy)
+        res.append([(out - x).detach(), blk.attn.fgate_proj.weight.grad[:, 1:], blk.attn.fgate_proj.bias.grad,
+                    blk.attn.v_proj.linear.weight.grad])
+        if hook is not None:
+            hook.remove()
+    tol = 12 * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
+    for a, b in zip(*res):
+        assert (a.float() - b.float()).norm() <= tol * b.float().norm()
