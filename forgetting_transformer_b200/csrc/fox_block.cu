@@ -35,7 +35,8 @@ template <bool kBf16>
 __device__ __forceinline__ float blk_load1(const uint16_t* p) {
   return unpack2<kBf16>(static_cast<uint32_t>(*p)).x;
 }
-__device__ __forceinline__ float blk_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+// (in full fp32, as torch.sigmoid: the mixing weights are few; __fdividef would give 0 where 1 + exp(-x) is above 2^126)
+__device__ __forceinline__ float blk_sigmoid(float x) { return __frcp_rn(1.f + expf(-x)); }
 __device__ __forceinline__ float head_sum(float x, int lanes) {
   for (int o = lanes >> 1; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;

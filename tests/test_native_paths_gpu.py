@@ -6,6 +6,7 @@ import torch.autograd.forward_ad as fwAD
 from torch.utils._python_dispatch import TorchDispatchMode
 
 import forgetting_transformer_b200 as fox
+from forgetting_transformer_b200 import _lib
 from oracle import fox_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -240,3 +241,35 @@ def test_gate_bias_is_added_before_the_projection_is_rounded(dtype):
     tol = 12 * (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12)
     for a, b in zip(*res):
         assert (a.float() - b.float()).norm() <= tol * b.float().norm()
+
+
+@pytest.mark.parametrize("kernel", ["step", "sequence"])
+def test_mixing_weights_are_full_fp32_sigmoids(kernel):
+    """sigmoid(-87.5) = 9.98e-39 against a previous value of 1e38 makes 0.998; the approximate division gives 0 there, since
+    1 + exp(87.5) lies above 2^126.  (Elsewhere it is a few fp32 ulp off, which the 16-bit result does not show.)"""
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    B, H, D = 1, 2, 16
+    C, ld = H * D, 4 * H * D + 8      # rows [q | k | v | ogate | fgate (H) | k mix (H) | v mix (H) | pad]
+    dt = torch.bfloat16
+    w = torch.ones(C, device="cuda")
+    if kernel == "step":
+        y = torch.zeros(B, ld, device="cuda")
+        y[:, 4 * C + 2 * H:4 * C + 3 * H] = -87.5
+        q, ks = torch.empty(B, C, device="cuda", dtype=dt), torch.ones(B, C, device="cuda", dtype=dt)
+        vs = torch.full((B, C), 1e38, device="cuda", dtype=dt)
+        k, v, g = torch.empty(B, H, 8, D, device="cuda", dtype=dt), torch.empty(B, H, 8, D, device="cuda", dtype=dt), torch.empty(B, H, 8, device="cuda")
+        rc = lib.fox_step_mix(0, st, _lib.FOX_DTYPE_BF16, B, H, D, y.data_ptr(), ld, w.data_ptr(), _lib.FOX_DTYPE_FP32, w.data_ptr(),
+                              _lib.FOX_DTYPE_FP32, 1e-6, None, 0, None, None, ks.data_ptr(), vs.data_ptr(), q.data_ptr(), k.data_ptr(),
+                              v.data_ptr(), g.data_ptr(), 8, 0)
+        got = v[:, :, 0]
+    else:
+        y = torch.zeros(2, ld, device="cuda", dtype=dt)
+        y[:, 4 * C + 2 * H:4 * C + 3 * H] = -87.5
+        y[0, 2 * C:3 * C] = 1e38
+        q, k, v = torch.empty(3, 2, C, device="cuda", dtype=dt)
+        rc = lib.fox_mix_fwd(0, st, _lib.FOX_DTYPE_BF16, B, 2, H, D, y.data_ptr(), ld, w.data_ptr(), w.data_ptr(), 1e-6, None,
+                             q.data_ptr(), k.data_ptr(), v.data_ptr(), None, None, None)
+        got = v[1]
+    assert rc == 0
+    ref = torch.sigmoid(torch.tensor(-87.5, dtype=torch.float64)).item() * torch.tensor(1e38).to(dt).double().item()
+    assert (got.double() - ref).abs().max() <= 2 ** -8 * ref
