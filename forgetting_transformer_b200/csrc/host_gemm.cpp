@@ -79,8 +79,8 @@ std::shared_ptr<const Plan> make_plan(cublasLtHandle_t h, const Key& key, bool t
   cublasLtMatmulPreference_t pref;
   lt(cublasLtMatmulPreferenceCreate(&pref), "cublasLtMatmulPreferenceCreate");
   const size_t ws = kGemmWorkspace;
-  // split reductions only in fp32
-  const uint32_t reductions = CUBLASLT_REDUCTION_SCHEME_NONE | CUBLASLT_REDUCTION_SCHEME_INPLACE | CUBLASLT_REDUCTION_SCHEME_COMPUTE_TYPE;
+  // split reductions only in fp32 (the in-place scheme adds partial sums in the output's 16 bits)
+  const uint32_t reductions = CUBLASLT_REDUCTION_SCHEME_NONE | CUBLASLT_REDUCTION_SCHEME_COMPUTE_TYPE;
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &ws, sizeof(ws));
   cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, &reductions, sizeof(reductions));
   for (auto attr : {CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES,

@@ -273,3 +273,28 @@ def test_mixing_weights_are_full_fp32_sigmoids(kernel):
     assert rc == 0
     ref = torch.sigmoid(torch.tensor(-87.5, dtype=torch.float64)).item() * torch.tensor(1e38).to(dt).double().item()
     assert (got.double() - ref).abs().max() <= 2 ** -8 * ref
+
+
+@pytest.mark.parametrize("C,H,inter", [(256, 4, 96), (256, 2, 512), (512, 8, 1408)])
+def test_long_sums_over_tokens_are_kept_in_fp32(C, H, inter):
+    """Weight gradient of down_proj over 16384 tokens: the first half adds about 10^6 to every element and the second takes it
+    away again.  Partial sums in fp16 overflow, whichever way the tokens are split; what is left, some thousands, does not."""
+    T = 16384
+    blk, x = _block(C, H, inter, torch.float16), _x(T, C, torch.float16)
+    with torch.no_grad():
+        blk.attn.o_proj.weight.zero_()          # the MLP's input is x itself
+        x[..., 0] = 8.0
+        blk.mlp.gate_proj.weight[:, 0] = 0.4
+    dy = torch.where(torch.arange(T, device="cuda") < T // 2, 20.0, -20.0).half()[None, :, None].expand(1, T, C).contiguous()
+    blk(x).backward(dy)
+    z = x[0].double()
+    m = z * torch.rsqrt(z.pow(2).mean(-1, keepdim=True) + blk.mlp_norm.eps) * blk.mlp_norm.weight.double()
+    g, u = (m @ blk.mlp.gate_proj.weight.double().t()).chunk(2, -1)
+    act = torch.nn.functional.silu(g) * u
+    ref = dy[0].double().t() @ act
+    assert (dy[0, :T // 2].double().t() @ act[:T // 2]).abs().min() > 4 * 65504 and ref.abs().max() < 65504
+    # act carries about two roundings to 11 bits per token, which add up as a random walk over the tokens; the result is
+    # rounded once
+    walk = 20.0 * act.abs().max() * 2 * 2.0 ** -12 * T ** 0.5
+    err = (blk.mlp.down_proj.weight.grad.double() - ref).abs().max()
+    assert err <= 4 * walk + 2.0 ** -11 * ref.abs().max(), (err.item(), walk.item())
