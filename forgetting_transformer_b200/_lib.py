@@ -214,8 +214,8 @@ def status_buffer(device: torch.device) -> torch.Tensor:
 
 
 def poll_status(device: torch.device) -> None:
-    """Non-synchronising check, made by every forward after a backward: raises FoxError when a bounded wait inside a
-    kernel of an earlier step has run out (the results of that step are incomplete)."""
+    """Non-synchronising check, made by every call: raises FoxError when a bounded wait inside a kernel of an earlier call
+    has run out (the results of that call are incomplete)."""
     host().status_poll(_ordinal(device))
 
 

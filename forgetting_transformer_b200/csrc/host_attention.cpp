@@ -177,7 +177,6 @@ void attn_backward_launch(const AttnCall& c, const AttnGradCall& g) {
                           c.gate_st[2], g.dgate, g.dgate_st[0], g.dgate_st[1], g.dgate_st[2], g.dbias,
                           g.two_kernel ? nullptr : dq_accum, c.sm_scale, g.two_kernel ? nullptr : &g.dq);
   });
-  status_pending(dev);
   if (debug_sync()) status_check(dev);
 }
 

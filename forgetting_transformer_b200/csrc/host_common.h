@@ -52,10 +52,10 @@ inline void launch(const char* name, cudaStream_t st, F&& f) {
 }
 
 // int32[4] in pinned host memory that a kernel writes when a bounded wait runs out (never otherwise), so that looking
-// at it costs the host a load instead of a queued copy and an event per step.
+// at it costs the host a load instead of a queued copy and an event per step.  Every call looks: the kernels that write may
+// still run at the first call after them.
 int32_t* status_words(int device);
-void status_pending(int device);   // a backward has been queued: the next call looks at the words
-void status_poll(int device);      // raises FoxError when a pending look finds a record
+void status_poll(int device);      // raises FoxError when there is a record, unless a graph is being captured
 void status_check(int device);     // synchronising look
 
 inline int dtype_code(at::ScalarType t) {

@@ -3,6 +3,9 @@
 // operator) against some 50 us of kernels; here the same work is direct C++ calls.
 #include "host_common.h"
 
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -58,7 +61,7 @@ namespace {
 constexpr int kMaxDevices = 64;
 struct Status {
   Tensor words;
-  bool pending = false;
+  std::atomic<int32_t*> ptr{nullptr};   // of `words`, once they are there
 };
 Status g_status[kMaxDevices];
 std::mutex g_status_mu;
@@ -71,11 +74,16 @@ Status& status_of(int device) {
 static const Tensor& status_tensor(int device) {
   Status& s = status_of(device);
   std::lock_guard<std::mutex> g(g_status_mu);
-  if (!s.words.defined()) s.words = at::zeros({4}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  if (!s.words.defined()) {
+    s.words = at::zeros({4}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    s.ptr = static_cast<int32_t*>(s.words.data_ptr());
+  }
   return s.words;
 }
-int32_t* status_words(int device) { return static_cast<int32_t*>(status_tensor(device).data_ptr()); }
-void status_pending(int device) { status_of(device).pending = true; }
+int32_t* status_words(int device) {
+  int32_t* p = status_of(device).ptr;
+  return p ? p : static_cast<int32_t*>(status_tensor(device).data_ptr());
+}
 
 static void report(int device, const char* when) {
   // (a record's first word is claimed before the others are written: let the kernel end)
@@ -88,18 +96,16 @@ static void report(int device, const char* when) {
             " thread=" + std::to_string(v[2]) + " detail=" + std::to_string(v[3]));
 }
 void status_poll(int device) {
-  Status& s = status_of(device);
-  if (!s.pending || !s.words.defined()) return;
-  s.pending = false;
-  volatile int32_t* w = status_words(device);
-  if (w[0] != 0) report(device, " in an earlier step");
+  volatile int32_t* w = status_of(device).ptr;
+  // (a report synchronises, which a capture does not allow: the record stays for the next call)
+  if (!w || w[0] == 0 || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return;
+  report(device, " in an earlier step");
 }
 void status_check(int device) {
-  Status& s = status_of(device);
-  if (!s.words.defined()) return;
+  volatile int32_t* w = status_of(device).ptr;
+  if (!w) return;
   c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
   C10_CUDA_CHECK(cudaDeviceSynchronize());
-  volatile int32_t* w = status_words(device);
   if (w[0] != 0) report(device, "");
 }
 
@@ -127,7 +133,7 @@ static FOX_PY(py_status_check) {
   HANDLE_TH_ERRORS
   const int only = static_cast<int>(PyLong_AsLong(args[0]));
   for (int d = 0; d < kMaxDevices; ++d)
-    if (g_status[d].words.defined() && (only < 0 || only == d)) status_check(d);
+    if (only < 0 || only == d) status_check(d);
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }

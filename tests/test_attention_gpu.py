@@ -389,9 +389,9 @@ def test_gate_logits_path_matches_the_log_gate_path(D, dtype):
 
 
 def test_expired_wait_is_reported_at_the_next_call():
-    """A kernel that gives up on a bounded wait leaves a record in the device's status words; the operator copies
-    them to pinned host memory after every backward and raises at the next call, without any synchronisation of
-    its own.  The record is made here by writing the status words from the host (no kernel is made to hang)."""
+    """A kernel that gives up on a bounded wait leaves a record in the device's status words, which lie in pinned host memory;
+    every call looks at them and raises, without any synchronisation of its own before it has found a record.  The record
+    is made here by writing the status words from the host (no kernel is made to hang)."""
     q, k, v, lf, do = [t.cuda() for t in _inputs(21, 1, 2, 256, 256, 64, torch.bfloat16)]
     dev = q.device
     for t in (q, k, v, lf):
@@ -400,8 +400,6 @@ def test_expired_wait_is_reported_at_the_next_call():
     torch.cuda.synchronize()
     fox.forgetting_attention(q, k, v, lf, head_first=True)          # nothing to report
     _lib.status_buffer(dev).copy_(torch.tensor([34, 5, 96, 7], dtype=torch.int32))
-    fox.forgetting_attention(q, k, v, lf, head_first=True).backward(do)   # queues the readback
-    torch.cuda.synchronize()
     with pytest.raises(fox.FoxError, match="site=34 cta=5 thread=96 detail=7"):
         fox.forgetting_attention(q, k, v, lf, head_first=True)
     fox.forgetting_attention(q, k, v, lf, head_first=True).backward(do)   # the record was cleared

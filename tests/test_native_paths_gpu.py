@@ -298,3 +298,25 @@ def test_long_sums_over_tokens_are_kept_in_fp32(C, H, inter):
     walk = 20.0 * act.abs().max() * 2 * 2.0 ** -12 * T ** 0.5
     err = (blk.mlp.down_proj.weight.grad.double() - ref).abs().max()
     assert err <= 4 * walk + 2.0 ** -11 * ref.abs().max(), (err.item(), walk.item())
+
+
+def test_expired_wait_after_the_last_backward_is_reported():
+    """The first call after a backward usually finds its kernels still running; a record they leave later is reported by the
+    calls after it, which need not be preceded by another backward, but not into a capture."""
+    q, k, v, g = _qkvg()
+    q.requires_grad_()
+    fox.forgetting_attention(q, k, v, g, head_first=True).sum().backward()
+    with torch.no_grad():
+        fox.forgetting_attention(q, k, v, g, head_first=True)
+        torch.cuda.synchronize()
+        words = _lib.status_buffer(q.device)
+        words.copy_(torch.tensor([34, 5, 96, 7], dtype=torch.int32))
+        try:
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                fox.forgetting_attention(q, k, v, g, head_first=True)
+            with pytest.raises(fox.FoxError, match="site=34 cta=5 thread=96 detail=7"):
+                fox.forgetting_attention(q, k, v, g, head_first=True)
+        finally:
+            words.zero_()
+        fox.forgetting_attention(q, k, v, g, head_first=True)
+    fox.check_status()
