@@ -464,15 +464,17 @@ struct BlockBackward : public torch::autograd::Node {
     static const B::Param mats[] = {B::kQ, B::kK, B::kV, B::kOGate, B::kFGate, B::kKMix, B::kVMix};
     bool any = false;
     for (B::Param m : mats) any = any || want(m);
-    if (any) {   // one product; the parameters' gradients are row ranges of it
+    if (any) {   // one product, taken apart
       const Tensor dstack = at::empty({s.ld, C}, o16);
       gemm(g, s.ld, C, n, t.dy, s.ld, true, a.hn, C, false, nullptr, 0, dstack.mutable_data_ptr(), C);
-      int64_t row = 0;
+      void* dst[7];
+      int64_t rows[7];
       for (int i = 0; i < 7; ++i) {
-        const int64_t rows = i < 4 ? C : s.H;
-        if (want(mats[i])) out[1 + mats[i]] = dstack.narrow(0, row, rows);
-        row += rows;
+        rows[i] = i < 4 ? C : s.H;
+        if (want(mats[i])) out[1 + mats[i]] = at::empty({rows[i], C}, o16);
+        dst[i] = want(mats[i]) ? out[1 + mats[i]].mutable_data_ptr() : nullptr;
       }
+      launch("fox_unpack", st, [&] { return fox_unpack(dev, st, 7, dst, rows, C, dstack.const_data_ptr()); });
     }
     gemm(g, n, C, s.ld, t.dy, s.ld, false, a.stack, C, false, nullptr, 0, t.dhn, C);
     const Tensor dx = at::empty(xt.sizes(), o16);

@@ -272,6 +272,11 @@ int fox_pack(int device, void* stream, int64_t n_mats, const void* const* mats, 
              int64_t cols, void* stack, int64_t n_vecs, const void* const* vecs, const int64_t* vec_len,
              const int32_t* vec_dtype, float* vecs_out, const void* bias, int64_t n_bias, int64_t bias_row, void* bias_out);
 
+/* The stacked matrix taken apart again: row ranges of stack (., cols) copied to up to 8 contiguous (mat_rows[i], cols) 16-bit
+ * matrices, one after another; a NULL matrix is left out. */
+int fox_unpack(int device, void* stream, int64_t n_mats, void* const* mats, const int64_t* mat_rows, int64_t cols,
+               const void* stack);
+
 /* outs[i][c] = sum over rows of parts[i] (rows[i], cols[i]) fp32, in out_dtype[i]; up to 6 arrays. */
 int fox_column_sums(int device, void* stream, int64_t n, const float* const* parts, const int64_t* rows,
                     const int64_t* cols, const int32_t* out_dtype, void* const* outs);

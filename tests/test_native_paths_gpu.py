@@ -320,3 +320,22 @@ def test_expired_wait_after_the_last_backward_is_reported():
             words.zero_()
         fox.forgetting_attention(q, k, v, g, head_first=True)
     fox.check_status()
+
+
+@pytest.mark.parametrize("frozen", [(), ("q_proj", "v_proj.shift_proj"), ("q_proj", "k_proj", "v_proj", "ogate_proj", "fgate_proj")])
+def test_block_gradients_have_memory_of_their_own(frozen):
+    """A gradient that is kept or saved holds no other parameter's memory; frozen parameters get none; what is there equals
+    the gradients of the block without frozen parameters."""
+    blk, x, dy = _block(), _x(), _x(seed=2)
+    blk(x).backward(dy)
+    ref = {n: p.grad for n, p in blk.named_parameters()}
+    blk.zero_grad(set_to_none=True)
+    for n, p in blk.named_parameters():
+        p.requires_grad_(not any(f in n for f in frozen))
+    blk(x).backward(dy)
+    for n, p in blk.named_parameters():
+        assert (p.grad is None) == any(f in n for f in frozen)
+        if p.grad is not None:
+            assert p.grad.untyped_storage().nbytes() == p.numel() * p.element_size(), n
+            # (sums by fp32 atomics in the attention: an ulp of the result's type here and there)
+            assert (p.grad.float() - ref[n].float()).norm() <= 2 ** -8 * ref[n].float().norm(), n
