@@ -191,10 +191,8 @@ class FoxProBlock(nn.Module):
         self.mlp_norm = RMSNorm(hidden_size, eps=norm_eps)
         self.mlp = FoxMLP(hidden_size, intermediate_size)
 
-    def _threshold(self, hidden_states: torch.Tensor) -> Optional[torch.Tensor]:
+    def _threshold(self, hidden_states: torch.Tensor) -> torch.Tensor:
         a = self.attn
-        if getattr(a, "log_pruning_tolerance", None) is None or not hasattr(a, "q_norm"):
-            return None
         return acp_threshold_from_qk_norm(a.q_norm.weight, a.k_norm.weight, a.num_heads, a.head_dim,
                                           hidden_states.shape[1], a.log_pruning_tolerance)
 
@@ -205,7 +203,7 @@ class FoxProBlock(nn.Module):
         Without a cache the whole block runs as one native forward and backward where its parts are the plain modules
         built here (no hooks, replaced submodules or autocast) in one 16-bit dtype; else module by module."""
         if past_key_values is None:
-            out = (_host or _load_host()).block(self, hidden_states, attention_mask, self._threshold(hidden_states))
+            out = (_host or _load_host()).block(self, hidden_states, attention_mask, self._threshold)
             if out is not None:
                 return out
         elif hidden_states.shape[1] == 1:     # a generated token: appended to the cache and taken through the block natively

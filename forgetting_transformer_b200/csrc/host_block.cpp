@@ -527,21 +527,29 @@ FOX_PY(py_set_block_classes) {
   END_HANDLE_TH_ERRORS
 }
 
-// block(self, hidden_states, attention_mask or None, threshold or None) -> out, or None where the modules' own forward
-// has to run
+// block(self, hidden_states, attention_mask or None, threshold) -> out, or None where the modules' own forward has to run.
+// threshold(hidden_states) gives the pruning threshold; it is called where there is one and the block runs here.
 FOX_PY(py_block) {
   HANDLE_TH_ERRORS
   Tensor x;
   Block b;
   if (!tensor(args[1], x) || !read_block(args[0], x, b)) Py_RETURN_NONE;
   if (args[2] != Py_None && !plain_tensor(args[2])) Py_RETURN_NONE;
-  const Tensor mask = unpack_opt(args[2], "attention_mask"), threshold = unpack_opt(args[3], "threshold");
-  if (b.pruned != threshold.defined() || x.size(1) < 2 || x.size(0) < 1) Py_RETURN_NONE;
+  const Tensor mask = unpack_opt(args[2], "attention_mask");
+  if (x.size(1) < 2 || x.size(0) < 1) Py_RETURN_NONE;
   if (mask.defined()) {
     const auto d = mask.scalar_type();
     if (mask.dim() != 2 || mask.size(0) != x.size(0) || mask.size(1) != x.size(1) || mask.device() != x.device() ||
         (d != at::kLong && d != at::kBool && d != at::kInt))
       Py_RETURN_NONE;
+  }
+  Tensor threshold;
+  if (b.pruned) {
+    PyObject* t = PyObject_CallOneArg(args[3], args[1]);
+    if (!t) throw python_error();
+    const bool ok = tensor(t, threshold);
+    Py_DECREF(t);
+    if (!ok) Py_RETURN_NONE;
   }
   Tensor out;
   {

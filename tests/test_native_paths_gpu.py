@@ -339,3 +339,14 @@ def test_block_gradients_have_memory_of_their_own(frozen):
             assert p.grad.untyped_storage().nbytes() == p.numel() * p.element_size(), n
             # (sums by fp32 atomics in the attention: an ulp of the result's type here and there)
             assert (p.grad.float() - ref[n].float()).norm() <= 2 ** -8 * ref[n].float().norm(), n
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_pruning_threshold_is_formed_once(native, monkeypatch):
+    blk, calls = _block(log_pruning_tolerance=-10.0), []
+    f = fox.block.acp_threshold_from_qk_norm
+    monkeypatch.setattr(fox.block, "acp_threshold_from_qk_norm", lambda *a: (calls.append(a), f(*a))[1])
+    if not native:
+        blk.attn.q_norm.register_forward_hook(lambda *a: None)
+    out = blk(_x())
+    assert len(calls) == 1 and ("FoxProBlockBackward" in out.grad_fn.name()) == native
