@@ -183,20 +183,42 @@ struct Arena {
   }
 };
 
-// what the forward leaves for the backward
+// what the forward makes, and leaves for the backward where there is one
 struct Acts {
   uint16_t *stack, *hn, *y, *qn, *kn, *vs, *o, *gated, *z, *m, *packed;
+  uint16_t *proj, *act;                               // o_proj's result and the MLP's product: not kept
   float *w_attn, *w_q, *w_k, *w_o, *w_mlp;            // norm weights as fp32, one after another
   uint16_t* bias;                                     // of the stacked product (ld), or null
   float *r_attn, *r_mlp, *r_q, *r_k, *r_o;            // reciprocal norms
   float *lam, *L, *norms;
   int64_t *start, *end, *seq;
-  int64_t norm_floats;
 };
-size_t lay_out(const Shape& s, char* base, Acts& a) {
-  Arena m{base};
+void lay_out_small(const Shape& s, Arena& m, Acts& a, bool keep) {
   const int64_t n = s.tokens, BH = s.B * s.H;
   a.stack = m.take<uint16_t>(s.ld * s.C);
+  a.w_attn = m.take<float>(5 * s.C);
+  a.w_q = a.w_attn + s.C;
+  a.w_k = a.w_q + s.C;
+  a.w_o = a.w_k + s.C;
+  a.w_mlp = a.w_o + s.C;
+  a.bias = s.bias ? m.take<uint16_t>(s.ld) : nullptr;
+  a.r_attn = m.take<float>(n);
+  a.r_mlp = m.take<float>(n);
+  a.r_q = keep ? m.take<float>(n * s.H) : nullptr;
+  a.r_k = keep ? m.take<float>(n * s.H) : nullptr;
+  a.r_o = m.take<float>(n * s.H);
+  a.lam = m.take<float>(BH * s.T);
+  a.L = m.take<float>(BH * s.T);
+  a.norms = m.take<float>(attn_norms(attn_shape(s), false).floats(BH));
+  a.seq = s.mask ? m.take<int64_t>(s.B) : nullptr;
+  a.start = s.pruned ? m.take<int64_t>(BH * attn_blocks(s.T)) : nullptr;
+  a.end = s.pruned && keep ? m.take<int64_t>(BH * attn_blocks(s.T)) : nullptr;
+}
+// For a backward: everything beside everything.
+size_t lay_out(const Shape& s, char* base, Acts& a) {
+  Arena m{base};
+  const int64_t n = s.tokens;
+  lay_out_small(s, m, a, true);
   a.hn = m.take<uint16_t>(n * s.C);
   a.y = m.take<uint16_t>(n * s.ld);
   a.qn = m.take<uint16_t>(n * s.C);
@@ -207,24 +229,27 @@ size_t lay_out(const Shape& s, char* base, Acts& a) {
   a.z = m.take<uint16_t>(n * s.C);
   a.m = m.take<uint16_t>(n * s.C);
   a.packed = m.take<uint16_t>(n * 2 * s.inter);
-  a.w_attn = m.take<float>(5 * s.C);
-  a.w_q = a.w_attn + s.C;
-  a.w_k = a.w_q + s.C;
-  a.w_o = a.w_k + s.C;
-  a.w_mlp = a.w_o + s.C;
-  a.bias = s.bias ? m.take<uint16_t>(s.ld) : nullptr;
-  a.r_attn = m.take<float>(n);
-  a.r_mlp = m.take<float>(n);
-  a.r_q = m.take<float>(n * s.H);
-  a.r_k = m.take<float>(n * s.H);
-  a.r_o = m.take<float>(n * s.H);
-  a.lam = m.take<float>(BH * s.T);
-  a.L = m.take<float>(BH * s.T);
-  a.norms = m.take<float>(attn_norms(attn_shape(s), false).floats(BH));
-  a.seq = s.mask ? m.take<int64_t>(s.B) : nullptr;
-  a.start = s.pruned ? m.take<int64_t>(BH * attn_blocks(s.T)) : nullptr;
-  a.end = s.pruned ? m.take<int64_t>(BH * attn_blocks(s.T)) : nullptr;
   return m.used;
+}
+// Without one: what is done with makes room.  The attention layer's arrays and the MLP's take turns in the same memory, o
+// lies over the normalised input, the gated output over q, o_proj's result over k.
+size_t lay_out_transient(const Shape& s, char* base, Acts& a) {
+  Arena m{base};
+  const int64_t n = s.tokens;
+  lay_out_small(s, m, a, false);
+  const size_t shared = m.used;
+  a.proj = a.kn = m.take<uint16_t>(n * s.C);   // (first: read while m and z behind it are written)
+  a.y = m.take<uint16_t>(n * s.ld);
+  a.o = a.hn = m.take<uint16_t>(n * s.C);
+  a.gated = a.qn = m.take<uint16_t>(n * s.C);
+  a.vs = m.take<uint16_t>(n * s.C);
+  const size_t attn_end = m.used;
+  m.used = shared;
+  a.act = m.take<uint16_t>(n * std::max(s.inter, s.C));   // (over proj, which the norm in front has read by then)
+  a.m = m.take<uint16_t>(n * s.C);
+  a.z = m.take<uint16_t>(n * s.C);
+  a.packed = m.take<uint16_t>(n * 2 * s.inter);
+  return std::max(attn_end, m.used);
 }
 
 // the backward's temporaries: the MLP's and the attention layer's take turns in the same memory
@@ -324,12 +349,13 @@ Forward forward(const Block& b, const Shape& s, const Tensor& x_in, const Tensor
   Forward f;
   const Tensor x = x_in.contiguous();
   Acts a;
-  f.acts = at::empty({static_cast<int64_t>(lay_out(s, nullptr, a))}, bytes);
-  lay_out(s, static_cast<char*>(f.acts.data_ptr()), a);
-  // [product workspace | o_proj's result, then the activations of the MLP]
-  const Tensor temp = at::empty({static_cast<int64_t>(kGemmWorkspace) + 2 * s.tokens * std::max(s.inter, s.C)}, bytes);
+  auto layout = [&](char* base) { return needs_grad ? lay_out(s, base, a) : lay_out_transient(s, base, a); };
+  f.acts = at::empty({static_cast<int64_t>(layout(nullptr))}, bytes);
+  layout(static_cast<char*>(f.acts.data_ptr()));
+  // [product workspace | with a backward: o_proj's result, then the MLP's product]
+  const Tensor temp = at::empty({static_cast<int64_t>(kGemmWorkspace) + (needs_grad ? 2 * s.tokens * std::max(s.inter, s.C) : 0)}, bytes);
   Gemm g{dev, code, st, temp.data_ptr()};
-  uint16_t* const act = reinterpret_cast<uint16_t*>(static_cast<char*>(temp.data_ptr()) + kGemmWorkspace);
+  if (needs_grad) a.proj = a.act = reinterpret_cast<uint16_t*>(static_cast<char*>(temp.data_ptr()) + kGemmWorkspace);
   f.out = at::empty(x_in.sizes(), x_in.options());
 
   pack(dev, st, b, s, a);
@@ -349,22 +375,21 @@ Forward forward(const Block& b, const Shape& s, const Tensor& x_in, const Tensor
   Tensor thr;
   if (threshold.defined()) thr = threshold.detach().to(x_in.device(), at::kFloat).expand({s.B, s.H});
   AttnCall c = attn_call(s, a, dev, st, code);
-  if (!needs_grad) c.end = nullptr;
   attn_forward_launch(c, attn_norms(c.s, false), a.norms, thr.defined() ? Threshold::kTensor : Threshold::kNone, 0.,
                       thr.defined() ? static_cast<float*>(thr.data_ptr()) : nullptr, thr.defined() ? thr.stride(0) : 0,
                       thr.defined() ? thr.stride(1) : 0);
   launch("fox_normgate_fwd", st, [&] {
     return fox_normgate_fwd_ld(dev, st, code, s.tokens, s.H, s.D, a.o, a.y + 3 * s.C, s.ld, a.w_o, b.o_eps, a.gated, a.r_o);
   });
-  gemm(g, s.tokens, s.C, s.C, a.gated, s.C, false, b.p[Block::kO].const_data_ptr(), s.C, true, nullptr, 0, act, s.C);
+  gemm(g, s.tokens, s.C, s.C, a.gated, s.C, false, b.p[Block::kO].const_data_ptr(), s.C, true, nullptr, 0, a.proj, s.C);
   launch("fox_rmsnorm_fwd", st, [&] {
-    return fox_rmsnorm_fwd(dev, st, code, s.tokens, s.C, act, x.const_data_ptr(), a.w_mlp, b.mlp_eps, a.m, a.z, a.r_mlp);
+    return fox_rmsnorm_fwd(dev, st, code, s.tokens, s.C, a.proj, x.const_data_ptr(), a.w_mlp, b.mlp_eps, a.m, a.z, a.r_mlp);
   });
   gemm(g, s.tokens, 2 * s.inter, s.C, a.m, s.C, false, b.p[Block::kGate].const_data_ptr(), s.C, true, nullptr, 0, a.packed, 2 * s.inter);
   launch("fox_swiglu_fwd", st, [&] {
-    return fox_swiglu_fwd(dev, st, code, s.tokens, s.inter, a.packed, 2 * s.inter, a.packed + s.inter, 2 * s.inter, act, s.inter);
+    return fox_swiglu_fwd(dev, st, code, s.tokens, s.inter, a.packed, 2 * s.inter, a.packed + s.inter, 2 * s.inter, a.act, s.inter);
   });
-  gemm(g, s.tokens, s.C, s.inter, act, s.inter, false, b.p[Block::kDown].const_data_ptr(), s.inter, true, a.z, s.C,
+  gemm(g, s.tokens, s.C, s.inter, a.act, s.inter, false, b.p[Block::kDown].const_data_ptr(), s.inter, true, a.z, s.C,
        f.out.mutable_data_ptr(), s.C);
   return f;
 }

@@ -350,3 +350,44 @@ def test_pruning_threshold_is_formed_once(native, monkeypatch):
         blk.attn.q_norm.register_forward_hook(lambda *a: None)
     out = blk(_x())
     assert len(calls) == 1 and ("FoxProBlockBackward" in out.grad_fn.name()) == native
+
+
+def _peak(f):
+    f()
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    f()
+    torch.cuda.synchronize()
+    return torch.cuda.max_memory_allocated() - before
+
+
+@pytest.mark.parametrize("C,H,inter,T", [(1536, 24, 4096, 8192), (768, 12, 2048, 16384), (512, 4, 1408, 16384)])
+def test_block_without_gradients_takes_no_more_memory_than_its_modules(C, H, inter, T):
+    """Beside the 32 MB of the products' workspace and the stacked weights, which do not grow with the tokens, and the few
+    fp32 values per head and token."""
+    blk, x = _block(C, H, inter), _x(T, C)
+    peak = []
+    for native in (True, False):
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        with torch.no_grad():
+            peak.append(_peak(lambda: blk(x)))
+        if hook is not None:
+            hook.remove()
+    fixed = (32 << 20) + 2 * (4 * C + 3 * H + 8) * C + 4 * (2 + 3 * H) * T + (1 << 20)
+    assert peak[0] <= peak[1] + fixed, [p >> 20 for p in peak]
+
+
+@pytest.mark.parametrize("C,H,inter", [(256, 4, 512), (512, 4, 96), (768, 12, 2048)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_block_gives_the_same_with_and_without_gradients(C, H, inter, padded):
+    """The same kernels on the same numbers, in memory that is used again without a backward: bit for bit."""
+    blk, x = _block(C, H, inter), _x(700, C, B=2)
+    mask = None
+    if padded:
+        mask = torch.ones(2, 700, dtype=torch.long, device="cuda")
+        mask[0, :333] = 0
+    ref = blk(x, mask)
+    with torch.no_grad():
+        out = blk(x, mask)
+    assert ref.grad_fn is not None and out.grad_fn is None and torch.equal(out, ref)
