@@ -10,6 +10,7 @@
 
 #include <ATen/autocast_mode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <torch/csrc/autograd/graph_task.h>
 
 #include <cmath>
 
@@ -214,8 +215,16 @@ void lay_out_small(const Shape& s, Arena& m, Acts& a, bool keep) {
   a.start = s.pruned ? m.take<int64_t>(BH * attn_blocks(s.T)) : nullptr;
   a.end = s.pruned && keep ? m.take<int64_t>(BH * attn_blocks(s.T)) : nullptr;
 }
-// For a backward: everything beside everything.
-size_t lay_out(const Shape& s, char* base, Acts& a) {
+// For a backward everything lies beside everything, what the MLP's part of it reads apart: that is released first.
+size_t lay_out_mlp(const Shape& s, char* base, Acts& a) {
+  Arena m{base};
+  const int64_t n = s.tokens;
+  a.z = m.take<uint16_t>(n * s.C);
+  a.m = m.take<uint16_t>(n * s.C);
+  a.packed = m.take<uint16_t>(n * 2 * s.inter);
+  return m.used;
+}
+size_t lay_out_attn(const Shape& s, char* base, Acts& a) {
   Arena m{base};
   const int64_t n = s.tokens;
   lay_out_small(s, m, a, true);
@@ -226,9 +235,6 @@ size_t lay_out(const Shape& s, char* base, Acts& a) {
   a.vs = m.take<uint16_t>(n * s.C);
   a.o = m.take<uint16_t>(n * s.C);
   a.gated = m.take<uint16_t>(n * s.C);
-  a.z = m.take<uint16_t>(n * s.C);
-  a.m = m.take<uint16_t>(n * s.C);
-  a.packed = m.take<uint16_t>(n * 2 * s.inter);
   return m.used;
 }
 // Without one: what is done with makes room.  The attention layer's arrays and the MLP's take turns in the same memory, o
@@ -252,36 +258,48 @@ size_t lay_out_transient(const Shape& s, char* base, Acts& a) {
   return std::max(attn_end, m.used);
 }
 
-// the backward's temporaries: the MLP's and the attention layer's take turns in the same memory
+// The backward's temporaries: what both parts use, the MLP's, the attention layer's.  The last two are never there together.
 struct Temps {
-  uint16_t *dz, *dm;
-  uint16_t *dact, *dpacked, *act;                       // MLP
-  uint16_t *dgated, *dy, *d_o, *dq, *dk, *dv, *dhn;     // attention layer
-  float *attn_work, *parts;
   void* gemm;
+  float* parts;
+  uint16_t* dz;
+  uint16_t *dact, *dpacked, *act, *dm;                           // MLP (dm over dact)
+  uint16_t *dgated, *dy, *d_o, *dq, *dk, *dv, *dhn, *dstack;     // attention layer (dq over dgated, dhn over d_o)
+  float* attn_work;
 };
-size_t lay_out(const Shape& s, char* base, int64_t part_floats, bool two_kernel, Temps& t) {
+size_t lay_out_shared(const Shape& s, char* base, int64_t part_floats, Temps& t) {
   Arena m{base};
-  const int64_t n = s.tokens;
   t.gemm = m.take<char>(static_cast<int64_t>(kGemmWorkspace));
   t.parts = m.take<float>(part_floats);
-  t.dz = m.take<uint16_t>(n * s.C);
-  const size_t shared = m.used;
-  t.dm = m.take<uint16_t>(n * s.C);
-  t.dact = m.take<uint16_t>(n * s.inter);
+  t.dz = m.take<uint16_t>(s.tokens * s.C);
+  return m.used;
+}
+size_t lay_out_mlp(const Shape& s, char* base, Temps& t) {
+  Arena m{base};
+  const int64_t n = s.tokens;
+  t.dm = t.dact = m.take<uint16_t>(n * std::max(s.inter, s.C));
   t.dpacked = m.take<uint16_t>(n * 2 * s.inter);
   t.act = m.take<uint16_t>(n * s.inter);
-  const size_t mlp_end = m.used;
-  m.used = shared;
-  t.dgated = m.take<uint16_t>(n * s.C);
+  return m.used;
+}
+size_t lay_out_attn(const Shape& s, char* base, bool two_kernel, Temps& t) {
+  Arena m{base};
+  const int64_t n = s.tokens;
+  t.dq = t.dgated = m.take<uint16_t>(n * s.C);
   t.dy = m.take<uint16_t>(n * s.ld);
-  t.d_o = m.take<uint16_t>(n * s.C);
-  t.dq = m.take<uint16_t>(n * s.C);
+  t.dhn = t.d_o = m.take<uint16_t>(n * s.C);
   t.dk = m.take<uint16_t>(n * s.C);
   t.dv = m.take<uint16_t>(n * s.C);
-  t.dhn = m.take<uint16_t>(n * s.C);
+  t.dstack = m.take<uint16_t>(s.ld * s.C);
   t.attn_work = m.take<float>(attn_backward_floats(attn_shape(s), two_kernel));
-  return std::max(mlp_end, m.used);
+  return m.used;
+}
+// memory for one of the layouts above, which lay(nullptr) sizes and lay(base) places
+template <typename F>
+Tensor allocate(const at::TensorOptions& bytes, F&& lay) {
+  const Tensor t = at::empty({static_cast<int64_t>(lay(nullptr))}, bytes);
+  lay(static_cast<char*>(t.data_ptr()));
+  return t;
 }
 
 AttnCall attn_call(const Shape& s, const Acts& a, int dev, cudaStream_t st, int code) {
@@ -335,7 +353,7 @@ void pack(int dev, cudaStream_t st, const Block& b, const Shape& s, const Acts& 
 }
 
 struct Forward {
-  Tensor out, acts, mask;
+  Tensor out, acts, mlp_acts, mask;
 };
 
 Forward forward(const Block& b, const Shape& s, const Tensor& x_in, const Tensor& mask, const Tensor& threshold, bool needs_grad) {
@@ -349,9 +367,12 @@ Forward forward(const Block& b, const Shape& s, const Tensor& x_in, const Tensor
   Forward f;
   const Tensor x = x_in.contiguous();
   Acts a;
-  auto layout = [&](char* base) { return needs_grad ? lay_out(s, base, a) : lay_out_transient(s, base, a); };
-  f.acts = at::empty({static_cast<int64_t>(layout(nullptr))}, bytes);
-  layout(static_cast<char*>(f.acts.data_ptr()));
+  if (needs_grad) {
+    f.acts = allocate(bytes, [&](char* base) { return lay_out_attn(s, base, a); });
+    f.mlp_acts = allocate(bytes, [&](char* base) { return lay_out_mlp(s, base, a); });
+  } else {
+    f.acts = allocate(bytes, [&](char* base) { return lay_out_transient(s, base, a); });
+  }
   // [product workspace | with a backward: o_proj's result, then the MLP's product]
   const Tensor temp = at::empty({static_cast<int64_t>(kGemmWorkspace) + (needs_grad ? 2 * s.tokens * std::max(s.inter, s.C) : 0)}, bytes);
   Gemm g{dev, code, st, temp.data_ptr()};
@@ -396,14 +417,14 @@ Forward forward(const Block& b, const Shape& s, const Tensor& x_in, const Tensor
 
 // ---------------------------------------------------------------- backward
 struct BlockBackward : public torch::autograd::Node {
-  SavedVariable x, acts, mask, w_o, w_gate, w_down;
+  SavedVariable x, acts, mlp_acts, mask, w_o, w_gate, w_down;
   at::ScalarType dtypes[Block::kCount];
   bool released = false;
   Shape s;
 
   std::string name() const override { return "FoxProBlockBackward"; }
   void release_variables() override {
-    for (SavedVariable* v : {&x, &acts, &mask, &w_o, &w_gate, &w_down}) v->reset_data();
+    for (SavedVariable* v : {&x, &acts, &mlp_acts, &mask, &w_o, &w_gate, &w_down}) v->reset_data();
     released = true;
   }
 
@@ -413,6 +434,7 @@ struct BlockBackward : public torch::autograd::Node {
     if (!grads[0].defined()) return out;
     if (released) throw std::runtime_error(torch::autograd::ERR_BACKWARD_TWICE);
     const Tensor xt = x.unpack().contiguous(), at_ = acts.unpack(), mt = mask.unpack();
+    Tensor mlp_at = mlp_acts.unpack();
     const Tensor wo = w_o.unpack(), wg = w_gate.unpack(), wd = w_down.unpack();
     const c10::cuda::CUDAGuard guard(xt.device());
     const at::AutoDispatchBelowADInplaceOrView no_autograd;
@@ -423,7 +445,8 @@ struct BlockBackward : public torch::autograd::Node {
     const auto o16 = xt.options();
     const int64_t n = s.tokens, C = s.C, I = s.inter;
     Acts a;
-    lay_out(s, static_cast<char*>(at_.data_ptr()), a);
+    lay_out_attn(s, static_cast<char*>(at_.data_ptr()), a);
+    lay_out_mlp(s, static_cast<char*>(mlp_at.data_ptr()), a);
     auto want = [&](int i) { return task_should_compute_output(1 + i); };
     const Tensor dout = grads[0].contiguous();
 
@@ -432,9 +455,10 @@ struct BlockBackward : public torch::autograd::Node {
     const int64_t mx = fox_mix_bwd_partials(n);
     const bool two_kernel = default_two_kernel(s.D);
     const int64_t part_floats = C * (2 * rn + ng + 2 * mx) + s.B * s.H;
+    const auto bytes = o16.dtype(at::kByte);
     Temps t;
-    const Tensor temp = at::empty({static_cast<int64_t>(lay_out(s, nullptr, part_floats, two_kernel, t))}, o16.dtype(at::kByte));
-    lay_out(s, static_cast<char*>(temp.data_ptr()), part_floats, two_kernel, t);
+    const Tensor shared = allocate(bytes, [&](char* base) { return lay_out_shared(s, base, part_floats, t); });
+    Tensor temp = allocate(bytes, [&](char* base) { return lay_out_mlp(s, base, t); });
     float* part_attn = t.parts;
     float* part_mlp = part_attn + rn * C;
     float* part_o = part_mlp + rn * C;
@@ -462,7 +486,11 @@ struct BlockBackward : public torch::autograd::Node {
     launch("fox_rmsnorm_bwd", st, [&] {
       return fox_rmsnorm_bwd(dev, st, code, n, C, a.z, a.w_mlp, a.r_mlp, t.dm, gout, t.dz, part_mlp, rn);
     });
-    // ---- attention layer
+    // ---- attention layer, in the memory that the MLP's part no longer needs (this stream's, so that reuse keeps the order)
+    temp.reset();
+    mlp_at.reset();
+    if (!torch::autograd::get_current_graph_task_keep_graph()) mlp_acts.reset_data();
+    temp = allocate(bytes, [&](char* base) { return lay_out_attn(s, base, two_kernel, t); });
     gemm(g, n, C, C, t.dz, C, false, wo.const_data_ptr(), C, false, nullptr, 0, t.dgated, C);
     weight_grad(B::kO, C, C, t.dz, a.gated);
     launch("fox_normgate_bwd", st, [&] {
@@ -490,8 +518,7 @@ struct BlockBackward : public torch::autograd::Node {
     bool any = false;
     for (B::Param m : mats) any = any || want(m);
     if (any) {   // one product, taken apart
-      const Tensor dstack = at::empty({s.ld, C}, o16);
-      gemm(g, s.ld, C, n, t.dy, s.ld, true, a.hn, C, false, nullptr, 0, dstack.mutable_data_ptr(), C);
+      gemm(g, s.ld, C, n, t.dy, s.ld, true, a.hn, C, false, nullptr, 0, t.dstack, C);
       void* dst[7];
       int64_t rows[7];
       for (int i = 0; i < 7; ++i) {
@@ -499,7 +526,7 @@ struct BlockBackward : public torch::autograd::Node {
         if (want(mats[i])) out[1 + mats[i]] = at::empty({rows[i], C}, o16);
         dst[i] = want(mats[i]) ? out[1 + mats[i]].mutable_data_ptr() : nullptr;
       }
-      launch("fox_unpack", st, [&] { return fox_unpack(dev, st, 7, dst, rows, C, dstack.const_data_ptr()); });
+      launch("fox_unpack", st, [&] { return fox_unpack(dev, st, 7, dst, rows, C, t.dstack); });
     }
     gemm(g, n, C, s.ld, t.dy, s.ld, false, a.stack, C, false, nullptr, 0, t.dhn, C);
     const Tensor dx = at::empty(xt.sizes(), o16);
@@ -599,6 +626,7 @@ FOX_PY(py_block) {
       torch::autograd::set_history(out, node);
       node->x = SavedVariable(x, false);
       node->acts = SavedVariable(f.acts, false);
+      node->mlp_acts = SavedVariable(f.mlp_acts, false);
       node->mask = SavedVariable(f.mask, false);
       node->w_o = SavedVariable(b.p[Block::kO], false);
       node->w_gate = SavedVariable(b.p[Block::kGate], false);

@@ -391,3 +391,39 @@ def test_block_gives_the_same_with_and_without_gradients(C, H, inter, padded):
     with torch.no_grad():
         out = blk(x, mask)
     assert ref.grad_fn is not None and out.grad_fn is None and torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("C,H,inter,T", [(1536, 24, 4096, 8192), (768, 12, 2048, 16384), (512, 4, 1408, 16384)])
+def test_block_step_takes_little_more_memory_than_its_modules(C, H, inter, T):
+    """A training step, beside the workspace of the products and the stack of weights and gradients.  The modules release
+    what they saved piece by piece; the block's one node in two pieces, for which 1/16 is allowed."""
+    blk, x, dy = _block(C, H, inter), _x(T, C).requires_grad_(), _x(T, C, seed=2)
+    peak = []
+    for native in (True, False):
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+
+        def step():
+            x.grad = None
+            blk.zero_grad(set_to_none=True)
+            blk(x).backward(dy)
+
+        peak.append(_peak(step))
+        if hook is not None:
+            hook.remove()
+    fixed = (32 << 20) + 2 * 2 * (4 * C + 3 * H + 8) * C
+    assert peak[0] <= peak[1] * 17 / 16 + fixed, [p >> 20 for p in peak]
+
+
+def test_block_backward_twice():
+    """retain_graph keeps what the first backward reads; without it a second one is refused."""
+    blk, x, dy = _block(), _x(300, B=2), _x(300, B=2, seed=2)
+    out = blk(x)
+    out.backward(dy, retain_graph=True)
+    first = {n: p.grad.clone() for n, p in blk.named_parameters()}
+    blk.zero_grad(set_to_none=True)
+    out.backward(dy)
+    for n, p in blk.named_parameters():
+        # (sums by fp32 atomics in the attention: an ulp of the result's type here and there)
+        assert (p.grad.float() - first[n].float()).norm() <= 2 ** -8 * first[n].float().norm(), n
+    with pytest.raises(RuntimeError, match="second time"):
+        out.backward(dy)
