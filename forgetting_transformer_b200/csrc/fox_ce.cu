@@ -280,8 +280,8 @@ static int ce_fwd_launch(int device, void* stream, int dtype, int64_t n_rows, in
   if (!logits || !labels || !losses || (!z_losses && !split) || !lse || n_rows <= 0 || n_cols <= 0 || di < 0)
     return FOX_ERR_BAD_ARG;
   if (total_classes < n_cols || class_start < 0 || class_start + n_cols > total_classes) return FOX_ERR_BAD_ARG;
-  if (n_rows > 2147483647LL || n_cols / 8 > 2147483647LL / 2) return FOX_ERR_TOO_LARGE;   // (16-byte pieces are counted in 32 bits)
   const int bytes = di == 2 ? 4 : 2;
+  if (n_rows > 2147483647LL || n_cols / (16 / bytes) > 2147483647LL / 2) return FOX_ERR_TOO_LARGE;   // (16-byte pieces are counted in 32 bits)
   if (reinterpret_cast<uintptr_t>(logits) % 16 || (row_stride * bytes) % 16 || row_stride < n_cols) return FOX_ERR_ALIGNMENT;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -302,8 +302,8 @@ static int ce_bwd_launch(int device, void* stream, int dtype, int64_t n_rows, in
   const int di = ce_dtype_index(dtype);
   if (!logits || !labels || !lse || !dloss || !dlogits || n_rows <= 0 || n_cols <= 0 || di < 0) return FOX_ERR_BAD_ARG;
   if (total_classes < n_cols || class_start < 0 || class_start + n_cols > total_classes) return FOX_ERR_BAD_ARG;
-  if (n_rows > 2147483647LL || n_cols / 8 > 2147483647LL / 2) return FOX_ERR_TOO_LARGE;   // (16-byte pieces are counted in 32 bits)
   const int bytes = di == 2 ? 4 : 2;
+  if (n_rows > 2147483647LL || n_cols / (16 / bytes) > 2147483647LL / 2) return FOX_ERR_TOO_LARGE;   // (16-byte pieces are counted in 32 bits)
   if (reinterpret_cast<uintptr_t>(logits) % 16 || (row_stride * bytes) % 16 || row_stride < n_cols ||
       reinterpret_cast<uintptr_t>(dlogits) % 16 || (dlogits_row_stride * bytes) % 16 || dlogits_row_stride < n_cols)
     return FOX_ERR_ALIGNMENT;

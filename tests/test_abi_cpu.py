@@ -77,6 +77,18 @@ def test_host_extension_of_another_pytorch_is_not_taken(tmp_path, monkeypatch):
         _lib.host()
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="looks at the refusal alone, on addresses that hold nothing")
+@pytest.mark.parametrize("dtype,per_piece", [(_lib.FOX_DTYPE_FP32, 4), (_lib.FOX_DTYPE_BF16, 8)])
+def test_cross_entropy_refuses_rows_of_too_many_pieces(dtype, per_piece):
+    """A thread counts a row's 16-byte pieces in 32 bits and steps past its end: rows of more than 2^30 pieces are refused
+    before anything is launched (there is no device here: smaller ones get as far as FOX_ERR_DEVICE)."""
+    lib = _lib.load()
+    for cols, rc in (((2 ** 30 + 1) * per_piece, -8), (2 ** 20 * per_piece, -7)):
+        f = lib.fox_cross_entropy_fwd(0, None, dtype, 1, cols, 4096, cols, 4096, 0.0, 1.0, 0.0, -100, 4096, 4096, 4096)
+        b = lib.fox_cross_entropy_bwd(0, None, dtype, 1, cols, 4096, cols, 4096, 4096, 4096, 1, 0.0, 1.0, 0.0, -100, 4096, cols)
+        assert (f, b) == (rc, rc)
+
+
 def _inputs(B=1, H=2, M=8, N=8, D=64, dtype=torch.bfloat16):
     q = torch.zeros(B, H, M, D, dtype=dtype)
     k = torch.zeros(B, H, N, D, dtype=dtype)
