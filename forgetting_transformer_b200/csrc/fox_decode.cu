@@ -33,7 +33,8 @@ constexpr int kDecThreads = 256, kDecWarps = kDecThreads / 32;
 constexpr int kDecTile = 1024;      // keys between two scans of the gates
 constexpr int kDecRows = 4;         // rows of K and of V in flight per lane
 constexpr int kDecMaxCluster = 8;
-constexpr int kDecMaxSplits = 512;
+constexpr int kDecMaxSplits = 1024;   // taken
+constexpr int kDecMostSplits = 512;   // asked for by fox_attn_decode_splits
 constexpr float kDecLog2e = 1.4426950408889634f;
 
 struct DecodeParams {
@@ -395,7 +396,7 @@ extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
   int64_t s = (148 * 4 + B * H - 1) / (B * H);
   const int64_t most = (N + 127) / 128;
   if (s > most) s = most;
-  if (s > kDecMaxSplits) s = kDecMaxSplits;
+  if (s > kDecMostSplits) s = kDecMostSplits;
   return s < 1 ? 1 : s;
 }
 

@@ -31,6 +31,29 @@ def test_decode_from_gates(B, H, N, D, padded):
     assert (err <= 2 ** -8 * ref.abs() + 2 ** -8 * ref.pow(2).mean().sqrt()).all(), err.max().item()
 
 
+@pytest.mark.parametrize("splits", [1, 8, 9, 512, 513, 1024])
+@pytest.mark.parametrize("N", [700, 2048])
+def test_decode_takes_any_number_of_ranges(splits, N):
+    """fox_attn_decode with ranges of the caller's choice, up to 1024: merged in a cluster (up to 8) or by the second kernel,
+    empty ranges among them.  bf16 rounds the result once."""
+    g = torch.Generator().manual_seed(N + splits)
+    B, H, D = 2, 3, 64
+    q, k, v = [torch.randn(B, H, t, D, generator=g).bfloat16().cuda() for t in (1, N, N)]
+    lam = torch.nn.functional.logsigmoid(torch.randn(B, H, N, generator=g) + 5).cuda().cumsum(-1).contiguous()
+    lib = _lib.load()
+    o, L = torch.empty_like(q), torch.empty(B, H, 1, device="cuda")
+    work = torch.empty(lib.fox_attn_decode_workspace_floats(B, H, D, splits), device="cuda")
+    rc = lib.fox_attn_decode(0, torch.cuda.current_stream().cuda_stream, _lib.FOX_DTYPE_BF16, B, H, N, D, _lib.t4(q), _lib.t4(k),
+                             _lib.t4(v), lam.data_ptr(), None, None, 0.125, _lib.t4(o), L.data_ptr(), work.data_ptr(), splits)
+    assert rc == 0
+    s = (q.double() @ k.double().transpose(-1, -2))[:, :, 0] / 8 + (lam[..., -1:] - lam).double()
+    ref = (s.softmax(-1)[:, :, None] @ v.double())
+    assert (o.double() - ref).abs().max() <= 2 ** -8 * ref.abs().max()
+    assert (L[..., 0].double() - s.logsumexp(-1)).abs().max() <= 1e-5 * s.abs().max()
+    assert lib.fox_attn_decode(0, None, _lib.FOX_DTYPE_BF16, B, H, N, D, _lib.t4(q), _lib.t4(k), _lib.t4(v), lam.data_ptr(), None, None,
+                               0.125, _lib.t4(o), L.data_ptr(), work.data_ptr(), 1025) == -1
+
+
 @pytest.mark.parametrize("B,C,H,I,N", [(1, 256, 4, 512, 1), (2, 512, 4, 1408, 130), (9, 768, 12, 2048, 64), (16, 256, 2, 96, 300)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("padded", [False, True])
