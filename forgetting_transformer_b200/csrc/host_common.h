@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
+#include <atomic>
 #include <string>
 
 #include "../../include/fox_b200.h"
@@ -35,20 +36,28 @@ inline void check_that(bool ok, const char* msg = "") {
 // fox_* return codes
 void check_rc(int rc, const char* what);
 
-// One stopwatch interval around a launch while a KernelTimer is active.
-extern bool g_timing;
-void timer_begin(const char* name, cudaStream_t st);
-void timer_end(cudaStream_t st);
+// One stopwatch interval around a launch while a KernelTimer is active (in any thread: an interval belongs to the launch that
+// opened it, and one whose launch fails is dropped).
+struct Interval {
+  const char* name = nullptr;
+  cudaEvent_t a = nullptr, b = nullptr;
+};
+extern std::atomic<bool> g_timing;
+Interval timer_begin(const char* name, cudaStream_t st);
+void timer_end(const Interval& iv, cudaStream_t st);
+void timer_drop(const Interval& iv);
 
 template <typename F>
 inline void launch(const char* name, cudaStream_t st, F&& f) {
-  if (!g_timing) {
+  if (!g_timing.load(std::memory_order_relaxed)) {
     check_rc(f(), name);
     return;
   }
-  timer_begin(name, st);
-  check_rc(f(), name);
-  timer_end(st);
+  const Interval iv = timer_begin(name, st);
+  const int rc = f();
+  if (rc == FOX_OK) timer_end(iv, st);
+  else timer_drop(iv);
+  check_rc(rc, name);
 }
 
 // int32[4] in pinned host memory that a kernel writes when a bounded wait runs out (never otherwise), so that looking

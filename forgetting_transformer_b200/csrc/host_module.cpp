@@ -5,7 +5,6 @@
 
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 
-#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -33,27 +32,27 @@ void check_rc(int rc, const char* what) {
 }
 
 // ---------------------------------------------------------------- stopwatch
-bool g_timing = false;
+std::atomic<bool> g_timing{false};
 namespace {
-struct Interval {
-  const char* name;
-  cudaEvent_t a, b;
-};
 std::mutex g_timer_mu;
 std::vector<Interval> g_intervals;
 }  // namespace
 
-void timer_begin(const char* name, cudaStream_t st) {
+Interval timer_begin(const char* name, cudaStream_t st) {
   Interval iv{name, nullptr, nullptr};
   C10_CUDA_CHECK(cudaEventCreate(&iv.a));
   C10_CUDA_CHECK(cudaEventCreate(&iv.b));
   C10_CUDA_CHECK(cudaEventRecord(iv.a, st));
+  return iv;
+}
+void timer_end(const Interval& iv, cudaStream_t st) {
+  C10_CUDA_CHECK(cudaEventRecord(iv.b, st));
   std::lock_guard<std::mutex> g(g_timer_mu);
   g_intervals.push_back(iv);
 }
-void timer_end(cudaStream_t st) {
-  std::lock_guard<std::mutex> g(g_timer_mu);
-  C10_CUDA_CHECK(cudaEventRecord(g_intervals.back().b, st));
+void timer_drop(const Interval& iv) {
+  cudaEventDestroy(iv.a);
+  cudaEventDestroy(iv.b);
 }
 
 // ---------------------------------------------------------------- status words
@@ -155,8 +154,7 @@ static FOX_PY(py_timer_take) {   // [(kernel, milliseconds), ...] of everything 
     float ms = 0.f;
     C10_CUDA_CHECK(cudaEventSynchronize(iv.b));
     C10_CUDA_CHECK(cudaEventElapsedTime(&ms, iv.a, iv.b));
-    cudaEventDestroy(iv.a);
-    cudaEventDestroy(iv.b);
+    timer_drop(iv);
     PyObject* t = Py_BuildValue("(sd)", iv.name, static_cast<double>(ms));
     PyList_Append(out, t);
     Py_DECREF(t);

@@ -47,7 +47,7 @@ class KernelTimer:
     active = None
 
     def __init__(self):
-        self.events = []
+        self.events, self._open = [], []    # (kernel, milliseconds); (kernel, start event, end event)
 
     def __enter__(self):
         KernelTimer.active = self
@@ -60,7 +60,8 @@ class KernelTimer:
 
     def summary(self):
         torch.cuda.synchronize()
-        self.events += _lib.host().timer_take()
+        self.events += _lib.host().timer_take() + [(name, a.elapsed_time(b)) for name, a, b in self._open]
+        self._open = []
         acc = {}
         for name, ms in self.events:
             n, t = acc.get(name, (0, 0.0))
@@ -69,8 +70,16 @@ class KernelTimer:
 
 
 def _call(name, fn, *args):
-    """Call one C-ABI entry point, raising on an error code."""
+    """Call one C-ABI entry point, raising on an error code; timed while a KernelTimer is active."""
+    timer = KernelTimer.active
+    if timer is None:
+        _lib.check(fn(*args), name)
+        return
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
     _lib.check(fn(*args), name)
+    b.record()
+    timer._open.append((name, a, b))
 
 
 def _stream() -> int:

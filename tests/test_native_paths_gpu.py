@@ -427,3 +427,35 @@ def test_block_backward_twice():
         assert (p.grad.float() - first[n].float()).norm() <= 2 ** -8 * first[n].float().norm(), n
     with pytest.raises(RuntimeError, match="second time"):
         out.backward(dy)
+
+
+def test_kernel_timer_times_every_launch():
+    """Launches of several threads, launches by way of Python, and none that failed."""
+    import threading
+    q, k, v, g = _qkvg()
+
+    def work():
+        x = [t.clone().requires_grad_() for t in (q, k, v, g)]
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                fox.forgetting_attention(*x, head_first=True).sum().backward()
+        torch.cuda.synchronize()
+
+    work()
+    with fox.ops.KernelTimer() as timer:
+        threads = [threading.Thread(target=work) for _ in range(3)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        fox.ops.max_row_norm(k)
+        fox.ops.log_lambda_cumsum(g, None)
+        many = _qkvg(B=4096, H=24, M=3, N=3, D=16)
+        out = fox.forgetting_attention(many[0].requires_grad_(), *many[1:], head_first=True)
+        with pytest.raises(fox.FoxError, match="TOO_LARGE"):       # (the backward takes 65535 heads at most)
+            out.sum().backward()
+    got = timer.summary()
+    assert {n: c for n, (c, _) in got.items()} == {
+        "fox_attn_prologue": 61, "fox_attn_fwd": 61, "fox_bwd_delta": 60, "fox_attn_bwd": 60, "fox_bwd_finish": 60,
+        "fox_max_row_norm": 1, "fox_cumsum_fwd": 1}
+    assert all(0 < ms < 1e3 for _, ms in got.values())
