@@ -782,6 +782,7 @@ FOX_PY(py_block_step) {
   if (at::GradMode::is_enabled()) {
     bool needs = x.requires_grad();
     for (const Tensor& t : b.p) needs = needs || (t.defined() && t.requires_grad());
+    for (const Tensor* t : {&c.k, &c.v, &c.g, &c.k_state, &c.v_state}) needs = needs || t->requires_grad();
     if (needs) Py_RETURN_NONE;
   }
   if (args[2] != Py_None && !plain_tensor(args[2])) Py_RETURN_NONE;

@@ -459,3 +459,17 @@ def test_kernel_timer_times_every_launch():
         "fox_attn_prologue": 61, "fox_attn_fwd": 61, "fox_bwd_delta": 60, "fox_attn_bwd": 60, "fox_bwd_finish": 60,
         "fox_max_row_norm": 1, "fox_cumsum_fwd": 1}
     assert all(0 < ms < 1e3 for _, ms in got.values())
+
+
+@pytest.mark.parametrize("what", [0, 1, 2])
+def test_token_step_against_a_history_with_gradients(what):
+    """Frozen blocks, but keys, values or log gates in the cache that need gradients (a learned prefix): the token's output
+    carries them."""
+    blk, x = _block().requires_grad_(False), _x(1)
+    cache, st = fox.FgateCache(), blk.attn.init_shift_state(1)
+    cache.update_shift_cache(st["key_shift"], st["value_shift"], 0)
+    hist = list(_qkvg(H=4, M=16, N=16)[1:])
+    hist[what].requires_grad_()
+    cache.update(*hist, 0)
+    blk(x, None, cache, 0).sum().backward()
+    assert hist[what].grad is not None and hist[what].grad.abs().sum() > 0
