@@ -38,7 +38,10 @@ struct Mod {
   PyObject* dict = nullptr;
   PyObject* get(PyObject* name) const { return PyDict_GetItem(dict, name); }
   bool flag(PyObject* name) const { PyObject* v = get(name); return v && PyObject_IsTrue(v) == 1; }
-  double number(PyObject* name) const { PyObject* v = get(name); return v ? PyFloat_AsDouble(v) : -1.; }
+  double number(PyObject* name) const {   // -1 for anything but a number, which is left to the modules
+    PyObject* v = get(name);
+    return v && (PyFloat_Check(v) || PyLong_Check(v)) ? PyFloat_AsDouble(v) : -1.;
+  }
   bool none(PyObject* name) const { PyObject* v = get(name); return v == Py_None; }
   PyObject* child(PyObject* name) const {
     PyObject* m = get(s__modules);

@@ -473,3 +473,15 @@ def test_token_step_against_a_history_with_gradients(what):
     cache.update(*hist, 0)
     blk(x, None, cache, 0).sum().backward()
     assert hist[what].grad is not None and hist[what].grad.abs().sum() > 0
+
+
+@pytest.mark.parametrize("eps", ["1e-6", torch.tensor(1e-6)])
+@pytest.mark.parametrize("T", [1, 64])
+def test_block_with_an_epsilon_that_is_no_number(eps, T):
+    """A configuration may give it as text or tensor; the modules take float() of it."""
+    blk, x, res = _block(), _x(T), []
+    for value in (1e-6, eps):
+        blk.attn_norm.eps = value
+        with torch.no_grad():
+            res.append(blk(x, *((None, _cache(blk), 0) if T == 1 else ())).float())
+    assert (res[0] - res[1]).norm() <= 2 ** -6 * res[0].norm()     # (native against modules: 8 roundings to 16 bits)
