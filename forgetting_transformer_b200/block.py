@@ -35,9 +35,8 @@ def _load_host():
     global _host
     host = _lib.host()
     m = torch.nn.modules.module
-    host.set_block_classes(FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear,
-                           FgateCache, _LayerStore, m._global_forward_hooks, m._global_forward_pre_hooks, m._global_backward_hooks,
-                           m._global_backward_pre_hooks)
+    host.set_block_classes(*_MODULE_CLASSES, FgateCache, _LayerStore, m._global_forward_hooks, m._global_forward_pre_hooks,
+                           m._global_backward_hooks, m._global_backward_pre_hooks, nn.Module, _MODULE_CALL, *_FORWARDS)
     _host = host
     return _host
 
@@ -214,3 +213,9 @@ class FoxProBlock(nn.Module):
         hidden_states = self.attn(self.attn_norm(hidden_states), attention_mask, past_key_values, layer_idx)
         hidden_states, residual = self.mlp_norm(hidden_states, residual, True)
         return residual + self.mlp(hidden_states)
+
+
+# what the native block stands in for, as it is when the package is loaded
+_MODULE_CLASSES = (FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear)
+_FORWARDS = tuple(c.forward for c in _MODULE_CLASSES)
+_MODULE_CALL = nn.Module.__call__

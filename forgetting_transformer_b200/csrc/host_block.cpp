@@ -19,7 +19,10 @@ namespace foxh {
 // ---------------------------------------------------------------- the module tree
 namespace {
 enum Class { kLayerCls, kMlpCls, kRmsCls, kGroupCls, kGatedCls, kShiftCls, kLinearCls, kCacheCls, kStoreCls, kClasses };
+constexpr int kModuleClasses = kCacheCls;   // those before it are modules
 PyObject* g_classes[kClasses] = {};
+PyObject* g_forwards[kModuleClasses] = {};   // their forward functions
+PyObject* g_module_call[2] = {};             // torch.nn.Module and its __call__
 PyObject* g_global_hooks[4] = {};   // torch.nn's global forward / pre / backward / backward pre hooks
 
 // interned attribute names
@@ -28,7 +31,7 @@ PyObject* g_global_hooks[4] = {};   // torch.nn's global forward / pre / backwar
   X(weight) X(bias) X(attn_norm) X(attn) X(mlp_norm) X(mlp) X(q_proj) X(k_proj) X(v_proj) X(o_proj) X(fgate_proj)             \
   X(ogate_proj) X(output_norm) X(q_norm) X(k_norm) X(linear) X(shift_proj) X(gate_proj) X(down_proj) X(eps) X(num_heads)      \
   X(log_pruning_tolerance) X(qk_norm) X(use_k_shift) X(use_v_shift) X(activation) X(is_rms_norm) X(num_groups)     \
-  X(_layers) X(key_shift_cache) X(value_shift_cache) X(_seen_tokens) X(k) X(v) X(g) X(length)
+  X(_layers) X(key_shift_cache) X(value_shift_cache) X(_seen_tokens) X(k) X(v) X(g) X(length) X(__call__)
 #define FOX_DECL(n) PyObject* s_##n;
 FOX_NAMES(FOX_DECL)
 #undef FOX_DECL
@@ -65,9 +68,16 @@ bool open(PyObject* obj, Mod& m) {
 }
 bool empty_dict(PyObject* d) { return !d || d == Py_None || (PyDict_Check(d) && PyDict_GET_SIZE(d) == 0); }
 
+// Is a class's attribute still the function it was when the package was loaded?  (Another one may have been put there.)
+bool unpatched(PyObject* cls, PyObject* name, PyObject* function) {
+  return PyDict_GetItem(reinterpret_cast<PyTypeObject*>(cls)->tp_dict, name) == function;
+}
+
 bool open_plain(const Mod& parent, PyObject* name, Class cls, Mod& m) {
   PyObject* obj = parent.child(name);
-  if (!obj || reinterpret_cast<PyObject*>(Py_TYPE(obj)) != g_classes[cls] || !open(obj, m)) return false;
+  if (!obj || reinterpret_cast<PyObject*>(Py_TYPE(obj)) != g_classes[cls] || !unpatched(g_classes[cls], s_forward, g_forwards[cls]) ||
+      !open(obj, m))
+    return false;
   return empty_dict(m.get(s__forward_hooks)) && empty_dict(m.get(s__forward_pre_hooks)) && empty_dict(m.get(s__backward_hooks)) &&
          empty_dict(m.get(s__backward_pre_hooks)) && !m.get(s_forward);
 }
@@ -122,6 +132,7 @@ bool read_block(PyObject* self, const Tensor& x, Block& b) {
   if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;   // (they are there to see the products)
   for (PyObject* h : g_global_hooks)
     if (!empty_dict(h)) return false;
+  if (!unpatched(g_module_call[0], s___call__, g_module_call[1])) return false;
   Mod blk, attn, mlp, m;
   if (!open(self, blk) || !open_plain(blk, s_attn, kLayerCls, attn) || !open_plain(blk, s_mlp, kMlpCls, mlp)) return false;
   const int64_t C = b.C = x.size(2), H = b.H = static_cast<int64_t>(attn.number(s_num_heads));
@@ -564,7 +575,8 @@ struct BlockBackward : public torch::autograd::Node {
 using namespace foxh;
 
 // set_block_classes(FoxProAttentionLayer, FoxMLP, RMSNorm, GroupNorm, FusedGroupNormGated, ShiftLinear, nn.Linear, FgateCache,
-//                   its layer store, the four global hook dictionaries of torch.nn.modules.module)
+//                   its layer store, the four global hook dictionaries of torch.nn.modules.module, nn.Module, its __call__,
+//                   the forward functions of the first seven)
 FOX_PY(py_set_block_classes) {
   HANDLE_TH_ERRORS
 #define FOX_INTERN(n) s_##n = PyUnicode_InternFromString(#n);
@@ -577,6 +589,15 @@ FOX_PY(py_set_block_classes) {
   for (int i = 0; i < 4; ++i) {
     Py_INCREF(args[kClasses + i]);
     g_global_hooks[i] = args[kClasses + i];
+  }
+  PyObject* const* rest = args + kClasses + 4;
+  for (int i = 0; i < 2; ++i) {
+    Py_INCREF(rest[i]);
+    g_module_call[i] = rest[i];
+  }
+  for (int i = 0; i < kModuleClasses; ++i) {
+    Py_INCREF(rest[2 + i]);
+    g_forwards[i] = rest[2 + i];
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS

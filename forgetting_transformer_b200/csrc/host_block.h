@@ -14,8 +14,8 @@ struct Block {
 };
 
 // Reads the module tree; false where any part of it is not the plain module this code stands in for (another class, a
-// hook, a patched forward, a tensor subclass, other dtypes or layouts, autocast, a forward-mode tangent) or under
-// torch.jit.trace or a dispatch mode: the modules' own forward then runs.
+// hook, a patched forward of the object or its class, a tensor subclass, other dtypes or layouts, autocast, a forward-mode
+// tangent) or under torch.jit.trace or a dispatch mode: the modules' own forward then runs.
 bool read_block(PyObject* self, const Tensor& x, Block& b);
 
 }  // namespace foxh

@@ -485,3 +485,19 @@ def test_block_with_an_epsilon_that_is_no_number(eps, T):
         with torch.no_grad():
             res.append(blk(x, *((None, _cache(blk), 0) if T == 1 else ())).float())
     assert (res[0] - res[1]).norm() <= 2 ** -6 * res[0].norm()     # (native against modules: 8 roundings to 16 bits)
+
+
+@pytest.mark.parametrize("cls", ["FoxProAttentionLayer", "FoxMLP", "RMSNorm", "GroupNorm", "FusedGroupNormGated", "ShiftLinear", "Linear",
+                                 "Module"])
+@pytest.mark.parametrize("T", [1, 64])
+def test_a_forward_put_on_a_class_takes_part(cls, T, monkeypatch):
+    """Tools replace nn.Linear.forward, a module class's forward or nn.Module.__call__ for every instance."""
+    blk, x, seen = _block(), _x(T), []
+    with torch.no_grad():
+        blk(x, *((None, _cache(blk), 0) if T == 1 else ()))
+        owner = getattr(fox.block, cls, None) or getattr(torch.nn, cls)
+        name = "__call__" if cls == "Module" else "forward"
+        f = getattr(owner, name)
+        monkeypatch.setattr(owner, name, lambda self, *a, **k: (seen.append(type(self)), f(self, *a, **k))[1])
+        blk.forward(x, *((None, _cache(blk), 0) if T == 1 else ()))
+    assert len(seen) > 0
