@@ -708,6 +708,8 @@ Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheL
   const Tensor x = x_in.contiguous();
   Tensor out = at::empty(x_in.sizes(), x_in.options()), mask64;
   if (mask.defined()) mask64 = mask.to(at::kLong).contiguous();
+  // written in place: what has saved one of them for a backward has to notice
+  for (const Tensor* t : {&c.k, &c.v, &c.g, &c.k_state, &c.v_state}) t->unsafeGetTensorImpl()->bump_version();
   const int64_t n = x.size(0), C = b.C, H = b.H, D = b.D, N = c.length + 1, cap = c.k.size(2);
   const AttnShape as{n, H, 1, N, D};
   const int64_t ld = (4 * C + 3 * H + 3) / 4 * 4;

@@ -501,3 +501,14 @@ def test_a_forward_put_on_a_class_takes_part(cls, T, monkeypatch):
         monkeypatch.setattr(owner, name, lambda self, *a, **k: (seen.append(type(self)), f(self, *a, **k))[1])
         blk.forward(x, *((None, _cache(blk), 0) if T == 1 else ()))
     assert len(seen) > 0
+
+
+def test_token_step_counts_as_a_change_in_place():
+    """Views of the cache and shift states that were saved for a backward are seen to have been written to."""
+    blk, x = _block(), _x(1)
+    cache = _cache(blk)
+    tensors = [*cache[0], cache.key_shift_cache[0], cache.value_shift_cache[0]]
+    before = [t._version for t in tensors]
+    with torch.no_grad():
+        blk(x, None, cache, 0)
+    assert all(t._version > v for t, v in zip(tensors, before))
