@@ -42,6 +42,8 @@ __device__ __forceinline__ float head_sum(float x, int lanes) {
   return x;
 }
 
+constexpr int kMixThreads = 256;   // rows of up to 2048 channels
+
 struct MixParams {
   const uint16_t* y;      // (tokens, ld): [q | k | v | ogate | fgate | k mix | v mix | pad]
   int64_t ld;
@@ -65,13 +67,12 @@ __device__ __forceinline__ void mix_load(const MixParams& p, int64_t t, bool on,
   }
 }
 
-// kThreads: 256 (rows of up to 2048 channels) or 512.  One CTA of 192 threads per 3 tokens' loads in flight is too little to
-// cover the chain load - sum over a head's lanes - store, so the narrow form takes one token at a time in 64 registers and
-// has 5 CTAs per SM, where two tokens in 116 registers left 2: 16384 x 1536 bf16 96 -> 71.5 us (4.2 TB/s), 2048 x 768 7.5 ->
+// One CTA of 192 threads per 3 tokens' loads in flight is too little to cover the chain load - sum over a head's lanes -
+// store, so it takes one token at a time in 64 registers and has 5 CTAs per SM, where two tokens in 116 registers left 2: 16384 x 1536 bf16 96 -> 71.5 us (4.2 TB/s), 2048 x 768 7.5 ->
 // 7.3 us.  (Two tokens in 80 registers: 67 and 8.1 us; one in 48 registers: 91 and 9.5 us; 4 channels a thread, which doubles
 // the instructions for addresses and sums: 199 and 13 us.)
-template <bool kBf16, int kThreads>
-__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) fox_mix_fwd_kernel(const MixParams p) {
+template <bool kBf16>
+__global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixParams p) {
   if (static_cast<int>(blockIdx.x) >= p.mix_blocks) {
     __shared__ unsigned long long s_sum;
     const int b = blockIdx.x - p.mix_blocks;
@@ -100,63 +101,51 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) fox_mix_fwd
   uint4 kp, vp;
   int pos = static_cast<int>(t0 % p.T);   // of the token in its sequence
   mix_load(p, t0 - 1, active && pos != 0, ch, C, kp, vp);
-  constexpr int kU = kThreads == 256 ? 1 : 2;   // tokens whose loads are in flight together
-  for (int64_t tb = t0; tb < t1; tb += kU) {
-    uint4 qr[kU], kr[kU], vr[kU];
-    float ak[kU], av[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int64_t t = tb + u;
-      const bool on = active && t < t1;
-      mix_load(p, t, on, ch, C, kr[u], vr[u]);
-      qr[u] = make_uint4(0, 0, 0, 0);
-      ak[u] = av[u] = 0.f;
-      if (on) {
-        const uint16_t* row = p.y + t * p.ld;
-        qr[u] = *reinterpret_cast<const uint4*>(row + ch);
-        ak[u] = blk_load1<kBf16>(row + 4 * C + p.H + h);
-        av[u] = blk_load1<kBf16>(row + 4 * C + 2 * p.H + h);
-      }
+  for (int64_t t = t0; t < t1; ++t) {
+    uint4 qr = make_uint4(0, 0, 0, 0), kr, vr;
+    float ak = 0.f, av = 0.f;
+    mix_load(p, t, active, ch, C, kr, vr);
+    if (active) {
+      const uint16_t* row = p.y + t * p.ld;
+      qr = *reinterpret_cast<const uint4*>(row + ch);
+      ak = blk_load1<kBf16>(row + 4 * C + p.H + h);
+      av = blk_load1<kBf16>(row + 4 * C + 2 * p.H + h);
     }
+    const bool first = pos == 0;   // no token before it
+    pos = pos + 1 == p.T ? 0 : pos + 1;
+    float q[8], k[8], v[8], kq[8], vq[8];
+    blk_unpack<kBf16>(qr, q);
+    blk_unpack<kBf16>(kr, k);
+    blk_unpack<kBf16>(vr, v);
+    blk_unpack<kBf16>(kp, kq);
+    blk_unpack<kBf16>(vp, vq);
+    const float a = blk_sigmoid(ak), c = blk_sigmoid(av);
+    float sq = 0.f, sk = 0.f;
 #pragma unroll
-    for (int u = 0; u < kU; ++u) {
-      const int64_t t = tb + u;
-      const bool first = pos == 0;   // no token before it
-      pos = pos + 1 == p.T ? 0 : pos + 1;
-      float q[8], k[8], v[8], kq[8], vq[8];
-      blk_unpack<kBf16>(qr[u], q);
-      blk_unpack<kBf16>(kr[u], k);
-      blk_unpack<kBf16>(vr[u], v);
-      blk_unpack<kBf16>(u == 0 ? kp : kr[u > 0 ? u - 1 : 0], kq);
-      blk_unpack<kBf16>(u == 0 ? vp : vr[u > 0 ? u - 1 : 0], vq);
-      const float a = blk_sigmoid(ak[u]), c = blk_sigmoid(av[u]);
-      float sq = 0.f, sk = 0.f;
+    for (int j = 0; j < 8; ++j) {
+      k[j] = k[j] * (1.f - a) + (first ? 0.f : kq[j] * a);
+      v[j] = v[j] * (1.f - c) + (first ? 0.f : vq[j] * c);
+      sq = fmaf(q[j], q[j], sq);
+      sk = fmaf(k[j], k[j], sk);
+    }
+    const float rq = rsqrtf(head_sum(sq, lanes) * inv_d + p.eps), rk = rsqrtf(head_sum(sk, lanes) * inv_d + p.eps);
+    if (active) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        k[j] = k[j] * (1.f - a) + (first ? 0.f : kq[j] * a);
-        v[j] = v[j] * (1.f - c) + (first ? 0.f : vq[j] * c);
-        sq = fmaf(q[j], q[j], sq);
-        sk = fmaf(k[j], k[j], sk);
+        q[j] *= rq * wq[j];
+        k[j] *= rk * wk[j];
       }
-      const float rq = rsqrtf(head_sum(sq, lanes) * inv_d + p.eps), rk = rsqrtf(head_sum(sk, lanes) * inv_d + p.eps);
-      if (active && t < t1) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          q[j] *= rq * wq[j];
-          k[j] *= rk * wk[j];
-        }
-        const int64_t o = t * C + ch;
-        *reinterpret_cast<uint4*>(p.q + o) = blk_pack<kBf16>(q);
-        *reinterpret_cast<uint4*>(p.k + o) = blk_pack<kBf16>(k);
-        *reinterpret_cast<uint4*>(p.v + o) = blk_pack<kBf16>(v);
-        if (sub == 0 && p.rstd_q) {
-          p.rstd_q[t * p.H + h] = rq;
-          p.rstd_k[t * p.H + h] = rk;
-        }
+      const int64_t o = t * C + ch;
+      *reinterpret_cast<uint4*>(p.q + o) = blk_pack<kBf16>(q);
+      *reinterpret_cast<uint4*>(p.k + o) = blk_pack<kBf16>(k);
+      *reinterpret_cast<uint4*>(p.v + o) = blk_pack<kBf16>(v);
+      if (sub == 0 && p.rstd_q) {
+        p.rstd_q[t * p.H + h] = rq;
+        p.rstd_k[t * p.H + h] = rk;
       }
     }
-    kp = kr[kU - 1];
-    vp = vr[kU - 1];
+    kp = kr;
+    vp = vr;
   }
 }
 
@@ -197,7 +186,7 @@ __device__ __forceinline__ void mix_bwd_load(const MixBwdParams& p, int64_t t, b
 // the token before in this order.  A CTA first forms the token after its range for that carry (1 / rows more reads).
 // The next token's rows are fetched before the current one is worked on.
 template <bool kBf16>
-__global__ void __launch_bounds__(512) fox_mix_bwd_kernel(const MixBwdParams p) {
+__global__ void __launch_bounds__(kMixThreads, 2) fox_mix_bwd_kernel(const MixBwdParams p) {
   const MixParams& f = p.f;
   const int lanes = f.D >> 3, C = f.H * f.D;
   const int h = threadIdx.x / lanes, sub = threadIdx.x % lanes;
@@ -435,7 +424,7 @@ static int mix_params(MixParams& p, int64_t B, int64_t T, int64_t H, int64_t D, 
                       const float* wk, const int64_t* mask, float eps) {
   if (!y || !wq || !wk || B <= 0 || T <= 0 || H <= 0) return FOX_ERR_BAD_ARG;
   if (D % 8 || D < 8 || D > 256 || (D & (D - 1))) return FOX_ERR_HEAD_DIM;
-  if (H * D > 4096 || T > 2147483647LL) return FOX_ERR_TOO_LARGE;   // (8 channels a thread, 512 threads)
+  if (H * D > 8 * kMixThreads || T > 2147483647LL) return FOX_ERR_TOO_LARGE;   // (8 channels a thread)
   if (reinterpret_cast<uintptr_t>(y) % 16 || ld % 8 || ld < 4 * H * D + 3 * H) return FOX_ERR_ALIGNMENT;
   p.y = (const uint16_t*)y; p.ld = ld; p.wq = wq; p.wk = wk; p.mask = mask; p.eps = eps;
   p.H = (int)H; p.D = (int)D; p.T = (int)T; p.tokens = B * T;
@@ -468,10 +457,8 @@ extern "C" int fox_mix_fwd(int device, void* stream, int dtype, int64_t B, int64
   p.seq_start = seq_start;
   p.mix_blocks = (int)((p.tokens + p.rows - 1) / p.rows);
   const unsigned grid = (unsigned)(p.mix_blocks + (seq_start ? B : 0));
-  const int threads = mix_threads(p);
-  auto kern = dtype == FOX_DTYPE_BF16 ? (threads <= 256 ? fox_mix_fwd_kernel<true, 256> : fox_mix_fwd_kernel<true, 512>)
-                                      : (threads <= 256 ? fox_mix_fwd_kernel<false, 256> : fox_mix_fwd_kernel<false, 512>);
-  kern<<<grid, threads, 0, (cudaStream_t)stream>>>(p);
+  if (dtype == FOX_DTYPE_BF16) fox_mix_fwd_kernel<true><<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
+  else fox_mix_fwd_kernel<false><<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
   return blk_rc();
 }
 
