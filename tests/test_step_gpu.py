@@ -126,3 +126,78 @@ def test_block_native_matches_modules(B, T, C, H, padded):
     for (n, a), (_, b) in zip(*res):
         a, b = a.float(), b.float()
         assert a.shape == b.shape and (a - b).norm() <= 12 * 2 ** -12 * b.norm() + 1e-6, (n, ((a - b).norm() / b.norm()).item())
+
+
+def _native_and_modules(blk, x, dy, mask=None):
+    """[(name, tensor)] of the native block and of its modules one by one (a forward hook turns the native path off)."""
+    res = []
+    for native in (True, False):
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        x.grad = None
+        blk.zero_grad(set_to_none=True)
+        out = blk(x, mask)
+        assert ("FoxProBlockBackward" in out.grad_fn.name()) == native
+        out.backward(dy)
+        res.append([("out", out.detach()), ("x", x.grad)] + [(n, p.grad) for n, p in blk.named_parameters()])
+        if hook is not None:
+            hook.remove()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    return res
+
+
+@pytest.mark.parametrize("B,T,C,H", [(1, 1100, 256, 4), (2, 1333, 512, 4), (1, 2500, 256, 16)])
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_pruned_block_native_matches_modules(B, T, C, H, padded, dtype):
+    """With log_pruning_tolerance and strong decay most key blocks are left out; head dims 64, 128 and 16, the key norms'
+    bound (from 1024 keys on), ragged lengths.  A dozen roundings, and e^-10 of a row's mass that either side may prune."""
+    torch.manual_seed(T)
+    blk = fox.FoxProBlock(C, H, 2 * C, fgate_bias=-1.0, log_pruning_tolerance=-10.0).cuda().to(dtype)
+    x = torch.randn(B, T, C, device="cuda").to(dtype).requires_grad_()
+    dy = torch.randn(B, T, C, device="cuda").to(dtype)
+    mask = None
+    if padded:
+        mask = torch.ones(B, T, dtype=torch.int32, device="cuda")
+        mask[0, :T // 3] = 0
+    tol = 12 * (2.0 ** -12 if dtype == torch.float16 else 2.0 ** -9) + 2 * 2.718 ** -10
+    for (n, a), (_, b) in zip(*_native_and_modules(blk, x, dy, mask)):
+        a, b = a.float(), b.float()
+        assert a.shape == b.shape and (a - b).norm() <= tol * b.norm() + 1e-6, (n, ((a - b).norm() / b.norm()).item())
+
+
+@pytest.mark.parametrize("B,T,C,H", [(1, 1200, 256, 4), (3, 1601, 256, 2), (1, 9472, 256, 4), (1, 12007, 512, 8)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_long_block_native_matches_modules(B, T, C, H, padded):
+    """Runs of 2 to 16 tokens per CTA in the token-shift kernels, and from 9472 tokens on a backward that walks several runs:
+    sequences' ends inside and between runs.  Both round intermediates to 11 bits at a dozen points."""
+    torch.manual_seed(T)
+    blk = fox.FoxProBlock(C, H, 2 * C, fgate_bias=4.0).cuda().to(torch.float16)
+    x = torch.randn(B, T, C, device="cuda").half().requires_grad_()
+    dy = torch.randn(B, T, C, device="cuda").half()
+    mask = None
+    if padded:
+        mask = torch.ones(B, T, dtype=torch.bool, device="cuda")
+        mask[B - 1, :T // 3] = False
+    for (n, a), (_, b) in zip(*_native_and_modules(blk, x, dy, mask)):
+        a, b = a.float(), b.float()
+        assert a.shape == b.shape and (a - b).norm() <= 12 * 2 ** -12 * b.norm() + 1e-6, (n, ((a - b).norm() / b.norm()).item())
+
+
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_block_under_checkpointing(reentrant):
+    from torch.utils.checkpoint import checkpoint
+    torch.manual_seed(3)
+    blk = fox.FoxProBlock(256, 4, 512, fgate_bias=2.0).cuda().to(torch.bfloat16)
+    x = torch.randn(2, 333, 256, device="cuda").bfloat16().requires_grad_()
+    dy = torch.randn(2, 333, 256, device="cuda").bfloat16()
+    res = []
+    for f in (blk, lambda x: checkpoint(blk, x, use_reentrant=reentrant)):
+        x.grad = None
+        blk.zero_grad(set_to_none=True)
+        out = f(x)
+        out.backward(dy)
+        res.append([out.detach(), x.grad] + [p.grad for p in blk.parameters()])
+    assert torch.equal(res[0][0], res[1][0])
+    for a, b in zip(*res):      # (sums by fp32 atomics in the attention: an ulp of the result's type here and there)
+        assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
