@@ -595,3 +595,29 @@ def test_forward_d128_half_tiles_with_a_moving_maximum(M, N, dtype):
     eps = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
     bound = 2 * (2 * eps + 1e-4) * v.float().abs().max().item()
     assert (out.double().cpu() - ref.double().nan_to_num(0.0)).abs().max().item() < bound
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_weights_are_relative_to_the_maximum_of_the_nearest_128_keys(D, dtype):
+    """A row's weights are rounded to 16 bits relative to a reference that covers the nearest 128 keys, so a dominant key among
+    them has weight 1 exactly and only the result is rounded.  Row i of 64 has its dominant key in the farther half of them,
+    with a logit of 3 to 5.4 over the others' 0 (not so far above them that the reference would be moved), and is looked at in
+    a channel that only this key has.  A value rounded once to b bits has an rms error of
+    2^(1-b) sqrt((1 - 1/4) / (2 ln 2) / 12) (log-uniform mantissas); weight and result rounded make that 1.41 times as much."""
+    g = torch.Generator().manual_seed(D)
+    H, M, N = 128, 64, 128
+    eye = torch.eye(64, D).expand(1, H, 64, D)
+    far = torch.zeros(1, H, 64, D)
+    q = (eye * (torch.rand(1, H, 64, 1, generator=g) * 2.4 + 3)).to(dtype)
+    k = torch.cat([eye, far], 2).to(dtype)
+    v = torch.cat([eye * torch.exp2(torch.rand(1, H, 64, 1, generator=g) * 8), far], 2).to(dtype)
+    with torch.no_grad():
+        out = fox.forgetting_attention(q.cuda(), k.cuda(), v.cuda(), torch.zeros(1, H, N).cuda(), head_first=True, sm_scale=1.0)
+    _lib.check_status()
+    s = q.double() @ k.double().transpose(-1, -2)
+    s.masked_fill_(torch.arange(N)[None] > torch.arange(M)[:, None] + N - M, -float("inf"))
+    got, ref = [t[0, :, :, :64].diagonal(dim1=1, dim2=2) for t in (out.double().cpu(), s.softmax(-1) @ v.double())]
+    rms = ((got - ref) / ref).pow(2).mean().sqrt().item()
+    once = 2.0 ** (-7 if dtype == torch.bfloat16 else -10) * (0.75 / (2 * 0.6931) / 12) ** 0.5
+    assert rms < 1.2 * once, rms / once
