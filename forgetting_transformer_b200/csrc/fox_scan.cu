@@ -350,9 +350,10 @@ fox_max_row_norm_kernel(const uint16_t* __restrict__ x, int64_t sb, int64_t sh, 
 // ------------------------------------------------------ before the attention forward
 // The prefix sum of the log gates and the largest key (and, for the automatic threshold, query) row norms in one
 // launch: they are independent, and each alone leaves most of the chip idle (one CTA per (b,h) scans, a scan of
-// 16384 gates takes 10 us).  blockIdx.y = 0 scans; blocks 1 .. n_k (n_k+1 .. n_k+n_q) each take every n_k-th
+// 16384 gates takes 10 us).  Block 0 of a (b, h) scans; blocks 1 .. n_k (n_k+1 .. n_k+n_q) each take every n_k-th
 // (n_q-th) group of rows and write ONE partial maximum, so nothing has to be zeroed first; the reader takes the
-// maximum of the parts.  (b, h) is the grid's x index: there may be more than the 65535 that y takes.
+// maximum of the parts.  All blocks lie on the grid's x axis, one (b, h) behind the other: y ends at 65535, and with the
+// parts on the slow axis the scans start first but the norms' reads spread over all (b, h), 1.5 % slower where they are long.
 struct NormSource {
   const uint16_t* x;
   int64_t sb, sh, st;
@@ -410,7 +411,7 @@ fox_prologue_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t
                     const int64_t* __restrict__ seq_start, float* __restrict__ lam,
                     const NormSource k, const NormSource q, int H, int N, int D) {
   __shared__ float red[32];
-  const int bh = blockIdx.x, x = blockIdx.y;
+  const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
   if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
   else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
   else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
@@ -649,7 +650,8 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
                                  int64_t n_k_parts, const fox_tensor4* q, float* q_parts, int64_t n_q_parts) {
   if (!gates || !log_lambda || B <= 0 || H <= 0 || N <= 0 || M <= 0 || M > N) return FOX_ERR_BAD_ARG;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
-  if (B * H > 2147483647LL || n_k_parts > 32767 || n_q_parts > 32767) return FOX_ERR_TOO_LARGE;
+  if (n_k_parts > 32767 || n_q_parts > 32767 || B * H > 2147483647LL / (1 + (k ? n_k_parts : 0) + (q ? n_q_parts : 0)))
+    return FOX_ERR_TOO_LARGE;
   if (!head_dim_ok(D)) return FOX_ERR_HEAD_DIM;
   NormSource ks{}, qs{};
   if (k) {
@@ -663,7 +665,7 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
     qs = NormSource{(const uint16_t*)q->ptr, q->sb, q->sh, q->st, (int)M, (int)n_q_parts, q_parts};
   }
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  dim3 grid((unsigned)(B * H), (unsigned)(1 + ks.n_parts + qs.n_parts));
+  const unsigned grid = (unsigned)(B * H * (1 + ks.n_parts + qs.n_parts));
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == FOX_DTYPE_BF16;
 #define FOX_PRO(K)                                                                                                       \
