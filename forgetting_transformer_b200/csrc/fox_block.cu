@@ -35,8 +35,13 @@ template <bool kBf16>
 __device__ __forceinline__ float blk_load1(const uint16_t* p) {
   return unpack2<kBf16>(static_cast<uint32_t>(*p)).x;
 }
-// (in full fp32, as torch.sigmoid: the mixing weights are few; __fdividef would give 0 where 1 + exp(-x) is above 2^126)
-__device__ __forceinline__ float blk_sigmoid(float x) { return __frcp_rn(1.f + expf(-x)); }
+// The two mixing weights of a head: its even lanes hold the logit of k's, the odd ones of v's, each warp forms both with one
+// sigmoid and hands them round.
+__device__ __forceinline__ float2 blk_mix_weights(float logit, int lanes) {
+  const float w = sigmoid_fp32(logit);
+  const int lane0 = (threadIdx.x & 31) & ~(lanes - 1);
+  return make_float2(__shfl_sync(0xffffffffu, w, lane0), __shfl_sync(0xffffffffu, w, lane0 + 1));
+}
 __device__ __forceinline__ float head_sum(float x, int lanes) {
   for (int o = lanes >> 1; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
@@ -103,13 +108,12 @@ __global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixPa
   mix_load(p, t0 - 1, active && pos != 0, ch, C, kp, vp);
   for (int64_t t = t0; t < t1; ++t) {
     uint4 qr = make_uint4(0, 0, 0, 0), kr, vr;
-    float ak = 0.f, av = 0.f;
+    float mix = 0.f;
     mix_load(p, t, active, ch, C, kr, vr);
     if (active) {
       const uint16_t* row = p.y + t * p.ld;
       qr = *reinterpret_cast<const uint4*>(row + ch);
-      ak = blk_load1<kBf16>(row + 4 * C + p.H + h);
-      av = blk_load1<kBf16>(row + 4 * C + 2 * p.H + h);
+      mix = blk_load1<kBf16>(row + 4 * C + (1 + (sub & 1)) * p.H + h);
     }
     const bool first = pos == 0;   // no token before it
     pos = pos + 1 == p.T ? 0 : pos + 1;
@@ -119,7 +123,8 @@ __global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixPa
     blk_unpack<kBf16>(vr, v);
     blk_unpack<kBf16>(kp, kq);
     blk_unpack<kBf16>(vp, vq);
-    const float a = blk_sigmoid(ak), c = blk_sigmoid(av);
+    const float2 w = blk_mix_weights(mix, lanes);
+    const float a = w.x, c = w.y;
     float sq = 0.f, sk = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -160,13 +165,13 @@ struct MixBwdParams {
 struct MixRow {
   uint4 q, dq, dk, dv;   // of token t
   uint4 kp, vp;          // k, v of token t - 1
-  float ak, av, rq, rk;
+  float mix, rq, rk;
 };
 
 template <bool kBf16>
-__device__ __forceinline__ void mix_bwd_load(const MixBwdParams& p, int64_t t, bool on, int ch, int C, int h, MixRow& r) {
+__device__ __forceinline__ void mix_bwd_load(const MixBwdParams& p, int64_t t, bool on, int ch, int C, int h, int sub, MixRow& r) {
   r.q = r.dq = r.dk = r.dv = make_uint4(0, 0, 0, 0);
-  r.ak = r.av = r.rq = r.rk = 0.f;
+  r.mix = r.rq = r.rk = 0.f;
   mix_load(p.f, t - 1, on && t > 0, ch, C, r.kp, r.vp);
   if (on) {
     const uint16_t* row = p.f.y + t * p.f.ld;
@@ -175,8 +180,7 @@ __device__ __forceinline__ void mix_bwd_load(const MixBwdParams& p, int64_t t, b
     r.dq = *reinterpret_cast<const uint4*>(p.dq + o);
     r.dk = *reinterpret_cast<const uint4*>(p.dk + o);
     r.dv = *reinterpret_cast<const uint4*>(p.dv + o);
-    r.ak = blk_load1<kBf16>(row + 4 * C + p.f.H + h);
-    r.av = blk_load1<kBf16>(row + 4 * C + 2 * p.f.H + h);
+    r.mix = blk_load1<kBf16>(row + 4 * C + (1 + (sub & 1)) * p.f.H + h);
     r.rq = p.f.rstd_q[t * p.f.H + h];
     r.rk = p.f.rstd_k[t * p.f.H + h];
   }
@@ -210,10 +214,10 @@ __global__ void __launch_bounds__(kMixThreads, 2) fox_mix_bwd_kernel(const MixBw
     uint4 kc, vc;   // k, v of the current token
     mix_load(f, last, active, ch, C, kc, vc);
     MixRow nx;
-    mix_bwd_load<kBf16>(p, last, active, ch, C, h, nx);
+    mix_bwd_load<kBf16>(p, last, active, ch, C, h, sub, nx);
     for (int64_t t = last; t >= t0; --t) {
       const MixRow r = nx;
-      mix_bwd_load<kBf16>(p, t - 1, active && t > t0, ch, C, h, nx);
+      mix_bwd_load<kBf16>(p, t - 1, active && t > t0, ch, C, h, sub, nx);
       const bool first = t % f.T == 0;
       const bool own = t < t1;
       float k[8], v[8], kq[8], vq[8], dk[8], dv[8];
@@ -223,7 +227,8 @@ __global__ void __launch_bounds__(kMixThreads, 2) fox_mix_bwd_kernel(const MixBw
       blk_unpack<kBf16>(r.vp, vq);
       blk_unpack<kBf16>(r.dk, dk);
       blk_unpack<kBf16>(r.dv, dv);
-      const float a = blk_sigmoid(r.ak), c = blk_sigmoid(r.av);
+      const float2 w = blk_mix_weights(r.mix, lanes);
+      const float a = w.x, c = w.y;
       float ks[8], wdy[8], c1 = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -423,7 +428,7 @@ static inline int blk_rc() { return cudaGetLastError() == cudaSuccess ? FOX_OK :
 static int mix_params(MixParams& p, int64_t B, int64_t T, int64_t H, int64_t D, const void* y, int64_t ld, const float* wq,
                       const float* wk, const int64_t* mask, float eps) {
   if (!y || !wq || !wk || B <= 0 || T <= 0 || H <= 0) return FOX_ERR_BAD_ARG;
-  if (D % 8 || D < 8 || D > 256 || (D & (D - 1))) return FOX_ERR_HEAD_DIM;
+  if (D < 16 || D > 256 || (D & (D - 1))) return FOX_ERR_HEAD_DIM;   // (two lanes a head at least)
   if (H * D > 8 * kMixThreads || T > 2147483647LL) return FOX_ERR_TOO_LARGE;   // (8 channels a thread)
   if (reinterpret_cast<uintptr_t>(y) % 16 || ld % 8 || ld < 4 * H * D + 3 * H) return FOX_ERR_ALIGNMENT;
   p.y = (const uint16_t*)y; p.ld = ld; p.wq = wq; p.wk = wk; p.mask = mask; p.eps = eps;

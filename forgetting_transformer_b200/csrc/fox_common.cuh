@@ -433,6 +433,15 @@ __device__ __forceinline__ uint4 ld_v4_here(const uint4* p) {
   return v;
 }
 
+// sigmoid to about two ulp over the whole range: exp(-|x|) is at most 1, so that the approximate reciprocal of 1 + exp(-|x|),
+// in [1, 2], needs one Newton step and no case of its own, and the left tail keeps its smallest values.
+__device__ __forceinline__ float sigmoid_fp32(float x) {
+  const float e = expf(-fabsf(x)), y = 1.f + e;
+  float r = __fdividef(1.f, y);
+  r = fmaf(r, fmaf(-y, r, 1.f), r);
+  return x >= 0.f ? r : e * r;
+}
+
 // three-input maximum (one instruction on sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;

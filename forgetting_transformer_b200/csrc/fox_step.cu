@@ -299,8 +299,7 @@ __global__ void __launch_bounds__(128) fox_step_mix_kernel(const StepMixParams p
   pdl_wait();
   pdl_launch();
   const float* y = p.y + b * p.ld;
-  auto sigmoid = [](float x) { return __frcp_rn(1.f + expf(-x)); };   // (full fp32, as torch.sigmoid)
-  const float ak = sigmoid(y[4 * C + p.H + h]), av = sigmoid(y[4 * C + 2 * p.H + h]);
+  const float ak = sigmoid_fp32(y[4 * C + p.H + h]), av = sigmoid_fp32(y[4 * C + 2 * p.H + h]);
   float q = 0.f, k = 0.f, v = 0.f;
   if (on) {
     q = y[ch];

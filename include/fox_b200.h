@@ -253,7 +253,7 @@ int fox_normgate_bwd_ld(int device, void* stream, int dtype, int64_t tokens, int
  * weights sigmoid(k mix), sigmoid(v mix) (token_shift.py:21-158, ShiftLinear, modeling_forgetting_transformer.py:44-95), then per-head RMSNorm of q
  * and k (layernorm.py:183-245) with fp32 weights wq, wk (C).  mask (B,T) int64 or NULL: 0 = padding, whose k and v rows
  * count as zero.  q, k, v: (B*T, C); rstd_q, rstd_k (B*T, H) fp32, both or neither; seq_start (B) or NULL receives
- * T - sum(mask[b]).  C <= 2048. */
+ * T - sum(mask[b]).  D a power of two from 16 to 256, C <= 2048. */
 int fox_mix_fwd(int device, void* stream, int dtype, int64_t B, int64_t T, int64_t H, int64_t D, const void* y, int64_t ld,
                 const float* wq, const float* wk, float eps, const int64_t* mask, void* q, void* k, void* v, float* rstd_q,
                 float* rstd_k, int64_t* seq_start);
