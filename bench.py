@@ -642,7 +642,8 @@ def run_ours(args, w, wname):
         lin_flops = 6.0 * tokens_b * (5 * hidden * hidden + 3 * hidden * inter + 3 * hidden * w["H"])
         block = {"shape": f"B{w['B']} T{w['T']} hidden {hidden}, {w['H']} heads, SwiGLU {inter}, bf16 weights",
                  "ms_per_step": ms_blk,
-                 "attention_kernels_ms": sum(v_[1] * v_[0] / n_blk for k_, v_ in bk.items()),
+                 "attention_kernels_ms": sum(v_[1] * v_[0] / n_blk for k_, v_ in bk.items()
+                                             if k_.startswith(("fox_attn_", "fox_find_index", "fox_bwd_"))),
                  "attention_flops": flops, "linear_flops": lin_flops,
                  "tflops_total": (flops + lin_flops) / (ms_blk * 1e-3) / 1e12}
         del blk, xb, dyb
@@ -758,10 +759,16 @@ def run_ours(args, w, wname):
             line["normgate"] = normgate
         n_vec = w["B"] * w["H"] * w["T"]
         aux = {}
-        for name, bytes_ in (("fox_cumsum_fwd", 8 * n_vec), ("fox_revcumsum", 12 * n_vec),
-                             ("fox_bwd_delta", 2 * 2 * n_vec * w["D"] + 4 * n_vec),
-                             ("fox_dq_convert", 6 * n_vec * w["D"])):
-            if name in kern:
+        # bytes a launch cannot do without.  fox_attn_prologue: gates in, prefixes out; k once for its row norms (from 1024
+        # keys on), q too for the automatic threshold.  fox_bwd_delta: out and dout in, delta out; for the one-pass backward
+        # it clears the fp32 dQ accumulator (64 columns at least) and the row sums.  fox_bwd_finish: both halves of the gate
+        # gradient in, the gradient out; for the one-pass backward the accumulator in, dQ out.
+        norms = (w["T"] >= 1024 or thr == "auto") + (thr == "auto")
+        acc = 0 if two_kernel else n_vec * max(w["D"], 64) * 4
+        for name, bytes_ in (("fox_attn_prologue", 8 * n_vec + norms * 2 * n_vec * w["D"]),
+                             ("fox_bwd_delta", 2 * 2 * n_vec * w["D"] + 4 * n_vec + (acc + 4 * n_vec if acc else 0)),
+                             ("fox_bwd_finish", 12 * n_vec + (acc + 2 * n_vec * w["D"] if acc else 0))):
+            if name in kern and not cp:     # (a context-parallel step launches them per chunk)
                 aux[name] = {"ms": kern[name][1], "gbs": bytes_ / (kern[name][1] * 1e-3) / 1e9}
         line["hbm_kernels"] = aux
         if world == 1 and not args.no_cpu:

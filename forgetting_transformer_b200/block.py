@@ -3,8 +3,12 @@
 Mirrors the data flow of upstream's ``ForgettingAttentionLayer`` / ``ForgettingTransformerMLP`` /
 ``ForgettingTransformerBlock`` (modeling_forgetting_transformer.py:98-430, 467-516, 519-622) in the "Pro"
 configuration: output gate + output norm, per-head QK-norm, data-dependent K and V token shift, full forget
-gate, no rotary embedding; training path and, with an ``FgateCache``, the prefill / generation path.  The matrix products are ``nn.Linear`` / ``F.linear`` (cuBLAS);
-everything between them is a kernel of this library:
+gate, no rotary embedding; training path and, with an ``FgateCache``, the prefill / generation path.
+
+A plain block without a cache, and a generated token with one, run natively (csrc/host_block.cpp): the projections of a
+sequence are one cuBLASLt product with stacked weights, those of a token kernels of this library.  Everything else runs the
+modules below one by one, with ``nn.Linear`` / ``F.linear`` (cuBLAS) for the products and a kernel of this library for what
+lies between them:
 
     x -> RMSNorm -> q_proj, ShiftLinear(k), ShiftLinear(v), fgate_proj, ogate_proj
       -> per-head RMSNorm(q), RMSNorm(k) -> forgetting_attention(log sigmoid(fgate))

@@ -281,8 +281,8 @@ def make_graphed(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_fgate: t
                  head_first: bool = False, seq_start: Optional[torch.Tensor] = None,
                  sm_scale: Optional[float] = None,
                  adaptive_threshold=None, num_warmup_iters: int = 3):
-    """CUDA-graph replay of a step for launch-bound shapes (B4 T512 H12 D64: 7 launches whose device time is a
-    fraction of their launch cost).  Returns ``f(q, k, v, log_fgate) -> out`` with the same autograd contract as
+    """CUDA-graph replay of a step for launch-bound shapes (B4 T512 H12 D64: five launches and the autograd engine's hand-over
+    between threads).  Returns ``f(q, k, v, log_fgate) -> out`` with the same autograd contract as
     ``forgetting_attention`` for tensors of exactly the sample arguments' shapes, dtypes and ``requires_grad``
     flags.  Every entry point of the library launches on the caller's current stream, allocates nothing and never
     synchronises, and the cached TMA descriptors are keyed by (pointer, shape, strides), so
