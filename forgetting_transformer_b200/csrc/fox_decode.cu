@@ -35,6 +35,8 @@ constexpr int kDecRows = 4;         // rows of K and of V in flight per lane
 constexpr int kDecMaxCluster = 8;
 constexpr int kDecMaxSplits = 1024;   // taken
 constexpr int kDecMostSplits = 512;   // asked for by fox_attn_decode_splits
+constexpr int64_t kDecSlots = 444, kDecClusterSlots = 400;                            // CTAs of a wave
+constexpr int64_t kDecStartKeys = 600, kDecMergeKeys = 120, kDecLeastKeys = 128;      // (at fox_attn_decode_splits)
 constexpr float kDecLog2e = 1.4426950408889634f;
 
 struct DecodeParams {
@@ -391,10 +393,27 @@ static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
 
 using namespace fox;
 
-// Ranges per (b,h): about four CTAs per SM over all (b,h), at least 128 keys each.
+// Ranges per (b,h), so that the CTAs come in whole waves: 444 (three per SM) where a second kernel merges, 400 where clusters
+// do (those find no room on the last SMs of a GPC: 72 x 5 CTAs 36.1 us, 72 x 6 52.1).  A (b,h) that is one range of a wave
+// takes the next wave too where its shorter ranges pay for the second start, some 600 keys (256 (b,h) of 4099 keys, head dim
+// 128: one range 105 us, three 94; of 1024 keys: 28.5 and 31.3).  Eight ranges need no merge kernel, which is worth some 120
+// keys.  At least 128 keys a range.  Four CTAs per SM on average, as before, left a last wave nearly empty: 24 x 65536 keys of
+// head dim 64 in 25 ranges 81.4 us, in 18 67.2; 48 x 8192 25.7 -> 22.6; 192 x 2048 26.2 -> 22.0; 72 x 5000 of 128 41.3 -> 36.1.
 extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
-  int64_t s = (148 * 4 + B * H - 1) / (B * H);
-  const int64_t most = (N + 127) / 128;
+  const int64_t bh = B * H;
+  auto fit = [&](int64_t waves) {
+    const int64_t s = waves * kDecSlots / bh;
+    return s > kDecMaxCluster ? s : waves * kDecClusterSlots / bh > 1 ? waves * kDecClusterSlots / bh : int64_t{1};
+  };
+  const int64_t waves = (bh + kDecSlots - 1) / kDecSlots;
+  int64_t s = fit(waves);
+  if (s == 1) {
+    const int64_t next = fit(waves + 1);
+    if ((waves + 1) * (N / next + kDecStartKeys) < waves * (N + kDecStartKeys)) s = next;
+  } else if (s > kDecMaxCluster && N / kDecMaxCluster < N / s + kDecMergeKeys) {
+    s = kDecMaxCluster;
+  }
+  const int64_t most = (N + kDecLeastKeys - 1) / kDecLeastKeys;
   if (s > most) s = most;
   if (s > kDecMostSplits) s = kDecMostSplits;
   return s < 1 ? 1 : s;

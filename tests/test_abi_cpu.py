@@ -177,3 +177,14 @@ def test_layer_glue_expressions():
     ws = fox.acp_threshold_from_qk_norm(wq[:D], wk[:D], H, D, T, tol, share_param_across_head=True)
     assert ws.dim() == 0 and ws.item() == (-(2 * wq[:D].abs().max() * wk[:D].abs().max() * math.sqrt(D)
                                               + math.log(T)) + tol).item()
+
+
+@pytest.mark.parametrize("bh", [1, 24, 49, 50, 72, 144, 223, 256, 400, 401, 444, 445, 512, 889, 65535])
+@pytest.mark.parametrize("n", [1, 256, 257, 2000, 70000, 2 ** 31 - 2048])
+def test_decode_ranges_fill_whole_waves(bh, n):
+    """Ranges of one-token attention: at least 128 keys each, and never more CTAs than the waves they are cut for hold (444 a
+    wave, 400 where clusters merge)."""
+    s = _lib.load().fox_attn_decode_splits(1, bh, n)
+    assert 1 <= s <= min(512, max(1, -(-n // 128)))
+    waves = -(-bh // 444) + (1 if -(-bh // 444) * 400 // bh <= 1 else 0)
+    assert s == 1 or bh * s <= waves * (444 if s > 8 else 400)
