@@ -86,38 +86,51 @@ def join_class_shards(loss_parts, lse_local, target, lse_square_scale, ignore_in
     return losses, z_losses, lse
 
 
+def _forward(ctx, logits, target, label_smoothing, logit_scale, lse_square_scale, ignore_index, inplace_backward, process_group):
+    """Forward of the functions below: (losses, z_losses, what the backward needs as tensors)."""
+    if not logits.is_cuda:
+        raise _lib.FoxError("cross_entropy_loss needs CUDA tensors on an sm_100 device; there is no CPU path")
+    n_rows, n_cols = logits.shape
+    assert target.shape == (n_rows,)
+    if logits.dtype not in _DTYPES:
+        raise _lib.FoxError(f"unsupported logits dtype {logits.dtype}")
+    world = 1 if process_group is None else dist.get_world_size(process_group)
+    rank = 0 if process_group is None else dist.get_rank(process_group)
+    total_classes, class_start = world * n_cols, rank * n_cols
+    es = logits.element_size()
+    if logits.stride(-1) != 1 or (logits.stride(0) * es) % 16 or logits.data_ptr() % 16:
+        logits = logits.contiguous()
+        if (logits.stride(0) * es) % 16:     # a class count whose rows cannot all start on 16 bytes: pad the stride
+            pad = torch.empty((n_rows, -(-n_cols * es // 16) * 16 // es), dtype=logits.dtype, device=logits.device)
+            pad[:, :n_cols] = logits
+            logits = pad[:, :n_cols]
+    target = target.to(torch.long).contiguous()
+    losses, z_losses, lse = _local_forward(logits, target, label_smoothing, logit_scale, lse_square_scale,
+                                           ignore_index, total_classes, class_start, world > 1)
+    if world > 1:
+        losses, z_losses, lse = join_class_shards(losses, lse, target, float(lse_square_scale), int(ignore_index),
+                                                  process_group)
+    ctx.args = (float(label_smoothing), float(logit_scale), float(lse_square_scale), int(ignore_index))
+    ctx.classes = (total_classes, class_start)
+    ctx.inplace_backward = inplace_backward
+    return losses, z_losses, (logits, lse, target)
+
+
+def _gradient(ctx, logits):
+    # (same row stride as the saved logits: a re-laid class count keeps its 16-byte aligned rows)
+    return logits if ctx.inplace_backward else torch.empty_strided(logits.shape, logits.stride(), dtype=logits.dtype,
+                                                                   device=logits.device)
+
+
 class CrossEntropyLossFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, logits, target, label_smoothing=0.0, logit_scale=1.0, lse_square_scale=0.0, ignore_index=-100,
                 inplace_backward=False, process_group=None):
-        if not logits.is_cuda:
-            raise _lib.FoxError("cross_entropy_loss needs CUDA tensors on an sm_100 device; there is no CPU path")
-        n_rows, n_cols = logits.shape
-        assert target.shape == (n_rows,)
-        if logits.dtype not in _DTYPES:
-            raise _lib.FoxError(f"unsupported logits dtype {logits.dtype}")
-        world = 1 if process_group is None else dist.get_world_size(process_group)
-        rank = 0 if process_group is None else dist.get_rank(process_group)
-        total_classes, class_start = world * n_cols, rank * n_cols
-        es = logits.element_size()
-        if logits.stride(-1) != 1 or (logits.stride(0) * es) % 16 or logits.data_ptr() % 16:
-            logits = logits.contiguous()
-            if (logits.stride(0) * es) % 16:     # a class count whose rows cannot all start on 16 bytes: pad the stride
-                pad = torch.empty((n_rows, -(-n_cols * es // 16) * 16 // es), dtype=logits.dtype, device=logits.device)
-                pad[:, :n_cols] = logits
-                logits = pad[:, :n_cols]
-        target = target.to(torch.long).contiguous()
-        losses, z_losses, lse = _local_forward(logits, target, label_smoothing, logit_scale, lse_square_scale,
-                                               ignore_index, total_classes, class_start, world > 1)
-        if world > 1:
-            losses, z_losses, lse = join_class_shards(losses, lse, target, float(lse_square_scale), int(ignore_index),
-                                                      process_group)
-        ctx.save_for_backward(logits, lse, target)
+        losses, z_losses, saved = _forward(ctx, logits, target, label_smoothing, logit_scale, lse_square_scale, ignore_index,
+                                           inplace_backward, process_group)
+        ctx.save_for_backward(*saved)
         ctx.mark_non_differentiable(z_losses)
-        ctx.args = (float(label_smoothing), float(logit_scale), float(lse_square_scale), int(ignore_index))
-        ctx.classes = (total_classes, class_start)
-        ctx.inplace_backward = inplace_backward
         return losses, z_losses
 
     @staticmethod
@@ -125,12 +138,41 @@ class CrossEntropyLossFunction(torch.autograd.Function):
         del grad_z_losses  # z_losses are for logging only, as upstream
         logits, lse, target = ctx.saved_tensors
         label_smoothing, logit_scale, lse_square_scale, ignore_index = ctx.args
-        # (same row stride as the saved logits: a re-laid class count keeps its 16-byte aligned rows)
-        dlogits = logits if ctx.inplace_backward else torch.empty_strided(logits.shape, logits.stride(),
-                                                                          dtype=logits.dtype, device=logits.device)
+        dlogits = _gradient(ctx, logits)
         _local_backward(logits, target, lse, grad_losses.float(), label_smoothing, logit_scale, lse_square_scale,
                         ignore_index, ctx.classes[0], ctx.classes[1], dlogits)
         return dlogits, None, None, None, None, None, None, None
+
+
+class _MeanLossFunction(torch.autograd.Function):
+    """The mean of the losses over the rows with a target, in one kernel behind the losses' own."""
+
+    @staticmethod
+    def forward(ctx, logits, target, label_smoothing, logit_scale, lse_square_scale, ignore_index, inplace_backward):
+        losses, _, (logits, lse, target) = _forward(ctx, logits, target, label_smoothing, logit_scale, lse_square_scale,
+                                                    ignore_index, inplace_backward, None)
+        dev = logits.device
+        with torch.cuda.device(dev):
+            mean, count = torch.empty((), dtype=torch.float32, device=dev), torch.empty((), dtype=torch.float32, device=dev)
+            _lib.check(_lib.load().fox_cross_entropy_mean(dev.index, _stream(), losses.shape[0], losses.data_ptr(),
+                                                          target.data_ptr(), int(ignore_index), mean.data_ptr(),
+                                                          count.data_ptr()), "fox_cross_entropy_mean")
+        ctx.save_for_backward(logits, lse, target, count)
+        return mean
+
+    @staticmethod
+    def backward(ctx, grad_mean):
+        logits, lse, target, count = ctx.saved_tensors
+        dlogits = _gradient(ctx, logits)
+        grad_mean = grad_mean.float()
+        dev = logits.device
+        with torch.cuda.device(dev):
+            _lib.check(_lib.load().fox_cross_entropy_bwd_mean(dev.index, _stream(), _DTYPES[logits.dtype], logits.shape[0],
+                                                              logits.shape[1], logits.data_ptr(), logits.stride(0),
+                                                              target.data_ptr(), lse.data_ptr(), grad_mean.data_ptr(),
+                                                              count.data_ptr(), *ctx.args, dlogits.data_ptr(),
+                                                              dlogits.stride(0)), "fox_cross_entropy_bwd_mean")
+        return dlogits, None, None, None, None, None, None
 
 
 def cross_entropy_loss(logits: torch.Tensor, target: torch.Tensor, label_smoothing: float = 0.0,
@@ -161,6 +203,9 @@ class FusedCrossEntropyLoss(nn.Module):
 
     def forward(self, input, target):
         assert input.is_cuda and target.is_cuda, "Only support CUDA tensors"
+        if self.reduction == "mean" and self.process_group is None and not self.return_z_loss:
+            return _MeanLossFunction.apply(input, target, self.label_smoothing, self.logit_scale, self.lse_square_scale,
+                                           self.ignore_index, self.inplace_backward)
         loss, z_loss = cross_entropy_loss(input, target, label_smoothing=self.label_smoothing,
                                           logit_scale=self.logit_scale, lse_square_scale=self.lse_square_scale,
                                           ignore_index=self.ignore_index, inplace_backward=self.inplace_backward,

@@ -351,6 +351,16 @@ int fox_cross_entropy_bwd(int device, void* stream, int dtype, int64_t n_rows, i
                           int64_t dloss_stride, float label_smoothing, float logit_scale, float lse_square_scale,
                           int64_t ignore_index, void* dlogits, int64_t dlogits_row_stride);
 
+/* The mean of the losses over the rows whose label is not ignore_index (FusedCrossEntropyLoss with reduction='mean',
+ * fused_cross_entropy.py:387-389) and the number of those rows, one fp32 each; and the backward through it: dloss of every
+ * row is *dmean / *count. */
+int fox_cross_entropy_mean(int device, void* stream, int64_t n_rows, const float* losses, const int64_t* labels,
+                           int64_t ignore_index, float* mean, float* count);
+int fox_cross_entropy_bwd_mean(int device, void* stream, int dtype, int64_t n_rows, int64_t n_cols, const void* logits,
+                               int64_t row_stride, const int64_t* labels, const float* lse, const float* dmean,
+                               const float* count, float label_smoothing, float logit_scale, float lse_square_scale,
+                               int64_t ignore_index, void* dlogits, int64_t dlogits_row_stride);
+
 /* The same loss with the classes split over ranks (tensor parallelism over the vocabulary; replaces the
  * `process_group` path of fused_cross_entropy.py:150-151, 196-226 and :229-273).  This rank holds n_cols of
  * total_classes classes, starting at class_start.  The forward writes the rank's own log-sum-exp (lse_local) and

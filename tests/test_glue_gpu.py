@@ -344,3 +344,28 @@ def test_cross_entropy_gradient_of_rows_that_are_not_finite():
     loss.sum().backward()
     assert (x.grad[0] == 0).all() and (x.grad[3] == 0).all()
     assert x.grad[1, 100].isnan() and x.grad[2, 7].isnan()
+
+
+@pytest.mark.parametrize("rows", [1, 31, 1025, 8192, 8193, 40007])
+def test_mean_cross_entropy_over_any_number_of_rows(rows):
+    """reduction='mean' at the edges of one CTA's trip and of the cluster: the loss is the fp64 mean of the rows' fp32 losses
+    rounded once, the gradient that of losses.sum() / count to an fp32 rounding, and no row with a target gives NaN."""
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, 40, generator=g).cuda()
+    labels = torch.randint(0, 40, (rows,), generator=g).cuda()
+    labels[3::5] = 7
+    for ignore in (7, -100):
+        xs = [x.clone().requires_grad_() for _ in range(2)]
+        mean = fox.FusedCrossEntropyLoss(ignore_index=ignore, label_smoothing=0.1)(xs[0], labels)
+        losses, _ = fox.cross_entropy_loss(xs[1], labels, 0.1, 1.0, 0.0, ignore)
+        count = (labels != ignore).sum()
+        assert mean.dtype == torch.float32 and mean.shape == ()
+        ref = losses.double().sum() / count
+        assert (mean - ref).abs() <= 2 ** -23 * ref.abs()
+        (mean * 3).backward()
+        (losses.sum() / count * 3).backward()
+        assert (xs[0].grad - xs[1].grad).abs().max() <= 2 ** -22 * xs[1].grad.abs().max()
+    none = fox.FusedCrossEntropyLoss(ignore_index=7)(x.requires_grad_(), torch.full_like(labels, 7))
+    assert none.isnan()
+    none.backward()
+    assert (x.grad == 0).all()
