@@ -433,6 +433,17 @@ __device__ __forceinline__ uint4 ld_v4_here(const uint4* p) {
   return v;
 }
 
+// Untiled copy into shared memory; both addresses 16-byte aligned, bytes a multiple of 16.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+// Asks for `bytes` (a multiple of 16) from p on (16-byte aligned) to be brought into L2.
+__device__ __forceinline__ void l2_request(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // sigmoid to about two ulp over the whole range: exp(-|x|) is at most 1, so that the approximate reciprocal of 1 + exp(-|x|),
 // in [1, 2], needs one Newton step and no case of its own, and the left tail keeps its smallest values.
 __device__ __forceinline__ float sigmoid_fp32(float x) {

@@ -22,6 +22,8 @@
 // launched early (programmatic dependent launch).
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "fox_common.cuh"
 #include "fox_host.h"
 
@@ -56,6 +58,44 @@ struct DecodeParams {
   bool pdl;                    // launched with programmatic stream serialization
 };
 
+// A token's way into the attention (fox_step_mix's work, kStep below): q comes from the projections, and the CTA that has the
+// last key puts it into the cache first.
+struct DecodeStep {
+  const float* y;              // (B, ld): [q | k | v | ogate | fgate | k mix | v mix]
+  int64_t ld;
+  const void *wq, *wk, *bias;  // (C), (C), (H) or nullptr
+  int wq_dtype, wk_dtype, bias_dtype;
+  float eps;
+  const int64_t* mask;         // (B, N) or nullptr: the first valid key is N - its sum
+  uint16_t *k_state, *v_state; // (B, C), replaced
+  uint16_t *k_cache, *v_cache; // (B, H, cap, D)
+  float* g_cache;              // (B, H, cap)
+  int64_t cap;
+};
+
+__device__ __forceinline__ float dec_load_any(const void* w, int dtype, int i) {
+  if (dtype == FOX_DTYPE_FP32) return static_cast<const float*>(w)[i];
+  const uint32_t u = static_cast<const uint16_t*>(w)[i];
+  return dtype == FOX_DTYPE_BF16 ? unpack2<true>(u).x : unpack2<false>(u).x;
+}
+template <bool kBf16>
+__device__ __forceinline__ uint4 dec_pack(const float* f) {
+  return make_uint4(pack2<kBf16>(f[0], f[1]), pack2<kBf16>(f[2], f[3]), pack2<kBf16>(f[4], f[5]), pack2<kBf16>(f[6], f[7]));
+}
+__device__ __forceinline__ void dec_load8(const float* p, float* f) {   // (16-byte aligned)
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+template <int kLanes>
+__device__ __forceinline__ float dec_norm(const float* f, float inv_d, float eps) {   // over the lanes that share a row
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) ss = fmaf(f[c], f[c], ss);
+#pragma unroll
+  for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  return rsqrtf(ss * inv_d + eps);
+}
+
 template <bool kBf16>
 __device__ __forceinline__ void dec_unpack(const uint4& v, float* f) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -84,9 +124,9 @@ __device__ __forceinline__ void dec_store(const DecodeParams& p, int b, int h, i
   p.o[b * p.o_sb + h * p.o_sh + d] = static_cast<uint16_t>(pk & 0xffffu);
 }
 
-template <bool kBf16, int D, bool kCluster>
+template <bool kBf16, int D, bool kCluster, bool kStep = false>
 __global__ void __launch_bounds__(kDecThreads, 3)
-fox_decode_kernel(const DecodeParams p) {
+fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeStep, char> step) {
   constexpr int LPR = D / 8, RPW = 32 / LPR;
   constexpr int kBatch = kDecWarps * RPW * kDecRows;   // keys a CTA takes per step
   __shared__ float s_bias[kDecTile];                   // (sum of the gates after key j, inside the range) * log2e
@@ -99,36 +139,44 @@ fox_decode_kernel(const DecodeParams p) {
   const int sub = lane % LPR, grp = lane / LPR;
   const int64_t bh = static_cast<int64_t>(b) * p.H + h;
   const int N = p.N;
-  // (no effect without programmatic serialization; what follows may start, and waits for this grid's end)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  int lo = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
-  if (p.start_index) {
-    const int64_t si = p.start_index[bh];
-    lo = max(lo, static_cast<int>(si < N ? si : N));
+  int lo = 0;
+  if constexpr (kStep) {
+    // Before the wait for the projections: what does not come from the kernel in front.  (A kernel of the chain lets the next
+    // one start after its own wait, so everything in front of the projections has ended: mask, cache and states are final.)
+    if (step.mask) {
+      __shared__ long long s_n[kDecWarps];
+      long long n = 0;
+      for (int i = tid; i < N; i += kDecThreads) n += step.mask[static_cast<int64_t>(b) * N + i];
+      for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+      if (lane == 0) s_n[warp] = n;
+      __syncthreads();
+      n = 0;
+      for (int w = 0; w < kDecWarps; ++w) n += s_n[w];
+      lo = static_cast<int>(max(min(static_cast<long long>(N) - n, static_cast<long long>(N)), 0LL));
+    }
+  } else {
+    // (no effect without programmatic serialization; what follows may start, and waits for this grid's end)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.seq_start) lo = static_cast<int>(p.seq_start[b]);
+    if (p.start_index) {
+      const int64_t si = p.start_index[bh];
+      lo = max(lo, static_cast<int>(si < N ? si : N));
+    }
+    lo = max(min(lo, N), 0);
   }
-  lo = max(min(lo, N), 0);
-  const int span = N - lo;
+  const int end = kStep ? N - 1 : N;   // (the token's own key is not read from the cache)
+  const int span = max(end - lo, 0);
   const int per = (span + p.splits - 1) / p.splits;
-  const int j0 = min(N, lo + split * per), j1 = min(N, j0 + per);
+  const int j0 = min(end, lo + split * per), j1 = min(end, j0 + per);
 
-  float qv[8];
-  dec_unpack<kBf16>(*reinterpret_cast<const uint4*>(p.q + b * p.q_sb + h * p.q_sh + sub * 8), qv);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) qv[c] *= p.qk_scale;
   const uint16_t* kb = p.k + b * p.k_sb + h * p.k_sh + sub * 8;
   const uint16_t* vb = p.v + b * p.v_sb + h * p.v_sh + sub * 8;
-  const float* lam = p.lam ? p.lam + bh * N : nullptr;
+  const float* lam = !kStep && p.lam ? p.lam + bh * N : nullptr;
   const float* gate = p.gate + b * p.g_sb + h * p.g_sh;
   const float lam_q = lam ? lam[N - 1] : 0.f;
-
-  float m = -INFINITY, l = 0.f, acc[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) acc[c] = 0.f;
   float carry = 0.f;   // sum of the range's gates right of the current tile
-  for (int e = j1; e > j0; e -= kDecTile) {
-    const int t0 = max(j0, e - kDecTile), n = e - t0;
-    // ---- bias of the tile's keys ----
+  auto bias = [&](int t0, int n) {
     __syncthreads();
     if (lam) {
       for (int i = tid; i < n; i += kDecThreads) s_bias[i] = (lam_q - lam[t0 + i]) * kDecLog2e;
@@ -164,47 +212,161 @@ fox_decode_kernel(const DecodeParams p) {
       }
     }
     __syncthreads();
-    // ---- the tile's keys ----
-    for (int i0 = 0; i0 < n; i0 += kBatch) {
-      uint4 kr[kDecRows], vr[kDecRows];
+  };
+  uint4 kr[kDecRows], vr[kDecRows];
+  auto load = [&](int t0, int n, int i0) {
 #pragma unroll
-      for (int u = 0; u < kDecRows; ++u) {
-        const int i = min(i0 + (u * kDecWarps + warp) * RPW + grp, n - 1);
-        kr[u] = *reinterpret_cast<const uint4*>(kb + static_cast<int64_t>(t0 + i) * p.k_st);
+    for (int u = 0; u < kDecRows; ++u) {
+      const int i = min(i0 + (u * kDecWarps + warp) * RPW + grp, n - 1);
+      kr[u] = *reinterpret_cast<const uint4*>(kb + static_cast<int64_t>(t0 + i) * p.k_st);
+    }
+#pragma unroll
+    for (int u = 0; u < kDecRows; ++u) {
+      const int i = min(i0 + (u * kDecWarps + warp) * RPW + grp, n - 1);
+      vr[u] = *reinterpret_cast<const uint4*>(vb + static_cast<int64_t>(t0 + i) * p.v_st);
+    }
+  };
+
+  float qv[8];
+  float g_new = 0.f;
+  const bool owner = kStep && split == p.splits - 1 && warp == 0;
+  // kStep: [norm weights of q, k | gate bias], the states' key and value, which the token's replace
+  __shared__ __align__(16) float s_w[kStep ? 2 * D + 1 : 1];
+  __shared__ uint4 s_new[2][kStep ? LPR : 1];
+  if constexpr (kStep) {
+    const int C = p.H * D;
+    for (int i = tid; i < 2 * D; i += kDecThreads)
+      s_w[i] = i < D ? dec_load_any(step.wq, step.wq_dtype, h * D + i) : dec_load_any(step.wk, step.wk_dtype, h * D + i - D);
+    if (tid == 0) s_w[2 * D] = step.bias ? dec_load_any(step.bias, step.bias_dtype, h) : 0.f;
+    if (tid < 2 * LPR)
+      s_new[tid / LPR][tid % LPR] = *reinterpret_cast<const uint4*>((tid < LPR ? step.k_state : step.v_state) +
+                                                                    static_cast<int64_t>(b) * C + h * D + (tid % LPR) * 8);
+    if (j1 > j0) {   // the first tile's gates and rows, and a request for what follows them
+      const int t0 = max(j0, j1 - kDecTile);
+      // (32 KB of each: 444 CTAs' requests stay well inside L2)
+      const uint32_t o = tid * 4096u, bytes = min(static_cast<uint32_t>(j1 - t0) * (D * 2), 32768u);
+      if (o < bytes) {
+        const int64_t at = (bh * step.cap + t0) * D;
+        l2_request(reinterpret_cast<const char*>(step.k_cache + at) + o, min(4096u, bytes - o));
+        l2_request(reinterpret_cast<const char*>(step.v_cache + at) + o, min(4096u, bytes - o));
       }
+      load(t0, j1 - t0, 0);
+      bias(t0, j1 - t0);
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const float inv_d = 1.f / static_cast<float>(D);
+    const int ch = h * D + sub * 8;
+    const float* y = step.y + b * step.ld;
+    dec_load8(y + ch, qv);
+    if (owner) {   // the token's key, value and gate; its projections replace the states
+      const int64_t so = static_cast<int64_t>(b) * C + ch;
+      float kp[8], vp[8], k_new[8], v_new[8];
+      dec_load8(y + C + ch, k_new);
+      dec_load8(y + 2 * C + ch, v_new);
+      const float f = y[4 * C + h] + s_w[2 * D], mk = y[4 * C + p.H + h], mv = y[4 * C + 2 * p.H + h];
+      dec_unpack<kBf16>(s_new[0][sub], kp);
+      dec_unpack<kBf16>(s_new[1][sub], vp);
+      const float ak = sigmoid_fp32(mk), av = sigmoid_fp32(mv);
+      const uint4 k16 = dec_pack<kBf16>(k_new), v16 = dec_pack<kBf16>(v_new);
+      dec_unpack<kBf16>(k16, k_new);
+      dec_unpack<kBf16>(v16, v_new);
 #pragma unroll
-      for (int u = 0; u < kDecRows; ++u) {
-        const int i = min(i0 + (u * kDecWarps + warp) * RPW + grp, n - 1);
-        vr[u] = *reinterpret_cast<const uint4*>(vb + static_cast<int64_t>(t0 + i) * p.v_st);
+      for (int c = 0; c < 8; ++c) {
+        k_new[c] = ak * kp[c] + (1.f - ak) * k_new[c];
+        v_new[c] = av * vp[c] + (1.f - av) * v_new[c];
       }
-      float s[kDecRows], mx = m;
+      const float rk = dec_norm<LPR>(k_new, inv_d, step.eps);
 #pragma unroll
-      for (int u = 0; u < kDecRows; ++u) {
-        float kv[8];
-        dec_unpack<kBf16>(kr[u], kv);
-        float x = 0.f;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) x = fmaf(qv[c], kv[c], x);
-#pragma unroll
-        for (int o = LPR / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        const int i = i0 + (u * kDecWarps + warp) * RPW + grp;
-        s[u] = i < n ? x + s_bias[min(i, n - 1)] : -INFINITY;
-        mx = fmaxf(mx, s[u]);
+      for (int c = 0; c < 8; ++c) k_new[c] *= rk * s_w[D + sub * 8 + c];
+      const uint4 kn = dec_pack<kBf16>(k_new), vn = dec_pack<kBf16>(v_new);
+      g_new = fminf(f, 0.f) - log1pf(expf(-fabsf(f)));
+      if (grp == 0) {
+        const int64_t row = (bh * step.cap + N - 1) * D + sub * 8;
+        *reinterpret_cast<uint4*>(step.k_cache + row) = kn;
+        *reinterpret_cast<uint4*>(step.v_cache + row) = vn;
+        *reinterpret_cast<uint4*>(step.k_state + so) = k16;
+        *reinterpret_cast<uint4*>(step.v_state + so) = v16;
       }
-      const float ref = mx == -INFINITY ? 0.f : mx;
-      const float alpha = fast_exp2(m - ref);   // 0 when m was -inf
-      m = mx;
-      l *= alpha;
+      if (lane == 0) step.g_cache[bh * step.cap + N - 1] = g_new;
+      __syncwarp();
+      if (grp == 0) {   // (read by this warp)
+        s_new[0][sub] = kn;
+        s_new[1][sub] = vn;
+      }
+    }
+    const float rq = dec_norm<LPR>(qv, inv_d, step.eps);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[c] *= alpha;
+    for (int c = 0; c < 8; ++c) qv[c] *= rq * s_w[sub * 8 + c];
+    const uint4 q16 = dec_pack<kBf16>(qv);
+    dec_unpack<kBf16>(q16, qv);
+  } else {
+    dec_unpack<kBf16>(*reinterpret_cast<const uint4*>(p.q + b * p.q_sb + h * p.q_sh + sub * 8), qv);
+  }
 #pragma unroll
-      for (int u = 0; u < kDecRows; ++u) {
-        const float w = fast_exp2(s[u] - ref);  // 0 past the end
-        float vv[8];
-        dec_unpack<kBf16>(vr[u], vv);
-        l += w;
+  for (int c = 0; c < 8; ++c) qv[c] *= p.qk_scale;
+
+  float m = -INFINITY, l = 0.f, acc[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[c] = fmaf(w, vv[c], acc[c]);
+  for (int c = 0; c < 8; ++c) acc[c] = 0.f;
+  auto use = [&](int n, int i0) {
+    float s[kDecRows], mx = m;
+#pragma unroll
+    for (int u = 0; u < kDecRows; ++u) {
+      float kv[8];
+      dec_unpack<kBf16>(kr[u], kv);
+      float x = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) x = fmaf(qv[c], kv[c], x);
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      const int i = i0 + (u * kDecWarps + warp) * RPW + grp;
+      s[u] = i < n ? x + s_bias[min(i, n - 1)] : -INFINITY;
+      mx = fmaxf(mx, s[u]);
+    }
+    const float ref = mx == -INFINITY ? 0.f : mx;
+    const float alpha = fast_exp2(m - ref);   // 0 when m was -inf
+    m = mx;
+    l *= alpha;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[c] *= alpha;
+#pragma unroll
+    for (int u = 0; u < kDecRows; ++u) {
+      const float w = fast_exp2(s[u] - ref);  // 0 past the end
+      float vv[8];
+      dec_unpack<kBf16>(vr[u], vv);
+      l += w;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[c] = fmaf(w, vv[c], acc[c]);
+    }
+  };
+  if (kStep && j1 > j0) use(min(j1 - j0, kDecTile), 0);
+  for (int e = j1; e > j0; e -= kDecTile) {
+    const int t0 = max(j0, e - kDecTile), n = e - t0;
+    const bool begun = kStep && e == j1;   // (its gates and first rows came before the wait)
+    if (!begun) bias(t0, n);
+    for (int i0 = begun ? kBatch : 0; i0 < n; i0 += kBatch) {
+      load(t0, n, i0);
+      use(n, i0);
+    }
+  }
+  if constexpr (kStep) {
+    // The token's own key.  The others' logits lack its gate, which is taken off its logit instead.
+    if (owner) {
+      float kv[8], vv[8], x = 0.f;
+      __syncwarp();
+      dec_unpack<kBf16>(s_new[0][sub], kv);
+      dec_unpack<kBf16>(s_new[1][sub], vv);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) x = fmaf(qv[c], kv[c], x);
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (grp == 0 && lo < N) {
+        float f_old, f_new;
+        dec_join(m, l, x - g_new * kDecLog2e, 1.f, f_old, f_new);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[c] = acc[c] * f_old + vv[c] * f_new;
       }
     }
   }
@@ -239,7 +401,7 @@ fox_decode_kernel(const DecodeParams p) {
   }
   if (p.splits == 1) {
     if (tid < D) dec_store<kBf16, D>(p, b, h, tid, x, lt);
-    if (tid == 0) p.L[bh] = lt > 0.f ? mx * 0.6931471805599453f + __logf(lt) : -INFINITY;
+    if (tid == 0 && p.L) p.L[bh] = lt > 0.f ? mx * 0.6931471805599453f + __logf(lt) : -INFINITY;
     return;
   }
   if constexpr (kCluster) {
@@ -252,14 +414,22 @@ fox_decode_kernel(const DecodeParams p) {
     }
     cluster.sync();
     if (split == 0) {
-      float ms[kDecMaxCluster], after = 0.f, top = -INFINITY;
+      // every remote value is asked for before the first is used
+      float ms[kDecMaxCluster], ls[kDecMaxCluster], gs[kDecMaxCluster], os[kDecMaxCluster];
+#pragma unroll
+      for (int r = 0; r < kDecMaxCluster; ++r) {
+        const float* rem = cluster.map_shared_rank(s_res, r < p.splits ? r : 0);
+        ms[r] = rem[D];
+        ls[r] = rem[D + 1];
+        gs[r] = rem[D + 2];
+        os[r] = rem[tid < D ? tid : 0];
+      }
+      float after = 0.f, top = -INFINITY;
 #pragma unroll
       for (int r = kDecMaxCluster - 1; r >= 0; --r) {
-        ms[r] = -INFINITY;
         if (r < p.splits) {
-          const float* rem = cluster.map_shared_rank(s_res, r);
-          ms[r] = rem[D] + after;
-          after += rem[D + 2];
+          ms[r] += after;
+          after += gs[r];
           top = fmaxf(top, ms[r]);
         }
       }
@@ -267,14 +437,13 @@ fox_decode_kernel(const DecodeParams p) {
 #pragma unroll
       for (int r = 0; r < kDecMaxCluster; ++r) {
         if (r < p.splits && ms[r] != -INFINITY) {
-          const float* rem = cluster.map_shared_rank(s_res, r);
           const float f = fast_exp2(ms[r] - top);
-          lsum = fmaf(rem[D + 1], f, lsum);
-          if (tid < D) osum = fmaf(rem[tid], f, osum);
+          lsum = fmaf(ls[r], f, lsum);
+          osum = fmaf(os[r], f, osum);
         }
       }
       if (tid < D) dec_store<kBf16, D>(p, b, h, tid, osum, lsum);
-      if (tid == 0) p.L[bh] = lsum > 0.f ? top * 0.6931471805599453f + __logf(lsum) : -INFINITY;
+      if (tid == 0 && p.L) p.L[bh] = lsum > 0.f ? top * 0.6931471805599453f + __logf(lsum) : -INFINITY;
     }
     cluster.sync();   // (the others' shared memory is read until here)
   } else {
@@ -356,6 +525,23 @@ __global__ void __launch_bounds__(256) fox_decode_merge_kernel(const DecodeParam
 }
 
 template <bool kBf16, int D>
+static int launch_step(const DecodeParams& p, const DecodeStep& step, int64_t B, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)p.splits, (unsigned)p.H, (unsigned)B);
+  cfg.blockDim = dim3(kDecThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = (unsigned)p.splits;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true, true>, p, step) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+}
+
+template <bool kBf16, int D>
 static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.splits, (unsigned)p.H, (unsigned)B);
@@ -376,10 +562,10 @@ static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
       ++n;
     }
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true>, p) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true>, p, '\0') == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
   }
   cfg.numAttrs = n;
-  if (cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, false>, p) != cudaSuccess) return FOX_ERR_LAUNCH;
+  if (cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, false>, p, '\0') != cudaSuccess) return FOX_ERR_LAUNCH;
   cfg.gridDim = dim3((unsigned)p.H, (unsigned)B);
   cfg.blockDim = dim3(256);
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -478,4 +664,45 @@ extern "C" int fox_attn_decode_gates(int device, void* stream, int dtype, int64_
   p.g_sb = sb; p.g_sh = sh; p.g_sn = sn;
   p.seq_start = seq_start;
   return decode(device, stream, dtype, B, H, N, D, q, k, v, p, sm_scale, o, L, workspace, splits);
+}
+
+// Ranges of fox_step_attn, or 0 where fox_step_mix and fox_attn_decode_gates are the better way: more CTAs than a wave (16
+// sequences x 32 heads of 8192 keys 694 us for two layers, 674 apart), or ranges so long that more than eight of them pay for
+// the two launches more (24 heads of 8000 keys 105 and 101 us).
+extern "C" int64_t fox_step_attn_splits(int64_t B, int64_t H, int64_t N) {
+  const int64_t s = fox_attn_decode_splits(B, H, N);
+  if (B * H * s > kDecSlots) return 0;
+  return s <= kDecMaxCluster ? s : N <= 8 * 768 ? 8 : 0;
+}
+
+extern "C" int fox_step_attn(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t D, const float* y, int64_t ld,
+                             const void* wq, int wq_dtype, const void* wk, int wk_dtype, float eps, const void* bias, int bias_dtype,
+                             const int64_t* mask, void* k_state, void* v_state, void* k_cache, void* v_cache, float* g_cache,
+                             int64_t capacity, int64_t pos, float sm_scale, void* o, int64_t splits) {
+  if (!y || !wq || !wk || !k_state || !v_state || !k_cache || !v_cache || !g_cache || !o || B <= 0 || H <= 0 || B > 65535 || H > 65535 ||
+      pos < 0 || pos >= capacity || pos >= 2147483647LL - kDecTile || splits <= 0 || splits > kDecMaxCluster)
+    return FOX_ERR_BAD_ARG;
+  if (D != 16 && D != 32 && D != 64 && D != 128) return FOX_ERR_HEAD_DIM;
+  if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
+  if (ld % 4 || ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(k_state) | reinterpret_cast<uintptr_t>(v_state) |
+                  reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) % 16))
+    return FOX_ERR_ALIGNMENT;
+  if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
+  DecodeParams p{};
+  p.k = (const uint16_t*)k_cache; p.v = (const uint16_t*)v_cache;
+  p.k_sb = p.v_sb = H * capacity * D; p.k_sh = p.v_sh = capacity * D; p.k_st = p.v_st = D;
+  p.gate = g_cache; p.g_sb = H * capacity; p.g_sh = capacity; p.g_sn = 1;
+  p.o = (uint16_t*)o; p.o_sb = H * D; p.o_sh = D;
+  p.H = (int)H; p.N = (int)(pos + 1); p.splits = (int)splits;
+  p.qk_scale = sm_scale * kDecLog2e;
+  const DecodeStep s{y, ld, wq, wk, bias, wq_dtype, wk_dtype, bias_dtype, eps, mask, (uint16_t*)k_state, (uint16_t*)v_state,
+                     (uint16_t*)k_cache, (uint16_t*)v_cache, g_cache, capacity};
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool bf = dtype == FOX_DTYPE_BF16;
+  switch (D) {
+    case 16: return bf ? launch_step<true, 16>(p, s, B, st) : launch_step<false, 16>(p, s, B, st);
+    case 32: return bf ? launch_step<true, 32>(p, s, B, st) : launch_step<false, 32>(p, s, B, st);
+    case 64: return bf ? launch_step<true, 64>(p, s, B, st) : launch_step<false, 64>(p, s, B, st);
+    default: return bf ? launch_step<true, 128>(p, s, B, st) : launch_step<false, 128>(p, s, B, st);
+  }
 }

@@ -10,18 +10,25 @@
 //   5. a = swiglu(rmsnorm(z) Wg^T)                                                   fox_step_product, rmsnorm -> swiglu
 //   6. y = z + a Wd^T                                                                fox_step_product, plain -> + z
 //
-// Bound by reading the weights once (47 MB a layer at hidden 1536: 7 us).  A CTA takes 8 rows of W; its 8 warps split K
-// in interleaved blocks of 32 columns, so that a row is read in 512-byte runs, and join their sums in shared memory.
+// Steps 2 and 3 are one kernel (fox_step_attn, fox_decode.cu) where a cluster can merge the keys' ranges.
+//
+// Bound by latency: a layer of hidden 1536 reads 61 MB of weights (9 us) through five kernels that wait for one another.  A CTA
+// takes 8 rows of W; its 8 warps split K in interleaved blocks of 32 columns and join their sums in shared memory.
 // The products are mma.sync m16n8k16 with the sequences (padded to 16) as A and the 8 weight rows as B: the matrix
 // units cost nothing here, and 2 x 16 fused multiply-adds per weight on the CUDA cores would bound the kernel above 4
 // sequences; tcgen05's 128-row tiles would be idle for all but a sixteenth.  The order of K inside a block of 32 is free,
-// so lane (g, t) holds the 16 bytes at columns 8t .. 8t+7 of row g, one load, and feeds them to two instructions.
+// so lane (g, t) holds the 16 bytes at columns 8t .. 8t+7 of row g and feeds them to two instructions.
 //
-// Every kernel is launched with programmatic stream serialization.  The products behind the first request their first
-// weights before they wait for the kernel in front, which does not write them, so that the load latency and the launch
-// hide behind it.  Each lets the next one start only after its own wait: a kernel's early reads then come after
-// everything in front of its predecessor has ended.  The first product follows a kernel of someone else's, which may
-// have written the weights, and requests them after the wait.
+// The weights' rows come by bulk copies into shared memory (kSmem).  Through registers, as large batches still take them,
+// a CTA held 64 to 128 registers a thread and the 512 and 777 CTAs of the gate and first products ran in two waves, the
+// second of which began its loads where the first ended: 40 us a layer of hidden 1536 with 2000 keys, 33 now.
+//
+// Every kernel is launched with programmatic stream serialization.  The products behind the first request their weights
+// before they wait for the kernel in front, which does not write them, so that the load latency and the launch hide behind
+// it; the gate product's CTAs leave no shared memory for the next one's, so they ask for its weights in L2.  Each lets the next
+// one start only after its own wait: a kernel's early reads then come after everything in front of its predecessor has
+// ended.  The first product follows a kernel of someone else's, which may have written the weights, and copies them after
+// the wait; what it asks for before is only brought into L2, where a later write still finds it.
 #include "fox_common.cuh"
 #include "fox_host.h"
 
@@ -30,6 +37,13 @@ namespace fox {
 constexpr int kStepThreads = 256, kStepWarps = 8;
 constexpr int kStepAhead = 8;    // blocks of 32 columns a warp has in flight
 constexpr int kStepMats = 7;
+constexpr uint32_t kStepChunk = 4096;         // bytes of one request for what a later product reads
+constexpr int kStepEarly = 296;               // CTAs that request the first product's weights
+// Input and weights of a CTA that may lie in shared memory together; more goes through registers.  (16 sequences of 1536 channels:
+// the gate product would need 99 KB, and a layer takes 126 us so, 114 through registers; 2 sequences' down product, 83 KB: 59
+// and 61 us a layer.)
+constexpr size_t kStepSmem = 88 * 1024;
+constexpr int kStepWaitSite = 91;
 
 enum StepInput { kInRms = 0, kInGated = 1, kInPlain = 2 };
 enum StepOutput { kOutFp32 = 0, kOutAdd16 = 1, kOutSwiglu = 2, kOutAdd32 = 3 };
@@ -49,6 +63,9 @@ struct StepParams {
   int64_t ldo;
   const void* res;                // kOutAdd16: (B, ldo) 16-bit; kOutAdd32: (B, ldo) fp32
   int half;                       // kOutSwiglu: rows of each half
+  const char* ahead;              // what a later product reads (16-byte aligned), or nullptr
+  uint32_t ahead_bytes;           // (a multiple of 16)
+  int* status;                    // where a wait that runs out is recorded; nullptr: weights through registers
 };
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -106,7 +123,10 @@ __device__ __forceinline__ void load_x8(const StepParams& p, int b, int c, float
   }
 }
 
-template <bool kBf16, int kIn, int kOut>
+// bytes between two rows of weights in shared memory: 64 modulo 128, so that eight rows' pieces of 64 bytes meet no bank twice
+__host__ __device__ __forceinline__ uint32_t step_row_bytes(int K) { return K * 2 + (K % 64 ? 0 : 64); }
+
+template <bool kBf16, int kIn, int kOut, bool kSmem>
 __global__ void __launch_bounds__(kStepThreads)
 fox_step_product_kernel(const StepParams p) {
   constexpr int NT = kOut == kOutSwiglu ? 2 : 1;   // 8-row tiles of a CTA
@@ -125,7 +145,27 @@ fox_step_product_kernel(const StepParams p) {
   for (int i = 0; i < NT; ++i)
     wp[i] = p.w[mat] + static_cast<int64_t>(min(row0 + g, p.rows[mat] - 1) + i * p.half) * p.K + t * 8;
 
-  uint4 wr[NT][kStepAhead];
+  const uint32_t w_row = step_row_bytes(p.K);
+  uint8_t* s_w = reinterpret_cast<uint8_t*>(s_x + p.B * stride);   // kSmem: (NT * 8 rows)
+  __shared__ uint64_t bar_w;
+  __shared__ int abort_flag;
+  if constexpr (kSmem) {
+    if (tid == 0) {
+      abort_flag = 0;
+      mbar_init(&bar_w, 1);
+      mbar_fence_init();
+      mbar_expect_tx(&bar_w, NT * 8 * p.K * 2);
+    }
+    __syncwarp();
+  }
+  auto copy = [&] {   // a lane of the first warp asks for a row
+    if (warp == 0 && lane < NT * 8) {
+      const int i = lane >> 3;
+      const uint16_t* src = p.w[mat] + static_cast<int64_t>(min(row0 + (lane & 7), p.rows[mat] - 1) + i * p.half) * p.K;
+      bulk_load(s_w + lane * w_row, src, p.K * 2, &bar_w);
+    }
+  };
+  uint4 wr[NT][kSmem ? 1 : kStepAhead];
   auto fetch = [&](int kb0) {   // blocks kb0 + 8 j + warp
 #pragma unroll
     for (int j = 0; j < kStepAhead; ++j) {
@@ -137,26 +177,52 @@ fox_step_product_kernel(const StepParams p) {
       }
     }
   };
-  if constexpr (kIn != kInRms || kOut != kOutFp32) fetch(0);
+  constexpr bool kFirst = kIn == kInRms && kOut == kOutFp32;
+  if constexpr (!kFirst) {
+    if constexpr (kSmem) copy();
+    else fetch(0);
+  } else {
+    // (a request into L2 may come before the weights are written: it is the copy that has to come after)
+    const int tile = static_cast<int>(blockIdx.x) + tid * kStepEarly, tiles = static_cast<int>(gridDim.x);
+    if (static_cast<int>(blockIdx.x) < kStepEarly && tile < tiles) {
+      int m = 0;
+      while (m + 1 < p.n_mats && tile >= p.tile0[m + 1]) ++m;
+      const int row = (tile - p.tile0[m]) * 8;
+      l2_request(p.w[m] + static_cast<int64_t>(row) * p.K, static_cast<uint32_t>(min(8, p.rows[m] - row)) * p.K * 2);
+    }
+  }
+  if (p.ahead) {
+    const uint32_t step = kStepThreads * gridDim.x * kStepChunk;
+    for (uint32_t o = (tid * gridDim.x + blockIdx.x) * kStepChunk; o < p.ahead_bytes; o += step)
+      l2_request(p.ahead + o, min(kStepChunk, p.ahead_bytes - o));
+  }
+  // one chunk of a row per lane at most: its norm weights come before the wait, its input stays in registers
+  int per = 8;   // warps that share a row
+  if constexpr (kIn == kInRms)
+    while (per > 1 && per * p.B > 8) per >>= 1;
+  const bool once = kSmem && kIn == kInRms && chunks <= per * 32;
+  float nw[8];
+  if (!kFirst && once && (warp % per) * 32 + lane < chunks) load_w8(p.norm_w, p.w_dtype, (warp % per) * 32 + lane, nw);
   pdl_wait();
   pdl_launch();
-  if constexpr (kIn == kInRms && kOut == kOutFp32) fetch(0);
+  if constexpr (kFirst) {
+    if constexpr (kSmem) copy();
+    else fetch(0);
+    if (once && (warp % per) * 32 + lane < chunks) load_w8(p.norm_w, p.w_dtype, (warp % per) * 32 + lane, nw);
+  }
 
   // ---- the input, once per CTA ----
   if constexpr (kIn == kInRms) {
     // `per` warps share a row; each row's sum of squares goes through shared memory
-    int per = 8;
-    while (per > 1 && per * p.B > 8) per >>= 1;
     const int rows_at_once = 8 / per, part = warp % per;
     for (int b0 = 0; b0 < p.B; b0 += rows_at_once) {
       const int b = b0 + warp / per;
-      float ss = 0.f;
+      float ss = 0.f, x0[8];
       if (b < p.B) {
         for (int c = part * 32 + lane; c < chunks; c += per * 32) {
-          float f[8];
-          load_x8<kBf16>(p, b, c, f);
+          load_x8<kBf16>(p, b, c, x0);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+          for (int j = 0; j < 8; ++j) ss = fmaf(x0[j], x0[j], ss);
         }
       }
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -166,7 +232,14 @@ fox_step_product_kernel(const StepParams p) {
       ss = 0.f;
       for (int i = 0; i < per; ++i) ss += s_ss[warp - part + i];
       const float r = 1.f / sqrtf(ss / static_cast<float>(p.K) + p.eps);
-      if (b < p.B) {
+      if (b < p.B && once) {
+        const int c = part * 32 + lane;
+        if (c < chunks) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x0[j] = x0[j] * r * nw[j];
+          s_x[b * stride + c] = pack8s<kBf16>(x0);
+        }
+      } else if (b < p.B) {
         for (int c = part * 32 + lane; c < chunks; c += per * 32) {
           float f[8], w[8];
           load_x8<kBf16>(p, b, c, f);
@@ -211,22 +284,39 @@ fox_step_product_kernel(const StepParams p) {
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
   const bool lo = g < p.B, hi = g + 8 < p.B;
   const uint4* xl = s_x + g * stride + t;
-  for (int kb0 = 0; kb0 < nkb; kb0 += kStepAhead * kStepWarps) {
+  if constexpr (kSmem) {
+    mbar_wait(&bar_w, 0, &abort_flag, p.status, kStepWaitSite);   // (one that runs out is recorded; what follows is then discarded)
+#pragma unroll 4
+    for (int kb = warp; kb < nkb; kb += kStepWarps) {
+      uint4 a = make_uint4(0, 0, 0, 0), a8 = a;
+      if (lo) a = xl[kb * 4];
+      if (hi) a8 = xl[8 * stride + kb * 4];
 #pragma unroll
-    for (int j = 0; j < kStepAhead; ++j) {
-      const int kb = kb0 + j * kStepWarps + warp;
-      if (kb < nkb) {
-        uint4 a = make_uint4(0, 0, 0, 0), a8 = a;
-        if (lo) a = xl[kb * 4];
-        if (hi) a8 = xl[8 * stride + kb * 4];
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          step_mma<kBf16>(acc[i], a.x, a8.x, a.y, a8.y, wr[i][j].x, wr[i][j].y);
-          step_mma<kBf16>(acc[i], a.z, a8.z, a.w, a8.w, wr[i][j].z, wr[i][j].w);
-        }
+      for (int i = 0; i < NT; ++i) {
+        const uint4 w = *reinterpret_cast<const uint4*>(s_w + (i * 8 + g) * w_row + kb * 64 + t * 16);
+        step_mma<kBf16>(acc[i], a.x, a8.x, a.y, a8.y, w.x, w.y);
+        step_mma<kBf16>(acc[i], a.z, a8.z, a.w, a8.w, w.z, w.w);
       }
     }
-    if (kb0 + kStepAhead * kStepWarps < nkb) fetch(kb0 + kStepAhead * kStepWarps);
+  }
+  if constexpr (!kSmem) {
+    for (int kb0 = 0; kb0 < nkb; kb0 += kStepAhead * kStepWarps) {
+#pragma unroll
+      for (int j = 0; j < kStepAhead; ++j) {
+        const int kb = kb0 + j * kStepWarps + warp;
+        if (kb < nkb) {
+          uint4 a = make_uint4(0, 0, 0, 0), a8 = a;
+          if (lo) a = xl[kb * 4];
+          if (hi) a8 = xl[8 * stride + kb * 4];
+#pragma unroll
+          for (int i = 0; i < NT; ++i) {
+            step_mma<kBf16>(acc[i], a.x, a8.x, a.y, a8.y, wr[i][j].x, wr[i][j].y);
+            step_mma<kBf16>(acc[i], a.z, a8.z, a.w, a8.w, wr[i][j].z, wr[i][j].w);
+          }
+        }
+      }
+      if (kb0 + kStepAhead * kStepWarps < nkb) fetch(kb0 + kStepAhead * kStepWarps);
+    }
   }
   // c0, c1: sequence g, weight rows 2t, 2t+1; c2, c3: sequence g + 8
 #pragma unroll
@@ -322,6 +412,7 @@ __global__ void __launch_bounds__(128) fox_step_mix_kernel(const StepMixParams p
   }
   if (p.mask && h == 0) {
     long long n = 0;
+#pragma unroll 8
     for (int64_t i = d; i <= p.pos; i += blockDim.x) n += p.mask[b * (p.pos + 1) + i];
     for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
     if (lane == 0) s_n[warp] = n;
@@ -365,11 +456,9 @@ static cudaLaunchConfig_t pdl_config(dim3 grid, int threads, size_t smem, cudaSt
   return cfg;
 }
 
-template <bool kBf16, int kIn, int kOut>
-static int launch_product(int device, cudaStream_t st, const StepParams& p) {
-  auto kern = fox_step_product_kernel<kBf16, kIn, kOut>;
-  const size_t smem = static_cast<size_t>(p.B) * ((p.K / 8 + 7) / 8 * 8 + 4) * 16;
-  if (smem > 200 * 1024) return FOX_ERR_TOO_LARGE;
+template <bool kBf16, int kIn, int kOut, bool kSmem>
+static int launch_product(int device, cudaStream_t st, const StepParams& p, size_t smem) {
+  auto kern = fox_step_product_kernel<kBf16, kIn, kOut, kSmem>;
   static bool configured[64] = {};
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;
   if (smem > 32 * 1024 && !configured[device]) {
@@ -380,15 +469,23 @@ static int launch_product(int device, cudaStream_t st, const StepParams& p) {
   const cudaLaunchConfig_t cfg = pdl_config(dim3((unsigned)p.tile0[p.n_mats]), kStepThreads, smem, st, &attr);
   return cudaLaunchKernelEx(&cfg, kern, p) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
+template <bool kBf16, int kIn, int kOut>
+static int choose_product(int device, cudaStream_t st, const StepParams& p) {
+  const size_t x = static_cast<size_t>(p.B) * ((p.K / 8 + 7) / 8 * 8 + 4) * 16;
+  const size_t w = static_cast<size_t>(kOut == kOutSwiglu ? 16 : 8) * step_row_bytes(p.K);
+  if (x > 200 * 1024) return FOX_ERR_TOO_LARGE;
+  return p.status && x + w <= kStepSmem ? launch_product<kBf16, kIn, kOut, true>(device, st, p, x + w)
+                                        : launch_product<kBf16, kIn, kOut, false>(device, st, p, x);
+}
 
 }  // namespace fox
 
 using namespace fox;
 
-extern "C" int fox_step_product(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K,
-                                const void* x, int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D,
-                                const float* gate, int64_t gate_ld, int64_t n_mats, const void* const* mats,
-                                const int64_t* mat_rows, const void* residual, void* out, int64_t ldo) {
+static int step_product(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K, const void* x, int x_fp32,
+                        const void* norm_w, int norm_w_dtype, float eps, int64_t D, const float* gate, int64_t gate_ld, int64_t n_mats,
+                        const void* const* mats, const int64_t* mat_rows, const void* residual, void* out, int64_t ldo,
+                        const void* ahead, int64_t ahead_bytes, int32_t* status) {
   if (!x || !out || !mats || n_mats <= 0 || n_mats > kStepMats || B <= 0 || B > 16 || K <= 0 || ldo <= 0) return FOX_ERR_BAD_ARG;
   if (K % 32) return FOX_ERR_HEAD_DIM;
   if (dtype != FOX_DTYPE_BF16 && dtype != FOX_DTYPE_FP16) return FOX_ERR_BAD_ARG;
@@ -413,19 +510,41 @@ extern "C" int fox_step_product(int device, void* stream, int dtype, int input, 
   }
   p.tile0[n_mats] = tile;
   if (align % 16) return FOX_ERR_ALIGNMENT;
+  if (ahead && (reinterpret_cast<uintptr_t>(ahead) % 16 || ahead_bytes < 0 || ahead_bytes % 16)) return FOX_ERR_ALIGNMENT;
+  p.ahead = (const char*)ahead;
+  p.ahead_bytes = (uint32_t)(ahead_bytes < (1LL << 30) ? ahead_bytes : 1LL << 30);   // (counted in 32 bits)
+  p.status = status;
   p.n_mats = (int)n_mats; p.B = (int)B; p.K = (int)K; p.D = (int)D;
   p.x = x; p.x_fp32 = x_fp32 != 0; p.norm_w = norm_w; p.w_dtype = norm_w_dtype; p.eps = eps;
   p.gate = gate; p.gate_ld = gate_ld; p.res = residual; p.out = out; p.ldo = ldo;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == FOX_DTYPE_BF16;
-#define FOX_STEP(I, O) if (input == I && output == O) return bf ? launch_product<true, I, O>(device, st, p) : launch_product<false, I, O>(device, st, p)
+#define FOX_STEP(I, O) if (input == I && output == O) return bf ? choose_product<true, I, O>(device, st, p) : choose_product<false, I, O>(device, st, p)
   FOX_STEP(kInRms, kOutFp32);
   FOX_STEP(kInGated, kOutAdd16);
   FOX_STEP(kInRms, kOutSwiglu);
   FOX_STEP(kInPlain, kOutAdd32);
 #undef FOX_STEP
   return FOX_ERR_BAD_ARG;
+}
+
+extern "C" int fox_step_product_ahead(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K,
+                                      const void* x, int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D,
+                                      const float* gate, int64_t gate_ld, int64_t n_mats, const void* const* mats,
+                                      const int64_t* mat_rows, const void* residual, void* out, int64_t ldo, const void* ahead,
+                                      int64_t ahead_bytes, int32_t* status) {
+  if (!status) return FOX_ERR_BAD_ARG;
+  return step_product(device, stream, dtype, input, output, B, K, x, x_fp32, norm_w, norm_w_dtype, eps, D, gate, gate_ld, n_mats, mats,
+                      mat_rows, residual, out, ldo, ahead, ahead_bytes, status);
+}
+
+extern "C" int fox_step_product(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K,
+                                const void* x, int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D,
+                                const float* gate, int64_t gate_ld, int64_t n_mats, const void* const* mats,
+                                const int64_t* mat_rows, const void* residual, void* out, int64_t ldo) {
+  return step_product(device, stream, dtype, input, output, B, K, x, x_fp32, norm_w, norm_w_dtype, eps, D, gate, gate_ld, n_mats, mats,
+                      mat_rows, residual, out, ldo, nullptr, 0, nullptr);
 }
 
 extern "C" int fox_step_mix(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t D, const float* y, int64_t ld,

@@ -713,6 +713,9 @@ Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheL
   for (const Tensor* t : {&c.k, &c.v, &c.g, &c.k_state, &c.v_state}) t->unsafeGetTensorImpl()->bump_version();
   const int64_t n = x.size(0), C = b.C, H = b.H, D = b.D, N = c.length + 1, cap = c.k.size(2);
   const AttnShape as{n, H, 1, N, D};
+  uintptr_t bits = 0;   // (fox_step_attn takes 16-byte pieces of states and cache; the two kernels take any state)
+  for (const Tensor* t : {&c.k, &c.v, &c.k_state, &c.v_state}) bits |= reinterpret_cast<uintptr_t>(t->data_ptr());
+  const int64_t splits = bits % 16 ? 0 : fox_step_attn_splits(n, H, N);
   const int64_t ld = (4 * C + 3 * H + 3) / 4 * 4;
   Tensor memory;
   float *y, *z, *L, *work;
@@ -723,7 +726,7 @@ Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheL
     y = m.take<float>(n * ld);
     z = m.take<float>(n * C);
     L = m.take<float>(n * H);
-    work = m.take<float>(attn_decode_floats(as));
+    work = m.take<float>(splits > 0 ? 0 : attn_decode_floats(as));
     q = m.take<uint16_t>(n * C);
     o = m.take<uint16_t>(n * C);
     act = m.take<uint16_t>(n * b.inter);
@@ -732,6 +735,7 @@ Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheL
     memory = at::empty({static_cast<int64_t>(m.used)}, x.options().dtype(at::kByte));
     base = static_cast<char*>(memory.data_ptr());
   }
+  int32_t* status = status_words(dev);
   auto dt = [&](B::Param p) { return dtype_code(b.p[p].scalar_type()); };
   auto ptr = [&](B::Param p) { return b.p[p].const_data_ptr(); };
 
@@ -743,48 +747,59 @@ Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheL
     rows[i] = b.p[first[i]].size(0);
   }
   launch("fox_step_product", st, [&] {
-    return fox_step_product(dev, st, code, 0, 0, n, C, x.const_data_ptr(), 0, ptr(B::kAttnNorm), dt(B::kAttnNorm), b.attn_eps, 0, nullptr,
-                            0, 7, mats, rows, nullptr, y, ld);
+    return fox_step_product_ahead(dev, st, code, 0, 0, n, C, x.const_data_ptr(), 0, ptr(B::kAttnNorm), dt(B::kAttnNorm), b.attn_eps, 0,
+                                  nullptr, 0, 7, mats, rows, nullptr, y, ld, nullptr, 0, status);
   });
   const bool bias = b.p[B::kFBias].defined();
-  launch("fox_step_mix", st, [&] {
-    return fox_step_mix(dev, st, code, n, H, D, y, ld, ptr(B::kQNorm), dt(B::kQNorm), ptr(B::kKNorm), dt(B::kKNorm), b.qk_eps,
-                        bias ? ptr(B::kFBias) : nullptr, bias ? dt(B::kFBias) : 0,
-                        mask64.defined() ? mask64.const_data_ptr<int64_t>() : nullptr, seq, c.k_state.data_ptr(), c.v_state.data_ptr(), q,
-                        c.k.data_ptr(), c.v.data_ptr(), c.g.mutable_data_ptr<float>(), cap, c.length);
-  });
-  AttnCall a;
-  a.device = dev;
-  a.st = st;
-  a.code = code;
-  a.s = as;
-  a.q = fox_tensor4{q, C, D, D};
-  a.o = fox_tensor4{o, C, D, D};
-  a.k = fox_tensor4{c.k.data_ptr(), H * cap * D, cap * D, D};
-  a.v = fox_tensor4{c.v.data_ptr(), H * cap * D, cap * D, D};
-  a.sm_scale = static_cast<float>(1. / std::sqrt(static_cast<double>(D)));
-  a.seq_start = mask64.defined() ? seq : nullptr;
-  a.gate = c.g.data_ptr();
-  a.gate_st[0] = H * cap;
-  a.gate_st[1] = cap;
-  a.gate_st[2] = 1;
-  a.L = L;
-  attn_decode_launch(a, false, work, true);
+  const int64_t* mask_p = mask64.defined() ? mask64.const_data_ptr<int64_t>() : nullptr;
+  const float sm_scale = static_cast<float>(1. / std::sqrt(static_cast<double>(D)));
+  if (splits > 0) {
+    launch("fox_step_attn", st, [&] {
+      return fox_step_attn(dev, st, code, n, H, D, y, ld, ptr(B::kQNorm), dt(B::kQNorm), ptr(B::kKNorm), dt(B::kKNorm), b.qk_eps,
+                           bias ? ptr(B::kFBias) : nullptr, bias ? dt(B::kFBias) : 0, mask_p, c.k_state.data_ptr(), c.v_state.data_ptr(),
+                           c.k.data_ptr(), c.v.data_ptr(), c.g.mutable_data_ptr<float>(), cap, c.length, sm_scale, o, splits);
+    });
+  } else {
+    launch("fox_step_mix", st, [&] {
+      return fox_step_mix(dev, st, code, n, H, D, y, ld, ptr(B::kQNorm), dt(B::kQNorm), ptr(B::kKNorm), dt(B::kKNorm), b.qk_eps,
+                          bias ? ptr(B::kFBias) : nullptr, bias ? dt(B::kFBias) : 0,
+                          mask_p, seq, c.k_state.data_ptr(), c.v_state.data_ptr(), q,
+                          c.k.data_ptr(), c.v.data_ptr(), c.g.mutable_data_ptr<float>(), cap, c.length);
+    });
+    AttnCall a;
+    a.device = dev;
+    a.st = st;
+    a.code = code;
+    a.s = as;
+    a.q = fox_tensor4{q, C, D, D};
+    a.o = fox_tensor4{o, C, D, D};
+    a.k = fox_tensor4{c.k.data_ptr(), H * cap * D, cap * D, D};
+    a.v = fox_tensor4{c.v.data_ptr(), H * cap * D, cap * D, D};
+    a.sm_scale = sm_scale;
+    a.seq_start = mask64.defined() ? seq : nullptr;
+    a.gate = c.g.data_ptr();
+    a.gate_st[0] = H * cap;
+    a.gate_st[1] = cap;
+    a.gate_st[2] = 1;
+    a.L = L;
+    attn_decode_launch(a, false, work, true);
+  }
   const void* m1[1] = {ptr(B::kO)};
   const int64_t r1[1] = {C};
   launch("fox_step_product", st, [&] {
-    return fox_step_product(dev, st, code, 1, 1, n, C, o, 0, ptr(B::kONorm), dt(B::kONorm), b.o_eps, D, y + 3 * C, ld, 1, m1, r1,
-                            x.const_data_ptr(), z, C);
+    return fox_step_product_ahead(dev, st, code, 1, 1, n, C, o, 0, ptr(B::kONorm), dt(B::kONorm), b.o_eps, D, y + 3 * C, ld, 1, m1, r1,
+                                  x.const_data_ptr(), z, C, nullptr, 0, status);
   });
   const void* m2[1] = {ptr(B::kGate)};
   const int64_t r2[1] = {2 * b.inter};
-  launch("fox_step_product", st, [&] {
-    return fox_step_product(dev, st, code, 0, 2, n, C, z, 1, ptr(B::kMlpNorm), dt(B::kMlpNorm), b.mlp_eps, 0, nullptr, 0, 1, m2, r2, nullptr,
-                            act, b.inter);
-  });
   const void* m3[1] = {ptr(B::kDown)};
   launch("fox_step_product", st, [&] {
-    return fox_step_product(dev, st, code, 2, 3, n, b.inter, act, 0, nullptr, 0, 0.f, 0, nullptr, 0, 1, m3, r1, z, out.mutable_data_ptr(), C);
+    return fox_step_product_ahead(dev, st, code, 0, 2, n, C, z, 1, ptr(B::kMlpNorm), dt(B::kMlpNorm), b.mlp_eps, 0, nullptr, 0, 1, m2, r2,
+                                  nullptr, act, b.inter, m3[0], C * b.inter * 2, status);
+  });
+  launch("fox_step_product", st, [&] {
+    return fox_step_product_ahead(dev, st, code, 2, 3, n, b.inter, act, 0, nullptr, 0, 0.f, 0, nullptr, 0, 1, m3, r1, z,
+                                  out.mutable_data_ptr(), C, nullptr, 0, status);
   });
   return out;
 }

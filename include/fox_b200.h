@@ -290,6 +290,13 @@ int fox_step_product(int device, void* stream, int dtype, int input, int output,
                      int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D, const float* gate,
                      int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
                      const void* residual, void* out, int64_t ldo);
+/* The same with the weights through shared memory where they fit; while it waits for its input it asks for an array that a
+ * later kernel reads (16-byte aligned, a multiple of 16 bytes, or NULL) to be brought into L2.  status: as fox_attn_fwd. */
+int fox_step_product_ahead(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K, const void* x,
+                           int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D, const float* gate,
+                           int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
+                           const void* residual, void* out, int64_t ldo, const void* ahead, int64_t ahead_bytes,
+                           int32_t* status);
 /* y (B,ld) fp32 as fox_mix_fwd's rows: token shift with the states k_state, v_state (B,C) 16-bit, which are replaced by
  * this token's projections, norms of q and k, and row pos of the caches k, v (B,H,capacity,D), log gates (B,H,capacity);
  * mask (B,pos+1) int64 or NULL: seq_start (B) receives pos + 1 - its sum. */
@@ -297,6 +304,15 @@ int fox_step_mix(int device, void* stream, int dtype, int64_t B, int64_t H, int6
                  const void* wq, int wq_dtype, const void* wk, int wk_dtype, float eps, const void* bias, int bias_dtype,
                  const int64_t* mask, int64_t* seq_start, void* k_state, void* v_state, void* q, void* k_cache,
                  void* v_cache, float* g_cache, int64_t capacity, int64_t pos);
+
+/* fox_step_mix and the attention behind it in one kernel: arguments of the first, o (B,H,D) 16-bit contiguous, the keys of a
+ * (b,h) in `splits` (1 to 8) ranges that a cluster merges.  fox_step_attn_splits: how many, or 0 where the two calls are
+ * the better way. */
+int fox_step_attn(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t D, const float* y, int64_t ld,
+                  const void* wq, int wq_dtype, const void* wk, int wk_dtype, float eps, const void* bias, int bias_dtype,
+                  const int64_t* mask, void* k_state, void* v_state, void* k_cache, void* v_cache, float* g_cache,
+                  int64_t capacity, int64_t pos, float sm_scale, void* o, int64_t splits);
+int64_t fox_step_attn_splits(int64_t B, int64_t H, int64_t N);
 
 /* Row-wise RMSNorm with optional residual add, forward: z = x + residual (fp32; residual may be
  * NULL), residual_out = z rounded to the input dtype (may be NULL), rstd = (mean z^2 + eps)^-1/2,

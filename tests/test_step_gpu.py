@@ -201,3 +201,45 @@ def test_block_under_checkpointing(reentrant):
     assert torch.equal(res[0][0], res[1][0])
     for a, b in zip(*res):      # (sums by fp32 atomics in the attention: an ulp of the result's type here and there)
         assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
+
+
+@pytest.mark.parametrize("B,C,H,I,N", [(1, 512, 8, 1408, 2001), (3, 256, 2, 512, 1030), (1, 256, 4, 512, 6400), (16, 1536, 24, 4096, 40),
+                                       (16, 512, 32, 512, 70), (2, 768, 48, 544, 129)])
+@pytest.mark.parametrize("case", ["plain", "padded", "nothing valid", "states off 16 bytes"])
+def test_token_through_every_route(B, C, H, I, N, case):
+    """One token by each of the step's routes: keys in 1 to 8 ranges merged by a cluster, in more or in more CTAs than a wave by
+    the separate kernels, which take states that do not start on 16 bytes too; weights through shared memory and through
+    registers; a sequence whose every key is padding.  Against the modules, with the tolerance of the test above (fp16)."""
+    torch.manual_seed(C + N)
+    blk = fox.FoxProBlock(C, H, I, fgate_bias=2.0).cuda().to(torch.float16)
+    x = torch.randn(B, 1, C, device="cuda").half()
+    k, v = torch.randn(2, B, H, N, C // H, device="cuda").half()
+    g = torch.nn.functional.logsigmoid(torch.randn(B, H, N, device="cuda") + 3)
+    mask = None
+    if case in ("padded", "nothing valid"):
+        mask = torch.ones(B, N + 1, dtype=torch.long, device="cuda")
+        mask[0, :N // 3] = 0
+        if case == "nothing valid":
+            mask[B - 1] = 0
+    res = []
+    for native in (True, False):
+        cache = fox.FgateCache(granule=128)
+        st = blk.attn.init_shift_state(B)
+        if case == "states off 16 bytes":
+            st = {n: torch.zeros(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view_as(t) for n, t in st.items()}
+        for i, t in enumerate(st.values()):
+            t.copy_(torch.linspace(-1 + i, 1, t.numel(), device="cuda").view_as(t))
+        cache.update_shift_cache(st["key_shift"], st["value_shift"], 0)
+        cache.update(k, v, g, 0)
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        with torch.no_grad():
+            out = blk(x, mask, cache, 0)
+        if hook is not None:
+            hook.remove()
+        res.append([out] + [t.clone() for t in cache[0]] + [st["key_shift"].clone(), st["value_shift"].clone()])
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for a, b in zip(*res):
+        a, b = a.float(), b.float()
+        assert (a - b).abs().max() <= 2 ** -9 * (b.abs().max() + 1)
+        assert (a - b).norm() <= 2 ** -9 * b.norm()
