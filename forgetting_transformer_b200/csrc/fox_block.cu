@@ -17,20 +17,20 @@
 
 namespace fox {
 
+// eight channels as four pairs, for packed two-wide fp32 arithmetic
 template <bool kBf16>
-__device__ __forceinline__ void blk_unpack(const uint4& v, float* f) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 t = unpack2<kBf16>(w[j]);
-    f[2 * j] = t.x;
-    f[2 * j + 1] = t.y;
-  }
+__device__ __forceinline__ void blk_unpack2(const uint4& v, float2* f) {
+  f[0] = unpack2<kBf16>(v.x);
+  f[1] = unpack2<kBf16>(v.y);
+  f[2] = unpack2<kBf16>(v.z);
+  f[3] = unpack2<kBf16>(v.w);
 }
 template <bool kBf16>
-__device__ __forceinline__ uint4 blk_pack(const float* f) {
-  return make_uint4(pack2<kBf16>(f[0], f[1]), pack2<kBf16>(f[2], f[3]), pack2<kBf16>(f[4], f[5]), pack2<kBf16>(f[6], f[7]));
+__device__ __forceinline__ uint4 blk_pack2(const float2* f) {
+  return make_uint4(pack2<kBf16>(f[0].x, f[0].y), pack2<kBf16>(f[1].x, f[1].y), pack2<kBf16>(f[2].x, f[2].y), pack2<kBf16>(f[3].x, f[3].y));
 }
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 neg2(float2 x) { return make_float2(-x.x, -x.y); }
 template <bool kBf16>
 __device__ __forceinline__ float blk_load1(const uint16_t* p) {
   return unpack2<kBf16>(static_cast<uint32_t>(*p)).x;
@@ -42,8 +42,15 @@ __device__ __forceinline__ float2 blk_mix_weights(float logit, int lanes) {
   const int lane0 = (threadIdx.x & 31) & ~(lanes - 1);
   return make_float2(__shfl_sync(0xffffffffu, w, lane0), __shfl_sync(0xffffffffu, w, lane0 + 1));
 }
+// over the lanes of a head (kLanes of them, where that is known)
+template <int kLanes>
 __device__ __forceinline__ float head_sum(float x, int lanes) {
-  for (int o = lanes >> 1; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  if constexpr (kLanes > 0) {
+#pragma unroll
+    for (int o = kLanes >> 1; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  } else {
+    for (int o = lanes >> 1; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  }
   return x;
 }
 
@@ -73,10 +80,10 @@ __device__ __forceinline__ void mix_load(const MixParams& p, int64_t t, bool on,
 }
 
 // One CTA of 192 threads per 3 tokens' loads in flight is too little to cover the chain load - sum over a head's lanes -
-// store, so it takes one token at a time in 64 registers and has 5 CTAs per SM, where two tokens in 116 registers left 2: 16384 x 1536 bf16 96 -> 71.5 us (4.2 TB/s), 2048 x 768 7.5 ->
-// 7.3 us.  (Two tokens in 80 registers: 67 and 8.1 us; one in 48 registers: 91 and 9.5 us; 4 channels a thread, which doubles
+// store, so it takes one token at a time in 64 registers and has 5 CTAs per SM, where two tokens in 116 registers left 2: 16384 x 1536 bf16 96 -> 71.5 us, with
+// packed arithmetic 67 (4.5 TB/s), 2048 x 768 7.5 -> 6.7 us.  (Two tokens in 80 registers: 67 and 8.1 us; one in 48 registers: 91 and 9.5 us; 4 channels a thread, which doubles
 // the instructions for addresses and sums: 199 and 13 us.)
-template <bool kBf16>
+template <bool kBf16, int kLanes>
 __global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixParams p) {
   if (static_cast<int>(blockIdx.x) >= p.mix_blocks) {
     __shared__ unsigned long long s_sum;
@@ -91,19 +98,19 @@ __global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixPa
     if (threadIdx.x == 0) p.seq_start[b] = p.T - static_cast<int64_t>(s_sum);
     return;
   }
-  const int lanes = p.D >> 3, C = p.H * p.D;
+  const int lanes = kLanes ? kLanes : p.D >> 3, C = p.H * p.D;
   const int h = threadIdx.x / lanes, sub = threadIdx.x % lanes;
   const bool active = h < p.H;
   const int ch = active ? h * p.D + sub * 8 : 0;
   const float inv_d = 1.f / static_cast<float>(p.D);
-  float wq[8], wk[8];
+  float2 wq[4], wk[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    wq[j] = active ? p.wq[ch + j] : 0.f;
-    wk[j] = active ? p.wk[ch + j] : 0.f;
+  for (int j = 0; j < 4; ++j) {
+    wq[j] = active ? make_float2(p.wq[ch + 2 * j], p.wq[ch + 2 * j + 1]) : both(0.f);
+    wk[j] = active ? make_float2(p.wk[ch + 2 * j], p.wk[ch + 2 * j + 1]) : both(0.f);
   }
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * p.rows, t1 = min(t0 + p.rows, p.tokens);
-  uint4 kp, vp;
+  uint4 kp, vp;                           // of the token before; zero where there is none
   int pos = static_cast<int>(t0 % p.T);   // of the token in its sequence
   mix_load(p, t0 - 1, active && pos != 0, ch, C, kp, vp);
   for (int64_t t = t0; t < t1; ++t) {
@@ -115,42 +122,42 @@ __global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixPa
       qr = *reinterpret_cast<const uint4*>(row + ch);
       mix = blk_load1<kBf16>(row + 4 * C + (1 + (sub & 1)) * p.H + h);
     }
-    const bool first = pos == 0;   // no token before it
     pos = pos + 1 == p.T ? 0 : pos + 1;
-    float q[8], k[8], v[8], kq[8], vq[8];
-    blk_unpack<kBf16>(qr, q);
-    blk_unpack<kBf16>(kr, k);
-    blk_unpack<kBf16>(vr, v);
-    blk_unpack<kBf16>(kp, kq);
-    blk_unpack<kBf16>(vp, vq);
+    float2 q[4], k[4], v[4], kq[4], vq[4];
+    blk_unpack2<kBf16>(qr, q);
+    blk_unpack2<kBf16>(kr, k);
+    blk_unpack2<kBf16>(vr, v);
+    blk_unpack2<kBf16>(kp, kq);
+    blk_unpack2<kBf16>(vp, vq);
     const float2 w = blk_mix_weights(mix, lanes);
-    const float a = w.x, c = w.y;
-    float sq = 0.f, sk = 0.f;
+    const float2 a = both(w.x), c = both(w.y), a1 = both(1.f - w.x), c1 = both(1.f - w.y);
+    float2 sq = both(0.f), sk = both(0.f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      k[j] = k[j] * (1.f - a) + (first ? 0.f : kq[j] * a);
-      v[j] = v[j] * (1.f - c) + (first ? 0.f : vq[j] * c);
-      sq = fmaf(q[j], q[j], sq);
-      sk = fmaf(k[j], k[j], sk);
+    for (int j = 0; j < 4; ++j) {
+      k[j] = __ffma2_rn(k[j], a1, __fmul2_rn(kq[j], a));
+      v[j] = __ffma2_rn(v[j], c1, __fmul2_rn(vq[j], c));
+      sq = __ffma2_rn(q[j], q[j], sq);
+      sk = __ffma2_rn(k[j], k[j], sk);
     }
-    const float rq = rsqrtf(head_sum(sq, lanes) * inv_d + p.eps), rk = rsqrtf(head_sum(sk, lanes) * inv_d + p.eps);
+    const float rq = rsqrtf(head_sum<kLanes>(sq.x + sq.y, lanes) * inv_d + p.eps),
+                rk = rsqrtf(head_sum<kLanes>(sk.x + sk.y, lanes) * inv_d + p.eps);
     if (active) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        q[j] *= rq * wq[j];
-        k[j] *= rk * wk[j];
+      for (int j = 0; j < 4; ++j) {
+        q[j] = __fmul2_rn(q[j], __fmul2_rn(both(rq), wq[j]));
+        k[j] = __fmul2_rn(k[j], __fmul2_rn(both(rk), wk[j]));
       }
       const int64_t o = t * C + ch;
-      *reinterpret_cast<uint4*>(p.q + o) = blk_pack<kBf16>(q);
-      *reinterpret_cast<uint4*>(p.k + o) = blk_pack<kBf16>(k);
-      *reinterpret_cast<uint4*>(p.v + o) = blk_pack<kBf16>(v);
+      *reinterpret_cast<uint4*>(p.q + o) = blk_pack2<kBf16>(q);
+      *reinterpret_cast<uint4*>(p.k + o) = blk_pack2<kBf16>(k);
+      *reinterpret_cast<uint4*>(p.v + o) = blk_pack2<kBf16>(v);
       if (sub == 0 && p.rstd_q) {
         p.rstd_q[t * p.H + h] = rq;
         p.rstd_k[t * p.H + h] = rk;
       }
     }
-    kp = kr;
-    vp = vr;
+    kp = pos == 0 ? make_uint4(0, 0, 0, 0) : kr;
+    vp = pos == 0 ? make_uint4(0, 0, 0, 0) : vr;
   }
 }
 
@@ -168,129 +175,179 @@ struct MixRow {
   float mix, rq, rk;
 };
 
+// A CTA's rows: pointers to its first token, the same for every thread, and 32-bit offsets from there.
+struct MixRows {
+  const uint16_t *y, *dq, *dk, *dv;
+  uint16_t* dy;
+  const int64_t* mask;
+  const float *rq, *rk;
+};
+__device__ __forceinline__ void mix_rows_kv(const MixRows& p, uint32_t i, uint32_t ld, uint32_t C, bool on, uint32_t ch, uint4& k, uint4& v) {
+  k = v = make_uint4(0, 0, 0, 0);
+  if (on && (!p.mask || p.mask[i] != 0)) {
+    k = *reinterpret_cast<const uint4*>(p.y + (i * ld + C + ch));
+    v = *reinterpret_cast<const uint4*>(p.y + (i * ld + 2 * C + ch));
+  }
+}
 template <bool kBf16>
-__device__ __forceinline__ void mix_bwd_load(const MixBwdParams& p, int64_t t, bool on, int ch, int C, int h, int sub, MixRow& r) {
+__device__ __forceinline__ void mix_rows_load(const MixRows& p, uint32_t i, uint32_t ld, uint32_t C, uint32_t H, bool on, bool before,
+                                              uint32_t ch, uint32_t h, uint32_t sub, MixRow& r) {
   r.q = r.dq = r.dk = r.dv = make_uint4(0, 0, 0, 0);
   r.mix = r.rq = r.rk = 0.f;
-  mix_load(p.f, t - 1, on && t > 0, ch, C, r.kp, r.vp);
+  mix_rows_kv(p, i - 1, ld, C, on && before, ch, r.kp, r.vp);
   if (on) {
-    const uint16_t* row = p.f.y + t * p.f.ld;
-    const int64_t o = t * C + ch;
-    r.q = *reinterpret_cast<const uint4*>(row + ch);
-    r.dq = *reinterpret_cast<const uint4*>(p.dq + o);
-    r.dk = *reinterpret_cast<const uint4*>(p.dk + o);
-    r.dv = *reinterpret_cast<const uint4*>(p.dv + o);
-    r.mix = blk_load1<kBf16>(row + 4 * C + (1 + (sub & 1)) * p.f.H + h);
-    r.rq = p.f.rstd_q[t * p.f.H + h];
-    r.rk = p.f.rstd_k[t * p.f.H + h];
+    r.q = *reinterpret_cast<const uint4*>(p.y + (i * ld + ch));
+    r.dq = *reinterpret_cast<const uint4*>(p.dq + (i * C + ch));
+    r.dk = *reinterpret_cast<const uint4*>(p.dk + (i * C + ch));
+    r.dv = *reinterpret_cast<const uint4*>(p.dv + (i * C + ch));
+    r.mix = blk_load1<kBf16>(p.y + (i * ld + 4 * C + (1 + (sub & 1)) * H + h));
+    r.rq = p.rq[i * H + h];
+    r.rk = p.rk[i * H + h];
   }
 }
 
 // Tokens are walked backwards: the gradient of k[t] is (1 - a[t]) dk'[t] + a[t+1] dk'[t+1], the second term carried from
 // the token before in this order.  A CTA first forms the token after its range for that carry (1 / rows more reads).
-// The next token's rows are fetched before the current one is worked on.
-template <bool kBf16>
+// Bound by instructions and the latency of a token's chain at 12 warps per SM: what costs registers costs warps.  So a token's
+// rows are not held twice (no prefetch), the norm weights are read from shared memory, addresses are 32-bit offsets, and the
+// arithmetic is packed two wide (800 instructions a warp and token before).  16384 x 1536 bf16: 174 -> 123 us; 2048 x 768: 20.2
+// -> 14.2 us.  (112 registers for a third CTA: 130 and 15.2 us; 96: 177; prefetching the next rows into L1: 122.)
+template <bool kBf16, int kLanes>
 __global__ void __launch_bounds__(kMixThreads, 2) fox_mix_bwd_kernel(const MixBwdParams p) {
   const MixParams& f = p.f;
-  const int lanes = f.D >> 3, C = f.H * f.D;
+  const int lanes = kLanes ? kLanes : f.D >> 3, C = f.H * f.D;
   const int h = threadIdx.x / lanes, sub = threadIdx.x % lanes;
   const bool active = h < f.H;
   const int ch = active ? h * f.D + sub * 8 : 0;
   const float inv_d = 1.f / static_cast<float>(f.D);
-  float wq[8], wk[8], dwq[8], dwk[8];
+  __shared__ float4 s_wq[2 * kMixThreads], s_wk[2 * kMixThreads];   // the norm weights, a thread's own
+  float2 dwq[4], dwk[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    wq[j] = active ? f.wq[ch + j] : 0.f;
-    wk[j] = active ? f.wk[ch + j] : 0.f;
-    dwq[j] = dwk[j] = 0.f;
+  for (int i = 0; i < 2; ++i) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    s_wq[i * kMixThreads + threadIdx.x] = active ? make_float4(f.wq[ch + 4 * i], f.wq[ch + 4 * i + 1], f.wq[ch + 4 * i + 2], f.wq[ch + 4 * i + 3]) : zero;
+    s_wk[i * kMixThreads + threadIdx.x] = active ? make_float4(f.wk[ch + 4 * i], f.wk[ch + 4 * i + 1], f.wk[ch + 4 * i + 2], f.wk[ch + 4 * i + 3]) : zero;
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) dwq[j] = dwk[j] = both(0.f);
+  auto weights = [&](const float4* w, float2* o) {
+    const float4 x = w[threadIdx.x], y = w[kMixThreads + threadIdx.x];
+    o[0] = make_float2(x.x, x.y);
+    o[1] = make_float2(x.z, x.w);
+    o[2] = make_float2(y.x, y.y);
+    o[3] = make_float2(y.z, y.w);
+  };
   for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * f.rows; t0 < f.tokens; t0 += static_cast<int64_t>(gridDim.x) * f.rows) {
     const int64_t t1 = min(t0 + f.rows, f.tokens);
     const bool halo = t1 < f.tokens && t1 % f.T != 0;
     const int64_t last = halo ? t1 : t1 - 1;
-    float ck[8], cv[8];
+    int pos = static_cast<int>(last % f.T);   // of the token in its sequence
+    float2 ck[4], cv[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ck[j] = cv[j] = 0.f;
+    for (int j = 0; j < 4; ++j) ck[j] = cv[j] = both(0.f);
+    const int64_t tb = t0 > 0 ? t0 - 1 : 0;   // (the row before the range is read too)
+    const MixRows rows{f.y + tb * f.ld, p.dq + tb * C, p.dk + tb * C, p.dv + tb * C, p.dy + tb * f.ld, f.mask ? f.mask + tb : nullptr,
+                       f.rstd_q + tb * f.H, f.rstd_k + tb * f.H};
+    const uint32_t ld = static_cast<uint32_t>(f.ld), i0 = static_cast<uint32_t>(t0 - tb), i1 = static_cast<uint32_t>(t1 - tb);
     uint4 kc, vc;   // k, v of the current token
-    mix_load(f, last, active, ch, C, kc, vc);
-    MixRow nx;
-    mix_bwd_load<kBf16>(p, last, active, ch, C, h, sub, nx);
-    for (int64_t t = last; t >= t0; --t) {
-      const MixRow r = nx;
-      mix_bwd_load<kBf16>(p, t - 1, active && t > t0, ch, C, h, sub, nx);
-      const bool first = t % f.T == 0;
-      const bool own = t < t1;
-      float k[8], v[8], kq[8], vq[8], dk[8], dv[8];
-      blk_unpack<kBf16>(kc, k);
-      blk_unpack<kBf16>(vc, v);
-      blk_unpack<kBf16>(r.kp, kq);
-      blk_unpack<kBf16>(r.vp, vq);
-      blk_unpack<kBf16>(r.dk, dk);
-      blk_unpack<kBf16>(r.dv, dv);
+    uint32_t i = static_cast<uint32_t>(last - tb);
+    mix_rows_kv(rows, i, ld, C, active, ch, kc, vc);
+    for (;; --i) {
+      MixRow r;
+      mix_rows_load<kBf16>(rows, i, ld, C, f.H, active, i > 0, ch, h, sub, r);
+      const bool first = pos == 0;   // (the row before is another sequence's)
+      pos = first ? f.T - 1 : pos - 1;
+      const bool own = i < i1;
       const float2 w = blk_mix_weights(r.mix, lanes);
-      const float a = w.x, c = w.y;
-      float ks[8], wdy[8], c1 = 0.f;
+      const bool live = !rows.mask || rows.mask[i] != 0;
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      const uint32_t row = i * ld;
+      float dc1;
+      {   // v
+        const float2 c = both(w.y), c1 = both(1.f - w.y);
+        float2 v[4], vq[4], dv[4], ov[4], dc = both(0.f);
+        blk_unpack2<kBf16>(vc, v);
+        blk_unpack2<kBf16>(first ? zero : r.vp, vq);
+        blk_unpack2<kBf16>(r.dv, dv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (first) kq[j] = vq[j] = 0.f;   // (the row before is another sequence's)
-        ks[j] = (k[j] * (1.f - a) + kq[j] * a) * r.rk;   // normalised k'
-        wdy[j] = wk[j] * dk[j];
-        if (own) dwk[j] = fmaf(dk[j], ks[j], dwk[j]);
-        c1 = fmaf(ks[j], wdy[j], c1);
-      }
-      c1 = head_sum(c1, lanes) * inv_d;
-      float da = 0.f, dc = 0.f;
-      float ok[8], ov[8];
-      const bool live = !f.mask || f.mask[t] != 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float g = (wdy[j] - ks[j] * c1) * r.rk;   // dk'
-        da = fmaf(g, kq[j] - k[j], da);
-        dc = fmaf(dv[j], vq[j] - v[j], dc);
-        ok[j] = live ? fmaf(g, 1.f - a, ck[j]) : 0.f;
-        ov[j] = live ? fmaf(dv[j], 1.f - c, cv[j]) : 0.f;
-        ck[j] = first ? 0.f : a * g;
-        cv[j] = first ? 0.f : c * dv[j];
-      }
-      da = head_sum(da, lanes);
-      dc = head_sum(dc, lanes);
-      if (own) {
-        float q[8], dq[8], c2 = 0.f;
-        blk_unpack<kBf16>(r.q, q);
-        blk_unpack<kBf16>(r.dq, dq);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          q[j] *= r.rq;
-          dwq[j] = fmaf(dq[j], q[j], dwq[j]);
-          dq[j] *= wq[j];
-          c2 = fmaf(q[j], dq[j], c2);
+        for (int j = 0; j < 4; ++j) {
+          dc = __ffma2_rn(dv[j], __fadd2_rn(vq[j], neg2(v[j])), dc);
+          ov[j] = __ffma2_rn(dv[j], c1, cv[j]);
+          cv[j] = __fmul2_rn(c, dv[j]);
         }
-        c2 = head_sum(c2, lanes) * inv_d;
+        dc1 = dc.x + dc.y;
+        if (own && active) *reinterpret_cast<uint4*>(rows.dy + (row + 2 * C + ch)) = live ? blk_pack2<kBf16>(ov) : zero;
+      }
+      float da1;
+      {   // k
+        const float2 a = both(w.x), a1 = both(1.f - w.x), rk = both(r.rk);
+        float2 k[4], kq[4], dk[4], ks[4], wdy[4], s1 = both(0.f), da = both(0.f);
+        blk_unpack2<kBf16>(kc, k);
+        blk_unpack2<kBf16>(first ? zero : r.kp, kq);
+        blk_unpack2<kBf16>(r.dk, dk);
+        weights(s_wk, wdy);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          ks[j] = __fmul2_rn(__ffma2_rn(k[j], a1, __fmul2_rn(kq[j], a)), rk);   // normalised k'
+          wdy[j] = __fmul2_rn(wdy[j], dk[j]);
+          s1 = __ffma2_rn(ks[j], wdy[j], s1);
+          if (own) dwk[j] = __ffma2_rn(dk[j], ks[j], dwk[j]);
+          k[j] = __fadd2_rn(kq[j], neg2(k[j]));
+        }
+        const float2 m1 = both(-head_sum<kLanes>(s1.x + s1.y, lanes) * inv_d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 g = __fmul2_rn(__ffma2_rn(ks[j], m1, wdy[j]), rk);   // dk'
+          da = __ffma2_rn(g, k[j], da);
+          ks[j] = __ffma2_rn(g, a1, ck[j]);
+          ck[j] = __fmul2_rn(a, g);
+        }
+        da1 = da.x + da.y;
+        if (own && active) *reinterpret_cast<uint4*>(rows.dy + (row + C + ch)) = live ? blk_pack2<kBf16>(ks) : zero;
+      }
+      if (first) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ck[j] = cv[j] = both(0.f);
+      }
+      if (own) {   // q, and the mixing weights' logits
+        float2 q[4], dq[4], wq[4], s2 = both(0.f);
+        blk_unpack2<kBf16>(r.q, q);
+        blk_unpack2<kBf16>(r.dq, dq);
+        weights(s_wq, wq);
+        const float2 rq = both(r.rq);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          q[j] = __fmul2_rn(q[j], rq);
+          dwq[j] = __ffma2_rn(dq[j], q[j], dwq[j]);
+          dq[j] = __fmul2_rn(dq[j], wq[j]);
+          s2 = __ffma2_rn(q[j], dq[j], s2);
+        }
+        da1 = head_sum<kLanes>(da1, lanes);
+        dc1 = head_sum<kLanes>(dc1, lanes);
+        const float2 m2 = both(-head_sum<kLanes>(s2.x + s2.y, lanes) * inv_d);
         if (active) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) dq[j] = (dq[j] - q[j] * c2) * r.rq;
-          uint16_t* row = p.dy + t * f.ld;
-          *reinterpret_cast<uint4*>(row + ch) = blk_pack<kBf16>(dq);
-          *reinterpret_cast<uint4*>(row + C + ch) = blk_pack<kBf16>(ok);
-          *reinterpret_cast<uint4*>(row + 2 * C + ch) = blk_pack<kBf16>(ov);
+          for (int j = 0; j < 4; ++j) dq[j] = __fmul2_rn(__ffma2_rn(q[j], m2, dq[j]), rq);
+          *reinterpret_cast<uint4*>(rows.dy + (row + ch)) = blk_pack2<kBf16>(dq);
           if (sub == 0) {
-            row[4 * C + f.H + h] = static_cast<uint16_t>(pack2<kBf16>(da * a * (1.f - a), 0.f) & 0xffffu);
-            row[4 * C + 2 * f.H + h] = static_cast<uint16_t>(pack2<kBf16>(dc * c * (1.f - c), 0.f) & 0xffffu);
+            rows.dy[row + 4 * C + f.H + h] = static_cast<uint16_t>(pack2<kBf16>(da1 * w.x * (1.f - w.x), 0.f) & 0xffffu);
+            rows.dy[row + 4 * C + 2 * f.H + h] = static_cast<uint16_t>(pack2<kBf16>(dc1 * w.y * (1.f - w.y), 0.f) & 0xffffu);
           }
         }
-        if (threadIdx.x < p.pad1 - p.pad0) p.dy[t * f.ld + p.pad0 + threadIdx.x] = 0;
+        if (threadIdx.x < p.pad1 - p.pad0) rows.dy[row + p.pad0 + threadIdx.x] = 0;
       }
       kc = r.kp;
       vc = r.vp;
+      if (i == i0) break;
     }
   }
   if (active) {
-    float* o = p.dwq + static_cast<int64_t>(blockIdx.x) * C + ch;
-    *reinterpret_cast<float4*>(o) = make_float4(dwq[0], dwq[1], dwq[2], dwq[3]);
-    *reinterpret_cast<float4*>(o + 4) = make_float4(dwq[4], dwq[5], dwq[6], dwq[7]);
-    o = p.dwk + static_cast<int64_t>(blockIdx.x) * C + ch;
-    *reinterpret_cast<float4*>(o) = make_float4(dwk[0], dwk[1], dwk[2], dwk[3]);
-    *reinterpret_cast<float4*>(o + 4) = make_float4(dwk[4], dwk[5], dwk[6], dwk[7]);
+    float4* o = reinterpret_cast<float4*>(p.dwq + static_cast<int64_t>(blockIdx.x) * C + ch);
+    o[0] = make_float4(dwq[0].x, dwq[0].y, dwq[1].x, dwq[1].y);
+    o[1] = make_float4(dwq[2].x, dwq[2].y, dwq[3].x, dwq[3].y);
+    o = reinterpret_cast<float4*>(p.dwk + static_cast<int64_t>(blockIdx.x) * C + ch);
+    o[0] = make_float4(dwk[0].x, dwk[0].y, dwk[1].x, dwk[1].y);
+    o[1] = make_float4(dwk[2].x, dwk[2].y, dwk[3].x, dwk[3].y);
   }
 }
 
@@ -462,13 +519,16 @@ extern "C" int fox_mix_fwd(int device, void* stream, int dtype, int64_t B, int64
   p.seq_start = seq_start;
   p.mix_blocks = (int)((p.tokens + p.rows - 1) / p.rows);
   const unsigned grid = (unsigned)(p.mix_blocks + (seq_start ? B : 0));
-  if (dtype == FOX_DTYPE_BF16) fox_mix_fwd_kernel<true><<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
-  else fox_mix_fwd_kernel<false><<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
+  const bool bf = dtype == FOX_DTYPE_BF16;
+  auto kern = D == 64 ? (bf ? fox_mix_fwd_kernel<true, 8> : fox_mix_fwd_kernel<false, 8>)
+              : D == 128 ? (bf ? fox_mix_fwd_kernel<true, 16> : fox_mix_fwd_kernel<false, 16>)
+                         : (bf ? fox_mix_fwd_kernel<true, 0> : fox_mix_fwd_kernel<false, 0>);
+  kern<<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
   return blk_rc();
 }
 
 extern "C" int64_t fox_mix_bwd_partials(int64_t tokens) {
-  const int rows = mix_rows(tokens, 148 * 2);
+  const int rows = mix_rows(tokens, 148 * 3);
   const int64_t n = (tokens + rows - 1) / rows;
   return n < 148 * 4 ? n : 148 * 4;
 }
@@ -489,9 +549,12 @@ extern "C" int fox_mix_bwd(int device, void* stream, int dtype, int64_t B, int64
   p.pad0 = (int)(4 * H * D + 3 * H); p.pad1 = (int)ld;
   if (p.pad1 - p.pad0 > 32) return FOX_ERR_BAD_ARG;   // (one thread per pad column)
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  p.f.rows = mix_rows(p.f.tokens, 148 * 2);
-  if (dtype == FOX_DTYPE_BF16) fox_mix_bwd_kernel<true><<<(unsigned)n_partials, mix_threads(p.f), 0, (cudaStream_t)stream>>>(p);
-  else fox_mix_bwd_kernel<false><<<(unsigned)n_partials, mix_threads(p.f), 0, (cudaStream_t)stream>>>(p);
+  p.f.rows = mix_rows(p.f.tokens, 148 * 3);
+  const bool bf = dtype == FOX_DTYPE_BF16;
+  auto kern = D == 64 ? (bf ? fox_mix_bwd_kernel<true, 8> : fox_mix_bwd_kernel<false, 8>)
+              : D == 128 ? (bf ? fox_mix_bwd_kernel<true, 16> : fox_mix_bwd_kernel<false, 16>)
+                         : (bf ? fox_mix_bwd_kernel<true, 0> : fox_mix_bwd_kernel<false, 0>);
+  kern<<<(unsigned)n_partials, mix_threads(p.f), 0, (cudaStream_t)stream>>>(p);
   return blk_rc();
 }
 
