@@ -621,3 +621,25 @@ def test_weights_are_relative_to_the_maximum_of_the_nearest_128_keys(D, dtype):
     rms = ((got - ref) / ref).pow(2).mean().sqrt().item()
     once = 2.0 ** (-7 if dtype == torch.bfloat16 else -10) * (0.75 / (2 * 0.6931) / 12) ** 0.5
     assert rms < 1.2 * once, rms / once
+
+
+@pytest.mark.parametrize("M,N,bm,bn", [(1, 1, 128, 128), (128, 128, 128, 128), (129, 700, 128, 128), (5000, 5000, 32, 32),
+                                       (4096, 20000, 32, 128), (17000, 17000, 128, 128)])
+@pytest.mark.parametrize("kind", ["falling", "flat", "rising in places", "minus infinity"])
+def test_pruning_indices_by_search_and_by_scan(M, N, bm, bn, kind):
+    """fox_find_index on prefixes that never rise (searched) and on others (upstream's carried scan), more blocks than threads,
+    single blocks and ragged ends: bit-identical to the restated scans."""
+    g = torch.Generator().manual_seed(M + N)
+    gates = torch.nn.functional.logsigmoid(torch.randn(2, 3, N, generator=g) * 2)
+    if kind == "flat":
+        gates[..., N // 3:] = 0.0
+    if kind == "rising in places":
+        gates[torch.rand(2, 3, N, generator=g) < 0.3] = 2.0
+        gates[..., -1] = -1e4        # (a column that stops every row: upstream's scan would not return otherwise)
+    if kind == "minus infinity":
+        gates[1, :, N // 2] = -math.inf
+    lam = gates.cumsum(-1)
+    thr = torch.tensor([[-0.5, -10.0, -1e5], [-3.0, -1e-3, -40.0]])
+    si, ei = ops.find_index(lam.cuda(), thr.cuda(), M, bm, bn, True, True)
+    assert np.array_equal(si.cpu().numpy(), orc.find_start_index(lam.numpy(), thr.numpy(), M, N, bm, bn))
+    assert np.array_equal(ei.cpu().numpy(), orc.find_end_index(lam.numpy(), thr.numpy(), M, N, bm, bn))
