@@ -9,17 +9,23 @@
 // 16 + 16 packed ones), so S^T(i+1) is issued as soon as S^T(i) has been read and runs under phase B(i) and the
 // dV / dK products.
 //
-// One CTA = one (batch, head, 128-row KV tile), one CTA per SM; K and V resident in shared memory:
+// An item is a (batch, head, 128-row KV tile); one CTA per SM, K and V of its item resident in shared memory:
 //   warps 0-15 : four elementwise warpgroups, thread = KV row (TMEM lane) x 32 of the tile's 128 query columns
 //                phase A: p^T = 2^(s^T c + e_i - b_j), kept in registers; S^T is free once it has been read
 //                phase B: dS^T = p^T (dP^T - delta_i); P^T and dS^T -> 16 bit over its own dP^T columns;
 //                         colsum(dS) in fp32
-//   warp 16    : TMA producer (K, V once; Q, dO tiles in rings of two; stages e_i = (Lambda_i - L_i) log2e, delta_i)
+//   warp 16    : TMA producer (K, V once per item; Q, dO tiles in rings of two, which dK and dV leave through; stages e_i = (Lambda_i - L_i) log2e, delta_i)
 //   warp 17    : tcgen05.mma issuer:
 //                wait S read(i): S^T(i+1) = K Q(i+1)^T | wait dS(i): dV += P^T(i) dO(i), dK += dS^T(i) Q(i),
 //                dP^T(i+1) = V dO(i+1)^T
 // TMEM (512 columns): S^T [0,128), dP^T [128,256), dK [256,384), dV [384,512).
 // Query tiles are walked upwards from the diagonal to end_index (lines 1003-1049).
+//
+// Pruned calls leave an item about two query tiles, so that with a CTA for each the launch, the barriers and TMEM's
+// allocation, the first loads and the way out of dK and dV were most of its time.  kLoop: a CTA goes on with further items
+// (ItemQueue), whose K, V and first tiles are loaded and first products issued while this one's accumulators are read, scaled
+// and stored.  B4 T16384 H16 D128 with 97 % of the tiles pruned: 600 -> 389-398 us.  Without pruning an item has 64 tiles on
+// average and the walk costs registers in the tile loop: 7.73 ms against 7.69 with a CTA for each item.
 #include "fox_common.cuh"
 #include "fox_host.h"
 
@@ -39,6 +45,7 @@ struct KvParams {
   void* dv; int64_t dv_sb, dv_sh, dv_st;
   int* status;
   int H, M, N;
+  int tiles, items;          // KV tiles of a (b,h); of all
   float sm_scale, qk_scale;
 };
 
@@ -46,25 +53,14 @@ struct KvParams {
 __device__ long long g_kv_trace[24 * 8 * 16];
 #define KVSTAMP(role, ev, it) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0 && (it) >= 32 && (it) < 48) g_kv_trace[((role) * 8 + (ev)) * 16 + (it) - 32] = clock64(); } while (0)
 extern "C" int fox_debug_read_kv_trace(long long* host) { return cudaMemcpyFromSymbol(host, g_kv_trace, sizeof(g_kv_trace)); }
-// CTA timeline: nanosecond stamps of up to 8192 CTAs (entry, after set-up, first S^T, last tile, products done,
-// stores done, exit) and the SM they ran on
-__device__ unsigned long long g_kv_cta[8192 * 8];
-__device__ __forceinline__ unsigned long long kv_now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-#define KVCTA(ev) do { const unsigned cta_ = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z); if (cta_ < 8192) g_kv_cta[cta_ * 8 + (ev)] = kv_now_ns(); } while (0)
-extern "C" int fox_debug_read_kv_cta(unsigned long long* host) { return cudaMemcpyFromSymbol(host, g_kv_cta, sizeof(g_kv_cta)); }
 #else
 #define KVSTAMP(role, ev, it)
-#define KVCTA(ev)
 #endif
 
 enum KvWaitSite { kKvSiteQ = 71, kKvSiteDO = 72, kKvSiteQE = 73, kKvSiteDOE = 74, kKvSiteS = 75, kKvSiteDP = 76,
-                  kKvSiteP = 77, kKvSiteDS = 78, kKvSiteDone = 79, kKvSiteVec = 80, kKvSiteCol = 81, kKvSiteKV = 82, kKvSiteEpi = 83 };
+                  kKvSiteP = 77, kKvSiteDS = 78, kKvSiteDone = 79, kKvSiteVec = 80, kKvSiteCol = 81, kKvSiteKV = 82, kKvSiteEpi = 83, kKvSiteItem = 84 };
 
-template <int D, bool kBf16>
+template <int D, bool kBf16, bool kLoop>
 __global__ void __launch_bounds__(576, 1)
 fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -84,11 +80,12 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t bar_q_full[kSt], bar_q_empty[kSt], bar_do_full[kSt], bar_do_empty[kSt], bar_vec[kVec], bar_s_full,
-      bar_dp_full, bar_s_read, bar_ds_full, bar_done, bar_kv, bar_colsum, bar_epi[2];
+      bar_dp_full, bar_s_read, bar_ds_full, bar_done, bar_kv, bar_kv_free, bar_colsum, bar_epi[2], bar_epi_free[2];
   __shared__ __align__(16) float s_e[kVec][BM];
   __shared__ __align__(16) float s_delta[kVec][BM];
-  __shared__ float s_part[kWG - 1][128];
+  __shared__ float s_part[2][kWG - 1][128];
   __shared__ uint32_t tmem_slot;
+  __shared__ __align__(16) ItemQueue items;
   __shared__ int abort_flag;
 
   uint8_t* sQ = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -97,33 +94,34 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint8_t* sV = sK + kTileBytes;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    KVCTA(0);
-#ifdef FOX_KV_TRACE
-    unsigned smid_;
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid_));
-    { const unsigned cta_ = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z); if (cta_ < 8192) g_kv_cta[cta_ * 8 + 7] = smid_; }
-#endif
-  }
-  const int nb = static_cast<int>(blockIdx.x);   // (KV tile 0 sees every query row: heavy tiles first)
-  const int h = blockIdx.y, b = blockIdx.z;
   const int M = p.M, N = p.N, P = N - M;
-  const int64_t bh = static_cast<int64_t>(b) * p.H + h;
-  const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
-  const int j0 = nb * kKvBN;
 
-  // ---- query-tile range of this KV tile (upstream lines 1003-1049) ----
-  int lo = max(j0 - P, 0);
-  lo = (lo / BM) * BM;
-  int hi = M;
-  if (p.end_index) {
-    const int64_t e = p.end_index[bh * gridDim.x + nb];
-    hi = static_cast<int>(e < static_cast<int64_t>(M) ? e : static_cast<int64_t>(M));
-  }
-  if (p.seq_start && !(j0 + kKvBN >= seq0 - 1)) hi = lo;
-  const int hb_lo = lo / BM;
-  const int hb_hi = (hi + BM - 1) / BM;
-  const int n_tiles = max(hb_hi - hb_lo, 0);
+  // An item: one KV tile of one (b,h) (KV tile 0 sees every query row: heavy tiles first) with its query tiles
+  // [hb_lo, hb_lo + n) (upstream lines 1003-1049).  kLoop: a CTA goes on with others, without: it has one.
+  struct Item {
+    int b, h, j0, hb_lo, n, seq0;
+    int64_t bh;
+  };
+  auto item_of = [&](int i) {
+    Item x;
+    const int nb = i % p.tiles, u = i / p.tiles;
+    x.h = u % p.H;
+    x.b = u / p.H;
+    x.bh = u;
+    x.j0 = nb * kKvBN;
+    x.seq0 = p.seq_start ? static_cast<int>(p.seq_start[x.b]) : 0;
+    int lo = max(x.j0 - P, 0);
+    lo = (lo / BM) * BM;
+    int hi = M;
+    if (p.end_index) {
+      const int64_t e = p.end_index[static_cast<int64_t>(u) * p.tiles + nb];
+      hi = static_cast<int>(e < static_cast<int64_t>(M) ? e : static_cast<int64_t>(M));
+    }
+    if (p.seq_start && !(x.j0 + kKvBN >= x.seq0 - 1)) hi = lo;
+    x.hb_lo = lo / BM;
+    x.n = max((hi + BM - 1) / BM - x.hb_lo, 0);
+    return x;
+  };
 
   if (tid == 0) {
     abort_flag = 0;
@@ -140,9 +138,13 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     mbar_init(&bar_ds_full, 128 * kWG);
     mbar_init(&bar_done, 1);
     mbar_init(&bar_kv, 1);
-    mbar_init(&bar_colsum, 128 * (kWG - 1));
+    mbar_init(&bar_kv_free, 1);
+    mbar_init(&bar_colsum, 128 * kWG);
     mbar_init(&bar_epi[0], 256);
     mbar_init(&bar_epi[1], 256);
+    mbar_init(&bar_epi_free[0], 1);
+    mbar_init(&bar_epi_free[1], 1);
+    if constexpr (kLoop) items_init(items, 17);
     mbar_fence_init();
   }
   if (warp == kTmaWarp) {
@@ -154,97 +156,159 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tc_fence_after();
   const uint32_t tbase = tmem_slot;
   volatile int* abortp = &abort_flag;
-  if (tid == 0) KVCTA(1);
 
   if (warp == kTmaWarp) {
     // ===================== TMA producer =====================
-    if (n_tiles > 0) {
+    // Q and dO stages are taken in turn by the items' query tiles and, behind an item's last one, by its dK and dV on
+    // their way out: that tile lies in the other stage, which is free for the next item's first tile as soon as the
+    // products have read it.
+    if (elect_one()) {
+      tma_prefetch_desc(&tmQ);
+      tma_prefetch_desc(&tmDO);
+      tma_prefetch_desc(&tmK);
+      tma_prefetch_desc(&tmV);
+    }
+    __syncwarp();
+    uint32_t pos = 0, tiles = 0, kv_loads = 0, epilogues = 0;
+    uint32_t taken0 = 0, taken1 = 0, q_loads0 = 0, q_loads1 = 0, do_loads0 = 0, do_loads1 = 0;   // per stage
+    int out_j0 = -1, out_h = 0, out_b = 0;    // an item whose dK and dV are to be stored
+    uint32_t out_st = 0;
+    auto store = [&]() -> bool {
+      if (out_j0 < 0) return true;
+      const uint32_t ph = epilogues & 1;
+      if (!mbar_wait_warp(&bar_epi[0], ph, abortp, p.status, kKvSiteEpi, out_j0)) return false;
+      if (!mbar_wait_warp(&bar_epi[1], ph, abortp, p.status, kKvSiteEpi, out_j0)) return false;
       if (elect_one()) {
-        tma_prefetch_desc(&tmQ);
-        tma_prefetch_desc(&tmDO);
-        tma_prefetch_desc(&tmK);
-        tma_prefetch_desc(&tmV);
-        mbar_expect_tx(&bar_kv, 2 * kTileBytes);
 #pragma unroll
         for (int s = 0; s < kSub; ++s) {
-          tma_load_4d(sK + s * kSubBytes, &tmK, &bar_kv, s * 64, j0, h, b);
-          tma_load_4d(sV + s * kSubBytes, &tmV, &bar_kv, s * 64, j0, h, b);
+          tma_store_4d(&tmDK, sQ + out_st * kTileBytes + s * kSubBytes, s * 64, out_j0, out_h, out_b);
+          tma_store_4d(&tmDV, sDO + out_st * kTileBytes + s * kSubBytes, s * 64, out_j0, out_h, out_b);
         }
+        tma_store_commit();
+        tma_store_wait_read<0>();   // the tiles must stay in shared memory until they have been read
+        mbar_arrive(&bar_q_empty[out_st]);
+        mbar_arrive(&bar_do_empty[out_st]);
+        mbar_arrive(&bar_epi_free[0]);
+        mbar_arrive(&bar_epi_free[1]);
       }
       __syncwarp();
-      const float* lam = p.lam + bh * N + P;
-      const float* Lp = p.L + bh * M;
-      const float* dl = p.delta + bh * M;
+      ++epilogues;
+      out_j0 = -1;
+      return true;
+    };
+    bool ok = true;
+    uint32_t item = 0, asked = 0;
+    for (int i = blockIdx.x; i >= 0 && ok;) {
+      if constexpr (kLoop) {
+        ok = items_ask(items, item, abortp, p.status, kKvSiteItem);
+        if (!ok) break;
+        ++asked;
+      }
+      const Item x = item_of(i);
+      if (x.n > 0) {
+        ok = mbar_wait_warp(&bar_kv_free, (kv_loads & 1) ^ 1, abortp, p.status, kKvSiteKV, i);
+        if (!ok) break;
+        if (elect_one()) {
+          mbar_expect_tx(&bar_kv, 2 * kTileBytes);
+#pragma unroll
+          for (int s = 0; s < kSub; ++s) {
+            tma_load_4d(sK + s * kSubBytes, &tmK, &bar_kv, s * 64, x.j0, x.h, x.b);
+            tma_load_4d(sV + s * kSubBytes, &tmV, &bar_kv, s * 64, x.j0, x.h, x.b);
+          }
+        }
+        __syncwarp();
+        ++kv_loads;
+      }
+      const float* lam = p.lam + x.bh * N + P;
+      const float* Lp = p.L + x.bh * M;
+      const float* dl = p.delta + x.bh * M;
       // prefixes relative to this KV tile's first key before the scaling by log2(e), as for negb below
-      const float lam_ref = p.lam[bh * N + min(j0, N - 1)];
+      const float lam_ref = p.lam[x.bh * N + min(x.j0, N - 1)];
       float ev[4], dv_[4];   // lane l holds query rows 4l .. 4l+3 of a tile
       auto fetch_vec = [&](int it) {
-        const int i0 = (hb_lo + it) * BM + 4 * lane;
+        const int i0 = (x.hb_lo + it) * BM + 4 * lane;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int i = i0 + e;
+          const int r = i0 + e;
           float Li = -INFINITY, la = 0.f, de = 0.f;
-          if (i < M) {
-            Li = ldg_f32_here(Lp + i);
-            la = ldg_f32_here(lam + i);
-            de = ldg_f32_here(dl + i);
+          if (r < M) {
+            Li = ldg_f32_here(Lp + r);
+            la = ldg_f32_here(lam + r);
+            de = ldg_f32_here(dl + r);
           }
           ev[e] = (Li == -INFINITY) ? -INFINITY : ((la - lam_ref) - Li) * kKvLog2e;
           dv_[e] = de;
         }
       };
-      auto stage_vec = [&](int it) {
-        const int slot = it % kVec;
+      auto stage_vec = [&](uint32_t slot) {
         *reinterpret_cast<float4*>(&s_e[slot][4 * lane]) = make_float4(ev[0], ev[1], ev[2], ev[3]);
         *reinterpret_cast<float4*>(&s_delta[slot][4 * lane]) = make_float4(dv_[0], dv_[1], dv_[2], dv_[3]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_vec[slot]);
         __syncwarp();
       };
-      fetch_vec(0);
-      int issued = 0;
-      for (int it = 0; it < n_tiles; ++it) {
-        const int i0 = (hb_lo + it) * BM;
-        const int st = it % kSt;
-        const uint32_t ph = ((it / kSt) & 1) ^ 1;
-        if (!mbar_wait_warp(&bar_q_empty[st], ph, abortp, p.status, kKvSiteQE, it)) break;
+      if (x.n > 0) fetch_vec(0);
+      for (int it = 0; it < x.n; ++it, ++pos, ++tiles) {
+        const int i0 = (x.hb_lo + it) * BM;
+        const uint32_t st = pos & 1, ph = ((st ? taken1 : taken0) & 1) ^ 1;
+        ok = mbar_wait_warp(&bar_q_empty[st], ph, abortp, p.status, kKvSiteQE, it);
+        if (!ok) break;
         if (elect_one()) {
           mbar_expect_tx(&bar_q_full[st], kTileBytes);
 #pragma unroll
-          for (int s = 0; s < kSub; ++s) tma_load_4d(sQ + st * kTileBytes + s * kSubBytes, &tmQ, &bar_q_full[st], s * 64, i0, h, b);
+          for (int s = 0; s < kSub; ++s) tma_load_4d(sQ + st * kTileBytes + s * kSubBytes, &tmQ, &bar_q_full[st], s * 64, i0, x.h, x.b);
         }
         __syncwarp();
-        if (!mbar_wait_warp(&bar_do_empty[st], ph, abortp, p.status, kKvSiteDOE, it)) {
-          issued = 2 * it + 1;
-          break;
-        }
+        if (st) ++q_loads1;
+        else ++q_loads0;
+        ok = mbar_wait_warp(&bar_do_empty[st], ph, abortp, p.status, kKvSiteDOE, it);
+        if (!ok) break;
         if (elect_one()) {
           mbar_expect_tx(&bar_do_full[st], kTileBytes);
 #pragma unroll
-          for (int s = 0; s < kSub; ++s) tma_load_4d(sDO + st * kTileBytes + s * kSubBytes, &tmDO, &bar_do_full[st], s * 64, i0, h, b);
+          for (int s = 0; s < kSub; ++s) tma_load_4d(sDO + st * kTileBytes + s * kSubBytes, &tmDO, &bar_do_full[st], s * 64, i0, x.h, x.b);
         }
         __syncwarp();
-        issued = 2 * it + 2;
-        // (slot it % 4 last held tile it-4; the Q stage just re-used was freed by dK(it-2), behind dS(it-2))
-        stage_vec(it);
-        if (it + 1 < n_tiles) fetch_vec(it + 1);
+        if (st) ++do_loads1, ++taken1;
+        else ++do_loads0, ++taken0;
+        // (a slot last held the tile four before; the Q stage just re-used was freed by the products of a later one, behind
+        // its dS)
+        stage_vec(tiles % kVec);
+        if (it + 1 < x.n) fetch_vec(it + 1);
+        if (it == 0) ok = store();   // (the item before)
+        if (!ok) break;
       }
-      if (*abortp && lane == 0) {
-        // error path only: let the copies already in flight land before the CTA retires
-        const long long t0 = clock64();
-        while (!mbar_try_wait(&bar_kv, 0) && clock64() - t0 < 200000000LL) {
+      if (x.n == 0) ok = store();
+      if (!ok) break;
+      out_j0 = x.j0;
+      out_h = x.h;
+      out_b = x.b;
+      out_st = pos & 1;
+      if (pos & 1) ++taken1;
+      else ++taken0;
+      ++pos;
+      if constexpr (!kLoop) break;
+      i = items_next(items, item++, true, abortp, p.status, kKvSiteItem);
+    }
+    if (ok) ok = store();
+    if (*abortp && lane == 0) {
+      // error path only: let the copies already in flight land before the CTA retires
+      const long long t0 = clock64();
+      auto land = [&](uint64_t* bar, uint32_t loads) {
+        while (loads > 0 && !mbar_try_wait(bar, (loads - 1) & 1) && clock64() - t0 < 200000000LL) {
         }
-        for (int c = max(issued - 2 * kSt, 0); c < issued; ++c) {
-          const int it = c >> 1;
-          uint64_t* bar = (c & 1) ? &bar_do_full[it % kSt] : &bar_q_full[it % kSt];
-          while (!mbar_try_wait(bar, (it / kSt) & 1) && clock64() - t0 < 200000000LL) {
-          }
-        }
-      }
+      };
+      land(&bar_kv, kv_loads);
+      land(&bar_q_full[0], q_loads0);
+      land(&bar_q_full[1], q_loads1);
+      land(&bar_do_full[0], do_loads0);
+      land(&bar_do_full[1], do_loads1);
+      land(&items.full[0], (asked + 1) >> 1);
+      land(&items.full[1], asked >> 1);
     }
   } else if (warp == kMmaWarp) {
     // ===================== MMA issuer =====================
-    if (n_tiles > 0) {
+    {
       constexpr uint32_t idS = umma_idesc(kFmt, 128, BM, 0, 0);    // S^T, dP^T: N = 128 query rows, B K-major
       constexpr uint32_t idKV = umma_idesc(kFmt, 128, D, 0, 1);    // dV, dK: N = D, B MN-major
       const uint64_t dKk = umma_desc_kmajor(smem_u32(sK));
@@ -253,9 +317,9 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const uint64_t dDOk = umma_desc_kmajor(smem_u32(sDO));
       const uint64_t dQmn = umma_desc_mnmajor(smem_u32(sQ), kSubBytes);
       const uint64_t dDOmn = umma_desc_mnmajor(smem_u32(sDO), kSubBytes);
-      auto issue_s = [&](int t) {
+      auto issue_s = [&](uint32_t st) {
         if (elect_one()) {
-          const uint64_t dq_ = umma_desc_advance(dQk, (t % kSt) * kTileBytes);
+          const uint64_t dq_ = umma_desc_advance(dQk, st * kTileBytes);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = (kk >> 2) * kSubBytes + (kk & 3) * 32;
@@ -265,100 +329,118 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         __syncwarp();
       };
-      auto issue_dp = [&](int t) {
+      auto issue_dp = [&](uint32_t st, bool last) {
         if (elect_one()) {
-          const uint64_t do_ = umma_desc_advance(dDOk, (t % kSt) * kTileBytes);
+          const uint64_t do_ = umma_desc_advance(dDOk, st * kTileBytes);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = (kk >> 2) * kSubBytes + (kk & 3) * 32;
             mma_ss_raw(tbase + kColDP, umma_desc_advance(dVk, off), umma_desc_advance(do_, off), idS, kk > 0);
           }
           tc_commit_raw(&bar_dp_full);
+          if (last) tc_commit_raw(&bar_kv_free);   // the item's last reader of K and V
         }
         __syncwarp();
       };
-      bool ok = mbar_wait_warp(&bar_kv, 0, abortp, p.status, kKvSiteKV);
-      if (ok) ok = mbar_wait_warp(&bar_q_full[0], 0, abortp, p.status, kKvSiteQ, 0);
-      if (ok) {
+      uint32_t pos = 0, tiles = 0, done = 0, full0 = 0, full1 = 0;   // full: tiles of a stage so far
+      auto wait_q = [&](uint32_t st, int it) {
+        const bool good = mbar_wait_warp(&bar_q_full[st], (st ? full1 : full0) & 1, abortp, p.status, kKvSiteQ, it);
         tc_fence_after();
-        issue_s(0);
-        ok = mbar_wait_warp(&bar_do_full[0], 0, abortp, p.status, kKvSiteDO, 0);
-      }
-      if (ok) {
+        return good;
+      };
+      auto wait_do = [&](uint32_t st, int it) {   // (behind wait_q of the same tile)
+        const bool good = mbar_wait_warp(&bar_do_full[st], (st ? full1 : full0) & 1, abortp, p.status, kKvSiteDO, it);
         tc_fence_after();
-        issue_dp(0);
-      }
-      for (int it = 0; it < n_tiles && ok; ++it) {
-        const int st = it % kSt;
-        KVSTAMP(17, 0, it);
-        // S^T(it) has been read into registers: S^T(it+1) may overwrite it
-        ok = mbar_wait_warp(&bar_s_read, it & 1, abortp, p.status, kKvSiteP, it);
-        if (!ok) break;
-        KVSTAMP(17, 1, it);
-        if (it + 1 < n_tiles) {
-          ok = mbar_wait_warp(&bar_q_full[(it + 1) % kSt], ((it + 1) / kSt) & 1, abortp, p.status, kKvSiteQ, it + 1);
+        if (st) ++full1;
+        else ++full0;
+        return good;
+      };
+      bool ok = true;
+      uint32_t item = 0;
+      for (int i = blockIdx.x; i >= 0 && ok;) {
+        const Item x = item_of(i);
+        if (x.n > 0) {
+          // (S^T's columns are free: the item before ended with its last tile read; dP^T's follow its last products)
+          ok = mbar_wait_warp(&bar_kv, done & 1, abortp, p.status, kKvSiteKV, i) && wait_q(pos & 1, 0);
           if (!ok) break;
-          tc_fence_after();
-          issue_s(it + 1);
-        }
-        KVSTAMP(17, 2, it);
-        ok = mbar_wait_warp(&bar_ds_full, it & 1, abortp, p.status, kKvSiteDS, it);
-        if (!ok) break;
-        KVSTAMP(17, 3, it);
-        tc_fence_after();
-        if (elect_one()) {
-          // warpgroup g's 32 dP^T columns now hold its 16-bit P^T (first 16) and dS^T (last 16);
-          // product step kk covers query columns [16 kk, 16 kk + 16): warpgroup kk / 2, half kk % 2
-          const uint64_t do_ = umma_desc_advance(dDOmn, st * kTileBytes);
-          const uint64_t dq_ = umma_desc_advance(dQmn, st * kTileBytes);
-#pragma unroll
-          for (int kk = 0; kk < BM / 16; ++kk)
-            mma_ts_raw(tbase + kColDV, tbase + kColDP + (kk >> 1) * CW + (kk & 1) * 8, umma_desc_advance(do_, kk * 2048), idKV,
-                       (it > 0 || kk > 0) ? 1u : 0u);
-          tc_commit_raw(&bar_do_empty[st]);
-#pragma unroll
-          for (int kk = 0; kk < BM / 16; ++kk)
-            mma_ts_raw(tbase + kColDK, tbase + kColDP + (kk >> 1) * CW + 16 + (kk & 1) * 8, umma_desc_advance(dq_, kk * 2048), idKV,
-                       (it > 0 || kk > 0) ? 1u : 0u);
-          tc_commit_raw(&bar_q_empty[st]);
-        }
-        __syncwarp();
-        if (it + 1 < n_tiles) {
-          ok = mbar_wait_warp(&bar_do_full[(it + 1) % kSt], ((it + 1) / kSt) & 1, abortp, p.status, kKvSiteDO, it + 1);
+          issue_s(pos & 1);
+          ok = wait_do(pos & 1, 0);
           if (!ok) break;
-          tc_fence_after();
-          issue_dp(it + 1);   // overwrites P^T(it), dS^T(it): ordered behind dV(it), dK(it) in the tensor pipe
+          issue_dp(pos & 1, x.n == 1);
+          for (int it = 0; it < x.n; ++it, ++pos, ++tiles) {
+            const uint32_t st = pos & 1, nx = st ^ 1, ph = tiles & 1;
+            // S^T(it) has been read into registers: S^T(it+1) may overwrite it
+            ok = mbar_wait_warp(&bar_s_read, ph, abortp, p.status, kKvSiteP, it);
+            if (!ok) break;
+            if (it + 1 < x.n) {
+              ok = wait_q(nx, it + 1);
+              if (!ok) break;
+              issue_s(nx);
+            }
+            ok = mbar_wait_warp(&bar_ds_full, ph, abortp, p.status, kKvSiteDS, it);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+              // warpgroup g's 32 dP^T columns now hold its 16-bit P^T (first 16) and dS^T (last 16);
+              // product step kk covers query columns [16 kk, 16 kk + 16): warpgroup kk / 2, half kk % 2
+              const uint64_t do_ = umma_desc_advance(dDOmn, st * kTileBytes);
+              const uint64_t dq_ = umma_desc_advance(dQmn, st * kTileBytes);
+#pragma unroll
+              for (int kk = 0; kk < BM / 16; ++kk)
+                mma_ts_raw(tbase + kColDV, tbase + kColDP + (kk >> 1) * CW + (kk & 1) * 8, umma_desc_advance(do_, kk * 2048), idKV,
+                           (it > 0 || kk > 0) ? 1u : 0u);
+              tc_commit_raw(&bar_do_empty[st]);
+#pragma unroll
+              for (int kk = 0; kk < BM / 16; ++kk)
+                mma_ts_raw(tbase + kColDK, tbase + kColDP + (kk >> 1) * CW + 16 + (kk & 1) * 8, umma_desc_advance(dq_, kk * 2048), idKV,
+                           (it > 0 || kk > 0) ? 1u : 0u);
+              tc_commit_raw(&bar_q_empty[st]);
+            }
+            __syncwarp();
+            if (it + 1 < x.n) {
+              ok = wait_do(nx, it + 1);
+              if (!ok) break;
+              issue_dp(nx, it + 2 == x.n);   // overwrites P^T(it), dS^T(it): ordered behind dV(it), dK(it) in the tensor pipe
+            }
+          }
+          if (!ok) break;
+          tc_commit(&bar_done);
+          ++done;
         }
-        KVSTAMP(17, 4, it);
+        ++pos;   // (the stage of the item's dK and dV)
+        if constexpr (!kLoop) break;
+      i = items_next(items, item++, false, abortp, p.status, kKvSiteItem);
       }
-      if (ok) tc_commit(&bar_done);
     }
   } else {
     // ===================== elementwise / epilogue =====================
     const int g = warp >> 2;
     const int r = tid & 127;
-    const int j = j0 + r;
-    const bool j_ok = j < N && j >= seq0;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    // Lambda_i - Lambda_j from prefixes relative to the tile's first key: scaling a prefix of -1e4 by log2(e)
-    // first would cost an absolute 2e-3 per logit
-    const float negb = j_ok ? (p.lam[bh * N + min(j0, N - 1)] - p.lam[bh * N + j]) * kKvLog2e : -INFINITY;
     const uint32_t tS = tbase + lane_base + kColS + g * CW, tDP = tbase + lane_base + kColDP + g * CW;
     const float2 scale2 = make_float2(p.qk_scale, p.qk_scale);
+    uint32_t tiles = 0, done = 0, epilogues = 0;
+    bool ok = true;
+    uint32_t item = 0;
+    for (int i = blockIdx.x; i >= 0 && ok;) {
+    const Item x = item_of(i);
+    const int j0 = x.j0, j = j0 + r;
+    const bool j_ok = j < N && j >= x.seq0;
+    // Lambda_i - Lambda_j from prefixes relative to the tile's first key: scaling a prefix of -1e4 by log2(e)
+    // first would cost an absolute 2e-3 per logit
+    const float negb = j_ok ? (p.lam[x.bh * N + min(j0, N - 1)] - p.lam[x.bh * N + j]) * kKvLog2e : -INFINITY;
     const float2 negb2 = make_float2(negb, negb);
     float2 colsum2 = make_float2(0.f, 0.f);
-    bool ok = true;
-    for (int it = 0; it < n_tiles; ++it) {
-      const int i0 = (hb_lo + it) * BM;
-      const int slot = it % kVec;
+    for (int it = 0; it < x.n; ++it, ++tiles) {
+      const int i0 = (x.hb_lo + it) * BM;
+      const uint32_t slot = tiles % kVec;
       // ---------------- phase A: p^T into registers ----------------
       KVSTAMP(warp, 0, it);
-      ok = mbar_wait(&bar_vec[slot], (it / kVec) & 1, abortp, p.status, kKvSiteVec, it);
-      ok = mbar_wait(&bar_s_full, it & 1, abortp, p.status, kKvSiteS, it) && ok;
+      ok = mbar_wait(&bar_vec[slot], (tiles / kVec) & 1, abortp, p.status, kKvSiteVec, it);
+      ok = mbar_wait(&bar_s_full, tiles & 1, abortp, p.status, kKvSiteS, it) && ok;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       KVSTAMP(warp, 1, it);
-      if (tid == 0 && it == 0) KVCTA(2);
       tc_fence_after();
       uint32_t sreg[32], pk[16];
       float2 pf[16];
@@ -389,7 +471,7 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
       KVSTAMP(warp, 2, it);
       // ---------------- phase B: P^T and dS^T, 16 bit, over this warpgroup's own dP^T columns ----------------
-      ok = mbar_wait(&bar_dp_full, it & 1, abortp, p.status, kKvSiteDP, it);
+      ok = mbar_wait(&bar_dp_full, tiles & 1, abortp, p.status, kKvSiteDP, it);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       KVSTAMP(warp, 3, it);
@@ -416,39 +498,38 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       KVSTAMP(warp, 4, it);
     }
     // ---- epilogue: dK * sm_scale, dV -> 16-bit -> global; -colsum(dS) ----
-    if (tid == 0) KVCTA(3);
+    if (!ok) break;
     float colsum = colsum2.x + colsum2.y;
-    if (g > 0) {
-      s_part[g - 1][r] = colsum;
+    if (x.n > 0) {
+      // (two arrays in turn, and every warpgroup waits for the others: none is more than one item ahead)
+      float (*part)[128] = s_part[done & 1];
+      if (g > 0) part[g - 1][r] = colsum;
       mbar_arrive(&bar_colsum);
-    } else {
-      ok = mbar_wait(&bar_colsum, 0, abortp, p.status, kKvSiteCol) && ok;
+      ok = mbar_wait(&bar_colsum, done & 1, abortp, p.status, kKvSiteCol);
       ok = __all_sync(0xffffffffu, ok);
-      if (ok) colsum += (s_part[0][r] + s_part[1][r]) + s_part[2][r];
+      if (ok && g == 0) colsum += (part[0][r] + part[1][r]) + part[2][r];
+      ok = mbar_wait(&bar_done, done & 1, abortp, p.status, kKvSiteDone) && ok;
+      ++done;
     }
-    if (n_tiles > 0 && ok) {
-      ok = mbar_wait(&bar_done, 0, abortp, p.status, kKvSiteDone);
-      ok = __all_sync(0xffffffffu, ok);
-    }
-    if (tid == 0) KVCTA(4);
-    if (ok) {
+    if (epilogues > 0) ok = mbar_wait(&bar_epi_free[g >> 1], (epilogues - 1) & 1, abortp, p.status, kKvSiteEpi) && ok;
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    {
       tc_fence_after();
-      // warpgroups 0, 1 hold the halves of dK, 2 and 3 those of dV.  The 16-bit tiles go through shared memory
-      // (the Q stages are idle: every product has retired) and leave as TMA stores, which write whole lines and
-      // clip the rows past N; a thread storing its own row 16 bytes at a time kept the CTA ~7 us in this epilogue.
+      // warpgroups 0, 1 hold the halves of dK, 2 and 3 those of dV.  The 16-bit tiles go through shared memory (a Q
+      // and a dO stage that nothing reads) and leave as TMA stores, which write whole lines and clip the rows past N;
+      // a thread storing its own row 16 bytes at a time kept the CTA ~7 us in this epilogue.
       constexpr int kHalf = D / 2;   // columns of dK or dV per warpgroup
       const int which = g >> 1, part_c = (g & 1) * kHalf;
-      const bool keep = j_ok && n_tiles > 0;
+      const bool keep = j_ok && x.n > 0;
       const uint32_t tcol = tbase + lane_base + (which == 0 ? kColDK : kColDV) + part_c;
       const float sc = which == 0 ? p.sm_scale : 1.f;
-      uint8_t* stile = sQ + which * kTileBytes;
+      uint8_t* stile = (which == 0 ? sQ : sDO) + ((tiles + epilogues) & 1) * kTileBytes;   // (see the producer)
 #pragma unroll
       for (int c = 0; c < kHalf; c += 32) {
-        uint32_t t0[32];
-        if (n_tiles > 0) {
-          tmem_ld32(tcol + c, t0);
-          tmem_ld_wait();
-        }
+        uint32_t t0[32];   // (of an item without query tiles: not kept)
+        tmem_ld32(tcol + c, t0);
+        tmem_ld_wait();
         const int col = part_c + c;
         uint8_t* srow = stile + (col >> 6) * kSubBytes + r * 128;
 #pragma unroll
@@ -464,27 +545,19 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
       }
       fence_proxy_async_smem();
+      tc_fence_before();   // (the accumulators are overwritten by the next item's products)
       mbar_arrive(&bar_epi[which]);
-      if ((g & 1) == 0 && (warp & 3) == 0) {
-        // (a bounded wait like every other one: a warp that gave up elsewhere never arrives)
-        if (mbar_wait_warp(&bar_epi[which], 0, abortp, p.status, kKvSiteEpi) && elect_one()) {
-#pragma unroll
-          for (int sub = 0; sub < kSub; ++sub)
-            tma_store_4d(which == 0 ? &tmDK : &tmDV, stile + sub * kSubBytes, sub * 64, j0, h, b);
-          tma_store_commit();
-          tma_store_wait_read<0>();   // the tile must stay in shared memory until it has been read
-        }
-        __syncwarp();
-      }
-      if (g == 0 && j < N) p.dlam_col[bh * N + j] = keep ? -colsum : 0.f;
+      if (g == 0 && j < N) p.dlam_col[x.bh * N + j] = keep ? -colsum : 0.f;
     }
-    if (tid == 0) KVCTA(5);
+    ++epilogues;
+    if constexpr (!kLoop) break;
+      i = items_next(items, item++, false, abortp, p.status, kKvSiteItem);
+    }
   }
 
   tc_fence_before();
   __syncthreads();
   if (warp == kTmaWarp) tmem_dealloc(tbase, kTmemCols);
-  if (tid == 0) KVCTA(6);
 }
 
 template <int D, bool kBf16>
@@ -509,15 +582,15 @@ static int launch_kv(int device, cudaStream_t stream, int64_t B, int64_t H, int6
   if ((rc = cached_tmap_4d(&tmDK, tdk, 2, false, kBf16, 64, kKvBN, true))) return rc;
   if ((rc = cached_tmap_4d(&tmDV, tdv, 2, false, kBf16, 64, kKvBN, true))) return rc;
   constexpr int smem = (2 * 2 + 2) * 128 * D * 2 + 1024;   // Q, dO in two stages each, K, V
-  auto kern = fox_attn_bwd_kv_kernel<D, kBf16>;
-  static bool configured[64] = {};
+  const bool loop = prm.end_index != nullptr;   // (see the head of this file)
+  auto kern = loop ? fox_attn_bwd_kv_kernel<D, kBf16, true> : fox_attn_bwd_kv_kernel<D, kBf16, false>;
+  static bool configured[2][64] = {};
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;
-  if (!configured[device]) {
+  if (!configured[loop][device]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
-    configured[device] = true;
+    configured[loop][device] = true;
   }
-  dim3 grid((unsigned)((N + kKvBN - 1) / kKvBN), (unsigned)H, (unsigned)B);
-  kern<<<grid, 576, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDK, tmDV, prm);
+  kern<<<(unsigned)prm.items, 576, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDK, tmDV, prm);
   return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 
@@ -534,6 +607,9 @@ int launch_bwd_kv(int device, cudaStream_t stream, bool bf16, int D, int64_t B, 
   prm.dv = dv->ptr; prm.dv_sb = dv->sb; prm.dv_sh = dv->sh; prm.dv_st = dv->st;
   prm.status = status;
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
+  const int64_t tiles = (N + kKvBN - 1) / kKvBN;
+  if (tiles * H * B > 2147483647LL - 65536) return FOX_ERR_TOO_LARGE;
+  prm.tiles = (int)tiles; prm.items = (int)(tiles * H * B);
   prm.sm_scale = sm_scale;
   prm.qk_scale = sm_scale * kKvLog2e;
   if (D == 64)

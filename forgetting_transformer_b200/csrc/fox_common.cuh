@@ -174,6 +174,55 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred px;\n\telect.sync _|px, 0xffffffff;\n\tselp.u32 %0, 1, 0, px;\n\t}" : "=r"(pred));
   return pred != 0;
 }
+
+// ---------------------------------------------------------------------- items
+// A grid of one CTA per item whose CTAs go on with items of CTAs that have not begun (cluster launch control): the items are
+// handed out in the grid's order to whichever CTA is free, as without it, but a CTA's set-up is paid once and the next
+// item's loads run under the end of this one.  One warp asks ahead for each item, the others read the answers; every lane
+// of a warp takes part in every call.
+struct ItemQueue {
+  uint4 answer[2];
+  uint64_t full[2], read[2];
+};
+__device__ __forceinline__ void items_init(ItemQueue& q, uint32_t reading_warps) {   // (without the asking one)
+  for (int i = 0; i < 2; ++i) {
+    mbar_init(&q.full[i], 1);
+    mbar_init(&q.read[i], reading_warps);
+  }
+}
+// asks for the item behind the k-th; never called again after an answer without one
+__device__ __forceinline__ bool items_ask(ItemQueue& q, uint32_t k, volatile int* abortp, int* status, int site) {
+  if (!mbar_wait_warp(&q.read[k & 1], ((k >> 1) & 1) ^ 1, abortp, status, site, static_cast<int>(k))) return false;
+  if (elect_one()) {
+    fence_proxy_async_smem();
+    mbar_expect_tx(&q.full[k & 1], 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(&q.answer[k & 1])), "r"(smem_u32(&q.full[k & 1]))
+                 : "memory");
+  }
+  __syncwarp();
+  return true;
+}
+// the item behind the k-th, or -1
+__device__ __forceinline__ int items_next(ItemQueue& q, uint32_t k, bool asking, volatile int* abortp, int* status, int site) {
+  if (!mbar_wait_warp(&q.full[k & 1], (k >> 1) & 1, abortp, status, site, static_cast<int>(k))) return -1;
+  int first, taken;
+  asm volatile(
+      "{\n\t.reg .b128 a;\n\t.reg .pred t;\n\t"
+      "ld.shared.b128 a, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 t, a;\n\t"
+      "selp.b32 %1, 1, 0, t;\n\t"
+      "mov.b32 %0, 0;\n\t"
+      "@t clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t}"
+      : "=r"(first), "=r"(taken)
+      : "r"(smem_u32(&q.answer[k & 1]))
+      : "memory");
+  fence_proxy_async_smem();   // (the next answer here comes by the async proxy)
+  __syncwarp();
+  if (!asking && elect_one()) mbar_arrive(&q.read[k & 1]);
+  __syncwarp();
+  return taken ? first : -1;
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
                "r"(ncols)

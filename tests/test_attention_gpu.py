@@ -643,3 +643,21 @@ def test_pruning_indices_by_search_and_by_scan(M, N, bm, bn, kind):
     si, ei = ops.find_index(lam.cuda(), thr.cuda(), M, bm, bn, True, True)
     assert np.array_equal(si.cpu().numpy(), orc.find_start_index(lam.numpy(), thr.numpy(), M, N, bm, bn))
     assert np.array_equal(ei.cpu().numpy(), orc.find_end_index(lam.numpy(), thr.numpy(), M, N, bm, bn))
+
+
+@pytest.mark.parametrize("M,N", [(2500, 2500), (1000, 3001), (129, 2560)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_pruned_backward_tiles_walked_by_a_cta_equal_tiles_of_their_own(M, N, dtype):
+    """The pruned D=128 backward walks its tiles, more than 148 here, with 148 CTAs: bit-identical to a call for each (b,h),
+    whose tiles have a CTA each.  Padding leaves a batch element without any key for most tiles and one with only its last."""
+    B, H = 3, 5
+    q, k, v, lf, do = _inputs(M + N, B, H, M, N, 128, dtype, mu=1.0, sigma=2.0)
+    lf[:, 3] = 0.0                                                  # (a head that nothing is pruned of)
+    seq = torch.tensor([0, N // 3, N - 1])
+    assert B * H * ((N + 127) // 128) > 2 * 148
+    whole = _run(q, k, v, lf, do, seq=seq, thr=-12.0)
+    for b in range(B):
+        for h in range(H):
+            part = _run(*[t[b:b + 1, h:h + 1] for t in (q, k, v, lf, do)], seq=seq[b:b + 1], thr=-12.0)
+            for name, x, y in zip(("out", "dq", "dk", "dv", "dlog_fgate"), whole, part):
+                assert torch.equal(x[b, h], y[0, 0]), (name, b, h)
