@@ -87,6 +87,7 @@ _SIGNATURES = {
                                  _F, c_int64, c_int64, _F, _F, _F, _F, c_int64]),
     "fox_step_product_ahead": (c_int, [c_int, c_void_p, c_int, c_int, c_int, c_int64, c_int64, _F, c_int, _F, c_int, c_float,
                                        c_int64, _F, c_int64, c_int64, _F, _F, _F, _F, c_int64, _F, c_int64, _F]),
+    "fox_step_ahead_offset": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
     "fox_step_mix": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, _F, c_int64, _F, c_int, _F, c_int, c_float, _F,
                              c_int, _F, _F, _F, _F, _F, _F, _F, _F, c_int64, c_int64]),
     "fox_step_attn": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, _F, c_int64, _F, c_int, _F, c_int, c_float, _F,

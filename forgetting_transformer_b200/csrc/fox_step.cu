@@ -64,9 +64,15 @@ struct StepParams {
   const void* res;                // kOutAdd16: (B, ldo) 16-bit; kOutAdd32: (B, ldo) fp32
   int half;                       // kOutSwiglu: rows of each half
   const char* ahead;              // what a later product reads (16-byte aligned), or nullptr
-  uint32_t ahead_bytes;           // (a multiple of 16)
+  uint64_t ahead_bytes;           // (a multiple of 16)
   int* status;                    // where a wait that runs out is recorded; nullptr: weights through registers
 };
+
+// Where the k-th request of a thread begins in what a later product reads.  In 64 bits: 256 threads of 4096 CTAs, the grid of an
+// intermediate size of 32768, ask for 2^32 bytes in one round.
+__host__ __device__ __forceinline__ uint64_t step_ahead_at(uint64_t grid, uint64_t block, uint64_t thread, uint64_t k) {
+  return ((k * kStepThreads + thread) * grid + block) * kStepChunk;
+}
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -192,9 +198,9 @@ fox_step_product_kernel(const StepParams p) {
     }
   }
   if (p.ahead) {
-    const uint32_t step = kStepThreads * gridDim.x * kStepChunk;
-    for (uint32_t o = (tid * gridDim.x + blockIdx.x) * kStepChunk; o < p.ahead_bytes; o += step)
-      l2_request(p.ahead + o, min(kStepChunk, p.ahead_bytes - o));
+    const uint64_t round = step_ahead_at(gridDim.x, 0, 0, 1);
+    for (uint64_t o = step_ahead_at(gridDim.x, blockIdx.x, tid, 0); o < p.ahead_bytes; o += round)
+      l2_request(p.ahead + o, static_cast<uint32_t>(min(static_cast<uint64_t>(kStepChunk), p.ahead_bytes - o)));
   }
   // one chunk of a row per lane at most: its norm weights come before the wait, its input stays in registers
   int per = 8;   // warps that share a row
@@ -512,7 +518,7 @@ static int step_product(int device, void* stream, int dtype, int input, int outp
   if (align % 16) return FOX_ERR_ALIGNMENT;
   if (ahead && (reinterpret_cast<uintptr_t>(ahead) % 16 || ahead_bytes < 0 || ahead_bytes % 16)) return FOX_ERR_ALIGNMENT;
   p.ahead = (const char*)ahead;
-  p.ahead_bytes = (uint32_t)(ahead_bytes < (1LL << 30) ? ahead_bytes : 1LL << 30);   // (counted in 32 bits)
+  p.ahead_bytes = (uint64_t)ahead_bytes;
   p.status = status;
   p.n_mats = (int)n_mats; p.B = (int)B; p.K = (int)K; p.D = (int)D;
   p.x = x; p.x_fp32 = x_fp32 != 0; p.norm_w = norm_w; p.w_dtype = norm_w_dtype; p.eps = eps;
@@ -527,6 +533,10 @@ static int step_product(int device, void* stream, int dtype, int input, int outp
   FOX_STEP(kInPlain, kOutAdd32);
 #undef FOX_STEP
   return FOX_ERR_BAD_ARG;
+}
+
+extern "C" int64_t fox_step_ahead_offset(int64_t grid, int64_t block, int64_t thread, int64_t k) {
+  return (int64_t)step_ahead_at((uint64_t)grid, (uint64_t)block, (uint64_t)thread, (uint64_t)k);
 }
 
 extern "C" int fox_step_product_ahead(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K,

@@ -297,6 +297,8 @@ int fox_step_product_ahead(int device, void* stream, int dtype, int input, int o
                            int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
                            const void* residual, void* out, int64_t ldo, const void* ahead, int64_t ahead_bytes,
                            int32_t* status);
+/* Offset in that array of the k-th request of a thread (of 256) of a CTA of a grid, 4096 bytes or what is left behind it. */
+int64_t fox_step_ahead_offset(int64_t grid, int64_t block, int64_t thread, int64_t k);
 /* y (B,ld) fp32 as fox_mix_fwd's rows: token shift with the states k_state, v_state (B,C) 16-bit, which are replaced by
  * this token's projections, norms of q and k, and row pos of the caches k, v (B,H,capacity,D), log gates (B,H,capacity);
  * mask (B,pos+1) int64 or NULL: seq_start (B) receives pos + 1 - its sum. */

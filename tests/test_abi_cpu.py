@@ -188,3 +188,18 @@ def test_decode_ranges_fill_whole_waves(bh, n):
     assert 1 <= s <= min(512, max(1, -(-n // 128)))
     waves = -(-bh // 444) + (1 if -(-bh // 444) * 400 // bh <= 1 else 0)
     assert s == 1 or bh * s <= waves * (444 if s > 8 else 400)
+
+
+@pytest.mark.parametrize("grid", [1, 176, 2048, 4095, 4096, 4097, 8192, 12288, 2 ** 20])
+def test_requests_ahead_of_a_token_product_cover_the_array_once(grid):
+    """fox_step_product_ahead's threads ask for one 4096-byte piece after another of what a later product reads: blocks follow
+    one another, then threads, then rounds, without a gap, a repetition or a round of no length, at grids beyond 2^32 bytes a
+    round (4096 CTAs of 256 threads) too."""
+    at = _lib.load().fox_step_ahead_offset
+    assert at(grid, 0, 0, 0) == 0
+    for k in (0, 1, 5):
+        for thread in range(256):
+            for block in {0, 1, grid // 2, grid - 2} & set(range(grid - 1)):
+                assert at(grid, block + 1, thread, k) == at(grid, block, thread, k) + 4096
+            after = at(grid, 0, thread + 1, k) if thread < 255 else at(grid, 0, 0, k + 1)
+            assert after == at(grid, grid - 1, thread, k) + 4096

@@ -243,3 +243,29 @@ def test_token_through_every_route(B, C, H, I, N, case):
         a, b = a.float(), b.float()
         assert (a - b).abs().max() <= 2 ** -9 * (b.abs().max() + 1)
         assert (a - b).norm() <= 2 ** -9 * b.norm()
+
+
+@pytest.mark.parametrize("B,I", [(1, 32768), (3, 32768), (1, 24608)])
+def test_token_through_a_wide_mlp(B, I):
+    """Gate products whose grid of I / 8 CTAs asks for 2^32 bytes a round, and for somewhat less, of what the down product
+    reads.  Against the modules, with the tolerance of the tests above (fp16)."""
+    torch.manual_seed(I)
+    blk = fox.FoxProBlock(256, 2, I, fgate_bias=2.0).cuda().to(torch.float16)
+    x = torch.randn(B, 1, 256, device="cuda").half()
+    k, v = torch.randn(2, B, 2, 70, 128, device="cuda").half()
+    g = torch.nn.functional.logsigmoid(torch.randn(B, 2, 70, device="cuda") + 3)
+    res = []
+    for native in (True, False):
+        cache = fox.FgateCache(granule=128)
+        st = blk.attn.init_shift_state(B)
+        cache.update_shift_cache(st["key_shift"], st["value_shift"], 0)
+        cache.update(k, v, g, 0)
+        hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+        with torch.no_grad():
+            res.append(blk(x, None, cache, 0).float())
+        if hook is not None:
+            hook.remove()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert (res[0] - res[1]).abs().max() <= 2 ** -9 * (res[1].abs().max() + 1)
+    assert (res[0] - res[1]).norm() <= 2 ** -9 * res[1].norm()
