@@ -363,8 +363,11 @@ fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeSt
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
       if (grp == 0 && lo < N) {
+        // (at -1e30 the others have no share left; minus infinity would make this logit infinite and its weight NaN.  Without
+        // others the gate has nothing to act on.)
+        const float g2 = lo < end ? g_new * kDecLog2e : 0.f;
         float f_old, f_new;
-        dec_join(m, l, x - g_new * kDecLog2e, 1.f, f_old, f_new);
+        dec_join(m, l, x - (g2 < -1e30f ? -1e30f : g2), 1.f, f_old, f_new);
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[c] = acc[c] * f_old + vv[c] * f_new;
       }

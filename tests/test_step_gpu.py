@@ -269,3 +269,42 @@ def test_token_through_a_wide_mlp(B, I):
     _lib.check_status()
     assert (res[0] - res[1]).abs().max() <= 2 ** -9 * (res[1].abs().max() + 1)
     assert (res[0] - res[1]).norm() <= 2 ** -9 * res[1].norm()
+
+
+@pytest.mark.parametrize("N", [1, 130, 2001])
+@pytest.mark.parametrize("route", ["one kernel", "separate kernels"])
+@pytest.mark.parametrize("padded", [False, True])
+def test_token_whose_gate_forgets_everything(N, route, padded):
+    """Forget logits of minus infinity, of a finite value whose multiple by log2(e) overflows, and of one that leaves the older
+    keys no share: the token's own value, by either route, as by the modules (bf16, eight roundings).  With a gate of NaN too:
+    it acts on the older keys, where there are any."""
+    torch.manual_seed(N)
+    B, C, H = 2, 256, 4
+    blk = fox.FoxProBlock(C, H, 512).cuda().to(torch.bfloat16)
+    x = torch.randn(B, 1, C, device="cuda").bfloat16()
+    k, v = torch.randn(2, B, H, N, C // H, device="cuda").bfloat16()
+    g = torch.nn.functional.logsigmoid(torch.randn(B, H, N, device="cuda") + 3)
+    mask = None
+    if padded:
+        mask = torch.ones(B, N + 1, dtype=torch.long, device="cuda")
+        mask[0, :N] = 0
+    for last in (2.0, float("nan")):
+        with torch.no_grad():
+            blk.attn.fgate_proj.bias.copy_(torch.tensor([float("-inf"), -3e38, -1e4, last]))
+        res = []
+        for native in (True, False):
+            cache = fox.FgateCache(granule=128)
+            st = blk.attn.init_shift_state(B)
+            if route == "separate kernels":   # (which take states that do not start on 16 bytes)
+                st = {n: torch.zeros(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view_as(t) for n, t in st.items()}
+            cache.update_shift_cache(st["key_shift"], st["value_shift"], 0)
+            cache.update(k, v, g, 0)
+            hook = None if native else blk.attn.q_norm.register_forward_hook(lambda *a: None)
+            with torch.no_grad():
+                res.append(blk(x, mask, cache, 0).float())
+            if hook is not None:
+                hook.remove()
+        assert res[1].isfinite().all() or last != last
+        assert torch.equal(res[0].isfinite(), res[1].isfinite())
+        a, b = res[0].nan_to_num(0, 0, 0), res[1].nan_to_num(0, 0, 0)
+        assert (a - b).norm() <= 2 ** -6 * b.norm(), last
