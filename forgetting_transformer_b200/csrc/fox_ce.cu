@@ -272,11 +272,11 @@ fox_ce_bwd_kernel(const void* __restrict__ logits, int64_t row_stride, const int
 // place of five elementwise and reduction kernels; sums in fp64, a cluster's CTAs through its shared memory.  Bound by
 // latency: 1024 threads take up to 8192 rows in one trip of eight loads each, more rows are spread over a cluster of eight
 // CTAs (a loss step of 8192 x 50304 bf16 406 -> 379 us; of 1000 x 32000, bound by the host's calls, 201 -> 147).
+// (Begins before the losses are written: no __restrict__, which would let its loads move in front of the wait.)
 constexpr int kMeanThreads = 1024, kMeanCluster = 8, kMeanRows = 8192;
 
 __global__ void __launch_bounds__(kMeanThreads)
-fox_ce_mean_kernel(const float* __restrict__ losses, const int64_t* __restrict__ labels, int64_t n_rows, int64_t ignore_index,
-                   float* __restrict__ mean, float* __restrict__ count) {
+fox_ce_mean_kernel(const float* losses, const int64_t* labels, int64_t n_rows, int64_t ignore_index, float* mean, float* count) {
   __shared__ double s_sum[32], s_total;
   __shared__ long long s_n[32], s_rows;
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -203,3 +203,18 @@ def test_requests_ahead_of_a_token_product_cover_the_array_once(grid):
                 assert at(grid, block + 1, thread, k) == at(grid, block, thread, k) + 4096
             after = at(grid, 0, thread + 1, k) if thread < 255 else at(grid, 0, 0, k + 1)
             assert after == at(grid, grid - 1, thread, k) + 4096
+
+
+def test_kernels_that_begin_early_take_no_invariant_pointers():
+    """A kernel with griddepcontrol.wait may begin before the kernel in front has written what it reads: a load through a
+    `const __restrict__` pointer, or by __ldg, is one that the compiler may move in front of the wait."""
+    found = 0
+    for name in build.SOURCES:
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(build.CSRC, name)).read())
+        for kernel in re.split(r"__global__", text)[1:]:
+            params, body = kernel.split("{", 1)
+            body = body.split("\n}\n", 1)[0]
+            if "griddepcontrol.wait" in body or "pdl_wait()" in body:
+                found += 1
+                assert "__restrict__" not in params + body and "__ldg" not in body, (name, params)
+    assert found == 5
