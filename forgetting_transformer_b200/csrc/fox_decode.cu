@@ -196,8 +196,10 @@ fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeSt
         if (lane >= o) incl += x;
       }
       if (lane == 31) s_scan[warp] = incl;
+      // (a gate of minus infinity cannot be taken off the sum again)
+      const float left = __shfl_up_sync(0xffffffffu, incl, 1);
       __syncthreads();
-      float before = carry + incl - own, total = 0.f;
+      float before = own > -INFINITY ? carry + incl - own : lane ? carry + left : carry, total = 0.f;
 #pragma unroll
       for (int w = 0; w < kDecWarps; ++w) {
         if (w < warp) before += s_scan[w];
@@ -488,8 +490,9 @@ __global__ void __launch_bounds__(256) fox_decode_merge_kernel(const DecodeParam
         const float x = __shfl_up_sync(0xffffffffu, incl, o);
         if (tid >= o) incl += x;
       }
+      const float left = __shfl_up_sync(0xffffffffu, incl, 1);   // (as for the keys' biases)
       if (s >= 0) {
-        const float mm = s_w[s] + after + incl - g;
+        const float mm = g > -INFINITY ? s_w[s] + after + incl - g : s_w[s] + after + (tid ? left : 0.f);
         s_w[s] = mm;
         top = fmaxf(top, mm);
       }

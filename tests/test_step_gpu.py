@@ -308,3 +308,24 @@ def test_token_whose_gate_forgets_everything(N, route, padded):
         assert torch.equal(res[0].isfinite(), res[1].isfinite())
         a, b = res[0].nan_to_num(0, 0, 0), res[1].nan_to_num(0, 0, 0)
         assert (a - b).norm() <= 2 ** -6 * b.norm(), last
+
+
+@pytest.mark.parametrize("N,D", [(2, 64), (130, 16), (1500, 128), (5000, 64), (30000, 64)])
+@pytest.mark.parametrize("at", [1, 2, 5, 70, 1100])
+def test_decode_from_gates_behind_one_of_minus_infinity(N, D, at):
+    """The key at whose gate everything is forgotten, and those behind it, share the row; the keys before it have no weight,
+    in the same range, tile and thread or in others.  Tolerance as for finite gates."""
+    g = torch.Generator().manual_seed(N + at)
+    at = min(at, N)
+    q, k, v = [torch.randn(1, 2, t, D, generator=g).bfloat16().cuda() for t in (1, N, N)]
+    lf = torch.nn.functional.logsigmoid(torch.randn(1, 2, N, generator=g) + 3).cuda()
+    lf[:, 0, N - at] = float("-inf")
+    with torch.no_grad():
+        out = fox.forgetting_attention(q, k, v, lf, head_first=True)
+    for h, n in ((0, at), (1, N)):
+        lam = lf[0, h, N - n + 1:].double().flip(0).cumsum(0).flip(0)
+        s = k[0, h, N - n:].double() @ q[0, h, 0].double() / D ** 0.5
+        s[:-1] += lam
+        ref = s.softmax(0) @ v[0, h, N - n:].double()
+        err = (out[0, h, 0].double() - ref).abs()
+        assert (err <= 2 ** -8 * ref.abs() + 2 ** -8 * ref.pow(2).mean().sqrt()).all(), (h, err.max().item())
