@@ -384,7 +384,7 @@ constexpr int kDq2BN = 128;
 enum Dq2WaitSite { kDq2SiteQ = 51, kDq2SiteK = 52, kDq2SiteV = 53, kDq2SiteKE = 54, kDq2SiteVE = 55, kDq2SiteS = 56,
                    kDq2SiteDP = 57, kDq2SiteDS = 58, kDq2SiteDone = 59, kDq2SiteNegB = 60, kDq2SiteRow = 61, kDq2SiteEpi = 62, kDq2SiteItem = 63 };
 
-template <int D, bool kBf16>
+template <int D, bool kBf16, bool kLoop>
 __global__ void __launch_bounds__(576, 1)
 fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -462,7 +462,7 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     mbar_init(&bar_epi_free, 1);
     mbar_init(&bar_q_free, 1);
     for (int i = 0; i < 3; ++i) mbar_init(&bar_negb[i], 1);
-    items_init(items, 17);
+    if constexpr (kLoop) items_init(items, 17);
     mbar_fence_init();
   }
   if (warp == kTmaWarp) {
@@ -507,11 +507,14 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     };
     bool ok = true;
     uint32_t item = 0, asked = 0;
-    for (int i = blockIdx.x; i >= 0 && ok;) {
+    auto ask = [&]() {
       ok = items_ask(items, item, abortp, p.status, kDq2SiteItem);
-      if (!ok) break;
-      ++asked;
+      if (ok) ++asked;
+      return ok;
+    };
+    for (int i = blockIdx.x; i >= 0 && ok;) {
       const Item x = item_of(i);
+      if (kLoop && x.n <= kAskTiles && !ask()) break;
       if (x.n > 0) {
         ok = mbar_wait_warp(&bar_q_free, (q_loads & 1) ^ 1, abortp, p.status, kDq2SiteQ, i);
         if (!ok) break;
@@ -548,6 +551,7 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       for (int it = 0; it < x.n; ++it, ++pos, ++tiles) {
         const int nb = x.nb_hi - 1 - it;
         const uint32_t ks = pos % kKS;
+        if (kLoop && it > 0 && it == x.n - kAskTiles && !ask()) break;
         ok = mbar_wait_warp(&bar_k_empty[ks], ((pos / kKS) & 1) ^ 1, abortp, p.status, kDq2SiteKE, it);
         if (!ok) break;
         if (elect_one()) {
@@ -585,6 +589,7 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       out_b = x.b;
       out_st = pos % kKS;
       ++pos;
+      if constexpr (!kLoop) break;
       i = items_next(items, item++, true, abortp, p.status, kDq2SiteItem);
     }
     if (ok) ok = store();
@@ -693,7 +698,8 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           ++done;
         }
         ++pos;   // (the stage of the item's dQ)
-      i = items_next(items, item++, false, abortp, p.status, kDq2SiteItem);
+        if constexpr (!kLoop) break;
+        i = items_next(items, item++, false, abortp, p.status, kDq2SiteItem);
       }
     }
   } else {
@@ -821,7 +827,8 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       ++epilogues;
       if (g == 0 && row_ok) p.dlam_row[x.bh * M + row] = rowsum;
     }
-      i = items_next(items, item++, false, abortp, p.status, kDq2SiteItem);
+    if constexpr (!kLoop) break;
+    i = items_next(items, item++, false, abortp, p.status, kDq2SiteItem);
     }
   }
 
@@ -883,12 +890,13 @@ static int launch_dq2(int device, cudaStream_t stream, int64_t B, int64_t H, int
   if (!tma_compatible(tdq, 2)) return FOX_ERR_ALIGNMENT;
   if ((rc = cached_tmap_4d(&tmDQ, tdq, 2, false, kBf16, 64, 128, true))) return rc;
   constexpr int smem = 2 * 128 * D * 2 + 4 * kDq2BN * D * 2 + 1024;
-  auto kern = fox_attn_bwd_dq2_kernel<D, kBf16>;
-  static bool configured[64] = {};
+  const bool loop = prm.items > kSms;   // (else every CTA has begun: there is none to ask for)
+  auto kern = loop ? fox_attn_bwd_dq2_kernel<D, kBf16, true> : fox_attn_bwd_dq2_kernel<D, kBf16, false>;
+  static bool configured[2][64] = {};
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;
-  if (!configured[device]) {
+  if (!configured[loop][device]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
-    configured[device] = true;
+    configured[loop][device] = true;
   }
   kern<<<(unsigned)prm.items, 576, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, prm);
   return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;

@@ -198,13 +198,14 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     };
     bool ok = true;
     uint32_t item = 0, asked = 0;
+    auto ask = [&]() {
+      ok = items_ask(items, item, abortp, p.status, kKvSiteItem);
+      if (ok) ++asked;
+      return ok;
+    };
     for (int i = blockIdx.x; i >= 0 && ok;) {
-      if constexpr (kLoop) {
-        ok = items_ask(items, item, abortp, p.status, kKvSiteItem);
-        if (!ok) break;
-        ++asked;
-      }
       const Item x = item_of(i);
+      if (kLoop && x.n <= kAskTiles && !ask()) break;
       if (x.n > 0) {
         ok = mbar_wait_warp(&bar_kv_free, (kv_loads & 1) ^ 1, abortp, p.status, kKvSiteKV, i);
         if (!ok) break;
@@ -251,6 +252,7 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       for (int it = 0; it < x.n; ++it, ++pos, ++tiles) {
         const int i0 = (x.hb_lo + it) * BM;
         const uint32_t st = pos & 1, ph = ((st ? taken1 : taken0) & 1) ^ 1;
+        if (kLoop && it > 0 && it == x.n - kAskTiles && !ask()) break;
         ok = mbar_wait_warp(&bar_q_empty[st], ph, abortp, p.status, kKvSiteQE, it);
         if (!ok) break;
         if (elect_one()) {
@@ -582,7 +584,7 @@ static int launch_kv(int device, cudaStream_t stream, int64_t B, int64_t H, int6
   if ((rc = cached_tmap_4d(&tmDK, tdk, 2, false, kBf16, 64, kKvBN, true))) return rc;
   if ((rc = cached_tmap_4d(&tmDV, tdv, 2, false, kBf16, 64, kKvBN, true))) return rc;
   constexpr int smem = (2 * 2 + 2) * 128 * D * 2 + 1024;   // Q, dO in two stages each, K, V
-  const bool loop = prm.end_index != nullptr;   // (see the head of this file)
+  const bool loop = prm.end_index != nullptr && prm.items > kSms;   // (see the head of this file)
   auto kern = loop ? fox_attn_bwd_kv_kernel<D, kBf16, true> : fox_attn_bwd_kv_kernel<D, kBf16, false>;
   static bool configured[2][64] = {};
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;

@@ -648,8 +648,9 @@ def test_pruning_indices_by_search_and_by_scan(M, N, bm, bn, kind):
 @pytest.mark.parametrize("M,N", [(2500, 2500), (1000, 3001), (129, 2560)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_pruned_backward_tiles_walked_by_a_cta_equal_tiles_of_their_own(M, N, dtype):
-    """The pruned D=128 backward walks its tiles, more than 148 here, with 148 CTAs: bit-identical to a call for each (b,h),
-    whose tiles have a CTA each.  Padding leaves a batch element without any key for most tiles and one with only its last."""
+    """A CTA of the pruned D=128 backward goes on with tiles of CTAs that have not begun where there are more tiles than the
+    148 that begin at once.  Bit-identical to a call for each (b,h), whose CTAs have one tile each, and within the oracle's bars.
+    Padding leaves a batch element without any key for most tiles and one with only its last."""
     B, H = 3, 5
     q, k, v, lf, do = _inputs(M + N, B, H, M, N, 128, dtype, mu=1.0, sigma=2.0)
     lf[:, 3] = 0.0                                                  # (a head that nothing is pruned of)
@@ -661,3 +662,17 @@ def test_pruned_backward_tiles_walked_by_a_cta_equal_tiles_of_their_own(M, N, dt
             part = _run(*[t[b:b + 1, h:h + 1] for t in (q, k, v, lf, do)], seq=seq[b:b + 1], thr=-12.0)
             for name, x, y in zip(("out", "dq", "dk", "dv", "dlog_fgate"), whole, part):
                 assert torch.equal(x[b, h], y[0, 0]), (name, b, h)
+            if h in (0, 3) and b != 1:
+                thr = np.full((1, 1), -12.0, dtype=np.float32)
+                si, ei = (f(part.lam.numpy(), thr, M, N, 128, 128) for f in (orc.find_start_index, orc.find_end_index))
+                _check_bf16(part, *[t[b:b + 1, h:h + 1] for t in (q, k, v, lf, do)], seq=seq[b:b + 1], start_index=si, end_index=ei)
+
+
+@pytest.mark.parametrize("B,H,M,N", [(2, 5, 2048, 2048), (1, 19, 2000, 2048), (4, 37, 128, 300), (1, 149, 100, 100)])
+def test_backward_that_could_prune_equals_one_that_cannot(B, H, M, N):
+    """A threshold that prunes nothing sends the D=128 backward over the same tiles as no threshold: the key side with CTAs that
+    go on with further tiles against one CTA a tile, few and many tiles of up to 16 steps.  Bit-identical gradients."""
+    args = _inputs(M + H, B, H, M, N, 128, torch.bfloat16, mu=4.0)
+    seq = torch.arange(B) * (N // 5)
+    for name, a, b in zip(("out", "dq", "dk", "dv", "dlog_fgate"), _run(*args, seq=seq, thr=-1e9), _run(*args, seq=seq)):
+        assert torch.equal(a, b), name
