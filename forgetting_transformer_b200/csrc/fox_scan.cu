@@ -252,11 +252,12 @@ __device__ __forceinline__ int block_running_max(int v, int carry, int* red, int
 // condition holds.  Where the staged prefix never rises (every log gate is at most 0), neither does a row's difference to a
 // later column fall, so that the condition fails from one column on and the carried scan is the running maximum of searches
 // that begin at 0: a thread takes a row, by bisection.  The comparisons are the same ones on the same values, so the arrays
-// are bit-identical.  A prefix that rises or is NaN somewhere, or a threshold that no column of some row stops at, goes through
+// are bit-identical.  A prefix that rises or is NaN somewhere, a threshold that no column of some row stops at, or few blocks go through
 // the carried scan itself, 32 blocks at a time by one warp (0: start_index (B,H,ceil(M/BM)); 1: end_index (B,H,ceil(N/BN))),
 // bound by its dependent steps:
 // 64 (b,h) of 128 x 128 blocks take 37-40 us by the scan and 6.6 by the searches.
 constexpr int kIndexThreads = 128;
+constexpr int kIndexScan = 4;   // up to so many blocks the scan is shorter than the searches' barriers (2 x 2: 2.8 us against 3.7)
 __global__ void __launch_bounds__(kIndexThreads)
 fox_find_index_kernel(const IndexParams p) {
   extern __shared__ float sm[];
@@ -292,13 +293,17 @@ fox_find_index_kernel(const IndexParams p) {
   __syncthreads();
   int64_t* start = p.start ? p.start + static_cast<int64_t>(bh) * nmb : nullptr;
   int64_t* end = p.end ? p.end + static_cast<int64_t>(bh) * nnb : nullptr;
-  bool falling = t == t && col_last[0] == col_last[0];
-  for (int i = threadIdx.x; i + 1 < nnb; i += blockDim.x) falling = falling && col_last[i + 1] <= col_last[i];
-  for (int i = threadIdx.x; i < nmb; i += blockDim.x) {
-    falling = falling && row_e[i + 1] <= row_e[i] && row_first[i] == row_first[i];
-    falling = falling && !(row_first[i] - col_last[nnb - 1] < t);   // (some column stops every row)
+  bool falling = false;
+  if (max(nmb, nnb) > kIndexScan) {
+    falling = t == t && col_last[0] == col_last[0];
+    for (int i = threadIdx.x; i + 1 < nnb; i += blockDim.x) falling = falling && col_last[i + 1] <= col_last[i];
+    for (int i = threadIdx.x; i < nmb; i += blockDim.x) {
+      falling = falling && row_e[i + 1] <= row_e[i] && row_first[i] == row_first[i];
+      falling = falling && !(row_first[i] - col_last[nnb - 1] < t);   // (some column stops every row)
+    }
+    falling = __syncthreads_and(falling);
   }
-  if (__syncthreads_and(falling)) {
+  if (falling) {
     if (start) {
       int carry = 0;
       for (int m0 = 0; m0 < nmb; m0 += kIndexThreads) {

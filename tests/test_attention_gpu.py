@@ -624,11 +624,12 @@ def test_weights_are_relative_to_the_maximum_of_the_nearest_128_keys(D, dtype):
 
 
 @pytest.mark.parametrize("M,N,bm,bn", [(1, 1, 128, 128), (128, 128, 128, 128), (129, 700, 128, 128), (5000, 5000, 32, 32),
-                                       (4096, 20000, 32, 128), (17000, 17000, 128, 128)])
+                                       (4096, 20000, 32, 128), (17000, 17000, 128, 128),
+                                       (512, 512, 128, 128), (513, 640, 128, 128)])
 @pytest.mark.parametrize("kind", ["falling", "flat", "rising in places", "minus infinity"])
 def test_pruning_indices_by_search_and_by_scan(M, N, bm, bn, kind):
-    """fox_find_index on prefixes that never rise (searched) and on others (upstream's carried scan), more blocks than threads,
-    single blocks and ragged ends: bit-identical to the restated scans."""
+    """fox_find_index on prefixes that never rise (searched, above four blocks) and on others (upstream's carried scan), more blocks than
+    threads, single blocks and ragged ends: bit-identical to the restated scans."""
     g = torch.Generator().manual_seed(M + N)
     gates = torch.nn.functional.logsigmoid(torch.randn(2, 3, N, generator=g) * 2)
     if kind == "flat":
