@@ -701,9 +701,21 @@ extern "C" int fox_bwd_finish(int device, void* stream, int dtype, int64_t B, in
 extern "C" int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D) {
   const int64_t rows_per_block = kScanThreads / (D / 8);
   int64_t n = (T + rows_per_block - 1) / rows_per_block;
-  const int64_t per_unit = (148 * 2) / (B * H) > 0 ? (148 * 2) / (B * H) : 1;
+  const int64_t per_unit = (kSms * 2) / (B * H) > 0 ? (kSms * 2) / (B * H) : 1;
   n = n < per_unit ? n : per_unit;
   return n < 32 ? n : 32;
+}
+
+// The same for keys alone, whose blocks share a launch with those of the prefix scans, one a (b,h).  Where fewer parts make the
+// two resident blocks per SM one wave, nearly full, that is faster than a few blocks in a second wave (48 (b,h) of 16384 x 64:
+// 36 -> 30 us; 24 of 11000 x 64: 16 -> 13), unless the parts left have to be much longer: 2 -> 1 part never (148 of 4096 x 128:
+// 42 -> 51), 3 -> 2 not with long rows in many (96 of 8192 x 128: 49 -> 53, of 4096 29 -> 28), and from four on it needs
+// a fuller wave (70 of 4096 x 128, 280 blocks: 20 -> 22; 71, 284 blocks: 22.3 -> 21.6).
+extern "C" int64_t fox_key_norm_parts(int64_t B, int64_t H, int64_t N, int64_t D) {
+  const int64_t n = fox_norm_parts(B, H, N, D), bh = B * H, places = 2 * kSms, fewer = places / bh - 1, blocks = (fewer + 1) * bh;
+  if (fewer >= n) return n;
+  const bool full = blocks >= places - (fewer >= 4 ? 16 : 12);
+  return full && (fewer >= 3 || (fewer == 2 && (N <= 4096 || D <= 64))) ? fewer : n;
 }
 
 extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M,

@@ -97,15 +97,11 @@ int64_t attn_blocks(int64_t n) { return (n + kBlock - 1) / kBlock; }
 // largest key norm per (b,h): the forward kernel's bound that lets most tiles skip the row-maximum pass
 AttnNorms attn_norms(const AttnShape& s, bool is_auto) {
   AttnNorms n;
-  if ((s.N >= 8 * kBlock && s.M > 1) || is_auto) n.n_k = fox_norm_parts(s.B, s.H, s.N, s.D);
   if (is_auto) {
+    n.n_k = fox_norm_parts(s.B, s.H, s.N, s.D);
     n.n_q = fox_norm_parts(s.B, s.H, s.M, s.D);
-  } else if (n.n_k > 1) {
-    // The blocks of the prefix scans share the launch: where fewer parts make the two resident blocks per SM one wave, nearly
-    // full, that is faster than a few blocks in a second one (48 (b,h) of 16384 x 64: 36 -> 30 us; 24 of 11000 x 64: 16 -> 13).
-    // 64 (b,h) of 16384 x 128 would leave 40 places empty (72 -> 80 us) and keep their parts.
-    const int64_t bh = s.B * s.H, one_wave = 296 / bh - 1;
-    if (one_wave >= 1 && one_wave < n.n_k && (1 + one_wave) * bh >= 280) n.n_k = one_wave;
+  } else if (s.N >= 8 * kBlock && s.M > 1) {
+    n.n_k = fox_key_norm_parts(s.B, s.H, s.N, s.D);
   }
   return n;
 }

@@ -116,8 +116,10 @@ int fox_max_row_norm(int device, void* stream, int dtype, int64_t B, int64_t H, 
 
 /* What the operator needs before its forward kernel, in one launch: the prefix sum of the gates (fox_cumsum_fwd /
  * fox_gate_prefix_fwd; gate_kind FOX_GATE_LOG or the dtype of gate logits) and, where k (q) is given, the largest row norm of
- * every (b,h) as n partial maxima, k_parts (B,H,n_k_parts), fully written; n from fox_norm_parts, <= 32. */
+ * every (b,h) as n partial maxima, k_parts (B,H,n_k_parts), fully written; n from fox_norm_parts, or for k without q from
+ * fox_key_norm_parts, <= 32. */
 int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D);
+int64_t fox_key_norm_parts(int64_t B, int64_t H, int64_t N, int64_t D);
 int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M, int64_t N,
                       int64_t D, const void* gates, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
                       float* log_lambda, const fox_tensor4* k, float* k_parts, int64_t n_k_parts, const fox_tensor4* q,
