@@ -38,6 +38,9 @@ constexpr int kStepThreads = 256, kStepWarps = 8;
 constexpr int kStepAhead = 8;    // blocks of 32 columns a warp has in flight
 constexpr int kStepMats = 7;
 constexpr uint32_t kStepChunk = 4096;         // bytes of one request for what a later product reads
+// The most that is asked for ahead: of more, L2 (126 MB) holds too little until it is read (2048 channels, intermediate size 16384,
+// 67 MB: 82 us a layer, without 88; 24576, 100 MB: 125 and 124; 32768, 134 MB: 139 and 135).
+constexpr int64_t kStepAheadMost = 96 << 20;
 constexpr int kStepEarly = 296;               // CTAs that request the first product's weights
 // Input and weights of a CTA that may lie in shared memory together; more goes through registers.  (16 sequences of 1536 channels:
 // the gate product would need 99 KB, and a layer takes 126 us so, 114 through registers; 2 sequences' down product, 83 KB: 59
@@ -522,6 +525,7 @@ static int step_product(int device, void* stream, int dtype, int input, int outp
   if (align % 16) return FOX_ERR_ALIGNMENT;
   if (ahead && (reinterpret_cast<uintptr_t>(ahead) % 16 || ahead_bytes < 0 || ahead_bytes % 16)) return FOX_ERR_ALIGNMENT;
   p.ahead = (const char*)ahead;
+  if (ahead_bytes > kStepAheadMost) p.ahead = nullptr;
   p.ahead_bytes = (uint64_t)ahead_bytes;
   p.status = status;
   p.n_mats = (int)n_mats; p.B = (int)B; p.K = (int)K; p.D = (int)D;

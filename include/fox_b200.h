@@ -293,7 +293,8 @@ int fox_step_product(int device, void* stream, int dtype, int input, int output,
                      int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
                      const void* residual, void* out, int64_t ldo);
 /* The same with the weights through shared memory where they fit; while it waits for its input it asks for an array that a
- * later kernel reads (16-byte aligned, a multiple of 16 bytes, or NULL) to be brought into L2.  status: as fox_attn_fwd. */
+ * later kernel reads (16-byte aligned, a multiple of 16 bytes, or NULL) to be brought into L2, unless it is larger than 96 MB.
+ * status: as fox_attn_fwd. */
 int fox_step_product_ahead(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K, const void* x,
                            int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D, const float* gate,
                            int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
