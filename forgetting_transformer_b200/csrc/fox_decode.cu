@@ -39,6 +39,7 @@ constexpr int kDecMaxSplits = 1024;   // taken
 constexpr int kDecMostSplits = 512;   // asked for by fox_attn_decode_splits
 constexpr int64_t kDecSlots = 444, kDecClusterSlots = 400;                            // CTAs of a wave
 constexpr int64_t kDecStartKeys = 600, kDecMergeKeys = 120, kDecLeastKeys = 128;      // (at fox_attn_decode_splits)
+constexpr int64_t kDecLongRange = 1024 * 64, kDecManyClusters = 384;   // keys times head dim; CTAs (at long_ranges)
 constexpr float kDecLog2e = 1.4426950408889634f;
 
 struct DecodeParams {
@@ -530,20 +531,38 @@ __global__ void __launch_bounds__(256) fox_decode_merge_kernel(const DecodeParam
   if (tid == 0) p.L[bh] = s_sum > 0.f ? s_top * 0.6931471805599453f + __logf(s_sum) : -INFINITY;
 }
 
+// A launch that begins while a product with much shared memory ends would find next to no L1, which its loads in flight need
+// (see fox_step.cu); one with long ranges waits for SMs that it can split anew.  Short ones are over before that pays: 24 (b,h) of
+// 250 keys a range 32.5 us a layer, 33.8 so; 192 of 2000 97 and 89, of 6000 178 and 148; 96 of 10000 235 and 185.  (Head dims
+// 16 and 32 are bound by their instructions: 160 of 6000 keys 48 and 50.)  Clusters that need nearly every place of their wave, and
+// those of eight, find them too late then: 80 x 5 of 2400 keys a range 82 and 88, 48 x 8 of 750, head dim 128, 92 and 99.
+static int long_ranges(cudaLaunchAttribute* attr, const DecodeParams& p, int64_t B, int D) {
+  const int64_t ctas = B * p.H * p.splits;
+  if (D < 64 || static_cast<int64_t>(p.N) * D < static_cast<int64_t>(p.splits) * kDecLongRange) return 0;
+  if (p.splits > 1 && (p.splits == kDecMaxCluster || (p.splits < kDecMaxCluster && ctas > kDecManyClusters && ctas <= kDecSlots))) return 0;
+  attr->id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attr->val.sharedMemCarveout = 20;   // (three CTAs' 9 to 12 KB of 228)
+  return 1;
+}
+
 template <bool kBf16, int D>
 static int launch_step(const DecodeParams& p, const DecodeStep& step, int64_t B, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.splits, (unsigned)p.H, (unsigned)B);
   cfg.blockDim = dim3(kDecThreads);
   cfg.stream = st;
-  cudaLaunchAttribute attrs[2] = {};
+  cudaLaunchAttribute attrs[3] = {};
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[0].val.programmaticStreamSerializationAllowed = 1;
-  attrs[1].id = cudaLaunchAttributeClusterDimension;
-  attrs[1].val.clusterDim.x = (unsigned)p.splits;
-  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  int n = 1 + long_ranges(&attrs[1], p, B, D);
+  if (p.splits > 1) {
+    attrs[n].id = cudaLaunchAttributeClusterDimension;
+    attrs[n].val.clusterDim.x = (unsigned)p.splits;
+    attrs[n].val.clusterDim.y = attrs[n].val.clusterDim.z = 1;
+    ++n;
+  }
   cfg.attrs = attrs;
-  cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true, true>, p, step) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 
@@ -553,11 +572,12 @@ static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
   cfg.gridDim = dim3((unsigned)p.splits, (unsigned)p.H, (unsigned)B);
   cfg.blockDim = dim3(kDecThreads);
   cfg.stream = st;
-  cudaLaunchAttribute attrs[2] = {}, attr{};
+  cudaLaunchAttribute attrs[3] = {}, attr{};
   int n = 0;
   if (p.pdl) {
     attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attrs[n++].val.programmaticStreamSerializationAllowed = 1;
+    n += long_ranges(&attrs[n], p, B, D);
   }
   cfg.attrs = attrs;
   if (p.splits <= kDecMaxCluster) {

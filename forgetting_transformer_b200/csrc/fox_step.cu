@@ -29,6 +29,8 @@
 // one start only after its own wait: a kernel's early reads then come after everything in front of its predecessor has
 // ended.  The first product follows a kernel of someone else's, which may have written the weights, and copies them after
 // the wait; what it asks for before is only brought into L2, where a later write still finds it.
+#include <algorithm>
+
 #include "fox_common.cuh"
 #include "fox_host.h"
 
@@ -47,6 +49,12 @@ constexpr int kStepEarly = 296;               // CTAs that request the first pro
 // and 61 us a layer.)
 constexpr size_t kStepSmem = 88 * 1024;
 constexpr int kStepWaitSite = 91;
+constexpr int64_t kSmSmem = 228 * 1024;       // of an SM
+constexpr int64_t kStepStatic = 10 * 1024;    // of a CTA beside input and weights: the sums' arrays and the system's share
+// A down product of so many weights, through registers behind a gate product through shared memory, waits for SMs with room for
+// its loads in L1 if its inputs leave a fifth (a layer of 2048 channels, intermediate size 16384: 82 -> 64 us, two sequences 88 ->
+// 71, five, whose inputs leave none, 113 -> 118; 12288: 66 -> 56; of 5632 the wait costs more than it gives: five 64.5 -> 67.8).
+constexpr int64_t kStepBigWeights = 16 << 20;
 
 enum StepInput { kInRms = 0, kInGated = 1, kInPlain = 2 };
 enum StepOutput { kOutFp32 = 0, kOutAdd16 = 1, kOutSwiglu = 2, kOutAdd32 = 3 };
@@ -469,6 +477,18 @@ static cudaLaunchConfig_t pdl_config(dim3 grid, int threads, size_t smem, cudaSt
   return cfg;
 }
 
+// Shared memory and L1 are one array per SM, split anew only while the SM is empty; kernels that begin early keep it from
+// that.  Left to itself the runtime gives these products all of it, and the attention behind them no room for its loads in flight
+// (48 (b,h) of 40000 keys 114 us, 78 behind products through registers).  Long attention asks for a split of its own
+// (fox_decode.cu).  The products do, all of a layer for the same, where the gate product's CTAs, as many to an SM as of the first
+// product, need no more than half: 16 sequences of 512 channels 35 -> 31 us a layer, one of 768 16.5 -> 15.4.  Above that it
+// takes the overlap of one product with the next: 16 of 1536 81 -> 92, one of 1024 19.8 -> 20.2.
+static size_t step_x_bytes(int64_t B, int64_t K) { return static_cast<size_t>(B) * ((K / 8 + 7) / 8 * 8 + 4) * 16; }
+static int step_carveout(int64_t ctas, int64_t bytes) {
+  return static_cast<int>(std::min<int64_t>((ctas * bytes * 100 + kSmSmem - 1) / kSmSmem, 100));
+}
+static int64_t step_per_sm(int64_t grid) { return std::min<int64_t>((grid + kSms - 1) / kSms, 4); }   // (4 by registers)
+
 template <bool kBf16, int kIn, int kOut, bool kSmem>
 static int launch_product(int device, cudaStream_t st, const StepParams& p, size_t smem) {
   auto kern = fox_step_product_kernel<kBf16, kIn, kOut, kSmem>;
@@ -478,13 +498,25 @@ static int launch_product(int device, cudaStream_t st, const StepParams& p, size
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return FOX_ERR_LAUNCH;
     configured[device] = true;
   }
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = pdl_config(dim3((unsigned)p.tile0[p.n_mats]), kStepThreads, smem, st, &attr);
+  cudaLaunchAttribute attrs[2] = {};
+  cudaLaunchConfig_t cfg = pdl_config(dim3((unsigned)p.tile0[p.n_mats]), kStepThreads, smem, st, attrs);
+  attrs[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  if (kSmem) {
+    const int64_t C = kIn == kInPlain ? p.rows[0] : p.K;
+    const int64_t gate = static_cast<int64_t>(step_x_bytes(p.B, C)) + 16 * step_row_bytes(static_cast<int>(C)) + kStepStatic;
+    const int share = step_carveout(step_per_sm(C / 2), gate);
+    attrs[1].val.sharedMemCarveout = share;
+    if (share <= 50) cfg.numAttrs = 2;
+  } else if (kIn == kInPlain && p.status && p.rows[0] * static_cast<int64_t>(p.K) >= kStepBigWeights) {
+    const int share = step_carveout(step_per_sm(p.tile0[p.n_mats]), static_cast<int64_t>(smem) + kStepStatic);
+    attrs[1].val.sharedMemCarveout = share;
+    if (share <= 80) cfg.numAttrs = 2;
+  }
   return cudaLaunchKernelEx(&cfg, kern, p) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 template <bool kBf16, int kIn, int kOut>
 static int choose_product(int device, cudaStream_t st, const StepParams& p) {
-  const size_t x = static_cast<size_t>(p.B) * ((p.K / 8 + 7) / 8 * 8 + 4) * 16;
+  const size_t x = step_x_bytes(p.B, p.K);
   const size_t w = static_cast<size_t>(kOut == kOutSwiglu ? 16 : 8) * step_row_bytes(p.K);
   if (x > 200 * 1024) return FOX_ERR_TOO_LARGE;
   return p.status && x + w <= kStepSmem ? launch_product<kBf16, kIn, kOut, true>(device, st, p, x + w)

@@ -204,7 +204,8 @@ def test_block_under_checkpointing(reentrant):
 
 
 @pytest.mark.parametrize("B,C,H,I,N", [(1, 512, 8, 1408, 2001), (3, 256, 2, 512, 1030), (1, 256, 4, 512, 6400), (16, 1536, 24, 4096, 40),
-                                       (16, 512, 32, 512, 70), (2, 768, 48, 544, 129)])
+                                       (16, 512, 32, 512, 70), (2, 768, 48, 544, 129), (16, 512, 8, 512, 3100),
+                                       (16, 512, 4, 512, 3100), (2, 2048, 16, 512, 5000), (1, 768, 6, 512, 4500)])
 @pytest.mark.parametrize("case", ["plain", "padded", "nothing valid", "states off 16 bytes"])
 def test_token_through_every_route(B, C, H, I, N, case):
     """One token by each of the step's routes: keys in 1 to 8 ranges merged by a cluster, in more or in more CTAs than a wave by
