@@ -715,7 +715,10 @@ Tensor step(const Block& b, const Tensor& x_in, const Tensor& mask, const CacheL
   const AttnShape as{n, H, 1, N, D};
   uintptr_t bits = 0;   // (fox_step_attn takes 16-byte pieces of states and cache; the two kernels take any state)
   for (const Tensor* t : {&c.k, &c.v, &c.k_state, &c.v_state}) bits |= reinterpret_cast<uintptr_t>(t->data_ptr());
-  const int64_t splits = bits % 16 ? 0 : fox_step_attn_splits(n, H, N);
+  int64_t splits = bits % 16 ? 0 : fox_step_attn_splits(n, H, N);
+  // Long ranges at head dim 128 are faster by the two kernels, except one or two CTAs to an SM (16 heads, one sequence of 6000 keys
+  // 61 and 58 us a layer, two 70 and 78, three 93 and 91, eight of 2000 110 and 103, of 12000 219 and 205; one of 2000 49 and 50).
+  if (D == 128 && N > splits * 512 && (n * H * splits < kSms || n * H * splits > 2 * kSms)) splits = 0;
   const int64_t ld = (4 * C + 3 * H + 3) / 4 * 4;
   Tensor memory;
   float *y, *z, *L, *work;

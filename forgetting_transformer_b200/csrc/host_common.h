@@ -25,6 +25,8 @@ namespace foxh {
 
 using at::Tensor;
 
+constexpr int64_t kSms = 148;
+
 // Python exceptions from code that may run without the interpreter lock (the autograd engine's threads among it).
 [[noreturn]] void raise_assert(const std::string& msg);   // AssertionError, as the Python mirror's asserts
 [[noreturn]] void raise_fox(const std::string& msg);      // forgetting_transformer_b200.FoxError
