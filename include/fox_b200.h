@@ -287,7 +287,9 @@ int fox_column_sums(int device, void* stream, int64_t n, const float* const* par
  * fox_step_product: out = f(in(x) W^T) for up to 7 contiguous 16-bit matrices (mat_rows[i], K), K a multiple of 32, their
  * outputs side by side.  input 0: rmsnorm(x) norm_w, x (B,K) 16-bit or (x_fp32) fp32; 1: per-head rmsnorm(x) norm_w
  * sigmoid(gate), head dim D, gate fp32 with row stride gate_ld; 2: x.  output 0: fp32 (B,ldo); 1: fp32, + residual
- * (16-bit); 2: silu(first half) * second half of one matrix's rows, 16-bit; 3: 16-bit, + residual (fp32). */
+ * (16-bit); 2: silu(first half) * second half of one matrix's rows, 16-bit; 3: 16-bit, + residual (fp32).  All but input 0 with
+ * output 0 read the matrices, fox_step_product_ahead norm_w too, before they wait for the launch in front, which may not write
+ * them. */
 int fox_step_product(int device, void* stream, int dtype, int input, int output, int64_t B, int64_t K, const void* x,
                      int x_fp32, const void* norm_w, int norm_w_dtype, float eps, int64_t D, const float* gate,
                      int64_t gate_ld, int64_t n_mats, const void* const* mats, const int64_t* mat_rows,
@@ -311,8 +313,11 @@ int fox_step_mix(int device, void* stream, int dtype, int64_t B, int64_t H, int6
                  void* v_cache, float* g_cache, int64_t capacity, int64_t pos);
 
 /* fox_step_mix and the attention behind it in one kernel: arguments of the first, o (B,H,D) 16-bit contiguous, the keys of a
- * (b,h) in `splits` (1 to 8) ranges that a cluster merges.  fox_step_attn_splits: how many, or 0 where the two calls are
- * the better way. */
+ * (b,h) in `splits` (1 to 8) ranges that a cluster merges.  It begins while the launch in front of it on the stream ends, and
+ * reads mask, states, caches, norm weights and bias before it waits for that one: the launch in front has to be the
+ * fox_step_product or fox_step_product_ahead that writes y, and all of those have to be written by launches or copies in front
+ * of that product.  (fox_step_mix reads everything but norm weights and bias behind its wait.)  fox_step_attn_splits: how many
+ * ranges, or 0 where the two calls are the better way. */
 int fox_step_attn(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t D, const float* y, int64_t ld,
                   const void* wq, int wq_dtype, const void* wk, int wk_dtype, float eps, const void* bias, int bias_dtype,
                   const int64_t* mask, void* k_state, void* v_state, void* k_cache, void* v_cache, float* g_cache,
