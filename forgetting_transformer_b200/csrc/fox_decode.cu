@@ -613,6 +613,7 @@ using namespace fox;
 // head dim 64 in 25 ranges 81.4 us, in 18 67.2; 48 x 8192 25.7 -> 22.6; 192 x 2048 26.2 -> 22.0; 72 x 5000 of 128 41.3 -> 36.1.
 extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
   const int64_t bh = B * H;
+  if (bh <= 0) return 1;   // (fox_attn_decode refuses such a call)
   auto fit = [&](int64_t waves) {
     const int64_t s = waves * kDecSlots / bh;
     return s > kDecMaxCluster ? s : waves * kDecClusterSlots / bh > 1 ? waves * kDecClusterSlots / bh : int64_t{1};
@@ -697,7 +698,7 @@ extern "C" int fox_attn_decode_gates(int device, void* stream, int dtype, int64_
 // the two launches more (24 heads of 8000 keys 105 and 101 us).
 extern "C" int64_t fox_step_attn_splits(int64_t B, int64_t H, int64_t N) {
   const int64_t s = fox_attn_decode_splits(B, H, N);
-  if (B * H * s > kDecSlots) return 0;
+  if (B <= 0 || H <= 0 || B * H * s > kDecSlots) return 0;
   return s <= kDecMaxCluster ? s : N <= 8 * 768 ? 8 : 0;
 }
 

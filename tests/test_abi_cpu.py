@@ -231,3 +231,11 @@ def test_key_norm_parts_fill_a_wave_and_stay_short(bh, n, d):
     if parts < most:
         assert 280 <= (1 + parts) * bh <= 296 and parts >= 2 and (parts >= 3 or n <= 4096 or d <= 64)
     assert bh not in (70, 140, 147, 148) or parts == most
+
+
+def test_sizes_for_calls_without_batch_or_heads():
+    """What the C interface says about launches for no (b,h) at all is an answer, not a division by zero."""
+    lib = _lib.load()
+    for b, h in ((0, 4), (4, 0), (0, 0)):
+        assert lib.fox_attn_decode_splits(b, h, 100) == 1 and lib.fox_step_attn_splits(b, h, 100) == 0
+        assert lib.fox_norm_parts(b, h, 2048, 64) == lib.fox_key_norm_parts(b, h, 2048, 64) == 1
