@@ -43,7 +43,7 @@ constexpr uint32_t kStepChunk = 4096;         // bytes of one request for what a
 // The most that is asked for ahead: of more, L2 (126 MB) holds too little until it is read (2048 channels, intermediate size 16384,
 // 67 MB: 82 us a layer, without 88; 24576, 100 MB: 125 and 124; 32768, 134 MB: 139 and 135).
 constexpr int64_t kStepAheadMost = 96 << 20;
-constexpr int kStepEarly = 296;               // CTAs that request the first product's weights
+constexpr int kStepEarly = 2 * kSms;          // CTAs that request the first product's weights
 // Input and weights of a CTA that may lie in shared memory together; more goes through registers.  (16 sequences of 1536 channels:
 // the gate product would need 99 KB, and a layer takes 126 us so, 114 through registers; 2 sequences' down product, 83 KB: 59
 // and 61 us a layer.)
@@ -393,9 +393,9 @@ __device__ __forceinline__ float load_any(const void* w, int dtype, int i) {
   return dtype == FOX_DTYPE_BF16 ? unpack2<true>(u).x : unpack2<false>(u).x;
 }
 
-// CTA = one head of one sequence, thread = channel; the few values make this a matter of latency only.  With a mask there are
-// more threads, for its sum: with one a channel 6200 keys of 8 heads of 64 took 27 us a layer, 23 now, 12000 of 24 67 and 47,
-// 40000 of 32 of 16 101 and 41.
+// CTA = one head of one sequence, thread = channel; the few values make this a matter of latency only.  With a mask there is a
+// thread for four of its elements at least, up to 512, for their sum: with one a channel 6200 keys of 8 heads of 64 took 27 us a
+// layer, 23 now, 12000 of 24 67 and 47, 40000 of 32 of 16 101 and 41.  (512 for 64 keys of 16 x 32 heads of 16: 34 for 32 us.)
 constexpr int kMaskThreads = 512;
 template <bool kBf16>
 __global__ void __launch_bounds__(kMaskThreads) fox_step_mix_kernel(const StepMixParams p) {
@@ -610,7 +610,9 @@ extern "C" int fox_step_mix(int device, void* stream, int dtype, int64_t B, int6
   const StepMixParams p{y, ld, wq, wk, bias, wq_dtype, wk_dtype, bias_dtype, eps, mask, seq_start, (uint16_t*)k_state, (uint16_t*)v_state,
                         (uint16_t*)q, (uint16_t*)k_cache, (uint16_t*)v_cache, g_cache, capacity, pos, (int)H, (int)D};
   cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = pdl_config(dim3((unsigned)H, (unsigned)B), mask ? kMaskThreads : D <= 32 ? 32 : (int)D, 0, (cudaStream_t)stream, &attr);
+  const int64_t summing = mask ? std::min<int64_t>((pos / 4 + 32) / 32 * 32, kMaskThreads) : 0;
+  const int threads = (int)std::max<int64_t>(summing, D <= 32 ? 32 : D);
+  const cudaLaunchConfig_t cfg = pdl_config(dim3((unsigned)H, (unsigned)B), threads, 0, (cudaStream_t)stream, &attr);
   const cudaError_t e = dtype == FOX_DTYPE_BF16 ? cudaLaunchKernelEx(&cfg, fox_step_mix_kernel<true>, p)
                                                 : cudaLaunchKernelEx(&cfg, fox_step_mix_kernel<false>, p);
   return e == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
