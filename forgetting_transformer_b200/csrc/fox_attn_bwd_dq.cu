@@ -379,7 +379,8 @@ fox_attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 // A CTA goes on with further (b, h, query tile) items (ItemQueue): the next one's Q, dO and first K, V are loaded while this
 // one's dQ is read, and dQ leaves through a K stage as TMA stores.  Of a pruned call's items, about two KV tiles long, set-up
 // and the way out of dQ were most of the time: B4 T16384 H16 D128 with 97 % of the tiles pruned 480 -> 318-325 us; unpruned
-// 5.48 -> 5.32 ms.  With a fixed stride over the items instead of the queue unpruned calls ended unevenly: 5.69-5.77.
+// 5.48 -> 5.32 ms.  With a fixed stride over the items instead of the queue unpruned calls ended unevenly: 5.69-5.77.  Up to 148
+// items begin at once and need no queue (128 of two tiles: 9.7 us with it, 9.3 without).
 constexpr int kDq2BN = 128;
 enum Dq2WaitSite { kDq2SiteQ = 51, kDq2SiteK = 52, kDq2SiteV = 53, kDq2SiteKE = 54, kDq2SiteVE = 55, kDq2SiteS = 56,
                    kDq2SiteDP = 57, kDq2SiteDS = 58, kDq2SiteDone = 59, kDq2SiteNegB = 60, kDq2SiteRow = 61, kDq2SiteEpi = 62, kDq2SiteItem = 63 };

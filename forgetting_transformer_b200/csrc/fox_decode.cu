@@ -37,7 +37,8 @@ constexpr int kDecRows = 4;         // rows of K and of V in flight per lane
 constexpr int kDecMaxCluster = 8;
 constexpr int kDecMaxSplits = 1024;   // taken
 constexpr int kDecMostSplits = 512;   // asked for by fox_attn_decode_splits
-constexpr int64_t kDecSlots = 444, kDecClusterSlots = 400;                            // CTAs of a wave
+constexpr int kDecPerSm = 3;                                                          // by the kernel's launch bounds
+constexpr int64_t kDecSlots = kSms * kDecPerSm, kDecClusterSlots = 400;               // CTAs of a wave
 constexpr int64_t kDecStartKeys = 600, kDecMergeKeys = 120, kDecLeastKeys = 128;      // (at fox_attn_decode_splits)
 constexpr int64_t kDecLongRange = 1024 * 64, kDecManyClusters = 384;   // keys times head dim; CTAs (at long_ranges)
 constexpr float kDecLog2e = 1.4426950408889634f;
@@ -126,7 +127,7 @@ __device__ __forceinline__ void dec_store(const DecodeParams& p, int b, int h, i
 }
 
 template <bool kBf16, int D, bool kCluster, bool kStep = false>
-__global__ void __launch_bounds__(kDecThreads, 3)
+__global__ void __launch_bounds__(kDecThreads, kDecPerSm)
 fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeStep, char> step) {
   constexpr int LPR = D / 8, RPW = 32 / LPR;
   constexpr int kBatch = kDecWarps * RPW * kDecRows;   // keys a CTA takes per step

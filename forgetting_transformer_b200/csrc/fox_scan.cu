@@ -707,11 +707,12 @@ extern "C" int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D) {
   return n < 32 ? n : 32;
 }
 
-// The same for keys alone, whose blocks share a launch with those of the prefix scans, one a (b,h).  Where fewer parts make the
-// two resident blocks per SM one wave, nearly full, that is faster than a few blocks in a second wave (48 (b,h) of 16384 x 64:
-// 36 -> 30 us; 24 of 11000 x 64: 16 -> 13), unless the parts left have to be much longer: 2 -> 1 part never (148 of 4096 x 128:
-// 42 -> 51), 3 -> 2 not with long rows in many (96 of 8192 x 128: 49 -> 53, of 4096 29 -> 28), and 4 -> 3 only in
-// a fuller wave (70 of 4096 x 128, 280 blocks: 20 -> 22; 71, 284 blocks: 22.3 -> 21.6).
+// The same for keys alone, whose blocks share a launch with those of the prefix scans, one a (b,h).  Where fewer parts make two
+// blocks per SM nearly full (at a time for fp16, one after the other for bf16, whose blocks take more than 32 registers a
+// thread), that is faster than a few blocks more behind them (48 (b,h) of 16384 x 64: 36 -> 30 us; 24 of 11000 x 64: 16 -> 13),
+// unless the parts left have to be much longer: 2 -> 1 part never (148 of 4096 x 128: 42 -> 51), 3 -> 2 not with long rows in many
+// (96 of 8192 x 128: 49 -> 53, of 4096 29 -> 28), and 4 -> 3 only in a fuller wave (70 of 4096 x 128, 280 blocks: 20 -> 22; 71, 284
+// blocks: 22.3 -> 21.6).
 extern "C" int64_t fox_key_norm_parts(int64_t B, int64_t H, int64_t N, int64_t D) {
   if (B <= 0 || H <= 0) return 1;
   const int64_t n = fox_norm_parts(B, H, N, D), bh = B * H, places = 2 * kSms, fewer = places / bh - 1, blocks = (fewer + 1) * bh;
