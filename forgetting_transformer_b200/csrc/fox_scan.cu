@@ -712,13 +712,14 @@ extern "C" int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D) {
 // thread), that is faster than a few blocks more behind them (48 (b,h) of 16384 x 64: 36 -> 30 us; 24 of 11000 x 64: 16 -> 13),
 // unless the parts left have to be much longer: 2 -> 1 part never (148 of 4096 x 128: 42 -> 51), 3 -> 2 not with long rows in many
 // (96 of 8192 x 128: 49 -> 53, of 4096 29 -> 28), and 4 -> 3 only in a fuller wave (70 of 4096 x 128, 280 blocks: 20 -> 22; 71, 284
-// blocks: 22.3 -> 21.6).
+// blocks: 22.3 -> 21.6).  Long rows of 16 or 32 channels keep theirs as well: their blocks are bound by instructions (fp16, 24 of
+// 12300 x 16: 16.9 -> 23.3, 20 of 16384 x 16 a third more).
 extern "C" int64_t fox_key_norm_parts(int64_t B, int64_t H, int64_t N, int64_t D) {
   if (B <= 0 || H <= 0) return 1;
   const int64_t n = fox_norm_parts(B, H, N, D), bh = B * H, places = 2 * kSms, fewer = places / bh - 1, blocks = (fewer + 1) * bh;
   if (fewer >= n) return n;
-  const bool full = blocks >= places - (fewer >= 4 ? 16 : 12);
-  return full && (fewer >= 3 || (fewer == 2 && (N <= 4096 || D <= 64))) ? fewer : n;
+  const bool full = blocks >= places - (fewer >= 4 ? 16 : 12) && (N <= 4096 || D >= 64);
+  return full && (fewer >= 3 || (fewer == 2 && (N <= 4096 || D == 64))) ? fewer : n;
 }
 
 extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_kind, int64_t B, int64_t H, int64_t M,
