@@ -73,6 +73,7 @@ struct BwdParams {
   int* status;
   long long* trace;          // optional (debug builds of the kernel only): clock64 stamps of CTA (0,0,0)
   int H, M, N;
+  ItemOrder order;   // units (b,h), KV tiles, the first one first
   bool tma_out;              // dK / dV leave through shared memory and TMA stores
   float sm_scale, qk_scale;
 };
@@ -88,7 +89,7 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
                : "memory");
 }
 
-template <int D, bool kBf16, bool kTrace, int kCWG, bool kNoDQ>
+template <int D, bool kBf16, bool kTrace, int kCWG, bool kNoDQ, bool kByLength>
 __global__ void __launch_bounds__((4 * kCWG + 6) * 32, 1)
 fox_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -144,7 +145,10 @@ fox_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* sStage = sdS + kDsBufs * 32768;        // kStageSub x [128 q][32 fp32], 128-byte swizzled, for the dQ reduction
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int unit = unit_here<kByLength>(p.order, p.H);
+  if (kByLength && unit >= p.order.units) return;
+  const int b = batch_of<kByLength>(p.order, unit), h = unit - b * p.H;
+  const int nb = rank_here<kByLength>();   // KV tile 0 sees every query row: long tiles first
   const int M = p.M, N = p.N, P = N - M;
   const int64_t bh = static_cast<int64_t>(b) * p.H + h;
   const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
@@ -154,7 +158,7 @@ fox_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   lo = (lo / kBwdBM) * kBwdBM;
   int hi = M;
   if (p.end_index) {
-    const int64_t e = p.end_index[bh * gridDim.x + nb];
+    const int64_t e = p.end_index[bh * p.order.tiles + nb];
     hi = static_cast<int>(e < static_cast<int64_t>(M) ? e : static_cast<int64_t>(M));
   }
   if (p.seq_start && !(nb * kBwdBN + kBwdBN >= seq0 - 1)) hi = lo;
@@ -832,23 +836,27 @@ static int launch_bwd(int device, cudaStream_t stream, int64_t B, int64_t H, int
   // fox_attn_bwd_kv_kernel replaced it)
   const bool tracing = prm.trace != nullptr;
   const bool nodq = prm.dq_accum == nullptr;
-  auto kern = tracing ? (nodq ? fox_attn_bwd_kernel<D, kBf16, true, kCWG, true> : fox_attn_bwd_kernel<D, kBf16, true, kCWG, false>)
-                      : (nodq ? fox_attn_bwd_kernel<D, kBf16, false, kCWG, true> : fox_attn_bwd_kernel<D, kBf16, false, kCWG, false>);
+  auto instance = [&](auto by) {
+    constexpr bool kBy = decltype(by)::value;
+    return tracing ? (nodq ? fox_attn_bwd_kernel<D, kBf16, true, kCWG, true, kBy> : fox_attn_bwd_kernel<D, kBf16, true, kCWG, false, kBy>)
+                   : (nodq ? fox_attn_bwd_kernel<D, kBf16, false, kCWG, true, kBy> : fox_attn_bwd_kernel<D, kBf16, false, kCWG, false, kBy>);
+  };
 #else
   constexpr bool tracing = false, nodq = false;
   if (prm.dq_accum == nullptr) return FOX_ERR_BAD_ARG;   // key-side-only calls go to fox_attn_bwd_kv_kernel
-  auto kern = fox_attn_bwd_kernel<D, kBf16, false, kCWG, false>;
+  auto instance = [](auto by) { return fox_attn_bwd_kernel<D, kBf16, false, kCWG, false, decltype(by)::value>; };
 #endif
+  const bool by_length = prm.order.group > 1;
+  auto kern = by_length ? instance(std::true_type{}) : instance(std::false_type{});
   const int threads = (4 * kCWG + 6) * 32;
-  static bool configured[4][64] = {};
+  static bool configured[8][64] = {};
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;
-  const int slot = tracing ? (nodq ? 3 : 1) : (nodq ? 2 : 0);
+  const int slot = (tracing ? (nodq ? 3 : 1) : (nodq ? 2 : 0)) + (by_length ? 4 : 0);
   if (!configured[slot][device]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
     configured[slot][device] = true;
   }
-  dim3 grid((unsigned)((N + kBwdBN - 1) / kBwdBN), (unsigned)H, (unsigned)B);
-  kern<<<grid, threads, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, tmDK, tmDV, prm);
+  kern<<<item_grid(prm.order, B, H), threads, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, tmDK, tmDV, prm);
   return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 
@@ -907,6 +915,8 @@ extern "C" int fox_attn_bwd(int device, void* stream, int dtype, int64_t B, int6
   prm.trace = nullptr;
 #endif
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
+  const int64_t tiles = (N + kBwdBN - 1) / kBwdBN;
+  prm.order = item_order(B * H, H, tiles, end_index ? 1 : item_group(B * H, tiles, M * (D < 64 ? 64 : D) * 8));
   prm.tma_out = end_index != nullptr || D < 64;
   prm.sm_scale = sm_scale;
   prm.qk_scale = sm_scale * 1.4426950408889634f;

@@ -33,7 +33,8 @@ struct DqParams {
   float* dlam_row;             // (B,H,M), fully written
   int* status;
   int H, M, N;
-  int tiles, items;            // query tiles of a (b,h); of all
+  int items;
+  ItemOrder order;             // units (b,h), query tiles, the last one first
   float qk_scale;              // sm_scale * log2(e)
   float sm_scale;
 };
@@ -427,16 +428,17 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   };
   auto item_of = [&](int i) {
     Item x;
-    const int u = i / p.tiles;
-    x.mb = p.tiles - 1 - i % p.tiles;
-    x.h = u % p.H;
-    x.b = u / p.H;
+    int u, rank;
+    item_at(p.order, i, u, rank);
+    x.mb = p.order.tiles - 1 - rank;
+    x.b = div_by(p.order.heads, u);
+    x.h = u - x.b * p.H;
     x.bh = u;
     const int hi = min(N, P + (x.mb + 1) * kDqBM);
     x.seq0 = p.seq_start ? static_cast<int>(p.seq_start[x.b]) : 0;
     int lo = min(x.seq0, hi);
     if (p.start_index) {
-      const int64_t si = p.start_index[static_cast<int64_t>(u) * p.tiles + x.mb];
+      const int64_t si = p.start_index[static_cast<int64_t>(u) * p.order.tiles + x.mb];
       lo = max(lo, static_cast<int>(si < static_cast<int64_t>(hi) ? si : static_cast<int64_t>(hi)));
     }
     x.nb_hi = (hi + BN - 1) / BN;
@@ -933,7 +935,8 @@ extern "C" int fox_attn_bwd_dq(int device, void* stream, int dtype, int64_t B, i
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
   const int64_t tiles = (M + kDqBM - 1) / kDqBM;
   if (tiles * H * B > 2147483647LL - 65536) return FOX_ERR_TOO_LARGE;
-  prm.tiles = (int)tiles; prm.items = (int)(tiles * H * B);
+  prm.items = (int)(tiles * H * B);
+  prm.order = item_order(B * H, H, tiles, start_index ? 1 : item_group(B * H, tiles, N * D * 4));
   prm.qk_scale = sm_scale * kDqLog2e;
   prm.sm_scale = sm_scale;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);

@@ -46,7 +46,8 @@ struct KvParams {
   void* dv; int64_t dv_sb, dv_sh, dv_st;
   int* status;
   int H, M, N;
-  int tiles, items;          // KV tiles of a (b,h); of all
+  int items;
+  ItemOrder order;           // units (b,h), KV tiles, the first one first
   float sm_scale, qk_scale;
 };
 
@@ -105,9 +106,10 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   };
   auto item_of = [&](int i) {
     Item x;
-    const int nb = i % p.tiles, u = i / p.tiles;
-    x.h = u % p.H;
-    x.b = u / p.H;
+    int u, nb;
+    item_at(p.order, i, u, nb);
+    x.b = div_by(p.order.heads, u);
+    x.h = u - x.b * p.H;
     x.bh = u;
     x.j0 = nb * kKvBN;
     x.seq0 = p.seq_start ? static_cast<int>(p.seq_start[x.b]) : 0;
@@ -115,7 +117,7 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     lo = (lo / BM) * BM;
     int hi = M;
     if (p.end_index) {
-      const int64_t e = p.end_index[static_cast<int64_t>(u) * p.tiles + nb];
+      const int64_t e = p.end_index[static_cast<int64_t>(u) * p.order.tiles + nb];
       hi = static_cast<int>(e < static_cast<int64_t>(M) ? e : static_cast<int64_t>(M));
     }
     if (p.seq_start && !(x.j0 + kKvBN >= x.seq0 - 1)) hi = lo;
@@ -612,7 +614,8 @@ int launch_bwd_kv(int device, cudaStream_t stream, bool bf16, int D, int64_t B, 
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
   const int64_t tiles = (N + kKvBN - 1) / kKvBN;
   if (tiles * H * B > 2147483647LL - 65536) return FOX_ERR_TOO_LARGE;
-  prm.tiles = (int)tiles; prm.items = (int)(tiles * H * B);
+  prm.items = (int)(tiles * H * B);
+  prm.order = item_order(B * H, H, tiles, end_index ? 1 : item_group(B * H, tiles, M * D * 4));
   prm.sm_scale = sm_scale;
   prm.qk_scale = sm_scale * kKvLog2e;
   if (D == 64)

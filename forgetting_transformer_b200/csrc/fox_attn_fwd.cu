@@ -47,6 +47,7 @@ struct FwdParams {
   float qk_scale;              // sm_scale * log2(e)
   const float* k_norm_max;     // (B,H,n_norm_parts) max_t ||k[b,h,t,:]||_2 in parts, or nullptr: lets a tile skip its maximum pass
   int n_norm_parts;            // <= 32
+  ItemOrder order;             // units (b,h), query tiles, the last one first
 };
 
 // How many of every 4 column pairs take the FMA-pipe exponential instead of the ex2 unit (measured best
@@ -73,7 +74,7 @@ enum FwdWaitSite {
   kSiteSFull = 16, kSitePFull = 17, kSiteODone = 18, kSiteDrain = 19, kSiteNegB = 20, kSiteMerge = 21, kSiteEpi = 22
 };
 
-template <int D, bool kBf16, int BN, int STAGES, int CTAS, int NWG, int SB, bool PREF>
+template <int D, bool kBf16, int BN, int STAGES, int CTAS, int NWG, int SB, bool PREF, bool kByLength>
 __global__ void __launch_bounds__(128 * NWG + 64, CTAS)
 fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -118,8 +119,10 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* sV = sK + STAGES * kTileBytes;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int mb = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);  // heavy tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int unit = unit_here<kByLength>(p.order, p.H);
+  if (kByLength && unit >= p.order.units) return;
+  const int b = batch_of<kByLength>(p.order, unit), h = unit - b * p.H;
+  const int mb = p.order.tiles - 1 - rank_here<kByLength>();   // long tiles first
   const int M = p.M, N = p.N, P = N - M;
 
   // ---- KV range of this query tile (upstream lines 591-613) ----
@@ -127,7 +130,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
   int lo = min(seq0, hi);
   if (p.start_index) {
-    const int64_t si = p.start_index[(static_cast<int64_t>(b) * p.H + h) * gridDim.x + mb];
+    const int64_t si = p.start_index[(static_cast<int64_t>(b) * p.H + h) * p.order.tiles + mb];
     lo = max(lo, static_cast<int>(si < static_cast<int64_t>(hi) ? si : static_cast<int64_t>(hi)));
   }
   lo = (lo / kFwdBN) * kFwdBN;
@@ -700,15 +703,16 @@ static int launch_fwd_t(int device, cudaStream_t stream, int64_t B, int64_t H, i
   if (!tma_compatible(to, 2)) return FOX_ERR_ALIGNMENT;
   if ((rc = cached_tmap_4d(&tmO, to, 2, false, kBf16, 64, 128, true))) return rc;
   constexpr int smem = 128 * D * 2 + 2 * STAGES * BN * D * 2 + 1024;
-  auto kern = fox_attn_fwd_kernel<D, kBf16, BN, STAGES, CTAS, NWG, SB, PREF>;
-  static bool configured[64] = {};  // per template instance and device
+  const bool by_length = prm.order.group > 1;
+  auto kern = by_length ? fox_attn_fwd_kernel<D, kBf16, BN, STAGES, CTAS, NWG, SB, PREF, true>
+                        : fox_attn_fwd_kernel<D, kBf16, BN, STAGES, CTAS, NWG, SB, PREF, false>;
+  static bool configured[2][64] = {};  // per template instance and device
   if (device < 0 || device >= 64) return FOX_ERR_DEVICE;
-  if (!configured[device]) {
+  if (!configured[by_length][device]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
-    configured[device] = true;
+    configured[by_length][device] = true;
   }
-  dim3 grid((unsigned)((M + kFwdBM - 1) / kFwdBM), (unsigned)H, (unsigned)B);
-  kern<<<grid, 128 * NWG + 64, smem, stream>>>(tmQ, tmK, tmV, tmO, prm);
+  kern<<<item_grid(prm.order, B, H), 128 * NWG + 64, smem, stream>>>(tmQ, tmK, tmV, tmO, prm);
   return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 
@@ -761,6 +765,8 @@ extern "C" int fox_attn_fwd_parts(int device, void* stream, int dtype, int64_t B
   prm.L = L;
   prm.status = status;
   prm.H = (int)H; prm.M = (int)M; prm.N = (int)N;
+  const int64_t tiles = (M + kFwdBM - 1) / kFwdBM;
+  prm.order = item_order(B * H, H, tiles, start_index ? 1 : item_group(B * H, tiles, N * D * 4));
   prm.qk_scale = sm_scale * 1.4426950408889634f;
   if (k_norm_parts && (n_norm_parts <= 0 || n_norm_parts > 32)) return FOX_ERR_BAD_ARG;
   prm.k_norm_max = k_norm_parts;

@@ -72,6 +72,20 @@ inline int make_tmap_4d(CUtensorMap* out, const Tensor4& t, int elem_bytes, bool
   return r == CUDA_SUCCESS ? FOX_OK : FOX_ERR_TENSORMAP;
 }
 
+// ------------------------------------------------------------- order of items
+// How many units go by length together (ItemOrder in fox_common.cuh): groups of even size whose rereads, unit_bytes a unit, stay in
+// L2 (126 MB; what is written takes its part).  Forward / backward kernels in us, unit by unit -> groups of 12, 24, 48 MB, all units:
+//   B2 H24 T16384 D64    2240 / 4724 -> 2151 / 4722, 2092 / 4697, 2079 / 4698, 2140 / 5191
+//   B2 H16 T4096 D64     138 / 278 -> 126 / 283, 117 / 251, 114 / 253, 115 / 259
+//   B4 H16 T16384 D128   4539 / 8273 + 5370 -> 16 MB 4457 / 8171 + 5316, 48 MB 4354 / 8148 + 5334, all 4788 / 8775 + 5837
+//   B4 H12 T512 D64      15.1 / 24.8 -> 12.4 / 21.0 (one group from 3 MB on)
+inline int64_t item_group(int64_t units, int64_t tiles, int64_t unit_bytes) {
+  constexpr int64_t kGroupBytes = 48 << 20;
+  const int64_t fit = unit_bytes < kGroupBytes ? kGroupBytes / unit_bytes : 1;
+  const int64_t groups = (units + fit - 1) / fit;
+  return tiles > 65535 || groups > 65535 ? 1 : (units + groups - 1) / groups;   // (what a grid can have)
+}
+
 // ------------------------------------------------------------- tensor-map cache
 struct TmapKey {
   uintptr_t ptr;

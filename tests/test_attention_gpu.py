@@ -677,3 +677,27 @@ def test_backward_that_could_prune_equals_one_that_cannot(B, H, M, N):
     seq = torch.arange(B) * (N // 5)
     for name, a, b in zip(("out", "dq", "dk", "dv", "dlog_fgate"), _run(*args, seq=seq, thr=-1e9), _run(*args, seq=seq)):
         assert torch.equal(a, b), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,T,D", [(13, 8200, 64), (25, 4100, 128), (3, 300, 64), (1, 1, 128)])
+def test_items_by_length_are_each_taken_once(H, T, D):
+    """Units go by tile length in groups that stay in L2 (13 of 4.2 MB and 25 of 2.1 MB: two uneven groups; fewer: one); a unit alone is
+    its own group.  The order decides nothing but when an item runs: the same bits (fp32 sums into dQ at D=64: in another order)."""
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    q, k, v, do = (torch.randn(1, H, T, D, generator=gen, device="cuda").bfloat16() for _ in range(4))
+    g = torch.nn.functional.logsigmoid(torch.randn(1, H, T, generator=gen, device="cuda") + 2)
+
+    def run(lo, hi):
+        x = [t[:, lo:hi].contiguous().requires_grad_() for t in (q, k, v, g)]
+        out = fox.forgetting_attention(*x, head_first=True)
+        out.backward(do[:, lo:hi].contiguous())
+        return [out] + [t.grad for t in x]
+
+    together = run(0, H)
+    for h in range(H):
+        for i, (a, b) in enumerate(zip(together, run(h, h + 1))):
+            if D == 64 and i in (1, 4):     # dQ, and the gate gradient through its row sums
+                assert (a[:, h:h + 1].double() - b.double()).norm() <= 2 ** -8 * b.double().norm() + 1e-30
+            else:
+                assert torch.equal(a[:, h:h + 1], b), (h, i)
