@@ -37,9 +37,11 @@ constexpr int kDecRows = 4;         // rows of K and of V in flight per lane
 constexpr int kDecMaxCluster = 8;
 constexpr int kDecMaxSplits = 1024;   // taken
 constexpr int kDecMostSplits = 512;   // asked for by fox_attn_decode_splits
-constexpr int kDecPerSm = 3;                                                          // by the kernel's launch bounds
-constexpr int64_t kDecSlots = kSms * kDecPerSm, kDecClusterSlots = 400;               // CTAs of a wave
+constexpr int kDecPerSm = 3, kDecMorePerSm = 4;                                       // by the kernels' launch bounds
+constexpr int64_t kDecSlots = kSms * kDecPerSm, kDecClusterSlots = 400;               // CTAs of a wave, three to an SM
+constexpr int64_t kDecMoreSlots = kSms * kDecMorePerSm, kDecMoreClusterSlots = 540;   // four
 constexpr int64_t kDecStartKeys = 600, kDecMergeKeys = 120, kDecLeastKeys = 128;      // (at fox_attn_decode_splits)
+constexpr int64_t kDecMoreLeastKeys = 640;
 constexpr int64_t kDecLongRange = 1024 * 64, kDecManyClusters = 384;   // keys times head dim; CTAs (at long_ranges)
 constexpr float kDecLog2e = 1.4426950408889634f;
 
@@ -126,8 +128,8 @@ __device__ __forceinline__ void dec_store(const DecodeParams& p, int b, int h, i
   p.o[b * p.o_sb + h * p.o_sh + d] = static_cast<uint16_t>(pk & 0xffffu);
 }
 
-template <bool kBf16, int D, bool kCluster, bool kStep = false>
-__global__ void __launch_bounds__(kDecThreads, kDecPerSm)
+template <bool kBf16, int D, bool kCluster, int kPerSm, bool kStep = false>
+__global__ void __launch_bounds__(kDecThreads, kPerSm)
 fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeStep, char> step) {
   constexpr int LPR = D / 8, RPW = 32 / LPR;
   constexpr int kBatch = kDecWarps * RPW * kDecRows;   // keys a CTA takes per step
@@ -564,11 +566,11 @@ static int launch_step(const DecodeParams& p, const DecodeStep& step, int64_t B,
   }
   cfg.attrs = attrs;
   cfg.numAttrs = n;
-  return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true, true>, p, step) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true, kDecPerSm, true>, p, step) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 
-template <bool kBf16, int D>
-static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
+template <bool kBf16, int D, int kPerSm>
+static int launch_decode_at(const DecodeParams& p, int64_t B, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.splits, (unsigned)p.H, (unsigned)B);
   cfg.blockDim = dim3(kDecThreads);
@@ -589,10 +591,10 @@ static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
       ++n;
     }
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true>, p, '\0') == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, true, kPerSm>, p, '\0') == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
   }
   cfg.numAttrs = n;
-  if (cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, false>, p, '\0') != cudaSuccess) return FOX_ERR_LAUNCH;
+  if (cudaLaunchKernelEx(&cfg, fox_decode_kernel<kBf16, D, false, kPerSm>, p, '\0') != cudaSuccess) return FOX_ERR_LAUNCH;
   cfg.gridDim = dim3((unsigned)p.H, (unsigned)B);
   cfg.blockDim = dim3(256);
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -602,24 +604,31 @@ static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, fox_decode_merge_kernel<kBf16, D>, p) == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
 }
 
-}  // namespace fox
-
-using namespace fox;
-
 // Ranges per (b,h), so that the CTAs come in whole waves: 444 (three per SM) where a second kernel merges, 400 where clusters
 // do (those find no room on the last SMs of a GPC: 72 x 5 CTAs 36.1 us, 72 x 6 52.1).  A (b,h) that is one range of a wave
 // takes the next wave too where its shorter ranges pay for the second start, some 600 keys (256 (b,h) of 4099 keys, head dim
 // 128: one range 105 us, three 94; of 1024 keys: 28.5 and 31.3).  Eight ranges need no merge kernel, which is worth some 120
 // keys.  At least 128 keys a range.  Four CTAs per SM on average, as before, left a last wave nearly empty: 24 x 65536 keys of
 // head dim 64 in 25 ranges 81.4 us, in 18 67.2; 48 x 8192 25.7 -> 22.6; 192 x 2048 26.2 -> 22.0; 72 x 5000 of 128 41.3 -> 36.1.
-extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
-  const int64_t bh = B * H;
-  if (bh <= 0) return 1;   // (fox_attn_decode refuses such a call)
+//
+// Four per SM (64 registers instead of 80, no spills) share the same bandwidth, so that a range takes a third longer; they are
+// taken where the waves are fewer by so much that this pays, counted in keys with 600 for a wave's start: 512 (b,h) of 4000
+// keys of 128 in one wave instead of three 192 -> 162 us, of 64 102 -> 86; 256 of 4099 of 128 in one instead of two 98 -> 91, of 2048
+// 54 -> 48.  With as many waves they pay where they fill one that three leave half empty and the ranges are long: 256 of 1500 of 128
+// in two ranges instead of one 43 -> 37, 144 of 2600 of 64 in three instead of two 24.7 -> 22.7, but 256 of 1000 of 64 17.8 and 18.5, 176 of
+// 1200 16.4 and 17.2.  Else they are no faster or slower: 384 of 8000 of 64 130 and 135, 32 of 3000 13.7 and 14.3, 4 of 30000 of 128 21.2
+// and 22.5, 768 of 2500 of 64 86 and 91; 24 x 65536 70.0 and 70.0.
+struct DecodePlan {
+  int64_t splits;
+  int per_sm;
+};
+static int64_t waves_of(int64_t ctas, int64_t slots) { return (ctas + slots - 1) / slots; }
+static int64_t fit_splits(int64_t bh, int64_t N, int64_t slots, int64_t cluster_slots) {
   auto fit = [&](int64_t waves) {
-    const int64_t s = waves * kDecSlots / bh;
-    return s > kDecMaxCluster ? s : waves * kDecClusterSlots / bh > 1 ? waves * kDecClusterSlots / bh : int64_t{1};
+    const int64_t s = waves * slots / bh;
+    return s > kDecMaxCluster ? s : waves * cluster_slots / bh > 1 ? waves * cluster_slots / bh : int64_t{1};
   };
-  const int64_t waves = (bh + kDecSlots - 1) / kDecSlots;
+  const int64_t waves = waves_of(bh, slots);
   int64_t s = fit(waves);
   if (s == 1) {
     const int64_t next = fit(waves + 1);
@@ -631,6 +640,29 @@ extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
   if (s > most) s = most;
   if (s > kDecMostSplits) s = kDecMostSplits;
   return s < 1 ? 1 : s;
+}
+static DecodePlan decode_plan(int64_t bh, int64_t N) {
+  const int64_t s3 = fit_splits(bh, N, kDecSlots, kDecClusterSlots), s4 = fit_splits(bh, N, kDecMoreSlots, kDecMoreClusterSlots);
+  auto waves = [&](int64_t s, int64_t slots, int64_t cluster_slots) { return waves_of(bh * s, s > 1 && s <= kDecMaxCluster ? cluster_slots : slots); };
+  const int64_t w3 = waves(s3, kDecSlots, kDecClusterSlots), w4 = waves(s4, kDecMoreSlots, kDecMoreClusterSlots);
+  const int64_t t3 = w3 * (N / s3 + kDecStartKeys), t4 = w4 * (N / s4 * kDecMorePerSm / kDecPerSm + kDecStartKeys);
+  const bool more = w4 < w3 ? t4 < t3 : w4 == w3 && t4 < t3 - t3 / 20 && N / s4 >= kDecMoreLeastKeys;
+  return more ? DecodePlan{s4, kDecMorePerSm} : DecodePlan{s3, kDecPerSm};
+}
+template <bool kBf16, int D>
+static int launch_decode(const DecodeParams& p, int64_t B, cudaStream_t st) {
+  const DecodePlan plan = decode_plan(B * p.H, p.N);   // (a caller may ask for other ranges than its)
+  return plan.per_sm == kDecMorePerSm && plan.splits == p.splits ? launch_decode_at<kBf16, D, kDecMorePerSm>(p, B, st)
+                                                                 : launch_decode_at<kBf16, D, kDecPerSm>(p, B, st);
+}
+
+}  // namespace fox
+
+using namespace fox;
+
+extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
+  if (B * H <= 0) return 1;   // (fox_attn_decode refuses such a call)
+  return decode_plan(B * H, N).splits;
 }
 
 // (none where the ranges are merged inside a cluster)
@@ -698,8 +730,9 @@ extern "C" int fox_attn_decode_gates(int device, void* stream, int dtype, int64_
 // sequences x 32 heads of 8192 keys 694 us for two layers, 674 apart), or ranges so long that more than eight of them pay for
 // the two launches more (24 heads of 8000 keys 105 and 101 us).
 extern "C" int64_t fox_step_attn_splits(int64_t B, int64_t H, int64_t N) {
-  const int64_t s = fox_attn_decode_splits(B, H, N);
-  if (B <= 0 || H <= 0 || B * H * s > kDecSlots) return 0;
+  if (B <= 0 || H <= 0) return 0;
+  const int64_t s = fit_splits(B * H, N, kDecSlots, kDecClusterSlots);
+  if (B * H * s > kDecSlots) return 0;
   return s <= kDecMaxCluster ? s : N <= 8 * 768 ? 8 : 0;
 }
 

@@ -330,3 +330,12 @@ def test_decode_from_gates_behind_one_of_minus_infinity(N, D, at):
         ref = s.softmax(0) @ v[0, h, N - n:].double()
         err = (out[0, h, 0].double() - ref).abs()
         assert (err <= 2 ** -8 * ref.abs() + 2 ** -8 * ref.pow(2).mean().sqrt()).all(), (h, err.max().item())
+
+
+@pytest.mark.parametrize("B,H,N,D,splits", [(16, 32, 513, 64, 1), (1, 592, 129, 32, 1), (2, 128, 2048, 128, 2), (10, 27, 2000, 16, 2)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_decode_by_four_ctas_of_an_sm(B, H, N, D, splits, padded):
+    """445 to 592 (b,h), one range each, and 223 to 270 in clusters of two: one wave of four CTAs to an SM in place of two or three of
+    three; the ranges of fewer CTAs to an SM would be others."""
+    assert _lib.load().fox_attn_decode_splits(B, H, N) == splits
+    test_decode_from_gates(B, H, N, D, padded)
