@@ -151,6 +151,7 @@ fox_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int nb = rank_here<kByLength>();   // KV tile 0 sees every query row: long tiles first
   const int M = p.M, N = p.N, P = N - M;
   const int64_t bh = static_cast<int64_t>(b) * p.H + h;
+  wait_for_kernel_in_front();   // (behind the barriers' set-up, as in the other kernels, it spills 120 bytes for 28 and gains no more)
   const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
 
   // ---- query-tile range of this KV tile (upstream lines 1003-1049) ----
@@ -856,8 +857,7 @@ static int launch_bwd(int device, cudaStream_t stream, int64_t B, int64_t H, int
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
     configured[slot][device] = true;
   }
-  kern<<<item_grid(prm.order, B, H), threads, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDQ, tmDK, tmDV, prm);
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  return launch_behind(kern, item_grid(prm.order, B, H), threads, smem, stream, tmQ, tmK, tmV, tmDO, tmDQ, tmDK, tmDV, prm);
 }
 
 }  // namespace fox

@@ -150,6 +150,7 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if constexpr (kLoop) items_init(items, 17);
     mbar_fence_init();
   }
+  wait_for_kernel_in_front();   // (no memory is read before this, and no TMEM held that the kernel in front might ask for)
   if (warp == kTmaWarp) {
     tmem_alloc(&tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -595,8 +596,7 @@ static int launch_kv(int device, cudaStream_t stream, int64_t B, int64_t H, int6
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
     configured[loop][device] = true;
   }
-  kern<<<(unsigned)prm.items, 576, smem, stream>>>(tmQ, tmK, tmV, tmDO, tmDK, tmDV, prm);
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  return launch_behind(kern, dim3((unsigned)prm.items), 576, smem, stream, tmQ, tmK, tmV, tmDO, tmDK, tmDV, prm);
 }
 
 // Key side (dk, dv, dlam_col); arguments as fox_attn_bwd's, already validated there.

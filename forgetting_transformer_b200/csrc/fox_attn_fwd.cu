@@ -125,19 +125,6 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int mb = p.order.tiles - 1 - rank_here<kByLength>();   // long tiles first
   const int M = p.M, N = p.N, P = N - M;
 
-  // ---- KV range of this query tile (upstream lines 591-613) ----
-  const int hi = min(N, P + (mb + 1) * kFwdBM);
-  const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
-  int lo = min(seq0, hi);
-  if (p.start_index) {
-    const int64_t si = p.start_index[(static_cast<int64_t>(b) * p.H + h) * p.order.tiles + mb];
-    lo = max(lo, static_cast<int>(si < static_cast<int64_t>(hi) ? si : static_cast<int64_t>(hi)));
-  }
-  lo = (lo / kFwdBN) * kFwdBN;
-  const int nb_lo = lo / BN;
-  const int nb_hi = (hi + BN - 1) / BN;  // exclusive
-  const int n_tiles = max(nb_hi - nb_lo, 0);
-
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&bar_q_full, 1);
@@ -157,6 +144,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     mbar_fence_init();
   }
+  wait_for_kernel_in_front();   // (no memory is read before this, and no TMEM held that the kernel in front might ask for)
   if (warp == kTmaWarp) {
     tmem_alloc(&tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -166,6 +154,19 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   const uint32_t tbase = tmem_slot;
   volatile int* abortp = &abort_flag;
+
+  // ---- KV range of this query tile (upstream lines 591-613) ----
+  const int hi = min(N, P + (mb + 1) * kFwdBM);
+  const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
+  int lo = min(seq0, hi);
+  if (p.start_index) {
+    const int64_t si = p.start_index[(static_cast<int64_t>(b) * p.H + h) * p.order.tiles + mb];
+    lo = max(lo, static_cast<int>(si < static_cast<int64_t>(hi) ? si : static_cast<int64_t>(hi)));
+  }
+  lo = (lo / kFwdBN) * kFwdBN;
+  const int nb_lo = lo / BN;
+  const int nb_hi = (hi + BN - 1) / BN;  // exclusive
+  const int n_tiles = max(nb_hi - nb_lo, 0);
 
   if (warp == kTmaWarp) {
     // ===================== TMA producer (whole warp converged, one elected lane issues) =====================
@@ -712,8 +713,7 @@ static int launch_fwd_t(int device, cudaStream_t stream, int64_t B, int64_t H, i
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return FOX_ERR_LAUNCH;
     configured[by_length][device] = true;
   }
-  kern<<<item_grid(prm.order, B, H), 128 * NWG + 64, smem, stream>>>(tmQ, tmK, tmV, tmO, prm);
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  return launch_behind(kern, item_grid(prm.order, B, H), 128 * NWG + 64, smem, stream, tmQ, tmK, tmV, tmO, prm);
 }
 
 template <int... A>

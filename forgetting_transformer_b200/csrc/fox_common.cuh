@@ -245,6 +245,10 @@ __device__ __forceinline__ int unit_here(const ItemOrder& o, int heads) {
 template <bool kByLength>
 __device__ __forceinline__ int batch_of(const ItemOrder& o, int unit) { return kByLength ? div_by(o.heads, unit) : blockIdx.z; }
 
+// What a kernel launched by launch_behind() does before it touches memory, by every thread: the kernel in front of it in the stream
+// has then ended and its writes are visible (and so are those of all before it, as that one began behind them or waited too).
+__device__ __forceinline__ void wait_for_kernel_in_front() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------- items
 // A grid of one CTA per item whose CTAs go on with items of CTAs that have not begun (cluster launch control): the items are
 // handed out in the grid's order to whichever CTA is free, as without it, but a CTA's set-up is paid once and the next

@@ -68,10 +68,8 @@ __device__ __forceinline__ float load_gate(const void* base, int64_t idx) {
 // One CTA per (b,h); chunks of 4096 elements with a carried running total.  With gate logits as input
 // (kIn < 3) the log gates themselves are formed on the fly and, if lf_out is given, written out (unmasked).
 template <int kIn>
-__device__ __forceinline__ void cumsum_rows(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
-                                            const int64_t* __restrict__ seq_start, const float* __restrict__ carry_in,
-                                            float* __restrict__ out, float* __restrict__ total_out,
-                                            float* __restrict__ lf_out, int H, int N, int bh, float* red) {
+__device__ __forceinline__ void cumsum_rows(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
+                                            const float* carry_in, float* out, float* total_out, float* lf_out, int H, int N, int bh, float* red) {
   const int b = bh / H, h = bh % H;
   const int64_t src0 = b * sb + h * sh;
   float* dst = out + static_cast<int64_t>(bh) * N;
@@ -269,6 +267,7 @@ fox_find_index_kernel(const IndexParams p) {
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* l = p.lam + static_cast<int64_t>(bh) * N;
+  wait_for_kernel_in_front();
   const int P = N - M;
   for (int i = threadIdx.x; i < nmb; i += blockDim.x) row_first[i] = l[P + i * BM];
   for (int i = threadIdx.x; i < nnb; i += blockDim.x) col_last[i] = l[min(N - 1, i * BN + BN - 1)];
@@ -469,11 +468,10 @@ __device__ __forceinline__ void norm_part(const NormSource& s, int D, int H, int
 
 template <int kIn, bool kBf16>
 __global__ void __launch_bounds__(kScanThreads)
-fox_prologue_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
-                    const int64_t* __restrict__ seq_start, float* __restrict__ lam,
-                    const NormSource k, const NormSource q, int H, int N, int D) {
+fox_prologue_kernel(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float* lam, const NormSource k, const NormSource q, int H, int N, int D) {
   __shared__ float red[32];
   const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
+  wait_for_kernel_in_front();
   if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
   else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
   else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
@@ -488,9 +486,8 @@ constexpr int kDeltaRows = 4;
 constexpr int kAccumCols = 64;
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
-fox_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int64_t o_st,
-                 const uint16_t* __restrict__ d_o, int64_t d_sb, int64_t d_sh, int64_t d_st, int H, int M, int D,
-                 float* __restrict__ delta, float* __restrict__ dq_acc, int acc_cols, float* __restrict__ dlam_row) {
+fox_delta_kernel(const uint16_t* o, int64_t o_sb, int64_t o_sh, int64_t o_st, const uint16_t* d_o, int64_t d_sb, int64_t d_sh,
+                 int64_t d_st, int H, int M, int D, float* delta, float* dq_acc, int acc_cols, float* dlam_row) {
   const int lanes_per_row = D / 8;
   const int rows_per_pass = 256 / lanes_per_row;
   const int bh = blockIdx.y, b = bh / H, h = bh % H;
@@ -499,6 +496,7 @@ fox_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int
   const uint16_t* ob = o + b * o_sb + h * o_sh + sub * 8;
   const uint16_t* gb = d_o + b * d_sb + h * d_sh + sub * 8;
   uint4 a[kDeltaRows], g[kDeltaRows];
+  wait_for_kernel_in_front();
 #pragma unroll
   for (int i = 0; i < kDeltaRows; ++i) {
     const int row = row0 + i * rows_per_pass;
@@ -584,6 +582,7 @@ template <int kIn, bool kBf16>
 __global__ void __launch_bounds__(kScanThreads)
 fox_bwd_finish_kernel(const RevParams rev, const ConvParams conv, int scan_blocks) {
   __shared__ float red[32];
+  wait_for_kernel_in_front();
   if (static_cast<int>(blockIdx.x) < scan_blocks) revcumsum_rows<kIn>(rev, blockIdx.x, red);
   else convert_rows<kBf16>(conv, blockIdx.x - scan_blocks);
 }
@@ -645,17 +644,16 @@ static int launch_finish(cudaStream_t st, int gate_kind, bool bf16, const RevPar
   const int64_t grid = scan_blocks + static_cast<int64_t>(conv.units) * conv.blocks_per_bh;
   if (grid <= 0 || grid > 2147483647LL) return FOX_ERR_TOO_LARGE;
   switch (gate_kind) {
-#define FOX_FIN(K)                                                                                          \
-  if (bf16) fox_bwd_finish_kernel<K, true><<<(unsigned)grid, kScanThreads, 0, st>>>(rev, conv, scan_blocks); \
-  else fox_bwd_finish_kernel<K, false><<<(unsigned)grid, kScanThreads, 0, st>>>(rev, conv, scan_blocks)
-    case FOX_DTYPE_FP16: FOX_FIN(0); break;
-    case FOX_DTYPE_BF16: FOX_FIN(1); break;
-    case FOX_DTYPE_FP32: FOX_FIN(2); break;
-    case FOX_GATE_LOG: FOX_FIN(3); break;
+#define FOX_FIN(K)                                                                                              \
+  return launch_behind(bf16 ? fox_bwd_finish_kernel<K, true> : fox_bwd_finish_kernel<K, false>, dim3((unsigned)grid), \
+                       kScanThreads, 0, st, rev, conv, scan_blocks)
+    case FOX_DTYPE_FP16: FOX_FIN(0);
+    case FOX_DTYPE_BF16: FOX_FIN(1);
+    case FOX_DTYPE_FP32: FOX_FIN(2);
+    case FOX_GATE_LOG: FOX_FIN(3);
 #undef FOX_FIN
     default: return FOX_ERR_BAD_ARG;
   }
-  return launch_rc();
 }
 
 extern "C" int fox_revcumsum(int device, void* stream, int64_t B, int64_t H, int64_t M, int64_t N,
@@ -746,18 +744,17 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
   const unsigned grid = (unsigned)(B * H * (1 + ks.n_parts + qs.n_parts));
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == FOX_DTYPE_BF16;
-#define FOX_PRO(K)                                                                                                       \
-  if (bf) fox_prologue_kernel<K, true><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D); \
-  else fox_prologue_kernel<K, false><<<grid, kScanThreads, 0, st>>>(gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D)
+#define FOX_PRO(K)                                                                                                        \
+  return launch_behind(bf ? fox_prologue_kernel<K, true> : fox_prologue_kernel<K, false>, dim3(grid), kScanThreads, 0, st, gates, \
+                       sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D)
   switch (gate_kind) {
-    case FOX_DTYPE_FP16: FOX_PRO(0); break;
-    case FOX_DTYPE_BF16: FOX_PRO(1); break;
-    case FOX_DTYPE_FP32: FOX_PRO(2); break;
-    case FOX_GATE_LOG: FOX_PRO(3); break;
+    case FOX_DTYPE_FP16: FOX_PRO(0);
+    case FOX_DTYPE_BF16: FOX_PRO(1);
+    case FOX_DTYPE_FP32: FOX_PRO(2);
+    case FOX_GATE_LOG: FOX_PRO(3);
     default: return FOX_ERR_BAD_ARG;
   }
 #undef FOX_PRO
-  return launch_rc();
 }
 
 static int launch_index(int device, cudaStream_t st, int64_t B, IndexParams p) {
@@ -770,8 +767,7 @@ static int launch_index(int device, cudaStream_t st, int64_t B, IndexParams p) {
     if (cudaFuncSetAttribute(fox_find_index_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return FOX_ERR_LAUNCH;
   }
-  fox_find_index_kernel<<<(unsigned)(B * p.H), kIndexThreads, smem, st>>>(p);
-  return launch_rc();
+  return launch_behind(fox_find_index_kernel, dim3((unsigned)(B * p.H)), kIndexThreads, (int)smem, st, p);
 }
 
 extern "C" int fox_attn_index(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N,
@@ -841,13 +837,9 @@ static int launch_delta(int device, void* stream, int dtype, int64_t B, int64_t 
   const int rows_per_block = kDeltaRows * 256 / (int)(D / 8);
   const int acc_cols = (int)(D > kAccumCols ? D : kAccumCols);
   dim3 grid((unsigned)((M + rows_per_block - 1) / rows_per_block), (unsigned)(B * H));
-#define FOX_DELTA(BF)                                                                                                  \
-  fox_delta_kernel<BF><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)o->ptr, o->sb, o->sh, o->st,             \
-      (const uint16_t*)d_o->ptr, d_o->sb, d_o->sh, d_o->st, (int)H, (int)M, (int)D, delta, dq_accum, acc_cols, dlam_row)
-  if (dtype == FOX_DTYPE_BF16) FOX_DELTA(true);
-  else FOX_DELTA(false);
-#undef FOX_DELTA
-  return launch_rc();
+  return launch_behind(dtype == FOX_DTYPE_BF16 ? fox_delta_kernel<true> : fox_delta_kernel<false>, grid, 256, 0, (cudaStream_t)stream,
+                       (const uint16_t*)o->ptr, o->sb, o->sh, o->st, (const uint16_t*)d_o->ptr, d_o->sb, d_o->sh, d_o->st, (int)H,
+                       (int)M, (int)D, delta, dq_accum, acc_cols, dlam_row);
 }
 
 extern "C" int fox_bwd_delta(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t D,

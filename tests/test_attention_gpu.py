@@ -701,3 +701,51 @@ def test_items_by_length_are_each_taken_once(H, T, D):
                 assert (a[:, h:h + 1].double() - b.double()).norm() <= 2 ** -8 * b.double().norm() + 1e-30
             else:
                 assert torch.equal(a[:, h:h + 1], b), (h, i)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("T,D,thr", [(100, 64, None), (700, 128, -6.0), (1500, 64, "auto"), (2100, 128, None)])
+def test_kernels_begun_behind_one_another_read_finished_inputs(T, D, thr, graph):
+    """The kernels of a pass take their SMs before the one in front has written back.  Inputs written by the kernels directly in front,
+    passes one behind the other into memory that the allocator hands on, and a capture that joins another stream in front: the
+    results of a pass that is alone, bit by bit (dQ at D=64, summed in any order: to rounding)."""
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    base = [torch.randn(1, 5, T, D, generator=gen, device="cuda").bfloat16() for _ in range(4)]
+    base.append(torch.nn.functional.logsigmoid(torch.randn(1, 5, T, generator=gen, device="cuda") + 1))
+    kw = {} if thr is None else dict(adaptive_threshold=thr)
+    scales = [1.0, 0.5, 2.0]
+
+    def run(scale):
+        q, k, v, do, g = [t * scale for t in base]
+        x = [t.requires_grad_() for t in (q, k, v, g)]
+        out = fox.forgetting_attention(*x, head_first=True, **kw)
+        return [out.detach(), *torch.autograd.grad(out, x, do)]
+
+    alone = []
+    for s in scales:
+        torch.cuda.synchronize()
+        alone.append(run(s))
+        torch.cuda.synchronize()
+    if graph:
+        main, side = torch.cuda.Stream(), torch.cuda.Stream()
+        g = torch.cuda.CUDAGraph()
+        main.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.graph(g, stream=main):
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                base[0].mul_(1.0)
+            main.wait_stream(side)
+            together = [run(s) for s in scales]
+        for _ in range(3):
+            g.replay()
+    else:
+        for _ in range(4):
+            together = [run(s) for s in scales]
+    torch.cuda.synchronize()
+    for a, b in zip(together, alone):
+        for i, (x, y) in enumerate(zip(a, b)):
+            if D == 64 and i in (1, 4):     # dQ, and the gate gradient through its row sums
+                assert (x.double() - y.double()).norm() <= 2 ** -8 * y.double().norm()
+            else:
+                assert torch.equal(x, y), i
