@@ -614,9 +614,9 @@ static int launch_decode_at(const DecodeParams& p, int64_t B, cudaStream_t st) {
 // Four per SM (64 registers instead of 80, no spills) share the same bandwidth, so that a range takes a third longer; they are
 // taken where the waves are fewer by so much that this pays, counted in keys with 600 for a wave's start: 512 (b,h) of 4000
 // keys of 128 in one wave instead of three 192 -> 162 us, of 64 102 -> 86; 256 of 4099 of 128 in one instead of two 98 -> 91, of 2048
-// 54 -> 48.  With as many waves they pay where they fill one that three leave half empty and the ranges are long: 256 of 1500 of 128
-// in two ranges instead of one 43 -> 37, 144 of 2600 of 64 in three instead of two 24.7 -> 22.7, but 256 of 1000 of 64 17.8 and 18.5, 176 of
-// 1200 16.4 and 17.2.  Else they are no faster or slower: 384 of 8000 of 64 130 and 135, 32 of 3000 13.7 and 14.3, 4 of 30000 of 128 21.2
+// 54 -> 48.  With as many waves they pay where they fill one that three leave half empty (a (b,h) in two ranges instead of one) and
+// the ranges are long: 256 of 1500 of 128 43 -> 37, but of 1000 of 64 17.8 and 18.5, 176 of 1200 16.4 and 17.2.  More ranges than two in
+// the same wave change little (144 of 2600 of 64 in three instead of two 24.7 and 22.7).  Else they are no faster or slower: 384 of 8000 of 64 130 and 135, 32 of 3000 13.7 and 14.3, 4 of 30000 of 128 21.2
 // and 22.5, 768 of 2500 of 64 86 and 91; 24 x 65536 70.0 and 70.0.
 struct DecodePlan {
   int64_t splits;
@@ -646,7 +646,7 @@ static DecodePlan decode_plan(int64_t bh, int64_t N) {
   auto waves = [&](int64_t s, int64_t slots, int64_t cluster_slots) { return waves_of(bh * s, s > 1 && s <= kDecMaxCluster ? cluster_slots : slots); };
   const int64_t w3 = waves(s3, kDecSlots, kDecClusterSlots), w4 = waves(s4, kDecMoreSlots, kDecMoreClusterSlots);
   const int64_t t3 = w3 * (N / s3 + kDecStartKeys), t4 = w4 * (N / s4 * kDecMorePerSm / kDecPerSm + kDecStartKeys);
-  const bool more = w4 < w3 ? t4 < t3 : w4 == w3 && t4 < t3 - t3 / 20 && N / s4 >= kDecMoreLeastKeys;
+  const bool more = w4 < w3 ? t4 < t3 : w4 == w3 && s3 == 1 && t4 < t3 - t3 / 20 && N / s4 >= kDecMoreLeastKeys;
   return more ? DecodePlan{s4, kDecMorePerSm} : DecodePlan{s3, kDecPerSm};
 }
 template <bool kBf16, int D>
