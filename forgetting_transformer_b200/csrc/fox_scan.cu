@@ -415,6 +415,9 @@ fox_max_row_norm_kernel(const uint16_t* __restrict__ x, int64_t sb, int64_t sh, 
 // (n_q-th) group of rows and write ONE partial maximum, so nothing has to be zeroed first; the reader takes the
 // maximum of the parts.  All blocks lie on the grid's x axis, one (b, h) behind the other: y ends at 65535, and with the
 // parts on the slow axis the scans start first but the norms' reads spread over all (b, h), 1.5 % slower where they are long.
+// Two blocks to an SM, at most 32 registers a thread: bf16 took 42 by itself and had one, whose loads and reductions took turns
+// (keys alone, 48 (b,h) of 16384 x 64: 30.0 -> 25.0 us, 512 of 2048 x 64 43.2 -> 34.4, 32 of 2048 x 128 9.5 -> 7.2; with queries, 64 of
+// 16384 x 128: 113.8 -> 101.4; 4 of 9000 x 128, whose scans are the longest, 8.4 and 8.7).
 struct NormSource {
   const uint16_t* x;
   int64_t sb, sh, st;
@@ -467,7 +470,7 @@ __device__ __forceinline__ void norm_part(const NormSource& s, int D, int H, int
 }
 
 template <int kIn, bool kBf16>
-__global__ void __launch_bounds__(kScanThreads)
+__global__ void __launch_bounds__(kScanThreads, 2)
 fox_prologue_kernel(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float* lam, const NormSource k, const NormSource q, int H, int N, int D) {
   __shared__ float red[32];
   const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
@@ -706,8 +709,7 @@ extern "C" int64_t fox_norm_parts(int64_t B, int64_t H, int64_t T, int64_t D) {
 }
 
 // The same for keys alone, whose blocks share a launch with those of the prefix scans, one a (b,h).  Where fewer parts make two
-// blocks per SM nearly full (at a time for fp16, one after the other for bf16, whose blocks take more than 32 registers a
-// thread), that is faster than a few blocks more behind them (48 (b,h) of 16384 x 64: 36 -> 30 us; 24 of 11000 x 64: 16 -> 13),
+// blocks per SM nearly full, that is faster than a few blocks more behind them (fp16; 24 (b,h) of 11000 x 64: 16 -> 13 us),
 // unless the parts left have to be much longer: 2 -> 1 part never (148 of 4096 x 128: 42 -> 51), 3 -> 2 not with long rows in many
 // (96 of 8192 x 128: 49 -> 53, of 4096 29 -> 28), and 4 -> 3 only in a fuller wave (70 of 4096 x 128, 280 blocks: 20 -> 22; 71, 284
 // blocks: 22.3 -> 21.6).  Long rows of 16 or 32 channels keep theirs as well: their blocks are bound by instructions (fp16, 24 of
