@@ -166,8 +166,8 @@ int fox_attn_decode(int device, void* stream, int dtype, int64_t B, int64_t H, i
                     float* L, float* workspace, int64_t splits);
 int64_t fox_attn_decode_workspace_floats(int64_t B, int64_t H, int64_t D, int64_t splits);
 /* The same from the log gates (fp32, element strides sb, sh, sn) instead of their prefix sum, without pruning.
- * splits for both from fox_attn_decode_splits; D in {16,32,64,128}.  programmatic != 0: launched with programmatic stream
- * serialization behind another kernel of this library. */
+ * splits for both from fox_attn_decode_splits; D in {16,32,64,128}.  programmatic != 0: one of a chain of
+ * this library's kernels, whose next may begin while this one runs (it waits for its end). */
 int fox_attn_decode_gates(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t N, int64_t D,
                           const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v, const float* log_fgate,
                           int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float sm_scale,

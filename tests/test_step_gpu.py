@@ -339,3 +339,29 @@ def test_decode_by_four_ctas_of_an_sm(B, H, N, D, splits, padded):
     three; the ranges of fewer CTAs to an SM would be others."""
     assert _lib.load().fox_attn_decode_splits(B, H, N) == splits
     test_decode_from_gates(B, H, N, D, padded)
+
+
+@pytest.mark.parametrize("B,H,N,D,thr", [(1, 2, 90, 64, None), (16, 30, 700, 64, None), (1, 3, 20000, 128, None), (2, 4, 3000, 64, -4.0)])
+def test_decode_calls_behind_one_another(B, H, N, D, thr):
+    """A call's kernels begin behind whatever is in front: inputs written just before, results in memory that the allocator hands on.
+    One range a (b,h), clusters, ranges merged by a second kernel, and a pruned call: the bits of calls that are alone."""
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v = (torch.randn(B, H, n, D, generator=gen, device="cuda").bfloat16() for n in (1, N, N))
+    g = torch.nn.functional.logsigmoid(torch.randn(B, H, N, generator=gen, device="cuda") + 3)
+    kw = {} if thr is None else dict(adaptive_threshold=thr)
+
+    def run(scale):
+        with torch.no_grad():
+            return fox.forgetting_attention(q * scale, k * scale, v * scale, g * scale, head_first=True, **kw)
+
+    scales = [1.0, 0.5, 2.0]
+    alone = []
+    for s in scales:
+        torch.cuda.synchronize()
+        alone.append(run(s))
+        torch.cuda.synchronize()
+    for _ in range(5):
+        together = [run(s) for s in scales]
+    torch.cuda.synchronize()
+    for a, b in zip(together, alone):
+        assert torch.equal(a, b)
