@@ -472,7 +472,7 @@ fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeSt
 template <bool kBf16, int D>
 __global__ void __launch_bounds__(256) fox_decode_merge_kernel(const DecodeParams p) {
   __shared__ float s_w[kDecMaxSplits], s_l[kDecMaxSplits], s_g[kDecMaxSplits], s_o[256], s_top, s_sum;
-  wait_for_kernel_in_front();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (p.chained) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int64_t bh = static_cast<int64_t>(b) * p.H + h;

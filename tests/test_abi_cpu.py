@@ -220,6 +220,26 @@ def test_kernels_that_begin_early_take_no_invariant_pointers():
     assert found == 5
 
 
+def test_kernels_launched_behind_another_take_no_invariant_pointers():
+    """The same for those that wait by wait_for_kernel_in_front(): each kernel that launch_behind() is given, and the functions it
+    calls in its file."""
+    waiting = set()
+    for name in build.SOURCES:
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(build.CSRC, name)).read())
+        for kernel in re.split(r"__global__", text)[1:]:
+            params, body = kernel.split("{", 1)
+            body = body.split("\n}\n", 1)[0]
+            if "wait_for_kernel_in_front()" in body:
+                waiting.add(re.search(r"(fox_\w+_kernel)\s*\(", params).group(1))
+                used = [f for f in re.split(r"__device__", text)[1:] if re.search(r"\b%s(<\w+>)?\(" % re.search(r"(\w+)\s*\(", f).group(1), body)]
+                assert not any("__restrict__" in f.split("\n}\n", 1)[0] or "__ldg" in f.split("\n}\n", 1)[0] for f in used), (name, params)
+                assert "__restrict__" not in params + body and "__ldg" not in body, (name, params)
+    assert {"fox_attn_fwd_kernel", "fox_attn_bwd_kernel", "fox_attn_bwd_kv_kernel", "fox_attn_bwd_dq2_kernel", "fox_find_index_kernel",
+            "fox_prologue_kernel", "fox_delta_kernel", "fox_bwd_finish_kernel"} <= waiting
+
+
 @pytest.mark.parametrize("bh", [1, 9, 10, 24, 35, 48, 60, 64, 70, 71, 96, 98, 99, 140, 147, 148, 149, 296, 297, 4000])
 @pytest.mark.parametrize("n,d", [(1024, 64), (4096, 128), (8192, 128), (16384, 64), (1024, 16), (12300, 16), (2 ** 24, 128)])
 def test_key_norm_parts_fill_a_wave_and_stay_short(bh, n, d):
