@@ -85,6 +85,7 @@ __device__ __forceinline__ void mix_load(const MixParams& p, int64_t t, bool on,
 // the instructions for addresses and sums: 199 and 13 us.)
 template <bool kBf16, int kLanes>
 __global__ void __launch_bounds__(kMixThreads, 4) fox_mix_fwd_kernel(const MixParams p) {
+  wait_for_kernel_in_front();
   if (static_cast<int>(blockIdx.x) >= p.mix_blocks) {
     __shared__ unsigned long long s_sum;
     const int b = blockIdx.x - p.mix_blocks;
@@ -214,6 +215,7 @@ __device__ __forceinline__ void mix_rows_load(const MixRows& p, uint32_t i, uint
 // -> 14.2 us.  (112 registers for a third CTA: 130 and 15.2 us; 96: 177; prefetching the next rows into L1: 122.)
 template <bool kBf16, int kLanes>
 __global__ void __launch_bounds__(kMixThreads, 2) fox_mix_bwd_kernel(const MixBwdParams p) {
+  wait_for_kernel_in_front();
   const MixParams& f = p.f;
   const int lanes = kLanes ? kLanes : f.D >> 3, C = f.H * f.D;
   const int h = threadIdx.x / lanes, sub = threadIdx.x % lanes;
@@ -372,6 +374,7 @@ struct PackParams {
 };
 
 __global__ void __launch_bounds__(256) fox_pack_kernel(const PackParams p) {
+  wait_for_kernel_in_front();
   if (static_cast<int>(blockIdx.x) < p.vec_blocks) {
     for (int i = 0; i < p.n_vecs; ++i) {
       for (int e = blockIdx.x * 256 + threadIdx.x; e < p.vec_len[i]; e += p.vec_blocks * 256) {
@@ -422,6 +425,7 @@ struct UnpackParams {
 };
 
 __global__ void __launch_bounds__(256) fox_unpack_kernel(const UnpackParams p) {
+  wait_for_kernel_in_front();
   const int per_row = p.C / 8;
   const int64_t total = static_cast<int64_t>(p.mat_row0[p.n_mats]) * per_row, step = static_cast<int64_t>(gridDim.x) * 256;
   constexpr int kU = 4;
@@ -454,6 +458,7 @@ struct SumParams {
 };
 
 __global__ void __launch_bounds__(1024) fox_column_sums_kernel(const SumParams p) {
+  wait_for_kernel_in_front();
   __shared__ float s[32][33];
   int i = 0;
   while (i + 1 < p.n && static_cast<int>(blockIdx.x) >= p.block0[i + 1]) ++i;
@@ -480,7 +485,6 @@ __global__ void __launch_bounds__(1024) fox_column_sums_kernel(const SumParams p
   }
 }
 
-static inline int blk_rc() { return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH; }
 
 static int mix_params(MixParams& p, int64_t B, int64_t T, int64_t H, int64_t D, const void* y, int64_t ld, const float* wq,
                       const float* wk, const int64_t* mask, float eps) {
@@ -523,8 +527,7 @@ extern "C" int fox_mix_fwd(int device, void* stream, int dtype, int64_t B, int64
   auto kern = D == 64 ? (bf ? fox_mix_fwd_kernel<true, 8> : fox_mix_fwd_kernel<false, 8>)
               : D == 128 ? (bf ? fox_mix_fwd_kernel<true, 16> : fox_mix_fwd_kernel<false, 16>)
                          : (bf ? fox_mix_fwd_kernel<true, 0> : fox_mix_fwd_kernel<false, 0>);
-  kern<<<grid, mix_threads(p), 0, (cudaStream_t)stream>>>(p);
-  return blk_rc();
+  return launch_behind(kern, dim3(grid), mix_threads(p), 0, (cudaStream_t)stream, p);
 }
 
 extern "C" int64_t fox_mix_bwd_partials(int64_t tokens) {
@@ -554,8 +557,7 @@ extern "C" int fox_mix_bwd(int device, void* stream, int dtype, int64_t B, int64
   auto kern = D == 64 ? (bf ? fox_mix_bwd_kernel<true, 8> : fox_mix_bwd_kernel<false, 8>)
               : D == 128 ? (bf ? fox_mix_bwd_kernel<true, 16> : fox_mix_bwd_kernel<false, 16>)
                          : (bf ? fox_mix_bwd_kernel<true, 0> : fox_mix_bwd_kernel<false, 0>);
-  kern<<<(unsigned)n_partials, mix_threads(p.f), 0, (cudaStream_t)stream>>>(p);
-  return blk_rc();
+  return launch_behind(kern, dim3((unsigned)n_partials), mix_threads(p.f), 0, (cudaStream_t)stream, p);
 }
 
 extern "C" int fox_pack(int device, void* stream, int64_t n_mats, const void* const* mats, const int64_t* mat_rows, int64_t rows,
@@ -591,8 +593,7 @@ extern "C" int fox_pack(int device, void* stream, int64_t n_mats, const void* co
   int64_t blocks = (rows * (cols / 8) + 256 * 4 - 1) / (256 * 4);
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks + p.vec_blocks == 0) return FOX_OK;
-  fox_pack_kernel<<<(unsigned)(blocks + p.vec_blocks), 256, 0, (cudaStream_t)stream>>>(p);
-  return blk_rc();
+  return launch_behind(fox_pack_kernel, dim3((unsigned)(blocks + p.vec_blocks)), 256, 0, (cudaStream_t)stream, p);
 }
 
 extern "C" int fox_unpack(int device, void* stream, int64_t n_mats, void* const* mats, const int64_t* mat_rows, int64_t cols,
@@ -614,8 +615,7 @@ extern "C" int fox_unpack(int device, void* stream, int64_t n_mats, void* const*
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   int64_t blocks = (row * (cols / 8) + 256 * 4 - 1) / (256 * 4);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  fox_unpack_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(p);
-  return blk_rc();
+  return launch_behind(fox_unpack_kernel, dim3((unsigned)blocks), 256, 0, (cudaStream_t)stream, p);
 }
 
 extern "C" int fox_column_sums(int device, void* stream, int64_t n, const float* const* parts, const int64_t* rows,
@@ -632,6 +632,5 @@ extern "C" int fox_column_sums(int device, void* stream, int64_t n, const float*
   p.block0[n] = (int)block;
   p.n = (int)n;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  fox_column_sums_kernel<<<(unsigned)block, 1024, 0, (cudaStream_t)stream>>>(p);
-  return blk_rc();
+  return launch_behind(fox_column_sums_kernel, dim3((unsigned)block), 1024, 0, (cudaStream_t)stream, p);
 }

@@ -39,8 +39,9 @@ __device__ __forceinline__ void glu_store8(uint16_t* p, const float* f) {
 
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
-fox_swiglu_fwd_kernel(const uint16_t* __restrict__ x, int64_t x_sr, const uint16_t* __restrict__ y, int64_t y_sr,
-                      uint16_t* __restrict__ z, int64_t z_sr, int64_t rows, int64_t cols) {
+fox_swiglu_fwd_kernel(const uint16_t* x, int64_t x_sr, const uint16_t* y, int64_t y_sr,
+                      uint16_t* z, int64_t z_sr, int64_t rows, int64_t cols) {
+  wait_for_kernel_in_front();
   const int64_t vec_per_row = cols >> 3;
   const int64_t n = rows * vec_per_row;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * 256) {
@@ -56,10 +57,11 @@ fox_swiglu_fwd_kernel(const uint16_t* __restrict__ x, int64_t x_sr, const uint16
 
 template <bool kBf16, bool kWithZ>
 __global__ void __launch_bounds__(256)
-fox_swiglu_bwd_kernel(const uint16_t* __restrict__ x, int64_t x_sr, const uint16_t* __restrict__ y, int64_t y_sr,
-                      const uint16_t* __restrict__ g, int64_t g_sr, uint16_t* __restrict__ dx, int64_t dx_sr,
-                      uint16_t* __restrict__ dy, int64_t dy_sr, uint16_t* __restrict__ z, int64_t z_sr, int64_t rows,
+fox_swiglu_bwd_kernel(const uint16_t* x, int64_t x_sr, const uint16_t* y, int64_t y_sr,
+                      const uint16_t* g, int64_t g_sr, uint16_t* dx, int64_t dx_sr,
+                      uint16_t* dy, int64_t dy_sr, uint16_t* z, int64_t z_sr, int64_t rows,
                       int64_t cols) {
+  wait_for_kernel_in_front();
   const int64_t vec_per_row = cols >> 3;
   const int64_t n = rows * vec_per_row;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * 256) {
@@ -107,11 +109,8 @@ extern "C" int fox_swiglu_fwd(int device, void* stream, int dtype, int64_t rows,
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   const unsigned grid = glu_grid(rows, cols);
   cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == FOX_DTYPE_BF16)
-    fox_swiglu_fwd_kernel<true><<<grid, 256, 0, st>>>((const uint16_t*)x, x_row_stride, (const uint16_t*)y, y_row_stride, (uint16_t*)z, z_row_stride, rows, cols);
-  else
-    fox_swiglu_fwd_kernel<false><<<grid, 256, 0, st>>>((const uint16_t*)x, x_row_stride, (const uint16_t*)y, y_row_stride, (uint16_t*)z, z_row_stride, rows, cols);
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  return launch_behind(dtype == FOX_DTYPE_BF16 ? fox_swiglu_fwd_kernel<true> : fox_swiglu_fwd_kernel<false>, dim3(grid), 256, 0, st,
+                       (const uint16_t*)x, x_row_stride, (const uint16_t*)y, y_row_stride, (uint16_t*)z, z_row_stride, rows, cols);
 }
 
 extern "C" int fox_swiglu_bwd(int device, void* stream, int dtype, int64_t rows, int64_t cols, const void* x,
@@ -125,15 +124,8 @@ extern "C" int fox_swiglu_bwd(int device, void* stream, int dtype, int64_t rows,
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   const unsigned grid = glu_grid(rows, cols);
   cudaStream_t st = (cudaStream_t)stream;
-#define FOX_GLU_BWD(BF, WZ)                                                                                          \
-  fox_swiglu_bwd_kernel<BF, WZ><<<grid, 256, 0, st>>>((const uint16_t*)x, x_row_stride, (const uint16_t*)y, y_row_stride, \
-                                                     (const uint16_t*)g, g_row_stride, (uint16_t*)dx, dx_row_stride,  \
-                                                     (uint16_t*)dy, dy_row_stride, (uint16_t*)z, z_row_stride, rows, cols)
-  if (dtype == FOX_DTYPE_BF16) {
-    if (z) FOX_GLU_BWD(true, true); else FOX_GLU_BWD(true, false);
-  } else {
-    if (z) FOX_GLU_BWD(false, true); else FOX_GLU_BWD(false, false);
-  }
-#undef FOX_GLU_BWD
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  auto kern = dtype == FOX_DTYPE_BF16 ? (z ? fox_swiglu_bwd_kernel<true, true> : fox_swiglu_bwd_kernel<true, false>)
+                                      : (z ? fox_swiglu_bwd_kernel<false, true> : fox_swiglu_bwd_kernel<false, false>);
+  return launch_behind(kern, dim3(grid), 256, 0, st, (const uint16_t*)x, x_row_stride, (const uint16_t*)y, y_row_stride, (const uint16_t*)g,
+                       g_row_stride, (uint16_t*)dx, dx_row_stride, (uint16_t*)dy, dy_row_stride, (uint16_t*)z, z_row_stride, rows, cols);
 }

@@ -61,14 +61,15 @@ __device__ __forceinline__ void store8(uint16_t* p, const float* f) {
 }
 
 template <bool kBf16, bool kGate>
-__global__ void fox_normgate_fwd_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ g,
-                                        const float* __restrict__ w, uint16_t* __restrict__ y,
-                                        float* __restrict__ rstd, int64_t tokens, int G, int D, float eps, int64_t g_ld) {
+__global__ void fox_normgate_fwd_kernel(const uint16_t* x, const uint16_t* g,
+                                        const float* w, uint16_t* y,
+                                        float* rstd, int64_t tokens, int G, int D, float eps, int64_t g_ld) {
   const int lanes = D >> 3;
   const int tid = threadIdx.x;
   const int h = tid / lanes, sub = tid % lanes;
   const bool active = h < G;
   const int ch = active ? h * D + sub * 8 : 0;
+  wait_for_kernel_in_front();
   float wv[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) wv[j] = active ? w[ch + j] : 0.f;
@@ -111,16 +112,17 @@ __global__ void fox_normgate_fwd_kernel(const uint16_t* __restrict__ x, const ui
 }
 
 template <bool kBf16, bool kGate>
-__global__ void fox_normgate_bwd_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ g,
-                                        const float* __restrict__ w, const float* __restrict__ rstd,
-                                        const uint16_t* __restrict__ dy, uint16_t* __restrict__ dx,
-                                        uint16_t* __restrict__ dg, float* __restrict__ dw_partial, int64_t tokens,
+__global__ void fox_normgate_bwd_kernel(const uint16_t* x, const uint16_t* g,
+                                        const float* w, const float* rstd,
+                                        const uint16_t* dy, uint16_t* dx,
+                                        uint16_t* dg, float* dw_partial, int64_t tokens,
                                         int G, int D, int64_t g_ld, int64_t dg_ld) {
   const int lanes = D >> 3;
   const int tid = threadIdx.x;
   const int h = tid / lanes, sub = tid % lanes;
   const bool active = h < G;
   const int ch = active ? h * D + sub * 8 : 0;
+  wait_for_kernel_in_front();
   float wv[8], dwv[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -196,16 +198,10 @@ extern "C" int fox_normgate_fwd_ld(int device, void* stream, int dtype, int64_t 
     return FOX_ERR_ALIGNMENT;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   const int64_t grid = tokens < 148 * 16 ? tokens : 148 * 16;
-#define FOX_NG_FWD(BF, GATE)                                                                      \
-  fox_normgate_fwd_kernel<BF, GATE><<<(unsigned)grid, threads, 0, (cudaStream_t)stream>>>(          \
-      (const uint16_t*)x, (const uint16_t*)g, w, (uint16_t*)y, rstd, tokens, (int)G, (int)D, eps, g_ld)
-  if (dtype == FOX_DTYPE_BF16) {
-    if (g) FOX_NG_FWD(true, true); else FOX_NG_FWD(true, false);
-  } else {
-    if (g) FOX_NG_FWD(false, true); else FOX_NG_FWD(false, false);
-  }
-#undef FOX_NG_FWD
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  auto kern = dtype == FOX_DTYPE_BF16 ? (g ? fox_normgate_fwd_kernel<true, true> : fox_normgate_fwd_kernel<true, false>)
+                                      : (g ? fox_normgate_fwd_kernel<false, true> : fox_normgate_fwd_kernel<false, false>);
+  return launch_behind(kern, dim3((unsigned)grid), threads, 0, (cudaStream_t)stream, (const uint16_t*)x, (const uint16_t*)g, w,
+                       (uint16_t*)y, rstd, tokens, (int)G, (int)D, eps, g_ld);
 }
 
 extern "C" int fox_normgate_bwd(int device, void* stream, int dtype, int64_t tokens, int64_t G, int64_t D,
@@ -229,15 +225,8 @@ extern "C" int fox_normgate_bwd_ld(int device, void* stream, int dtype, int64_t 
        reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dg) | reinterpret_cast<uintptr_t>(dw_partial)) % 16)
     return FOX_ERR_ALIGNMENT;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-#define FOX_NG_BWD(BF, GATE)                                                                          \
-  fox_normgate_bwd_kernel<BF, GATE><<<(unsigned)n_partials, threads, 0, (cudaStream_t)stream>>>(        \
-      (const uint16_t*)x, (const uint16_t*)g, w, rstd, (const uint16_t*)dy, (uint16_t*)dx, (uint16_t*)dg, \
-      dw_partial, tokens, (int)G, (int)D, g_ld, dg_ld)
-  if (dtype == FOX_DTYPE_BF16) {
-    if (g) FOX_NG_BWD(true, true); else FOX_NG_BWD(true, false);
-  } else {
-    if (g) FOX_NG_BWD(false, true); else FOX_NG_BWD(false, false);
-  }
-#undef FOX_NG_BWD
-  return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH;
+  auto kern = dtype == FOX_DTYPE_BF16 ? (g ? fox_normgate_bwd_kernel<true, true> : fox_normgate_bwd_kernel<true, false>)
+                                      : (g ? fox_normgate_bwd_kernel<false, true> : fox_normgate_bwd_kernel<false, false>);
+  return launch_behind(kern, dim3((unsigned)n_partials), threads, 0, (cudaStream_t)stream, (const uint16_t*)x, (const uint16_t*)g, w, rstd,
+                       (const uint16_t*)dy, (uint16_t*)dx, (uint16_t*)dg, dw_partial, tokens, (int)G, (int)D, g_ld, dg_ld);
 }

@@ -237,7 +237,9 @@ def test_kernels_launched_behind_another_take_no_invariant_pointers():
                 assert not any("__restrict__" in f.split("\n}\n", 1)[0] or "__ldg" in f.split("\n}\n", 1)[0] for f in used), (name, params)
                 assert "__restrict__" not in params + body and "__ldg" not in body, (name, params)
     assert {"fox_attn_fwd_kernel", "fox_attn_bwd_kernel", "fox_attn_bwd_kv_kernel", "fox_attn_bwd_dq2_kernel", "fox_find_index_kernel",
-            "fox_prologue_kernel", "fox_delta_kernel", "fox_bwd_finish_kernel"} <= waiting
+            "fox_prologue_kernel", "fox_delta_kernel", "fox_bwd_finish_kernel", "fox_mix_fwd_kernel", "fox_mix_bwd_kernel", "fox_pack_kernel",
+            "fox_unpack_kernel", "fox_column_sums_kernel", "fox_swiglu_fwd_kernel", "fox_swiglu_bwd_kernel", "fox_normgate_fwd_kernel",
+            "fox_normgate_bwd_kernel"} <= waiting
 
 
 @pytest.mark.parametrize("bh", [1, 9, 10, 24, 35, 48, 60, 64, 70, 71, 96, 98, 99, 140, 147, 148, 149, 296, 297, 4000])
