@@ -102,6 +102,10 @@ fox_rmsnorm_bwd_kernel(const uint16_t* __restrict__ z_saved, const float* __rest
   for (int64_t row = static_cast<int64_t>(blockIdx.x) * kRnWarps + warp; row < rows;
        row += static_cast<int64_t>(gridDim.x) * kRnWarps) {
     const float r = rstd[row];
+    // 1024 channels: the weights are read again for each row (from L1).  Kept in registers across rows they made it 155 a thread and one CTA
+    // to an SM; with 128 there are two (4096 rows 21.5 -> 9.8 us, 8192 30.7 -> 13.6).  768 channels have two either way, 1280 and more one.
+    const float* wr = w;
+    if (VPL == 4) asm volatile("" : "+l"(wr));
     float xhat[VPL][8], wdy[VPL][8];
     float c1 = 0.f;
 #pragma unroll
@@ -111,7 +115,7 @@ fox_rmsnorm_bwd_kernel(const uint16_t* __restrict__ z_saved, const float* __rest
       float zz[8], d[8];
       rn_load8<kBf16>(z_saved + off, zz);
       rn_load8<kBf16>(dy + off, d);
-      const float4 w0 = *reinterpret_cast<const float4*>(w + col), w1 = *reinterpret_cast<const float4*>(w + col + 4);
+      const float4 w0 = *reinterpret_cast<const float4*>(wr + col), w1 = *reinterpret_cast<const float4*>(wr + col + 4);
       const float wv[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
