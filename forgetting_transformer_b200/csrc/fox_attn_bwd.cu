@@ -240,9 +240,9 @@ fox_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int i = mb_ * kBwdBM + rr * 32 + lane;
           const bool in = i < M;
           const int ic = in ? i : 0;
-          const float l_ = ldg_f32_here(p.L + bh * M + ic);
-          const float a_ = ldg_f32_here(p.lam + bh * N + P + ic);
-          const float d_ = ldg_f32_here(p.delta + bh * M + ic);
+          const float l_ = ld_f32_here(p.L + bh * M + ic);
+          const float a_ = ld_f32_here(p.lam + bh * N + P + ic);
+          const float d_ = ld_f32_here(p.delta + bh * M + ic);
           rawL[slot][rr] = in ? l_ : -INFINITY;
           rawLam[slot][rr] = a_;
           rawD[slot][rr] = in ? d_ : 0.f;

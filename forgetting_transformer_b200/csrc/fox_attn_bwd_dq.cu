@@ -145,7 +145,7 @@ fox_attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       auto fetch_lam = [&](int it) {
         const int c0 = (nb_hi - 1 - it) * BN + 2 * lane;
 #pragma unroll
-        for (int e = 0; e < 2; ++e) lamv[e] = (c0 + e < N) ? ldg_f32_here(lam + c0 + e) : 0.f;
+        for (int e = 0; e < 2; ++e) lamv[e] = (c0 + e < N) ? ld_f32_here(lam + c0 + e) : 0.f;
       };
       auto stage_negb = [&](int it) {
         const int slot = it % 3;
@@ -541,7 +541,7 @@ fox_attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       auto fetch_lam = [&](int it, float* v) {
         const int c0 = (x.nb_hi - 1 - it) * BN + 4 * lane;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = (c0 + e < N) ? ldg_f32_here(lam + c0 + e) : 0.f;
+        for (int e = 0; e < 4; ++e) v[e] = (c0 + e < N) ? ld_f32_here(lam + c0 + e) : 0.f;
       };
       auto stage_negb = [&](uint32_t slot, const float* v) {
         *reinterpret_cast<float4*>(&s_negb[slot][4 * lane]) =

@@ -237,9 +237,9 @@ fox_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           const int r = i0 + e;
           float Li = -INFINITY, la = 0.f, de = 0.f;
           if (r < M) {
-            Li = ldg_f32_here(Lp + r);
-            la = ldg_f32_here(lam + r);
-            de = ldg_f32_here(dl + r);
+            Li = ld_f32_here(Lp + r);
+            la = ld_f32_here(lam + r);
+            de = ld_f32_here(dl + r);
           }
           ev[e] = (Li == -INFINITY) ? -INFINITY : ((la - lam_ref) - Li) * kKvLog2e;
           dv_[e] = de;

@@ -212,7 +212,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       auto fetch_lam = [&](int it) {
         const int c0 = (nb_hi - 1 - it) * BN + 4 * lane;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) lamv[e] = (4 * lane < BN && c0 + e < N) ? ldg_f32_here(lam + c0 + e) : 0.f;
+        for (int e = 0; e < 4; ++e) lamv[e] = (4 * lane < BN && c0 + e < N) ? ld_f32_here(lam + c0 + e) : 0.f;
       };
       auto stage_negb = [&](int it) {  // from lamv, fetched earlier for this tile
         const int slot = it % 3;

@@ -540,11 +540,12 @@ __device__ __forceinline__ float2 poly_exp2_x2(float2 x) {
   return r;
 }
 
-// Read-only global load that stays where it is written: the compiler may sink a plain load down to its
-// first use, which puts the whole memory latency in front of that use; a volatile asm is not moved.
-__device__ __forceinline__ float ldg_f32_here(const float* p) {
+// Global loads that stay where they are written: the compiler may sink a plain load down to its first use, which puts the whole
+// memory latency in front of that use; a volatile asm is not moved.  The read-only path (.nc) is for memory that nothing writes while
+// the kernel runs: not for what a kernel that begins behind another reads of that one's results, nor for what it writes itself.
+__device__ __forceinline__ float ld_f32_here(const float* p) {
   float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -553,7 +554,6 @@ __device__ __forceinline__ uint4 ldg_v4_here(const uint4* p) {
   asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-// (memory that the same kernel writes)
 __device__ __forceinline__ uint4 ld_v4_here(const uint4* p) {
   uint4 v;
   asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");

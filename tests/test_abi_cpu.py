@@ -205,41 +205,87 @@ def test_requests_ahead_of_a_token_product_cover_the_array_once(grid):
             assert after == at(grid, grid - 1, thread, k) + 4096
 
 
+def _device_functions(text):
+    """name -> parameters and body of every __global__ and __device__ function of a source without comments."""
+    found = {}
+    for start in re.finditer(r"__(?:global|device)__", text):
+        name = re.compile(r"(\w+)\s*\(").search(text, start.end())
+        while name and name.group(1) == "__launch_bounds__":
+            name = re.compile(r"(\w+)\s*\(").search(text, text.index(")", name.end()))
+        if not name or ";" in text[start.end():name.start()]:
+            continue
+        at, depth = name.end(), 1
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[at], 0)
+            at += 1
+        if not text[at:].lstrip().startswith("{"):
+            continue
+        at = text.index("{", at) + 1
+        depth = 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        found[name.group(1)] = found.get(name.group(1), "") + text[name.start():at]
+    return found
+
+
+def _sources():
+    strip = lambda name: re.sub(r"//[^\n]*", "", open(os.path.join(build.CSRC, name)).read())
+    common = _device_functions(strip("fox_common.cuh"))
+    for name in build.SOURCES:
+        yield name, strip(name), common
+
+
+def _with_all_it_calls(kernel, functions):
+    """The kernel, the functions that it names, those that they name, and so on."""
+    reached, todo = {}, [kernel]
+    while todo:
+        name = todo.pop()
+        reached[name] = functions[name]
+        todo += [f for f in set(re.findall(r"\w+", functions[name])) & set(functions) if f not in reached and f not in todo]
+    return reached
+
+
+WAITS = ("griddepcontrol.wait", "pdl_wait()", "wait_for_kernel_in_front()")
+
+
 def test_kernels_that_begin_early_take_no_invariant_pointers():
     """A kernel with griddepcontrol.wait may begin before the kernel in front has written what it reads: a load through a
-    `const __restrict__` pointer, or by __ldg, is one that the compiler may move in front of the wait."""
-    found = 0
-    for name in build.SOURCES:
-        text = re.sub(r"//[^\n]*", "", open(os.path.join(build.CSRC, name)).read())
-        for kernel in re.split(r"__global__", text)[1:]:
-            params, body = kernel.split("{", 1)
-            body = body.split("\n}\n", 1)[0]
-            if "griddepcontrol.wait" in body or "pdl_wait()" in body:
-                found += 1
-                assert "__restrict__" not in params + body and "__ldg" not in body, (name, params)
-    assert found == 5
+    `const __restrict__` pointer, by __ldg or on the read-only path (.nc) is one that may be done in front of the wait.  None in
+    such a kernel, nor in any function that it reaches, but for a token product's weights, which no kernel writes."""
+    waiting, helpers = set(), set()
+    for name, text, common in _sources():
+        functions = {**common, **_device_functions(text)}
+        for kernel in functions:
+            if not re.search(r"__global__[^;{]*\b%s\s*\(" % kernel, text) or not any(w in functions[kernel] for w in WAITS):
+                continue
+            waiting.add(kernel)
+            for f, body in _with_all_it_calls(kernel, functions).items():
+                helpers.add(f)
+                assert not any(x in body for x in ("__restrict__", "__ldg", ".nc.")) or f == "ldg_stream", (name, kernel, f)
+    assert len(waiting) >= 22
+    # the walk sees helpers of the common header, of two template arguments, and those that only helpers call
+    assert {"ld_f32_here", "dec_store", "load_gate", "norm_part", "tma_load_4d"} <= helpers and "ldg_v4_here" not in helpers
 
 
-def test_kernels_launched_behind_another_take_no_invariant_pointers():
-    """The same for those that wait by wait_for_kernel_in_front(): each kernel that launch_behind() is given, and the functions it
-    calls in its file."""
-    waiting = set()
-    for name in build.SOURCES:
-        if not name.endswith(".cu"):
-            continue
-        text = re.sub(r"//[^\n]*", "", open(os.path.join(build.CSRC, name)).read())
-        for kernel in re.split(r"__global__", text)[1:]:
-            params, body = kernel.split("{", 1)
-            body = body.split("\n}\n", 1)[0]
-            if "wait_for_kernel_in_front()" in body:
-                waiting.add(re.search(r"(fox_\w+_kernel)\s*\(", params).group(1))
-                used = [f for f in re.split(r"__device__", text)[1:] if re.search(r"\b%s(<\w+>)?\(" % re.search(r"(\w+)\s*\(", f).group(1), body)]
-                assert not any("__restrict__" in f.split("\n}\n", 1)[0] or "__ldg" in f.split("\n}\n", 1)[0] for f in used), (name, params)
-                assert "__restrict__" not in params + body and "__ldg" not in body, (name, params)
+def test_kernels_launched_behind_another_wait_for_it():
+    """Each kernel that a host function gives to launch_behind(), or to cudaLaunchKernelEx with its attributes, waits in its own body."""
+    launched = set()
+    for name, text, _ in _sources():
+        functions = _device_functions(text)
+        for host in text.split("\n}\n"):
+            if "launch_behind(" in host or "cudaLaunchKernelEx(" in host:
+                assert "<<<" not in host, name     # (or the names below would not all be launched so)
+                kernels = set(re.findall(r"\bfox_\w+_kernel\b", host))
+                assert kernels, (name, host[-200:])
+                for k in kernels:
+                    assert any(w in functions[k] for w in WAITS), (name, k)
+                launched |= kernels
     assert {"fox_attn_fwd_kernel", "fox_attn_bwd_kernel", "fox_attn_bwd_kv_kernel", "fox_attn_bwd_dq2_kernel", "fox_find_index_kernel",
             "fox_prologue_kernel", "fox_delta_kernel", "fox_bwd_finish_kernel", "fox_mix_fwd_kernel", "fox_mix_bwd_kernel", "fox_pack_kernel",
             "fox_unpack_kernel", "fox_column_sums_kernel", "fox_swiglu_fwd_kernel", "fox_swiglu_bwd_kernel", "fox_normgate_fwd_kernel",
-            "fox_normgate_bwd_kernel"} <= waiting
+            "fox_normgate_bwd_kernel", "fox_decode_kernel", "fox_decode_merge_kernel", "fox_step_product_kernel", "fox_step_mix_kernel",
+            "fox_ce_mean_kernel"} <= launched
 
 
 @pytest.mark.parametrize("bh", [1, 9, 10, 24, 35, 48, 60, 64, 70, 71, 96, 98, 99, 140, 147, 148, 149, 296, 297, 4000])
