@@ -52,6 +52,7 @@ _SIGNATURES = {
                              _F, _F, _F, c_float, _T4P, _F, _F, _F]),
     "fox_attn_fwd_parts": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P,
                                    _F, _F, _F, c_float, _T4P, _F, _F, c_int64, _F]),
+    "fox_attn_item_group": (c_int64, [c_int64, c_int64, c_int64]),
     "fox_norm_parts": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
     "fox_key_norm_parts": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
     "fox_attn_prologue": (c_int, [c_int, c_void_p, c_int, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _F, c_int64,

@@ -742,6 +742,10 @@ extern "C" int fox_attn_fwd(int device, void* stream, int dtype, int64_t B, int6
                             L, k_norm_max, 1, status);
 }
 
+extern "C" int64_t fox_attn_item_group(int64_t units, int64_t tiles, int64_t unit_bytes) {
+  return units <= 0 || tiles <= 0 || unit_bytes <= 0 ? 1 : fox::item_group(units, tiles, unit_bytes);
+}
+
 extern "C" int fox_attn_fwd_parts(int device, void* stream, int dtype, int64_t B, int64_t H, int64_t M, int64_t N,
                                   int64_t D, const fox_tensor4* q, const fox_tensor4* k, const fox_tensor4* v,
                                   const float* log_lambda, const int64_t* seq_start, const int64_t* start_index,

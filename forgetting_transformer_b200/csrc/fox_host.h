@@ -79,8 +79,13 @@ inline int make_tmap_4d(CUtensorMap* out, const Tensor4& t, int elem_bytes, bool
 //   B2 H16 T4096 D64     138 / 278 -> 126 / 283, 117 / 251, 114 / 253, 115 / 259
 //   B4 H16 T16384 D128   4539 / 8273 + 5370 -> 16 MB 4457 / 8171 + 5316, 48 MB 4354 / 8148 + 5334, all 4788 / 8775 + 5837
 //   B4 H12 T512 D64      15.1 / 24.8 -> 12.4 / 21.0 (one group from 3 MB on)
+// Items that all have an SM to themselves are one group whatever they read: groups of uneven sizes are padded with CTAs that have no
+// item, and those took places that the last items then shared with others (37 (b,h) of 512 x 8000, 148 items and 4 such CTAs: forward at
+// D64 77 -> 107 us by two groups, 77 by one; at D128 109 -> 131, 109).  More units than an int counts stay unit by unit.
 inline int64_t item_group(int64_t units, int64_t tiles, int64_t unit_bytes) {
   constexpr int64_t kGroupBytes = 48 << 20;
+  if (units * tiles <= 148) return units;
+  if (units > 2147483647LL - 65536) return 1;
   const int64_t fit = unit_bytes < kGroupBytes ? kGroupBytes / unit_bytes : 1;
   const int64_t groups = (units + fit - 1) / fit;
   return tiles > 65535 || groups > 65535 ? 1 : (units + groups - 1) / groups;   // (what a grid can have)

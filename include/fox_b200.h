@@ -152,6 +152,9 @@ int fox_attn_fwd_parts(int device, void* stream, int dtype, int64_t B, int64_t H
                  const int64_t* seq_start, const int64_t* start_index, float sm_scale, const fox_tensor4* o,
                  float* L, const float* k_norm_parts,
                        int64_t n_norm_parts, int32_t* status);
+/* How many of `units` (b,h) with `tiles` tiles each, that read unit_bytes each, the attention kernels go through together, the
+ * longest tiles first, where no threshold is given: as many as stay in L2, or all where each tile has an SM to itself. */
+int64_t fox_attn_item_group(int64_t units, int64_t tiles, int64_t unit_bytes);
 
 /* Forward attention for ONE query row per (b,h) -- a generation step against a cache of N keys, the
  * seqlen_q = 1 case of the same upstream kernel (forgetting_attention.py:148-153, 591-693; cache:

@@ -288,6 +288,25 @@ def test_kernels_launched_behind_another_wait_for_it():
             "fox_ce_mean_kernel"} <= launched
 
 
+@pytest.mark.parametrize("units,tiles", [(1, 1), (1, 148), (37, 4), (148, 1), (74, 2), (49, 3), (1, 149), (37, 5), (150, 1), (28, 65), (65535, 7),
+                                         (100000, 1), (3, 70000), (2 ** 31 - 70000, 1), (2 ** 31 + 5, 1), (2 ** 32 - 131071, 1)])
+@pytest.mark.parametrize("mb", [0.001, 1.9, 5, 24, 25, 60])
+def test_groups_of_items_by_length(units, tiles, mb):
+    """Units that go by length together: all of them where every tile has an SM to itself, so that no CTA without an item takes a
+    place there; else as many as stay in 48 MB, in groups that differ by less than their number, at most 65535 of them, whose
+    padded size stays below 2^31.  Units that an int does not count go one by one."""
+    group = _lib.load().fox_attn_item_group(units, tiles, int(mb * 2 ** 20))
+    assert 1 <= group <= units
+    if units * tiles <= 148:
+        assert group == units
+    elif group > 1:
+        groups = -(-units // group)
+        assert group * mb * 2 ** 20 <= 48 * 2 ** 20 + group and groups <= 65535 and tiles <= 65535
+        assert groups * group - units < group and groups * group < 2 ** 31
+    if units > 2 ** 31 - 65536:
+        assert group == 1
+
+
 @pytest.mark.parametrize("bh", [1, 9, 10, 24, 35, 48, 60, 64, 70, 71, 96, 98, 99, 140, 147, 148, 149, 296, 297, 4000])
 @pytest.mark.parametrize("n,d", [(1024, 64), (4096, 128), (8192, 128), (16384, 64), (1024, 16), (12300, 16), (2 ** 24, 128)])
 def test_key_norm_parts_fill_a_wave_and_stay_short(bh, n, d):
