@@ -125,6 +125,28 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int mb = p.order.tiles - 1 - rank_here<kByLength>();   // long tiles first
   const int M = p.M, N = p.N, P = N - M;
 
+  // ---- KV range of this query tile (upstream lines 591-613) ----
+  int seq0, nb_lo, nb_hi, n_tiles;   // (nb_hi exclusive)
+  auto set_range = [&] {
+    const int hi = min(N, P + (mb + 1) * kFwdBM);
+    seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
+    int lo = min(seq0, hi);
+    if (p.start_index) {
+      const int64_t si = p.start_index[(static_cast<int64_t>(b) * p.H + h) * p.order.tiles + mb];
+      lo = max(lo, static_cast<int>(si < static_cast<int64_t>(hi) ? si : static_cast<int64_t>(hi)));
+    }
+    lo = (lo / kFwdBN) * kFwdBN;
+    nb_lo = lo / BN;
+    nb_hi = (hi + BN - 1) / BN;
+    n_tiles = max(nb_hi - nb_lo, 0);
+  };
+  // Unit by unit the range is there before the barriers are: behind them, as by length, the same source makes a slower tile loop at head
+  // dim 128 (1 x 2 of 4096 x 16384 that a threshold could prune and does not: 237 us behind, 206 before; 4 heads 238 and 207; by length,
+  // either way, 205), for 0.2 us of set-up that the kernel in front would cover.
+  if constexpr (!kByLength) {
+    wait_for_kernel_in_front();
+    set_range();
+  }
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&bar_q_full, 1);
@@ -144,7 +166,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     mbar_fence_init();
   }
-  wait_for_kernel_in_front();   // (no memory is read before this, and no TMEM held that the kernel in front might ask for)
+  if constexpr (kByLength) wait_for_kernel_in_front();   // (no memory is read before this, and no TMEM held that the kernel in front might ask for)
   if (warp == kTmaWarp) {
     tmem_alloc(&tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -155,18 +177,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tbase = tmem_slot;
   volatile int* abortp = &abort_flag;
 
-  // ---- KV range of this query tile (upstream lines 591-613) ----
-  const int hi = min(N, P + (mb + 1) * kFwdBM);
-  const int seq0 = p.seq_start ? static_cast<int>(p.seq_start[b]) : 0;
-  int lo = min(seq0, hi);
-  if (p.start_index) {
-    const int64_t si = p.start_index[(static_cast<int64_t>(b) * p.H + h) * p.order.tiles + mb];
-    lo = max(lo, static_cast<int>(si < static_cast<int64_t>(hi) ? si : static_cast<int64_t>(hi)));
-  }
-  lo = (lo / kFwdBN) * kFwdBN;
-  const int nb_lo = lo / BN;
-  const int nb_hi = (hi + BN - 1) / BN;  // exclusive
-  const int n_tiles = max(nb_hi - nb_lo, 0);
+  if constexpr (kByLength) set_range();
 
   if (warp == kTmaWarp) {
     // ===================== TMA producer (whole warp converged, one elected lane issues) =====================
