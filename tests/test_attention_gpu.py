@@ -680,27 +680,32 @@ def test_backward_that_could_prune_equals_one_that_cannot(B, H, M, N):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("H,T,D", [(13, 8200, 64), (25, 4100, 128), (3, 300, 64), (1, 1, 128)])
-def test_items_by_length_are_each_taken_once(H, T, D):
-    """Units go by tile length in groups that stay in L2 (13 of 4.2 MB and 25 of 2.1 MB: two uneven groups; fewer: one); a unit alone is
-    its own group.  The order decides nothing but when an item runs: the same bits (fp32 sums into dQ at D=64: in another order)."""
+@pytest.mark.parametrize("B,H,T,D,padded", [(1, 13, 8200, 64, False), (1, 25, 4100, 128, False), (1, 3, 300, 64, False), (4, 7, 8200, 64, True),
+                                            (3, 9, 4100, 128, True)])
+def test_items_by_length_are_each_taken_once(B, H, T, D, padded):
+    """Units (b,h) go by tile length in groups that stay in L2 (13 of 4.2 MB and 25 of 2.1 MB: two uneven groups; 4 x 7 and 3 x 9: three
+    and two, none of whole batches; 3 small ones: one); a unit alone is its own group.  The order decides nothing but when an item
+    runs: the same bits (fp32 sums into dQ at D=64: in another order)."""
     gen = torch.Generator(device="cuda").manual_seed(H)
-    q, k, v, do = (torch.randn(1, H, T, D, generator=gen, device="cuda").bfloat16() for _ in range(4))
-    g = torch.nn.functional.logsigmoid(torch.randn(1, H, T, generator=gen, device="cuda") + 2)
+    q, k, v, do = (torch.randn(B, H, T, D, generator=gen, device="cuda").bfloat16() for _ in range(4))
+    g = torch.nn.functional.logsigmoid(torch.randn(B, H, T, generator=gen, device="cuda") + 2)
+    start = torch.arange(B, device="cuda") * (T // (B + 1)) if padded else None
 
-    def run(lo, hi):
-        x = [t[:, lo:hi].contiguous().requires_grad_() for t in (q, k, v, g)]
-        out = fox.forgetting_attention(*x, head_first=True)
-        out.backward(do[:, lo:hi].contiguous())
+    def run(b, h):
+        x = [t[b, h].contiguous().requires_grad_() for t in (q, k, v, g)]
+        out = fox.forgetting_attention(*x, head_first=True, seq_start=None if start is None else start[b])
+        out.backward(do[b, h].contiguous())
         return [out] + [t.grad for t in x]
 
-    together = run(0, H)
-    for h in range(H):
-        for i, (a, b) in enumerate(zip(together, run(h, h + 1))):
-            if D == 64 and i in (1, 4):     # dQ, and the gate gradient through its row sums
-                assert (a[:, h:h + 1].double() - b.double()).norm() <= 2 ** -8 * b.double().norm() + 1e-30
-            else:
-                assert torch.equal(a[:, h:h + 1], b), (h, i)
+    together = run(slice(0, B), slice(0, H))
+    for b in range(B):
+        for h in range(H):
+            for i, (x, y) in enumerate(zip(together, run(slice(b, b + 1), slice(h, h + 1)))):
+                x = x[b:b + 1, h:h + 1]
+                if D == 64 and i in (1, 4):     # dQ, and the gate gradient through its row sums
+                    assert (x.double() - y.double()).norm() <= 2 ** -8 * y.double().norm() + 1e-30
+                else:
+                    assert torch.equal(x, y), (b, h, i)
 
 
 @pytest.mark.gpu
@@ -708,44 +713,61 @@ def test_items_by_length_are_each_taken_once(H, T, D):
 @pytest.mark.parametrize("T,D,thr", [(100, 64, None), (700, 128, -6.0), (1500, 64, "auto"), (2100, 128, None)])
 def test_kernels_begun_behind_one_another_read_finished_inputs(T, D, thr, graph):
     """The kernels of a pass take their SMs before the one in front has written back.  Inputs written by the kernels directly in front,
-    passes one behind the other into memory that the allocator hands on, and a capture that joins another stream in front: the
-    results of a pass that is alone, bit by bit (dQ at D=64, summed in any order: to rounding)."""
+    passes one behind the other into memory that the allocator hands on, and a captured pass whose inputs another stream, joined in front
+    of its first kernel, writes late and anew for each replay: the results of a pass that is alone, bit by bit (dQ at D=64,
+    summed in any order: to rounding)."""
     gen = torch.Generator(device="cuda").manual_seed(T)
     base = [torch.randn(1, 5, T, D, generator=gen, device="cuda").bfloat16() for _ in range(4)]
     base.append(torch.nn.functional.logsigmoid(torch.randn(1, 5, T, generator=gen, device="cuda") + 1))
     kw = {} if thr is None else dict(adaptive_threshold=thr)
-    scales = [1.0, 0.5, 2.0]
 
-    def run(scale):
-        q, k, v, do, g = [t * scale for t in base]
+    def run(inputs):
+        q, k, v, do, g = inputs
         x = [t.requires_grad_() for t in (q, k, v, g)]
         out = fox.forgetting_attention(*x, head_first=True, **kw)
         return [out.detach(), *torch.autograd.grad(out, x, do)]
 
-    alone = []
-    for s in scales:
-        torch.cuda.synchronize()
-        alone.append(run(s))
-        torch.cuda.synchronize()
-    if graph:
-        main, side = torch.cuda.Stream(), torch.cuda.Stream()
-        g = torch.cuda.CUDAGraph()
-        main.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.graph(g, stream=main):
-            side.wait_stream(main)
-            with torch.cuda.stream(side):
-                base[0].mul_(1.0)
-            main.wait_stream(side)
-            together = [run(s) for s in scales]
-        for _ in range(3):
-            g.replay()
-    else:
-        for _ in range(4):
-            together = [run(s) for s in scales]
-    torch.cuda.synchronize()
-    for a, b in zip(together, alone):
-        for i, (x, y) in enumerate(zip(a, b)):
+    def scaled(scale):
+        return [t * scale for t in base]
+
+    def check(got, want):
+        for i, (x, y) in enumerate(zip(got, want)):
             if D == 64 and i in (1, 4):     # dQ, and the gate gradient through its row sums
                 assert (x.double() - y.double()).norm() <= 2 ** -8 * y.double().norm()
             else:
                 assert torch.equal(x, y), i
+
+    scales = [1.0, 0.5, 2.0]
+    alone = []
+    for s in scales:
+        inputs = scaled(s)
+        torch.cuda.synchronize()
+        alone.append(run(inputs))
+        torch.cuda.synchronize()
+    if graph:
+        main, side = torch.cuda.Stream(), torch.cuda.Stream()
+        g = torch.cuda.CUDAGraph()
+        source, inputs = scaled(0.0), scaled(0.0)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=main):
+            for t in inputs:
+                t.detach().fill_(float("nan"))
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(100_000)
+                for t, s in zip(inputs, source):
+                    t.detach().copy_(s)
+            main.wait_stream(side)
+            got = run(inputs)
+        for s, want in list(zip(scales, alone)) * 2:
+            for t, x in zip(source, scaled(s)):
+                t.copy_(x)
+            g.replay()
+            torch.cuda.synchronize()
+            check(got, want)
+    else:
+        for _ in range(4):
+            together = [run(scaled(s)) for s in scales]
+        torch.cuda.synchronize()
+        for got, want in zip(together, alone):
+            check(got, want)

@@ -512,3 +512,74 @@ def test_token_step_counts_as_a_change_in_place():
     with torch.no_grad():
         blk(x, None, cache, 0)
     assert all(t._version > v for t, v in zip(tensors, before))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("B,T,C,H", [(2, 100, 256, 2), (1, 700, 512, 4), (2, 300, 256, 4)])
+def test_block_passes_behind_one_another(B, T, C, H, graph):
+    """Packing, mix, gated norm, SwiGLU, unpacking and column sums take their SMs before the kernel in front has written back.  Passes whose
+    input a kernel directly in front has written, with weights changed by one between them, into memory that the allocator hands on, and a
+    capture of all three: the outputs and gradients of passes that are alone, bit by bit (head dim 64, whose dQ is summed in any order: what
+    depends on it to rounding)."""
+    blk, base, dy = _block(C, H, 2 * C), _x(T, C, B=B), _x(T, C, seed=2, B=B)
+    mask = torch.ones(B, T, dtype=torch.long, device="cuda")
+    mask[0, :T // 5] = 0
+    params = list(blk.parameters())
+    norm = blk.mlp_norm.weight
+    first = norm.detach().clone()
+
+    def run(scale):
+        with torch.no_grad():
+            torch.mul(first, scale, out=norm.data)
+        x = (base * scale).requires_grad_()
+        out = blk(x, mask)
+        return [out.detach(), *torch.autograd.grad(out, [x, *params], dy * scale)]
+
+    scales, alone = [1.0, 0.5, 2.0], []
+    for s in scales:
+        torch.cuda.synchronize()
+        alone.append(run(s))
+        torch.cuda.synchronize()
+    if graph:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            together = [run(s) for s in scales]
+        for _ in range(3):
+            g.replay()
+    else:
+        for _ in range(4):
+            together = [run(s) for s in scales]
+    torch.cuda.synchronize()
+    for got, want in zip(together, alone):
+        assert torch.equal(got[0], want[0])
+        for i, (a, b) in enumerate(zip(got[1:], want[1:])):
+            if C // H == 64:
+                assert (a.double() - b.double()).norm() <= 2 ** -7 * b.double().norm(), i
+            else:
+                assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("rows", [3, 300, 5000])
+def test_norm_gate_and_swiglu_behind_one_another(rows):
+    """The same for the two operators called by themselves, whose inputs a kernel directly in front has written."""
+    C, H = 512, 4
+    base = [_x(rows, C, seed=i)[0] for i in range(3)]
+    w = torch.rand(C, device="cuda") + 0.5
+
+    def run(scale):
+        x, y, dz = [t * scale for t in base]
+        x, y, wx = x.requires_grad_(), y.requires_grad_(), (w * scale).requires_grad_()
+        z = fox.swiglu(fox.group_norm_gated(x, y, wx, activation="sigmoid", is_rms_norm=True, num_groups=H), y)
+        return [z.detach(), *torch.autograd.grad(z, (x, y, wx), dz)]
+
+    scales, alone = [1.0, 0.5, 2.0], []
+    for s in scales:
+        torch.cuda.synchronize()
+        alone.append(run(s))
+        torch.cuda.synchronize()
+    for _ in range(4):
+        together = [run(s) for s in scales]
+    torch.cuda.synchronize()
+    for got, want in zip(together, alone):
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
