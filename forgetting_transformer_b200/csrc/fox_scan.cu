@@ -71,11 +71,14 @@ __device__ __forceinline__ float log_gate(float raw) {
 // log_lambda[b,h,t] = carry_in[b,h] + sum_{u<=t, u>=seq_start[b]} log_fgate[b,h,u]
 // One CTA per (b,h); chunks of 4096 elements with a carried running total.  With gate logits as input
 // (kIn < 3) the log gates themselves are formed on the fly and, if lf_out is given, written out (unmasked).
-// Bound by the chain of a chunk's load, scan and three barriers, 2.2 us of which the load is a third: the next chunk's gates are
-// asked for before the scan (prologue, bf16: one row of 65536 gates 35.9 -> 22.9 us, 24 rows of 11000 13.5 -> 11.3, 4 of 9000 8.7 ->
-// 7.0; up to 4096, one chunk, unchanged).  In the reverse scan, with three arrays, it takes more registers than two blocks of 1024
-// threads have, spills, and loses: 24 rows of 16384 24.0 and 24.0 us, from logits 24.5 and 28.7.
-template <int kIn>
+// Bound by the chain of a chunk's load, scan and three barriers, 2.2 us of which the load is a third: with kAhead the next chunk's gates
+// are asked for before the scan (prologue, bf16: one row of 65536 gates 35.9 -> 22.9 us, 24 rows of 11000 13.5 -> 11.3, 4 of 9000 8.7 ->
+// 7.0; up to 4096, one chunk, unchanged).  From logits the chunk in hand is then formed by every thread, with gates or without; without
+// kAhead a thread that has none (past the row's end, in front of seq_start) leaves the logarithms out, which is worth more up to four
+// chunks (24 rows of 4097 7.9 us before, 9.9 ahead, 8.2 so; 11000 with half of it padding 11.8, 14.7, 12.4; 48 of 16384 23.6, 21.1, 21.1; one of
+// 65536 38.1, 34.6).  In the reverse scan, with three arrays, it takes more registers than two blocks of 1024 threads have, spills,
+// and loses: 24 rows of 16384 24.0 and 24.0 us, from logits 24.5 and 28.7.
+template <int kIn, bool kAhead>
 __device__ __forceinline__ void cumsum_rows(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
                                             const float* carry_in, float* out, float* total_out, float* lf_out, int H, int N, int bh, float* red) {
   const int b = bh / H, h = bh % H;
@@ -92,19 +95,24 @@ __device__ __forceinline__ void cumsum_rows(const void* lf, int64_t sb, int64_t 
       if (static_cast<unsigned>(t) < static_cast<unsigned>(N) && (t >= s0 || (kIn < 3 && lf_out))) next[j] = load_gate<kIn>(lf, src0 + static_cast<int64_t>(t) * sn);
     }
   };
-  load(0);
+  if (kAhead) load(0);
   for (int base = 0; base < N; base += kScanChunk) {
     const int t0 = base + threadIdx.x * kScanPerThread;
     float x[kScanPerThread];
+    if (!kAhead) load(base);
 #pragma unroll
     for (int j = 0; j < kScanPerThread; ++j) x[j] = next[j];
-    load(base + kScanChunk);
+    if (kAhead) load(base + kScanChunk);
+    if (kIn == 3 || kAhead || (t0 < N && (t0 + kScanPerThread > s0 || lf_out))) {   // (a thread without gates has no logarithms to take)
 #pragma unroll
-    for (int j = 0; j < kScanPerThread; ++j) {
-      const int t = t0 + j;
-      const float g = log_gate<kIn>(x[j]);
-      if (kIn < 3 && lf_out && t < N) lf_out[static_cast<int64_t>(bh) * N + t] = g;
-      x[j] = (t < N && t >= s0) ? g : 0.f;
+      for (int j = 0; j < kScanPerThread; ++j) {
+        const int t = t0 + j;
+        const float g = log_gate<kIn>(x[j]);
+        if (kIn < 3 && lf_out && t < N) lf_out[static_cast<int64_t>(bh) * N + t] = g;
+        // (a log gate that was not loaded is 0 already; with the next ones in flight the choice costs nothing and without it the
+        // additions wait for them: 148 rows of 16384 7.4 us, 7.9 without)
+        x[j] = (kIn == 3 && !kAhead) || (t < N && t >= s0) ? g : 0.f;
+      }
     }
 #pragma unroll
     for (int j = 1; j < kScanPerThread; ++j) x[j] += x[j - 1];
@@ -121,13 +129,13 @@ __device__ __forceinline__ void cumsum_rows(const void* lf, int64_t sb, int64_t 
   if (total_out && threadIdx.x == 0) total_out[bh] = carry;
 }
 
-template <int kIn>
-__global__ void __launch_bounds__(kScanThreads)
+template <int kIn, bool kAhead>
+__global__ void __launch_bounds__(kScanThreads, kAhead ? 0 : 2)
 fox_cumsum_kernel(const void* __restrict__ lf, int64_t sb, int64_t sh, int64_t sn,
                   const int64_t* __restrict__ seq_start, const float* __restrict__ carry_in,
                   float* __restrict__ out, float* __restrict__ total_out, float* __restrict__ lf_out, int H, int N) {
   __shared__ float red[32];
-  cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, carry_in, out, total_out, lf_out, H, N, blockIdx.x, red);
+  cumsum_rows<kIn, kAhead>(lf, sb, sh, sn, seq_start, carry_in, out, total_out, lf_out, H, N, blockIdx.x, red);
 }
 
 // dlog_fgate[t] = carry_in + sum_{u >= t} (dcol[u] + drow[u - P] if u >= P)
@@ -495,7 +503,10 @@ fox_prologue_kernel(const void* lf, int64_t sb, int64_t sh, int64_t sn, const in
   __shared__ float red[32];
   const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
   wait_for_kernel_in_front();
-  if (x == 0) cumsum_rows<kIn>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+  if (x == 0) {
+    if (kIn == 3 || N > 4 * kScanChunk) cumsum_rows<kIn, true>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+    else cumsum_rows<kIn, false>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+  }
   else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
   else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
 }
@@ -615,6 +626,19 @@ static inline bool aligned16(const fox_tensor4* t) {
   return t && t->ptr && reinterpret_cast<uintptr_t>(t->ptr) % 16 == 0 && (t->sb * 2) % 16 == 0 &&
          (t->sh * 2) % 16 == 0 && (t->st * 2) % 16 == 0;
 }
+// The prefix sums by themselves.  Loading ahead takes 38 to 41 registers, one block to an SM instead of two: log gates where the rows
+// have an SM each or are so long that it pays all the same (148 rows of 4097 4.4 us without, 4.2 ahead, of 16384 9.1 and 7.4; 149 of 8192 8.1
+// and 7.6, but 1024 23.6 and 26.1; 1024 of 16384 45.4 and 42.6; 512 of 100 6.0 and 8.8); logits, whose threads without gates have no
+// logarithms to take without it, later and in one round of blocks only (148 of 8192 7.1 and 6.6, of 16384 12.8 and 12.1; 149 of 16384 19.9 and 21.4;
+// 1024 of 4096 21.9 and 27.8).
+template <int kIn>
+static void launch_cumsum(cudaStream_t st, unsigned rows, const void* gates, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
+                          const float* carry_in, float* out, float* total_out, float* lf_out, int H, int N) {
+  const bool ahead = kIn == 3 ? N > kScanChunk && (rows <= kSms || N >= 4 * kScanChunk) : rows <= kSms && N >= 3 * kScanChunk;
+  (ahead ? fox_cumsum_kernel<kIn, true> : fox_cumsum_kernel<kIn, false>)<<<rows, kScanThreads, 0, st>>>(
+      gates, sb, sh, sn, seq_start, carry_in, out, total_out, lf_out, H, N);
+}
+
 static inline int launch_rc() { return cudaGetLastError() == cudaSuccess ? FOX_OK : FOX_ERR_LAUNCH; }
 
 }  // namespace fox
@@ -628,8 +652,8 @@ extern "C" int fox_cumsum_fwd(int device, void* stream, int64_t B, int64_t H, in
                               const float* carry_in, float* log_lambda, float* total_out) {
   if (!log_fgate || !log_lambda || B <= 0 || H <= 0 || N <= 0) return FOX_ERR_BAD_ARG;
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
-  fox_cumsum_kernel<3><<<(unsigned)(B * H), kScanThreads, 0, (cudaStream_t)stream>>>(
-      log_fgate, sb, sh, sn, seq_start, carry_in, log_lambda, total_out, nullptr, (int)H, (int)N);
+  launch_cumsum<3>((cudaStream_t)stream, (unsigned)(B * H), log_fgate, sb, sh, sn, seq_start, carry_in, log_lambda, total_out, nullptr,
+                   (int)H, (int)N);
   return launch_rc();
 }
 
@@ -641,12 +665,8 @@ extern "C" int fox_gate_prefix_fwd(int device, void* stream, int dtype, int64_t 
   if (cudaSetDevice(device) != cudaSuccess) return FOX_ERR_DEVICE;
   const unsigned grid = (unsigned)(B * H);
   cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == FOX_DTYPE_FP16)
-    fox_cumsum_kernel<0><<<grid, kScanThreads, 0, st>>>(fgate_logit, sb, sh, sn, seq_start, nullptr, log_lambda, nullptr, log_fgate_out, (int)H, (int)N);
-  else if (dtype == FOX_DTYPE_BF16)
-    fox_cumsum_kernel<1><<<grid, kScanThreads, 0, st>>>(fgate_logit, sb, sh, sn, seq_start, nullptr, log_lambda, nullptr, log_fgate_out, (int)H, (int)N);
-  else
-    fox_cumsum_kernel<2><<<grid, kScanThreads, 0, st>>>(fgate_logit, sb, sh, sn, seq_start, nullptr, log_lambda, nullptr, log_fgate_out, (int)H, (int)N);
+  auto launch = dtype == FOX_DTYPE_FP16 ? launch_cumsum<0> : dtype == FOX_DTYPE_BF16 ? launch_cumsum<1> : launch_cumsum<2>;
+  launch(st, grid, fgate_logit, sb, sh, sn, seq_start, nullptr, log_lambda, nullptr, log_fgate_out, (int)H, (int)N);
   return launch_rc();
 }
 

@@ -307,6 +307,18 @@ def test_groups_of_items_by_length(units, tiles, mb):
         assert group == 1
 
 
+def test_scan_kernels_leave_room_for_a_second_block(tmp_path):
+    """Blocks of 1024 threads: 32 registers a thread let two be on an SM.  Prologue, backward's end, and the prefix sums that do not load
+    ahead (which those that do give up knowingly)."""
+    import subprocess
+    out = subprocess.run([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17",
+                          "-Xptxas", "-v", "-c", os.path.join(build.CSRC, "fox_scan.cu"), "-o", str(tmp_path / "scan.o")],
+                         capture_output=True, text=True, check=True).stderr
+    used = dict(re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", out, re.S))
+    two = {k: int(r) for k, r in used.items() if re.search(r"fox_(prologue|bwd_finish)_kernel|fox_cumsum_kernelILi\dELb0E", k)}
+    assert len(two) == 8 + 8 + 4 and all(r <= 32 for r in two.values()), two
+
+
 @pytest.mark.parametrize("bh", [1, 9, 10, 24, 35, 48, 60, 64, 70, 71, 96, 98, 99, 140, 147, 148, 149, 296, 297, 4000])
 @pytest.mark.parametrize("n,d", [(1024, 64), (4096, 128), (8192, 128), (16384, 64), (1024, 16), (12300, 16), (2 ** 24, 128)])
 def test_key_norm_parts_fill_a_wave_and_stay_short(bh, n, d):

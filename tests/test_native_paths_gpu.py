@@ -6,7 +6,7 @@ import torch.autograd.forward_ad as fwAD
 from torch.utils._python_dispatch import TorchDispatchMode
 
 import forgetting_transformer_b200 as fox
-from forgetting_transformer_b200 import _lib
+from forgetting_transformer_b200 import _lib, ops
 from oracle import fox_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -583,3 +583,36 @@ def test_norm_gate_and_swiglu_behind_one_another(rows):
     for got, want in zip(together, alone):
         for a, b in zip(got, want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows,N", [(1, 1), (3, 4095), (148, 4096), (148, 4097), (149, 4097), (2, 12287), (2, 12288), (149, 12290), (149, 16383), (149, 16384),
+                                    (150, 20000), (5, 33000)])
+@pytest.mark.parametrize("dtype", ["log", torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("padded", [False, True])
+def test_prefix_sums_with_and_without_loading_ahead(rows, N, dtype, padded):
+    """By themselves and in a call's prologue, at the lines between the two ways: against float64, each sum to the roundings of its
+    fp32 additions (4 in a thread, 10 in a block, one a chunk) and of the logarithms (4 ulp each)."""
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(1, rows, N, generator=gen, device="cuda") * 2 + 1
+    x[:, :, N // 3] = -40.0
+    start = 3 * N // 4 if padded else 0
+    seq = torch.full((1,), start, dtype=torch.long, device="cuda") if padded else None
+    if dtype == "log":
+        x = torch.nn.functional.logsigmoid(x)
+        lam, ref = ops.log_lambda_cumsum(x, seq), x.double()
+    else:
+        x = x.to(dtype)
+        lam, ref = ops.gate_prefix_from_logits(x, seq), torch.nn.functional.logsigmoid(x.double())
+    ref[:, :, :start] = 0
+    bound = (14 + N / 4096 + 4) * 2.0 ** -23 * ref.abs().cumsum(-1)
+    assert ((lam.double() - ref.cumsum(-1)).abs() <= bound).all()
+    if rows > 5 or N == 1:
+        return
+    k = torch.randn(1, rows, N, 64, generator=gen, device="cuda").bfloat16()
+    with torch.no_grad():    # (two query rows: one is a decode call, without a prologue)
+        call = fox.forgetting_attention if dtype == "log" else fox.forgetting_attention_from_gate_logits
+        out = call(k[:, :, -2:], k, k, x, head_first=True, seq_start=seq)[:, :, -1].double()
+    s = (k.double() @ k[:, :, -1:].double().transpose(2, 3))[..., 0] / 8 + (ref.cumsum(-1)[:, :, -1:] - ref.cumsum(-1))
+    s[:, :, :start] = float("-inf")
+    want = (s.softmax(-1)[..., None] * k.double()).sum(2)
+    assert (out - want).norm() <= 2 ** -7 * want.norm()
