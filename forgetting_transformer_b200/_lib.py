@@ -67,6 +67,7 @@ _SIGNATURES = {
     "fox_attn_decode_gates": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P, _F, c_int64,
                                       c_int64, c_int64, _F, c_float, _T4P, _F, _F, c_int64, c_int]),
     "fox_attn_decode_splits": (c_int64, [c_int64, c_int64, c_int64]),
+    "fox_attn_decode_per_sm": (c_int64, [c_int64, c_int64, c_int64]),
     "fox_attn_decode_workspace_floats": (c_int64, [c_int64, c_int64, c_int64, c_int64]),
     "fox_attn_bwd": (c_int, [c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_int64, _T4P, _T4P, _T4P,
                              _T4P, _F, _F, _F, _F, _F, c_float, _F, _F, _F, _T4P, _T4P, _F]),

@@ -472,7 +472,7 @@ fox_decode_kernel(const DecodeParams p, const std::conditional_t<kStep, DecodeSt
 template <bool kBf16, int D>
 __global__ void __launch_bounds__(256) fox_decode_merge_kernel(const DecodeParams p) {
   __shared__ float s_w[kDecMaxSplits], s_l[kDecMaxSplits], s_g[kDecMaxSplits], s_o[256], s_top, s_sum;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_for_kernel_in_front();
   if (p.chained) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int64_t bh = static_cast<int64_t>(b) * p.H + h;
@@ -539,13 +539,15 @@ __global__ void __launch_bounds__(256) fox_decode_merge_kernel(const DecodeParam
 // (see fox_step.cu); one with long ranges waits for SMs that it can split anew.  Short ones are over before that pays: 24 (b,h) of
 // 250 keys a range 32.5 us a layer, 33.8 so; 192 of 2000 97 and 89, of 6000 178 and 148; 96 of 10000 235 and 185.  (Head dims
 // 16 and 32 are bound by their instructions: 160 of 6000 keys 48 and 50.)  Clusters that need nearly every place of their wave, and
-// those of eight, find them too late then: 80 x 5 of 2400 keys a range 82 and 88, 48 x 8 of 750, head dim 128, 92 and 99.
+// those of eight, find them too late then: 80 x 5 of 2400 keys a range 82 and 88, 48 x 8 of 750, head dim 128, 92 and 99.  Not so the
+// clusters of two that come four CTAs to an SM, 446 to 540 of them: two layers of 240 (b,h) of 4200 keys 205 us without, 187 so; of 256 of 3000 181
+// and 166, of 6000 256 and 225; 512 single ranges of 4200 447 and 437.
 static int long_ranges(cudaLaunchAttribute* attr, const DecodeParams& p, int64_t B, int D) {
   const int64_t ctas = B * p.H * p.splits;
   if (D < 64 || static_cast<int64_t>(p.N) * D < static_cast<int64_t>(p.splits) * kDecLongRange) return 0;
   if (p.splits > 1 && (p.splits == kDecMaxCluster || (p.splits < kDecMaxCluster && ctas > kDecManyClusters && ctas <= kDecSlots))) return 0;
   attr->id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-  attr->val.sharedMemCarveout = 20;   // (three CTAs' 9 to 12 KB of 228)
+  attr->val.sharedMemCarveout = 20;   // (of 228 KB, where four CTAs take 9 to 12 each)
   return 1;
 }
 
@@ -617,9 +619,10 @@ static int launch_decode_at(const DecodeParams& p, int64_t B, cudaStream_t st) {
 // taken where the waves are fewer by so much that this pays, counted in keys with 600 for a wave's start: 512 (b,h) of 4000
 // keys of 128 in one wave instead of three 192 -> 162 us, of 64 102 -> 86; 256 of 4099 of 128 in one instead of two 98 -> 91, of 2048
 // 54 -> 48.  With as many waves they pay where they fill one that three leave half empty (a (b,h) in two ranges instead of one) and
-// the ranges are long: 256 of 1500 of 128 43 -> 37, but of 1000 of 64 17.8 and 18.5, 176 of 1200 16.4 and 17.2.  More ranges than two in
-// the same wave change little (144 of 2600 of 64 in three instead of two 24.7 and 22.7).  Else they are no faster or slower: 384 of 8000 of 64 130 and 135, 32 of 3000 13.7 and 14.3, 4 of 30000 of 128 21.2
-// and 22.5, 768 of 2500 of 64 86 and 91; 24 x 65536 70.0 and 70.0.
+// the ranges are long: 256 of 1500 of 128 43 -> 37, but of 1000 of 64 17.8 and 18.5, 176 of 1200 16.4 and 17.2.  Three ranges
+// instead of two in the same wave are not taken, though the one shape timed gained (144 of 2600 of 64 24.7 and 22.7).  Else they are no
+// faster or slower: 384 of 8000 of 64 130 and 135, 32 of 3000 13.7 and 14.3, 4 of 30000 of 128 21.2 and 22.5, 768 of 2500 of 64 86 and 91; 24 x
+// 65536 70.0 and 70.0.  (Head dim 16, whose ranges are bound by instructions, loses where they are shortest: 256 of 1300 10.4 and 11.0.)
 struct DecodePlan {
   int64_t splits;
   int per_sm;
@@ -666,6 +669,8 @@ extern "C" int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N) {
   if (B * H <= 0) return 1;   // (fox_attn_decode refuses such a call)
   return decode_plan(B * H, N).splits;
 }
+
+extern "C" int64_t fox_attn_decode_per_sm(int64_t B, int64_t H, int64_t N) { return B * H <= 0 ? kDecPerSm : decode_plan(B * H, N).per_sm; }
 
 // (none where the ranges are merged inside a cluster)
 extern "C" int64_t fox_attn_decode_workspace_floats(int64_t B, int64_t H, int64_t D, int64_t splits) {

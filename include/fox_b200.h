@@ -176,6 +176,8 @@ int fox_attn_decode_gates(int device, void* stream, int dtype, int64_t B, int64_
                           int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float sm_scale,
                           const fox_tensor4* o, float* L, float* workspace, int64_t splits, int programmatic);
 int64_t fox_attn_decode_splits(int64_t B, int64_t H, int64_t N);
+/* CTAs to an SM that these ranges are cut for, and launched with: 3 or 4. */
+int64_t fox_attn_decode_per_sm(int64_t B, int64_t H, int64_t N);
 
 /* delta[b,h,m] = sum_d o[b,h,m,d] * d_o[b,h,m,d] in fp32: replaces _bwd_preprocess
  * (forgetting_attention.py:267-277, kernel 902-943). */

@@ -179,15 +179,22 @@ def test_layer_glue_expressions():
                                               + math.log(T)) + tol).item()
 
 
-@pytest.mark.parametrize("bh", [1, 24, 49, 50, 72, 144, 223, 256, 400, 401, 444, 445, 512, 889, 65535])
-@pytest.mark.parametrize("n", [1, 256, 257, 2000, 70000, 2 ** 31 - 2048])
+@pytest.mark.parametrize("bh", [1, 24, 49, 50, 72, 144, 223, 256, 270, 271, 400, 401, 444, 445, 512, 540, 541, 592, 593, 889, 65535])
+@pytest.mark.parametrize("n", [1, 256, 257, 1279, 1500, 2000, 4099, 70000, 2 ** 31 - 2048])
 def test_decode_ranges_fill_whole_waves(bh, n):
-    """Ranges of one-token attention: at least 128 keys each, and never more CTAs than the waves they are cut for hold (444 a
-    wave, 400 where clusters merge)."""
-    s = _lib.load().fox_attn_decode_splits(1, bh, n)
-    assert 1 <= s <= min(512, max(1, -(-n // 128)))
-    waves = -(-bh // 444) + (1 if -(-bh // 444) * 400 // bh <= 1 else 0)
-    assert s == 1 or bh * s <= waves * (444 if s > 8 else 400)
+    """Ranges of one-token attention: at least 128 keys each, and never more CTAs than the waves they are cut for hold: 444 a wave, 400
+    where clusters merge, or 592 and 540 where they come four to an SM.  Those are chosen only where more (b,h) than one range of a
+    wave of three holds make them few, and the waves do not become more."""
+    lib = _lib.load()
+    s, per = lib.fox_attn_decode_splits(1, bh, n), lib.fox_attn_decode_per_sm(1, bh, n)
+    assert 1 <= s <= min(512, max(1, -(-n // 128))) and per in (3, 4)
+    full, clustered = (444, 400) if per == 3 else (592, 540)
+    waves = -(-bh // full) + (1 if -(-bh // full) * clustered // bh <= 1 else 0)
+    assert s == 1 or bh * s <= waves * (full if s > 8 else clustered)
+    if per == 4:
+        assert bh > 222 and -(-bh * s // (clustered if 1 < s <= 8 else full)) <= -(-bh // 444) + 1
+    if bh in (270, 592) and n in (1500, 2000, 4099):
+        assert (s, per) == ({270: 2, 592: 1}[bh], 4)
 
 
 @pytest.mark.parametrize("grid", [1, 176, 2048, 4095, 4096, 4097, 8192, 12288, 2 ** 20])

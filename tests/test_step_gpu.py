@@ -336,8 +336,9 @@ def test_decode_from_gates_behind_one_of_minus_infinity(N, D, at):
 @pytest.mark.parametrize("padded", [False, True])
 def test_decode_by_four_ctas_of_an_sm(B, H, N, D, splits, padded):
     """445 to 592 (b,h), one range each, and 223 to 270 in clusters of two: one wave of four CTAs to an SM in place of two or three of
-    three; the ranges of fewer CTAs to an SM would be others."""
-    assert _lib.load().fox_attn_decode_splits(B, H, N) == splits
+    three, launched so."""
+    lib = _lib.load()
+    assert lib.fox_attn_decode_splits(B, H, N) == splits and lib.fox_attn_decode_per_sm(B, H, N) == 4
     test_decode_from_gates(B, H, N, D, padded)
 
 
