@@ -74,10 +74,10 @@ __device__ __forceinline__ float log_gate(float raw) {
 // Bound by the chain of a chunk's load, scan and three barriers, 2.2 us of which the load is a third: with kAhead the next chunk's gates
 // are asked for before the scan (prologue, bf16: one row of 65536 gates 35.9 -> 22.9 us, 24 rows of 11000 13.5 -> 11.3, 4 of 9000 8.7 ->
 // 7.0; up to 4096, one chunk, unchanged).  From logits the chunk in hand is then formed by every thread, with gates or without; without
-// kAhead a thread that has none (past the row's end, in front of seq_start) leaves the logarithms out, which is worth more up to four
-// chunks (24 rows of 4097 7.9 us before, 9.9 ahead, 8.2 so; 11000 with half of it padding 11.8, 14.7, 12.4; 48 of 16384 23.6, 21.1, 21.1; one of
-// 65536 38.1, 34.6).  In the reverse scan, with three arrays, it takes more registers than two blocks of 1024 threads have, spills,
-// and loses: 24 rows of 16384 24.0 and 24.0 us, from logits 24.5 and 28.7.
+// kAhead a thread that has none (past the row's end, in front of seq_start) leaves the logarithms out, which is worth more below four
+// chunks (24 rows of 4097 7.9 us before, 9.9 ahead, 8.2 so; 11000 12.8, 14.5, 13.6, with half of it padding 11.8, 14.7, 12.4; but 8 of 16384
+// 20.0, 17.4, 18.8, one of 65536 38.1, 34.6, 37.7).  In the reverse scan, with three arrays, it takes more registers than two blocks of
+// 1024 threads have, spills, and loses: 24 rows of 16384 24.0 and 24.0 us, from logits 24.5 and 28.7.
 template <int kIn, bool kAhead>
 __device__ __forceinline__ void cumsum_rows(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
                                             const float* carry_in, float* out, float* total_out, float* lf_out, int H, int N, int bh, float* red) {
@@ -504,7 +504,7 @@ fox_prologue_kernel(const void* lf, int64_t sb, int64_t sh, int64_t sn, const in
   const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
   wait_for_kernel_in_front();
   if (x == 0) {
-    if (kIn == 3 || N > 4 * kScanChunk) cumsum_rows<kIn, true>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+    if (kIn == 3 || N >= 4 * kScanChunk) cumsum_rows<kIn, true>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
     else cumsum_rows<kIn, false>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
   }
   else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);

@@ -585,7 +585,7 @@ def test_norm_gate_and_swiglu_behind_one_another(rows):
             assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("rows,N", [(1, 1), (3, 4095), (148, 4096), (148, 4097), (149, 4097), (2, 12287), (2, 12288), (149, 12290), (149, 16383), (149, 16384),
+@pytest.mark.parametrize("rows,N", [(1, 1), (3, 4095), (148, 4096), (148, 4097), (149, 4097), (2, 12287), (2, 12288), (149, 12290), (2, 16383), (2, 16384), (149, 16383), (149, 16384),
                                     (150, 20000), (5, 33000)])
 @pytest.mark.parametrize("dtype", ["log", torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("padded", [False, True])
