@@ -12,6 +12,8 @@
 //   vector_norm(...).max(...) .............. lines 95-96
 #include <math.h>
 
+#include <type_traits>
+
 #include "fox_common.cuh"
 #include "fox_host.h"
 
@@ -74,10 +76,11 @@ __device__ __forceinline__ float log_gate(float raw) {
 // Bound by the chain of a chunk's load, scan and three barriers, 2.2 us of which the load is a third: with kAhead the next chunk's gates
 // are asked for before the scan (prologue, bf16: one row of 65536 gates 35.9 -> 22.9 us, 24 rows of 11000 13.5 -> 11.3, 4 of 9000 8.7 ->
 // 7.0; up to 4096, one chunk, unchanged).  From logits the chunk in hand is then formed by every thread, with gates or without; without
-// kAhead a thread that has none (past the row's end, in front of seq_start) leaves the logarithms out, which is worth more below four
-// chunks (24 rows of 4097 7.9 us before, 9.9 ahead, 8.2 so; 11000 12.8, 14.5, 13.6, with half of it padding 11.8, 14.7, 12.4; but 8 of 16384
-// 20.0, 17.4, 18.8, one of 65536 38.1, 34.6, 37.7).  In the reverse scan, with three arrays, it takes more registers than two blocks of
-// 1024 threads have, spills, and loses: 24 rows of 16384 24.0 and 24.0 us, from logits 24.5 and 28.7.
+// kAhead a thread that has none (past the row's end, in front of seq_start) leaves the logarithms out, which is worth more up to
+// eleven quarters of a chunk (24 rows of 4097 7.9 us before, 9.9 ahead, 8.2 so; 8192 10.8, 11.3, 10.3; 11000 12.8, 14.5, 13.6, with half of it
+// padding 11.8, 14.7, 12.4; but 16 of 12000 17.0, 16.3, 17.0, 8 of 16384 20.0, 17.4, 18.8, one of 65536 38.1, 34.6, 37.7); from fp32 logits, whose
+// loads take longer, up to seven (4 of 8192 7.6, 6.9, 8.2).  In the reverse scan, with three arrays, it takes more registers than two
+// blocks of 1024 threads have, spills, and loses: 24 rows of 16384 24.0 and 24.0 us, from logits 24.5 and 28.7.
 template <int kIn, bool kAhead>
 __device__ __forceinline__ void cumsum_rows(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start,
                                             const float* carry_in, float* out, float* total_out, float* lf_out, int H, int N, int bh, float* red) {
@@ -446,6 +449,11 @@ fox_max_row_norm_kernel(const uint16_t* __restrict__ x, int64_t sb, int64_t sh, 
 // Two blocks to an SM, at most 32 registers a thread: bf16 took 42 by itself and had one, whose loads and reductions took turns
 // (keys alone, 48 (b,h) of 16384 x 64: 30.0 -> 25.0 us, 512 of 2048 x 64 43.2 -> 34.4, 32 of 2048 x 128 9.5 -> 7.2; with queries, 64 of
 // 16384 x 128: 113.8 -> 101.4; 4 of 9000 x 128, whose scans are the longest, 8.4 and 8.7).
+// From some 24 (b, h) on two scans then share an SM here and there, and the launch waits for them (24 of 16384 x 64 from a block's
+// logits 21.3 us with one block to an SM, 29.1 with two).  With kFirst the scans are the first blocks, one to an SM: 18.5.  It is taken
+// where blocks share SMs at all and each scan finds one of its own, from logits (8 (b,h) 5 % less, 12 and 16 6 %, 32 13 %; strided ones
+// of 64 3 %) and from strided log gates (24 of 16384 26.8 -> 18.9, 32 8 %, 8 to 16 within 2 %); contiguous log gates lose 1 to 5 %,
+// the compiler's order of their loads being a worse one there.
 struct NormSource {
   const uint16_t* x;
   int64_t sb, sh, st;
@@ -497,18 +505,26 @@ __device__ __forceinline__ void norm_part(const NormSource& s, int D, int H, int
   }
 }
 
-template <int kIn, bool kBf16>
+template <int kIn, bool kBf16, bool kAhead, bool kFirst>
 __global__ void __launch_bounds__(kScanThreads, 2)
-fox_prologue_kernel(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float* lam, const NormSource k, const NormSource q, int H, int N, int D) {
+fox_prologue_kernel(const void* lf, int64_t sb, int64_t sh, int64_t sn, const int64_t* seq_start, float* lam, const NormSource k, const NormSource q, int units, int H, int N, int D) {
   __shared__ float red[32];
-  const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
-  wait_for_kernel_in_front();
-  if (x == 0) {
-    if (kIn == 3 || N >= 4 * kScanChunk) cumsum_rows<kIn, true>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
-    else cumsum_rows<kIn, false>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+  if constexpr (kFirst) {
+    wait_for_kernel_in_front();
+    if (static_cast<int>(blockIdx.x) < units) {
+      cumsum_rows<kIn, kAhead>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, blockIdx.x, red);
+    } else {
+      const int parts = k.n_parts + q.n_parts, i = blockIdx.x - units, bh = i / parts, x = i % parts;
+      if (x < k.n_parts) norm_part<kBf16>(k, D, H, bh, x, red);
+      else norm_part<kBf16>(q, D, H, bh, x - k.n_parts, red);
+    }
+  } else {
+    const int parts = 1 + k.n_parts + q.n_parts, bh = blockIdx.x / parts, x = blockIdx.x % parts;
+    wait_for_kernel_in_front();
+    if (x == 0) cumsum_rows<kIn, kAhead>(lf, sb, sh, sn, seq_start, nullptr, lam, nullptr, nullptr, H, N, bh, red);
+    else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
+    else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
   }
-  else if (x <= k.n_parts) norm_part<kBf16>(k, D, H, bh, x - 1, red);
-  else norm_part<kBf16>(q, D, H, bh, x - 1 - k.n_parts, red);
 }
 
 // ------------------------------------------------------ delta = rowsum(O * dO)
@@ -786,17 +802,24 @@ extern "C" int fox_attn_prologue(int device, void* stream, int dtype, int gate_k
   const unsigned grid = (unsigned)(B * H * (1 + ks.n_parts + qs.n_parts));
   cudaStream_t st = (cudaStream_t)stream;
   const bool bf = dtype == FOX_DTYPE_BF16;
-#define FOX_PRO(K)                                                                                                        \
-  return launch_behind(bf ? fox_prologue_kernel<K, true> : fox_prologue_kernel<K, false>, dim3(grid), kScanThreads, 0, st, gates, \
-                       sb, sh, sn, seq_start, log_lambda, ks, qs, (int)H, (int)N, (int)D)
+  const int64_t units = B * H, quarters = (N * 4 + kScanChunk - 1) / kScanChunk;   // (of a chunk)
+  const bool first = grid > kSms && units <= kSms && (gate_kind != FOX_GATE_LOG || (sn != 1 && units > 16));
+  const bool ahead = gate_kind == FOX_GATE_LOG || quarters > (gate_kind == FOX_DTYPE_FP32 ? 7 : 11);
+  auto launch = [&](auto gates_in, auto ahead_c) {
+    constexpr int kIn = decltype(gates_in)::value;
+    constexpr bool kAhead = decltype(ahead_c)::value;
+    auto kern = first ? (bf ? fox_prologue_kernel<kIn, true, kAhead, true> : fox_prologue_kernel<kIn, false, kAhead, true>)
+                      : (bf ? fox_prologue_kernel<kIn, true, kAhead, false> : fox_prologue_kernel<kIn, false, kAhead, false>);
+    return launch_behind(kern, dim3(grid), kScanThreads, 0, st, gates, sb, sh, sn, seq_start, log_lambda, ks, qs, (int)units, (int)H, (int)N, (int)D);
+  };
+  auto either = [&](auto gates_in) { return ahead ? launch(gates_in, std::true_type{}) : launch(gates_in, std::false_type{}); };
   switch (gate_kind) {
-    case FOX_DTYPE_FP16: FOX_PRO(0);
-    case FOX_DTYPE_BF16: FOX_PRO(1);
-    case FOX_DTYPE_FP32: FOX_PRO(2);
-    case FOX_GATE_LOG: FOX_PRO(3);
+    case FOX_DTYPE_FP16: return either(std::integral_constant<int, 0>{});
+    case FOX_DTYPE_BF16: return either(std::integral_constant<int, 1>{});
+    case FOX_DTYPE_FP32: return either(std::integral_constant<int, 2>{});
+    case FOX_GATE_LOG: return launch(std::integral_constant<int, 3>{}, std::true_type{});
     default: return FOX_ERR_BAD_ARG;
   }
-#undef FOX_PRO
 }
 
 static int launch_index(int device, cudaStream_t st, int64_t B, IndexParams p) {
