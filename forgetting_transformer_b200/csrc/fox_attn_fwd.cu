@@ -140,10 +140,12 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     nb_hi = (hi + BN - 1) / BN;
     n_tiles = max(nb_hi - nb_lo, 0);
   };
-  // Unit by unit the range is there before the barriers are: behind them, as by length, the same source makes a slower tile loop at head
-  // dim 128 (1 x 2 of 4096 x 16384 that a threshold could prune and does not: 237 us behind, 206 before; 4 heads 238 and 207; by length,
-  // either way, 205), for 0.2 us of set-up that the kernel in front would cover.
-  if constexpr (!kByLength) {
+  // Head dim 128, unit by unit: the range is there before the barriers are.  Behind them, as everywhere else, the same source makes a
+  // slower tile loop there (1 x 2 of 4096 x 16384 that a threshold could prune and does not: 237 us behind, 206 before; 4 heads 238 and 207; by
+  // length, either way, 205); it costs 0.2 us of set-up that the kernel in front would cover (at head dim 64 48 of 700 x 5000, pruned,
+  // 26.2 us before, 25.8 behind).
+  constexpr bool kRangeFirst = !kByLength && D > 64;
+  if constexpr (kRangeFirst) {
     wait_for_kernel_in_front();
     set_range();
   }
@@ -166,7 +168,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     mbar_fence_init();
   }
-  if constexpr (kByLength) wait_for_kernel_in_front();   // (no memory is read before this, and no TMEM held that the kernel in front might ask for)
+  if constexpr (!kRangeFirst) wait_for_kernel_in_front();   // (no memory is read before this, and no TMEM held that the kernel in front might ask for)
   if (warp == kTmaWarp) {
     tmem_alloc(&tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -177,7 +179,7 @@ fox_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tbase = tmem_slot;
   volatile int* abortp = &abort_flag;
 
-  if constexpr (kByLength) set_range();
+  if constexpr (!kRangeFirst) set_range();
 
   if (warp == kTmaWarp) {
     // ===================== TMA producer (whole warp converged, one elected lane issues) =====================
