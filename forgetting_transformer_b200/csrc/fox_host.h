@@ -144,7 +144,7 @@ inline int cached_tmap_4d(CUtensorMap* out, const Tensor4& t, int elem_bytes, bo
 
 // Launches a kernel whose CTAs may take their SMs and set up their barriers as soon as the last CTA of the kernel in front has ended,
 // before its results are written back; the kernel calls wait_for_kernel_in_front() before it reads or writes memory (its loads must
-// not be __restrict__ ones, which may move in front of the wait).  A launch behind another by stream order alone costs 1.5-2 us from
+// not be __restrict__ or .nc ones, which may be done in front of the wait).  A launch behind another by stream order alone costs 1.5-2 us from
 // the end of the first to the first load of the second; a pass of the attention is 5 to 7 kernels.  Forward and backward
 // together, back to back, stream order -> this: B1 H2 T128 D64 30.9 -> 22.4 us, B4 H12 T512 D64 51.2 -> 41.0, B2 H16 T2048 D128
 // 215 -> 203, B1 H24 T4096 D64 313 -> 301; from some 500 us a pass on within the noise.  None of the kernels lets the next begin
